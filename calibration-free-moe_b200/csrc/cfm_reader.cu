@@ -2875,9 +2875,10 @@ int cfm_build_sketch(const cfm_layer* layer, const void* gate_up, const int8_t* 
   const int64_t H = layer->hidden, I = layer->width, E = layer->experts;
   if (H <= 0 || H % kBlock || I <= 0 || I % 16 || E < 1 || E > 65535 || 2 * I / kBuildRows > 65535)
     return CFM_E_SHAPE;
-  const dim3 grid(static_cast<unsigned>(H / kBlock), static_cast<unsigned>(2 * I / kBuildRows),
+  const int64_t row_tiles = (2 * I / kBuildRows + kBuildWarps - 1) / kBuildWarps;
+  const dim3 grid(static_cast<unsigned>(H / kBlock), static_cast<unsigned>(row_tiles),
                   static_cast<unsigned>(E));
-  k_build_sketch<<<grid, kBuildRows * 32, 0, static_cast<cudaStream_t>(stream)>>>(
+  k_build_sketch<<<grid, kBuildWarps * 32, 0, static_cast<cudaStream_t>(stream)>>>(
       static_cast<int>(H), static_cast<int>(I), static_cast<const __nv_bfloat16*>(gate_up), signs,
       sketch, sketch_grouped, static_cast<__half*>(statistics));
   return launched();
