@@ -17,10 +17,11 @@ PACKAGE = Path(__file__).resolve().parent
 SOURCES = [PACKAGE / "csrc" / "cfm_reader.cu"]
 HEADERS = [PACKAGE / "csrc" / "cfm_device.cuh", PACKAGE / "csrc" / "cfm_grouped.cuh",
            PACKAGE / "csrc" / "cfm_exchange.cuh", PACKAGE / "csrc" / "cfm_select.cuh",
-           PACKAGE / "csrc" / "cfm_build.cuh", PACKAGE / "csrc" / "cfm_screen_rows32.cuh",
+           PACKAGE / "csrc" / "cfm_build.cuh", PACKAGE / "csrc" / "cfm_screen.cuh",
+           PACKAGE / "csrc" / "cfm_screen_tc.cuh", PACKAGE / "csrc" / "cfm_prepare.cuh",
            PACKAGE.parent / "include" / "cfm_b200.h"]
 LIBRARY = PACKAGE / "libcfm_b200.so"
-ABI_VERSION = 10
+ABI_VERSION = 11
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
@@ -111,7 +112,7 @@ _LAYOUT_ARRAYS = (
     "ids", "weights", "norms", "planes", "coordinates", "quantized", "exponents", "parts",
     "counters", "partial", "scores", "selected", "completed", "candidate_ids", "counts",
     "starts", "tile_starts", "activations", "exact", "down_parts", "encoder_parts", "latent",
-    "status", "limbs", "group_offsets", "group_pairs", "cuts", "variances", "unscales", "zero_limbs",
+    "status", "limbs", "group_offsets", "group_pairs", "cuts", "variances", "features", "pass_work", "busy_experts", "work_counts",
     "tile_list", "tile_count",
 )
 

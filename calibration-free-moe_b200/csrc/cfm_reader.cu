@@ -32,6 +32,7 @@ namespace cfm {
 // ---------------------------------------------------------------------------
 // Workspace binding
 // ---------------------------------------------------------------------------
+struct Pass;
 struct Workspace {
   int32_t* ids;
   float* weights;
@@ -51,6 +52,7 @@ struct Workspace {
   int32_t* starts;
   int32_t* tile_starts;
   __nv_bfloat16* activations;
+  __nv_bfloat16* features;
   float* exact;
   float* down_parts;
   float* encoder_parts;
@@ -61,8 +63,9 @@ struct Workspace {
   int32_t* group_pairs;
   int32_t* cuts;
   float* variances;
-  float* unscales;
-  int8_t* zero_limbs;
+  Pass* pass_work;
+  int32_t* busy_experts;
+  int32_t* work_counts;
   int32_t* tile_list;
   int32_t* tile_count;
   int32_t parts_tokens;
@@ -95,10 +98,6 @@ __device__ __forceinline__ int slot_of(const Layer& L, int i) {
   return L.width_magic ? static_cast<int>(__umulhi(static_cast<uint32_t>(i), L.width_magic))
                        : i / L.I;
 }
-
-// Score of candidate i (slot's channel c of local expert e) of token t; defined with the select kernel.
-__device__ __forceinline__ float candidate_score(const Layer& L, const Workspace& ws, int t, int i,
-                                                 int e, int c, float weight);
 
 static int64_t align256(int64_t v) { return (v + 255) / 256 * 256; }
 
@@ -158,8 +157,11 @@ static int make_layout(const cfm_layer* l, int32_t capacity, cfm_workspace_layou
   o->group_pairs = take(4 * C * K);
   o->cuts = take(4 * C * (K + 1));
   o->variances = take(4 * C * 2 * N);
-  o->unscales = take(4 * C * B);
-  o->zero_limbs = take(B * 3 * kBlock);
+  const int64_t E = std::max<int64_t>(l->experts, 1);
+  o->features = take(2 * C * N);
+  o->pass_work = take(16 * (C * K / 8 + std::min(E, C * K)));  // of at least eight pairs
+  o->busy_experts = take(4 * E);
+  o->work_counts = take(16);
   o->tile_list = take(32 * C * ((F + kDownTileRows - 1) / kDownTileRows + K));
   o->tile_count = take(16);
   o->bytes = at;
@@ -197,8 +199,10 @@ static Workspace bind(const cfm_workspace_layout& o, void* base, int32_t capacit
   w.group_pairs = reinterpret_cast<int32_t*>(p + o.group_pairs);
   w.cuts = reinterpret_cast<int32_t*>(p + o.cuts);
   w.variances = reinterpret_cast<float*>(p + o.variances);
-  w.unscales = reinterpret_cast<float*>(p + o.unscales);
-  w.zero_limbs = reinterpret_cast<int8_t*>(p + o.zero_limbs);
+  w.features = reinterpret_cast<__nv_bfloat16*>(p + o.features);
+  w.pass_work = reinterpret_cast<Pass*>(p + o.pass_work);
+  w.busy_experts = reinterpret_cast<int32_t*>(p + o.busy_experts);
+  w.work_counts = reinterpret_cast<int32_t*>(p + o.work_counts);
   w.tile_list = reinterpret_cast<int32_t*>(p + o.tile_list);
   w.tile_count = reinterpret_cast<int32_t*>(p + o.tile_count);
   w.parts_tokens = o.parts_tokens;
@@ -247,148 +251,9 @@ static Layer device_layer(const cfm_layer* l) {
 }
 
 #include "cfm_exchange.cuh"
-
-// ---------------------------------------------------------------------------
-// prepare: rotation, partial-screen mask, fixed-point copy
-// ---------------------------------------------------------------------------
-// grid (T, B), 128 threads: one thread per coordinate of one rotation block.
-__global__ void __launch_bounds__(kBlock) k_prepare(Layer L, Workspace ws,
-                                                    const __nv_bfloat16* hidden,
-                                                    const uint8_t* padding) {
-  const int t = blockIdx.x, b = blockIdx.y, c = threadIdx.x;
-  if (padding && padding[t]) return;
-  __shared__ float sm[kBlock];
-  __shared__ int warp_i[4];
-  __shared__ float warp_f[4];
-  const int lane = c & 31, warp = c >> 5;
-
-  const size_t at = static_cast<size_t>(t) * L.H + b * kBlock + c;
-  float v = __fmul_rn(__bfloat162float(hidden[at]),
-                      static_cast<float>(L.signs[b * kBlock + c]));
-  // Butterfly, half-widths 1..64: the member with the bit clear takes the sum,
-  // the member with the bit set takes (partner - own).
-#pragma unroll
-  for (int w = 1; w < 32; w <<= 1) {
-    const float o = __shfl_xor_sync(kFull, v, w);
-    v = (c & w) ? __fsub_rn(o, v) : __fadd_rn(v, o);
-  }
-#pragma unroll
-  for (int w = 32; w < kBlock; w <<= 1) {
-    sm[c] = v;
-    __syncthreads();
-    const float o = sm[c ^ w];
-    __syncthreads();
-    v = (c & w) ? __fsub_rn(o, v) : __fadd_rn(v, o);
-  }
-  v = __fmul_rn(v, 0.0883883461f);  // float(1 / sqrt(128))
-
-  // Rank by magnitude, ties to the lower coordinate.
-  const float a = fabsf(v);
-  sm[c] = a;
-  __syncthreads();
-  bool kept = true;
-  if (L.KEEP < kBlock) {
-    int rank = 0;
-#pragma unroll 8
-    for (int j = 0; j < kBlock; ++j) {
-      const float o = sm[j];
-      rank += (o > a) || (o == a && j < c);
-    }
-    kept = rank < L.KEEP;
-  }
-  // Compact kept coordinates in ascending coordinate order.
-  const unsigned ballot = __ballot_sync(kFull, kept);
-  if (lane == 0) warp_i[warp] = __popc(ballot);
-  // Block maximum magnitude (kept values are the largest, so this is theirs).
-  float m = a;
-#pragma unroll
-  for (int w = 16; w; w >>= 1) m = fmaxf(m, __shfl_xor_sync(kFull, m, w));
-  if (lane == 0) warp_f[warp] = m;
-  __syncthreads();
-  int position = __popc(ballot & ((1u << lane) - 1));
-  for (int w = 0; w < warp; ++w) position += warp_i[w];
-  m = fmaxf(fmaxf(warp_f[0], warp_f[1]), fmaxf(warp_f[2], warp_f[3]));
-  __syncthreads();
-
-  // Fixed point: q = rint(v * 2^(21 - e)), e = floor(log2 m) clamped to +-100.
-  int e = static_cast<int>((__float_as_uint(m) >> 23) & 0xff) - 127;
-  e = max(-100, min(100, e));
-  int q = 0;
-  float energy = 0.0f;
-  if (kept) {
-    const float scale = __uint_as_float(static_cast<uint32_t>(127 + kQuantBits - e) << 23);
-    q = (m > 0.0f) ? __float2int_rn(__fmul_rn(v, scale)) : 0;
-    q = max(-(1 << 22), min(1 << 22, q));
-    energy = __fmul_rn(v, v);
-    const size_t out = (static_cast<size_t>(t) * L.B + b) * L.KEEP + position;
-    ws.planes[out] = v;
-    ws.coordinates[out] = c;
-    ws.quantized[out] = q;
-  }
-  {
-    // Balanced base-256 digits of q (zero for dropped coordinates), in natural
-    // coordinate order: q = l0 + 256 l1 + 65536 l2, each digit an int8.
-    const int l0 = static_cast<int8_t>(q & 0xff);
-    const int q1 = (q - l0) >> 8;
-    const int l1 = static_cast<int8_t>(q1 & 0xff);
-    const int l2 = (q1 - l1) >> 8;
-    int8_t* limb = ws.limbs + (static_cast<size_t>(t) * L.B + b) * 3 * kBlock + c;
-    limb[0] = static_cast<int8_t>(l0);
-    limb[kBlock] = static_cast<int8_t>(l1);
-    limb[2 * kBlock] = static_cast<int8_t>(l2);
-  }
-  int qsum = q;
-#pragma unroll
-  for (int w = 16; w; w >>= 1) qsum += __shfl_xor_sync(kFull, qsum, w);
-  if (lane == 0) warp_i[warp] = qsum;
-  sm[c] = energy;  // squares of the kept values, zero elsewhere
-  __syncthreads();
-  if (c == 0) {
-    const size_t row = static_cast<size_t>(t) * L.B + b;
-    ws.exponents[2 * row] = e;
-    ws.exponents[2 * row + 1] = warp_i[0] + warp_i[1] + warp_i[2] + warp_i[3];
-    ws.unscales[row] = __uint_as_float(static_cast<uint32_t>(127 + e - kQuantBits) << 23);
-    // Energy of the kept coordinates, summed in coordinate order (pinned).
-    float total = 0.0f;
-    for (int j = 0; j < kBlock; ++j) total = __fadd_rn(total, sm[j]);
-    ws.norms[row] = total;
-  }
-}
-
-// ---------------------------------------------------------------------------
-// route: stable ascending sort of a token's experts
-// ---------------------------------------------------------------------------
-// grid (T), 32 threads.
-__global__ void __launch_bounds__(32) k_route(Layer L, Workspace ws, const void* ids,
-                                              int ids64, const void* weights, int wbf16) {
-  const int t = blockIdx.x, lane = threadIdx.x;
-  long long id = 0x7fffffffffffffffLL;
-  float w = 0.0f;
-  if (lane < L.K) {
-    const size_t at = static_cast<size_t>(t) * L.K + lane;
-    id = ids64 ? static_cast<const long long*>(ids)[at]
-               : static_cast<long long>(static_cast<const int32_t*>(ids)[at]);
-    w = wbf16 ? __bfloat162float(static_cast<const __nv_bfloat16*>(weights)[at])
-              : static_cast<const float*>(weights)[at];
-  }
-  int rank = 0;
-  for (int j = 0; j < L.K; ++j) {
-    const long long o = __shfl_sync(kFull, id, j);
-    rank += (o < id) || (o == id && j < lane);
-  }
-  if (lane < L.K) {
-    int local = -1;
-    if (L.expert_map) {
-      if (id >= 0 && id < L.global_experts) local = L.expert_map[id];
-    } else if (id >= 0 && id < L.E) {
-      local = static_cast<int>(id);
-    }
-    if (local >= L.E) local = -1;
-    const size_t out = static_cast<size_t>(t) * L.K + rank;
-    ws.ids[out] = local;
-    ws.weights[out] = w;
-  }
-}
+#include "cfm_prepare.cuh"
+#include "cfm_screen.cuh"
+#include "cfm_screen_tc.cuh"
 
 // ---------------------------------------------------------------------------
 // adopt: a selection made on the token's home rank, cut down to this rank's experts
@@ -498,7 +363,7 @@ __global__ void __launch_bounds__(256) k_adopt(Layer L, Workspace ws, const void
 }
 
 // ---------------------------------------------------------------------------
-// screen: sketch GEMV + score
+// screen of layers without a row-major sketch: sketch GEMV + score
 // ---------------------------------------------------------------------------
 // grid (T*K pairs, S splits of the rotation blocks), W*CG threads.  Thread
 // (cg, wi) owns sketch word wi (16 rows) and the kept coordinates j = cg mod CG
@@ -506,6 +371,7 @@ __global__ void __launch_bounds__(256) k_adopt(Layer L, Workspace ws, const void
 // shared memory; each thread then finishes 16/CG rows.
 template <int CG>
 __global__ void __launch_bounds__(512) k_screen(Layer L, Workspace ws, const uint8_t* padding, int S) {
+  grid_dependency_wait();     // the kept values and the routes are complete
   grid_dependency_release();  // the selection may be scheduled; it waits for this grid
   constexpr int RPT = kWordRows / CG;  // rows a thread finishes per block
   constexpr int U = 8;                 // words in flight per thread
@@ -612,12 +478,25 @@ __global__ void __launch_bounds__(512) k_screen(Layer L, Workspace ws, const uin
 
   float* gate_out = ws.partial + static_cast<size_t>(t) * 2 * L.N + static_cast<size_t>(slot) * L.I;
   float* up_out = gate_out + L.N;
+  // Scores and features of the pair, once the CTA's threads have written its projections (the
+  // library-scratch screen has no place for them).
+  auto finish = [&]() {
+    if (!ws.scores) return;
+    __syncthreads();
+    const float* variance = ws.variances + static_cast<size_t>(t) * 2 * L.N +
+                            static_cast<size_t>(slot) * L.I;
+    const bool risk = L.score != CFM_SCORE_POINT;
+    for (int c = tid; c < L.I; c += threads)
+      finish_candidate(L, ws, pair, e, c, gate_out[c], up_out[c], risk ? variance[c] : 0.0f,
+                       risk ? variance[L.N + c] : 0.0f);
+  };
   if (S == 1) {
 #pragma unroll
     for (int r = 0; r < RPT; ++r) {
       const int row = row0 + r;
       (row < L.I ? gate_out[row] : up_out[row - L.I]) = run[r];
     }
+    finish();
     return;
   }
   __threadfence();
@@ -637,535 +516,19 @@ __global__ void __launch_bounds__(512) k_screen(Layer L, Workspace ws, const uin
     for (int b = 0; b < L.B; ++b) s = __fadd_rn(s, __ldcg(p + static_cast<size_t>(b) * rows));
     (row < L.I ? gate_out[row] : up_out[row - L.I]) = s;
   }
-}
-
-// ---------------------------------------------------------------------------
-// grouped screen: pairs grouped by expert, int8 tensor-core dot products
-// ---------------------------------------------------------------------------
-// Lists the active (token, slot) pairs of every local expert.  One CTA; dynamic
-// shared memory: 2 * E counters.  The order of an expert's pairs is whatever the
-// atomics produce; every pair's result is independent of it.
-__global__ void __launch_bounds__(1024) k_group(Layer L, Workspace ws, const uint8_t* padding,
-                                                int T) {
-  extern __shared__ int group_smem[];
-  int* count = group_smem;
-  int* cursor = group_smem + L.E;
-  const int tid = threadIdx.x, pairs = T * L.K;
-  for (int e = tid; e < L.E; e += blockDim.x) count[e] = 0;
-  __syncthreads();
-  for (int p = tid; p < pairs; p += blockDim.x) {
-    const int e = ws.ids[p];
-    if (e >= 0 && !(padding && padding[p / L.K])) atomicAdd(&count[e], 1);
-  }
-  __syncthreads();
-  if (tid < 32) {  // exclusive scan over experts, one warp
-    int carry = 0;
-    for (int base = 0; base < L.E; base += 32) {
-      const int e = base + tid;
-      const int mine = e < L.E ? count[e] : 0;
-      int scan = mine;
-#pragma unroll
-      for (int w = 1; w < 32; w <<= 1) {
-        const int o = __shfl_up_sync(kFull, scan, w);
-        if (tid >= w) scan += o;
-      }
-      if (e < L.E) {
-        cursor[e] = carry + scan - mine;
-        ws.group_offsets[e] = carry + scan - mine;
-      }
-      carry += __shfl_sync(kFull, scan, 31);
-    }
-    if (tid == 0) ws.group_offsets[L.E] = carry;
-  }
-  __syncthreads();
-  for (int p = tid; p < pairs; p += blockDim.x) {
-    const int e = ws.ids[p];
-    if (e >= 0 && !(padding && padding[p / L.K])) {
-      ws.group_pairs[atomicAdd(&cursor[e], 1)] = p;
-    }
-  }
-}
-
-// Sixteen 2-bit codes of one 32-bit word -> four int8x4 registers of trits.
-// The grouped layout stores coordinate c of a word at bit 4c (c < 4),
-// 4(c-4)+2 (c < 8), 16+4(c-8) (c < 12), 18+4(c-12) otherwise, so that four
-// masked shifts yield byte-permute selectors; the permute picks -1, 0, +1 from
-// a register table.
-__device__ __forceinline__ void decode_word(uint32_t w, uint32_t& c0, uint32_t& c1, uint32_t& c2,
-                                            uint32_t& c3) {
-  constexpr uint32_t table = 0x000100ffu;  // byte 0 = -1, byte 1 = 0, byte 2 = +1
-  c0 = __byte_perm(table, 0u, w & 0x3333u);
-  c1 = __byte_perm(table, 0u, (w >> 2) & 0x3333u);
-  c2 = __byte_perm(table, 0u, (w >> 16) & 0x3333u);
-  c3 = __byte_perm(table, 0u, (w >> 18) & 0x3333u);
-}
-
-__device__ __forceinline__ void mma_s8(int (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2,
-                                       uint32_t a3, uint32_t b0, uint32_t b1) {
-  asm("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
-      "{%0,%1,%2,%3};"
-      : "+r"(d[0]), "+r"(d[1]), "+r"(d[2]), "+r"(d[3])
-      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+  finish();
 }
 
 #include "cfm_build.cuh"
 
-constexpr int kGroupWarps = 8;  // 16 sketch rows per warp
-
-// m16n8k32 int8 MMA whose accumulator starts at zero.
-__device__ __forceinline__ void mma_s8_first(int (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2,
-                                             uint32_t a3, uint32_t b0, uint32_t b1) {
-  asm("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
-      "{%10,%10,%10,%10};"
-      : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3])
-      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "r"(0));
-}
-
-// Everything a lane needs for one rotation block, fetched one block ahead.
-struct GroupFetch {
-  uint2 word_a, word_b;  // 32 coordinates of rows g and g + 8
-  uint4 digit[3][2];     // this lane's 32 coordinates of the three digits of token g
-  __half scale_a, scale_b;
-  float unscale[2];      // 2^(e - 21) of the two tokens this lane finishes (2 tq, 2 tq + 1)
-};
-
-// grid (ceil(2I / 128), E, passes), 256 threads, no shared memory, no barrier.  A warp
-// owns 16 sketch rows of one expert and walks the rotation blocks in order.  Per
-// block it decodes 16 rows x 128 coordinates into int8 fragments and multiplies
-// them with the int8 digits of up to eight of the expert's tokens (m16n8k32,
-// exact int32 sums; one 8-column tile per digit).  Lane (g, tq) holds
-// coordinates 32 tq .. 32 tq + 31 of rows g and g + 8 and of token g's digits,
-// so k-step m uses coordinates 32 tq + 8 m .. + 7 of all of them; the digits
-// come straight from global memory (L1/L2 resident, 32 contiguous bytes per
-// lane and digit).  The next block's words, digits, scales and exponents are
-// in flight in registers while the current block computes.  Experts with more
-// than eight tokens take further passes of eight, spread over grid.z.
-__global__ void __launch_bounds__(kGroupWarps * 32, 2) k_screen_grouped(Layer L, Workspace ws) {
-  grid_dependency_release();  // the selection may be scheduled; it waits for this grid
-  constexpr int kGroupRows = kGroupWarps * 16;  // rows per CTA
-  const int e = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int g = lane >> 2, tq = lane & 3;
-  const int first = ws.group_offsets[e], total = ws.group_offsets[e + 1] - first;
-  const int rows = 2 * L.I;
-  const int r0 = blockIdx.x * kGroupRows + warp * 16;
-  if (total == 0 || r0 >= rows) return;  // whole warps are in or out: 2I is a multiple of 32
-  const int row_a = r0 + g, row_b = r0 + g + 8;
-  const uint2* sketch = reinterpret_cast<const uint2*>(L.sketch_grouped) + tq;
-  const size_t sketch_block = static_cast<size_t>(rows) * (kBlock / 32);  // uint2 per block
-  const size_t sketch_a = (static_cast<size_t>(e) * L.B * rows + row_a) * (kBlock / 32);
-  const size_t sketch_b = (static_cast<size_t>(e) * L.B * rows + row_b) * (kBlock / 32);
-  const __half* scales = L.statistics + static_cast<size_t>(e) * L.B * 2 * rows;
-
-  for (int base = 8 * blockIdx.z; base < total; base += 8 * gridDim.z) {
-    const int count = min(8, total - base);
-    // Pair of the token whose digits this lane feeds (column g of the tiles).
-    const int pair_g = g < count ? ws.group_pairs[first + base + g] : -1;
-    // Pairs of the two tokens whose results this lane finishes.
-    const int pair_0 = __shfl_sync(kFull, pair_g, (2 * tq) * 4);
-    const int pair_1 = __shfl_sync(kFull, pair_g, (2 * tq + 1) * 4);
-    // Running pointers, advanced by one rotation block per fetch.  Empty token
-    // slots read a block of zero digits kept in the workspace (never written).
-    const uint2* next_a = sketch + sketch_a;
-    const uint2* next_b = sketch + sketch_b;
-    const __half* next_scale_a = scales + row_a;
-    const __half* next_scale_b = scales + row_b;
-    const uint4* next_digits = reinterpret_cast<const uint4*>(
-        (pair_g >= 0 ? ws.limbs + static_cast<size_t>(pair_g / L.K) * L.B * 3 * kBlock
-                     : ws.zero_limbs) + 32 * tq);
-    const float* next_unscale_0 = ws.unscales + static_cast<size_t>(max(pair_0, 0) / L.K) * L.B;
-    const float* next_unscale_1 = ws.unscales + static_cast<size_t>(max(pair_1, 0) / L.K) * L.B;
-    auto fetch = [&]() {
-      GroupFetch f;
-      f.word_a = *next_a;
-      f.word_b = *next_b;
-      f.scale_a = *next_scale_a;
-      f.scale_b = *next_scale_b;
-#pragma unroll
-      for (int j = 0; j < 3; ++j) {
-        f.digit[j][0] = next_digits[j * (kBlock / 16)];
-        f.digit[j][1] = next_digits[j * (kBlock / 16) + 1];
-      }
-      f.unscale[0] = *next_unscale_0;
-      f.unscale[1] = *next_unscale_1;
-      next_a += sketch_block;
-      next_b += sketch_block;
-      next_scale_a += 2 * rows;
-      next_scale_b += 2 * rows;
-      next_digits += 3 * kBlock / 16;
-      ++next_unscale_0;
-      ++next_unscale_1;
-      return f;
-    };
-
-    float run[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-    auto compute = [&](const GroupFetch& cur) {
-      uint32_t fa[8], fb[8];
-      decode_word(cur.word_a.x, fa[0], fa[1], fa[2], fa[3]);
-      decode_word(cur.word_a.y, fa[4], fa[5], fa[6], fa[7]);
-      decode_word(cur.word_b.x, fb[0], fb[1], fb[2], fb[3]);
-      decode_word(cur.word_b.y, fb[4], fb[5], fb[6], fb[7]);
-      int acc[3][4];
-#pragma unroll
-      for (int j = 0; j < 3; ++j) {
-        const uint4 lo = cur.digit[j][0], hi = cur.digit[j][1];
-        mma_s8_first(acc[j], fa[0], fb[0], fa[1], fb[1], lo.x, lo.y);
-        mma_s8(acc[j], fa[2], fb[2], fa[3], fb[3], lo.z, lo.w);
-        mma_s8(acc[j], fa[4], fb[4], fa[5], fb[5], hi.x, hi.y);
-        mma_s8(acc[j], fa[6], fb[6], fa[7], fb[7], hi.z, hi.w);
-      }
-      const float scale_a = __half2float(cur.scale_a), scale_b = __half2float(cur.scale_b);
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const int dot = acc[0][i] + acc[1][i] * 256 + acc[2][i] * 65536;
-        const float d = __fmul_rn(__int2float_rn(dot), cur.unscale[i & 1]);
-        run[i] = __fadd_rn(run[i], __fmul_rn(i < 2 ? scale_a : scale_b, d));
-      }
-    };
-    // Two fetch buffers used in turn, so that no block's data is copied between
-    // registers: while one block computes the next one's loads are in flight.
-    GroupFetch even = fetch(), odd;
-    for (int b = 0; b < L.B; b += 2) {
-      if (b + 1 < L.B) odd = fetch();
-      compute(even);
-      if (b + 2 < L.B) even = fetch();
-      if (b + 1 < L.B) compute(odd);
-    }
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int pair = (i & 1) ? pair_1 : pair_0;
-      if (pair < 0) continue;
-      const int row = (i < 2) ? row_a : row_b;
-      const int t = pair / L.K, slot = pair - t * L.K;
-      float* out = ws.partial + static_cast<size_t>(t) * 2 * L.N + static_cast<size_t>(slot) * L.I;
-      (row < L.I ? out[row] : out[L.N + row - L.I]) = run[i];
-    }
-  }
-}
-
-// ---------------------------------------------------------------------------
-// grouped screen on the 5th-generation tensor cores (tcgen05, TMEM accumulators)
-// ---------------------------------------------------------------------------
-// Same arithmetic as k_screen_grouped (int8 trits x int8 digits -> exact int32
-// block dots), as one M128 x N32 x K32 `tcgen05.mma.kind::i8` per 32 coordinates.
-// A CTA owns 128 sketch rows of one expert and up to ten of its tokens per pass.
-// Per rotation block one ring stage in shared memory holds
-//   A  the 128 rows x 128 coordinates decoded to int8 (K-major canonical layout,
-//      no swizzle: core matrices of 8 rows x 16 bytes, 128 bytes apart along K,
-//      256 bytes apart along M; four K = 32 steps of 4 KiB), and
-//   B  the three int8 digits of the tokens for those 128 coordinates (column
-//      3 token + digit, same layout, four steps of 1 KiB);
-// both written by eight producer warps (a thread decodes 64 coordinates of one
-// row and forwards one 16-byte piece of digits, all fetched one block ahead).
-// One warp issues the MMAs into one of four 32-column int32 accumulators in
-// tensor memory; four epilogue warps read them back (`tcgen05.ld`), rescale per
-// block and keep the running projections in registers.  Stages and
-// accumulators are handed over with mbarriers; every wait is bounded (about a
-// second) and on expiry sets `status[0]`, makes all roles leave, and the CTA
-// still frees its tensor memory.
-namespace tc {
-
-constexpr int kRows = 128;            // sketch rows per CTA (MMA M)
-constexpr int kCols = 32;             // accumulator columns (MMA N)
-constexpr int kTokens = 10;           // tokens per pass: 3 digit columns each
-constexpr int kStages = 4;            // ring stages = accumulators in flight
-constexpr int kStepBytes = kRows * 32;          // one K = 32 step of A
-constexpr int kDigitStepBytes = kCols * 32;     // one K = 32 step of B
-constexpr int kStageBytes = 4 * (kStepBytes + kDigitStepBytes);  // one rotation block
-constexpr int kProducers = 256;                 // eight producer warps
-constexpr int kThreads = 13 * 32;               // 8 producer, 4 epilogue, 1 MMA warp
-constexpr long long kWaitCycles = 2000000000LL;  // bound of every barrier wait
-
-__device__ __forceinline__ uint32_t shared_address(const void* p) {
-  return static_cast<uint32_t>(__cvta_generic_to_shared(p));
-}
-
-__device__ __forceinline__ void barrier_init(uint32_t bar, int count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
-}
-
-__device__ __forceinline__ void barrier_arrive(uint32_t bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
-}
-
-// Waits for the phase with the given parity; false when the wait ran out or
-// another role already gave up.
-__device__ __forceinline__ bool barrier_wait(uint32_t bar, uint32_t parity, volatile int* abort) {
-  const long long start = clock64();
-  for (;;) {
-    uint32_t done;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(done)
-        : "r"(bar), "r"(parity)
-        : "memory");
-    if (done) return true;
-    if (*abort || clock64() - start > kWaitCycles) {
-      *abort = 1;
-      return false;
-    }
-  }
-}
-
-// Shared-memory matrix descriptor: K-major, no swizzle, 128 bytes between the
-// two 16-byte K chunks of a core-matrix row group, 256 bytes between row groups.
-__device__ __forceinline__ uint64_t matrix_descriptor(uint32_t address) {
-  uint64_t d = 0;
-  d |= static_cast<uint64_t>((address & 0x3ffffu) >> 4);  // start address
-  d |= static_cast<uint64_t>(128 >> 4) << 16;             // leading (K) byte offset
-  d |= static_cast<uint64_t>(256 >> 4) << 32;             // stride (M/N) byte offset
-  d |= static_cast<uint64_t>(1) << 46;                    // descriptor version of sm_100
-  return d;
-}
-
-// Instruction descriptor: int32 accumulate, signed int8 A and B, both K-major.
-__host__ __device__ constexpr uint32_t instruction_descriptor() {
-  return (2u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>(kCols >> 3) << 17) |
-         (static_cast<uint32_t>(kRows >> 4) << 24);
-}
-
-__device__ __forceinline__ void mma_i8(uint32_t tmem, uint64_t a, uint64_t b, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, {%5, %5, %5, %5}, p;\n\t}"
-      :
-      : "r"(tmem), "l"(a), "l"(b), "r"(instruction_descriptor()), "r"(accumulate), "r"(0)
-      : "memory");
-}
-
-__device__ __forceinline__ void mma_commit(uint32_t bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar)
-               : "memory");
-}
-
-__host__ __device__ inline size_t shared_bytes(int B) {
-  return static_cast<size_t>(kStages) * kStageBytes + sizeof(float) * kTokens * B + 256;
-}
-
-}  // namespace tc
-
-// grid (ceil(2I / 128), E, passes), 416 threads, dynamic shared memory
-// tc::shared_bytes(B).
-__global__ void __launch_bounds__(tc::kThreads) k_screen_tc(Layer L, Workspace ws) {
-  using namespace tc;
-  extern __shared__ __align__(1024) uint8_t tc_shared[];
-  uint8_t* ring = tc_shared;  // [kStages][A 16 KiB | B 4 KiB]
-  float* unscale = reinterpret_cast<float*>(ring + kStages * kStageBytes);  // [kTokens][B]
-  uint8_t* tail = reinterpret_cast<uint8_t*>(unscale + kTokens * L.B);
-  uint64_t* barriers = reinterpret_cast<uint64_t*>(tail);  // full, empty, ready, freed x stages
-  int* pairs = reinterpret_cast<int*>(tail + 128);         // [kTokens]
-  uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(tail + 192);
-  volatile int* abort = reinterpret_cast<volatile int*>(tail + 196);
-
-  const int e = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int first = ws.group_offsets[e], total = ws.group_offsets[e + 1] - first;
-  if (total <= static_cast<int>(blockIdx.z) * kTokens) return;  // no pass for this CTA
-  const int rows = 2 * L.I;
-  const uint32_t full = shared_address(barriers), empty = full + 8 * kStages,
-                 ready = empty + 8 * kStages, freed = ready + 8 * kStages;
-
-  if (tid == 0) {
-    *abort = 0;
-    for (int s = 0; s < kStages; ++s) {
-      barrier_init(full + 8 * s, kProducers / 32);  // one lane of every producer warp arrives
-      barrier_init(empty + 8 * s, 1);               // the MMA commit arrives
-      barrier_init(ready + 8 * s, 1);               // the MMA commit arrives
-      barrier_init(freed + 8 * s, 4);               // one lane of every epilogue warp arrives
-    }
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-  }
-  if (warp == 12) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
-                     shared_address(tmem_holder)),
-                 "r"(kStages * kCols)
-                 : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-  }
-  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-  __syncthreads();
-  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  const uint32_t tmem = *tmem_holder;
-
-  int iteration = 0;  // rotation blocks processed so far, over all passes
-  for (int base = kTokens * blockIdx.z; base < total; base += kTokens * gridDim.z) {
-    const int count = min(kTokens, total - base);
-    if (tid < kTokens) pairs[tid] = tid < count ? ws.group_pairs[first + base + tid] : -1;
-    __syncthreads();
-    for (int index = tid; index < kTokens * L.B; index += kThreads) {
-      const int token = index / L.B, b = index - token * L.B;
-      const int pair = pairs[token];
-      const int be =
-          pair >= 0 ? ws.exponents[2 * (static_cast<size_t>(pair / L.K) * L.B + b)] : kQuantBits;
-      unscale[index] = __uint_as_float(static_cast<uint32_t>(127 + be - kQuantBits) << 23);
-    }
-    __syncthreads();
-
-    if (warp < 8) {
-      // ---- producers.  Thread (half, local row): coordinates 64 half .. + 63 of
-      // the row (four words, K steps 2 half and 2 half + 1); it also forwards the
-      // 16-byte piece `piece` of digit column `column` of the block.
-      const int half = tid >> 7, local = tid & 127;
-      const int row = blockIdx.x * kRows + local;
-      const bool inside = row < rows;
-      const uint4* source =
-          reinterpret_cast<const uint4*>(L.sketch_grouped +
-                                         (static_cast<size_t>(e) * L.B * rows + (inside ? row : 0)) *
-                                             (kBlock / 16)) + half;
-      const size_t block_stride = static_cast<size_t>(rows) * (kBlock / 16) / 4;  // uint4 per block
-      const int column = tid >> 3, piece = tid & 7;  // 32 columns x 8 pieces
-      const int token = column / 3, digit = column - 3 * token;
-      const int pair = token < kTokens ? pairs[token] : -1;
-      const uint4* digits =
-          pair >= 0 ? reinterpret_cast<const uint4*>(
-                          ws.limbs + (static_cast<size_t>(pair / L.K) * L.B * 3 + digit) * kBlock) + piece
-                    : nullptr;
-      const size_t digit_stride = 3 * kBlock / 16;  // uint4 per block
-      uint8_t* a_dst = ring + (2 * half) * kStepBytes + (local >> 3) * 256 + (local & 7) * 16;
-      uint8_t* b_dst = ring + 4 * kStepBytes + (piece >> 1) * kDigitStepBytes + (column >> 3) * 256 +
-                       (piece & 1) * 128 + (column & 7) * 16;
-      uint4 next_words = inside ? source[0] : make_uint4(0, 0, 0, 0);
-      uint4 next_digits = digits ? digits[0] : make_uint4(0, 0, 0, 0);
-      for (int b = 0; b < L.B && !*abort; ++b) {
-        const int it = iteration + b, stage = it % kStages;
-        const uint4 words = next_words, piece_bytes = next_digits;
-        if (b + 1 < L.B) {
-          if (inside) next_words = source[(b + 1) * block_stride];
-          if (digits) next_digits = digits[(b + 1) * digit_stride];
-        }
-        if (!barrier_wait(empty + 8 * stage, ((it / kStages) & 1) ^ 1, abort)) break;
-        uint8_t* a_out = a_dst + stage * kStageBytes;
-        const uint32_t four[4] = {words.x, words.y, words.z, words.w};
-#pragma unroll
-        for (int w = 0; w < 4; ++w) {  // word w = coordinates 64 half + 16 w .. + 15
-          uint4 bytes;
-          decode_word(four[w], bytes.x, bytes.y, bytes.z, bytes.w);
-          *reinterpret_cast<uint4*>(a_out + (w >> 1) * kStepBytes + (w & 1) * 128) = bytes;
-        }
-        *reinterpret_cast<uint4*>(b_dst + stage * kStageBytes) = piece_bytes;
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        __syncwarp();
-        if (lane == 0) barrier_arrive(full + 8 * stage);
-      }
-    } else if (warp == 12) {
-      // ---- MMA issue: one lane; four K = 32 steps per rotation block.
-      if (lane == 0) {
-        for (int b = 0; b < L.B && !*abort; ++b) {
-          const int it = iteration + b, stage = it % kStages;
-          const uint32_t parity = (it / kStages) & 1;
-          if (!barrier_wait(full + 8 * stage, parity, abort)) break;
-          if (!barrier_wait(freed + 8 * stage, parity ^ 1, abort)) break;
-          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          const uint32_t a_base = shared_address(ring + stage * kStageBytes);
-          const uint32_t b_base = a_base + 4 * kStepBytes;
-#pragma unroll
-          for (int step = 0; step < 4; ++step)
-            mma_i8(tmem + stage * kCols, matrix_descriptor(a_base + step * kStepBytes),
-                   matrix_descriptor(b_base + step * kDigitStepBytes), step > 0);
-          mma_commit(empty + 8 * stage);  // the stage may be refilled
-          mma_commit(ready + 8 * stage);  // the accumulator may be read
-        }
-      }
-    } else {
-      // ---- epilogue: thread = accumulator lane = sketch row.
-      const int quarter = warp - 8, local = quarter * 32 + lane;
-      const int row = blockIdx.x * kRows + local;
-      const bool inside = row < rows;
-      const __half* scales =
-          L.statistics + static_cast<size_t>(e) * L.B * 2 * rows + (inside ? row : 0);
-      float run[kTokens];
-#pragma unroll
-      for (int t = 0; t < kTokens; ++t) run[t] = 0.0f;
-      float scale = inside ? __half2float(scales[0]) : 0.0f;
-      for (int b = 0; b < L.B && !*abort; ++b) {
-        const int it = iteration + b, stage = it % kStages;
-        const float scale_now = scale;
-        if (inside && b + 1 < L.B)
-          scale = __half2float(scales[static_cast<size_t>(b + 1) * 2 * rows]);
-        if (!barrier_wait(ready + 8 * stage, (it / kStages) & 1, abort)) break;
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        uint32_t c[kCols];
-        const uint32_t address = tmem + (static_cast<uint32_t>(quarter * 32) << 16) + stage * kCols;
-        asm volatile(
-            "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-            "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-            "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
-            : "=r"(c[0]), "=r"(c[1]), "=r"(c[2]), "=r"(c[3]), "=r"(c[4]), "=r"(c[5]), "=r"(c[6]),
-              "=r"(c[7]), "=r"(c[8]), "=r"(c[9]), "=r"(c[10]), "=r"(c[11]), "=r"(c[12]),
-              "=r"(c[13]), "=r"(c[14]), "=r"(c[15]), "=r"(c[16]), "=r"(c[17]), "=r"(c[18]),
-              "=r"(c[19]), "=r"(c[20]), "=r"(c[21]), "=r"(c[22]), "=r"(c[23]), "=r"(c[24]),
-              "=r"(c[25]), "=r"(c[26]), "=r"(c[27]), "=r"(c[28]), "=r"(c[29]), "=r"(c[30]),
-              "=r"(c[31])
-            : "r"(address)
-            : "memory");
-        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-        __syncwarp();
-        if (lane == 0) barrier_arrive(freed + 8 * stage);
-#pragma unroll
-        for (int t = 0; t < kTokens; ++t) {
-          if (t < count) {
-            const int dot = static_cast<int>(c[3 * t]) + static_cast<int>(c[3 * t + 1]) * 256 +
-                            static_cast<int>(c[3 * t + 2]) * 65536;
-            const float d = __fmul_rn(__int2float_rn(dot), unscale[t * L.B + b]);
-            run[t] = __fadd_rn(run[t], __fmul_rn(scale_now, d));
-          }
-        }
-      }
-      if (inside && !*abort) {
-#pragma unroll
-        for (int t = 0; t < kTokens; ++t) {
-          if (t < count) {
-            const int pair = pairs[t];
-            const int token = pair / L.K, slot = pair - token * L.K;
-            float* out = ws.partial + static_cast<size_t>(token) * 2 * L.N +
-                         static_cast<size_t>(slot) * L.I;
-            (row < L.I ? out[row] : out[L.N + row - L.I]) = run[t];
-          }
-        }
-      }
-    }
-    iteration += L.B;
-    __syncthreads();
-    if (*abort) break;
-  }
-  if (*abort && tid == 0) atomicExch(&ws.status[0], 1);
-  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-  __syncthreads();
-  if (warp == 12) {
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem),
-                 "r"(kStages * kCols)
-                 : "memory");
-  }
-}
-
-#include "cfm_screen_rows32.cuh"
-
-// grid (T, ceil(N / 256)), 256 threads: zero the projections of remote or padded
-// slots (the grouped screen writes only live pairs).
-__global__ void k_clear_dead(Layer L, Workspace ws, const uint8_t* padding) {
-  const int t = blockIdx.x, i = blockIdx.y * blockDim.x + threadIdx.x;
-  if (i >= L.N) return;
-  const int slot = i / L.I;
-  if ((padding && padding[t]) || ws.ids[static_cast<size_t>(t) * L.K + slot] < 0) {
-    ws.partial[static_cast<size_t>(t) * 2 * L.N + i] = 0.0f;
-    ws.partial[static_cast<size_t>(t) * 2 * L.N + L.N + i] = 0.0f;
-  }
-}
-
-// grid (T, ceil(N / 256)), 256 threads: scores from projections (used when the
-// scores are exchanged between ranks before selection).
+// grid (T, ceil(N / 256)), 256 threads: zero the scores of remote or padded slots (used when the
+// scores are exchanged between ranks before selection; the screen has written the others).
 __global__ void k_score(Layer L, Workspace ws, const uint8_t* padding) {
   const int t = blockIdx.x, i = blockIdx.y * blockDim.x + threadIdx.x;
   if (i >= L.N) return;
-  const int slot = i / L.I, c = i - slot * L.I;
-  const int e = ws.ids[static_cast<size_t>(t) * L.K + slot];
-  float value = 0.0f;
-  if (e >= 0 && !(padding && padding[t]))
-    value = candidate_score(L, ws, t, i, e, c, ws.weights[static_cast<size_t>(t) * L.K + slot]);
-  ws.scores[static_cast<size_t>(t) * L.N + i] = value;
+  const int slot = i / L.I;
+  if ((padding && padding[t]) || ws.ids[static_cast<size_t>(t) * L.K + slot] < 0)
+    ws.scores[static_cast<size_t>(t) * L.N + i] = 0.0f;
 }
 
 // Residual variance of every candidate's sketch projections (recovery-aware
@@ -1188,22 +551,6 @@ __global__ void __launch_bounds__(256) k_variance(Layer L, Workspace ws, const u
   }
   float* out = ws.variances + static_cast<size_t>(t) * 2 * L.N + static_cast<size_t>(slot) * L.I;
   (row < L.I ? out[row] : out[L.N + row - L.I]) = sum;
-}
-
-// Score of candidate i of token t from its projections (and variances).
-__device__ __forceinline__ float candidate_score(const Layer& L, const Workspace& ws, int t, int i,
-                                                 int e, int c, float weight) {
-  const float* gate = ws.partial + static_cast<size_t>(t) * 2 * L.N;
-  const float norm = L.norms[static_cast<size_t>(e) * L.I + c];
-  if (L.score == CFM_SCORE_POINT) return point_score(gate[i], gate[L.N + i], norm, weight, L.activation);
-  const float* variance = ws.variances + static_cast<size_t>(t) * 2 * L.N;
-  float alpha = 0.0f, beta = 0.0f;
-  if (L.geometry) {
-    alpha = L.geometry[(static_cast<size_t>(e) * L.I + c) * 2];
-    beta = L.geometry[(static_cast<size_t>(e) * L.I + c) * 2 + 1];
-  }
-  return risk_score(gate[i], gate[L.N + i], variance[i], variance[L.N + i], norm, alpha, beta,
-                    weight, L.activation);
 }
 
 // ---------------------------------------------------------------------------
@@ -1347,15 +694,11 @@ __global__ void __launch_bounds__(kSelectThreads)
     if (scores_ready) {
       for (int i = tid; i < N; i += kSelectThreads) keys[i] = __float_as_uint(score[i]);
     } else {
-      // Score every candidate from its sketch projections (zero for remote slots).
+      // The screen's scores; zero for remote slots.
       for (int i = tid; i < N; i += kSelectThreads) {
-        const int slot = slot_of(L, i), c = i - slot * I;
-        const int e = ws.ids[static_cast<size_t>(t) * K + slot];
-        float value = 0.0f;
-        if (e >= 0)
-          value = candidate_score(L, ws, t, i, e, c, ws.weights[static_cast<size_t>(t) * K + slot]);
-        score[i] = value;
-        keys[i] = __float_as_uint(value);
+        const bool live = ws.ids[static_cast<size_t>(t) * K + slot_of(L, i)] >= 0;
+        keys[i] = live ? __float_as_uint(score[i]) : 0u;
+        if (!live) score[i] = 0.0f;
       }
     }
     // Radix search for the F-th largest key: digits of 11, 11 and 10 bits from
@@ -1747,22 +1090,6 @@ constexpr int kDownStages = 4;      // rows in flight per warp (3, 4 and 6 measu
 constexpr int kDownRowBytes = kDownColumns * 2;  // one row's share of a CTA: 2 KiB per warp and row
 constexpr int down_ring_bytes(int stages) { return 4 * stages * kDownRowBytes; }  // per CTA
 
-// 16 bytes global -> shared memory, past L1, completing in the thread's current
-// cp.async group.
-__device__ __forceinline__ void copy_async16(void* shared, const void* global) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
-                   static_cast<uint32_t>(__cvta_generic_to_shared(shared))),
-               "l"(global)
-               : "memory");
-}
-__device__ __forceinline__ void copy_async_commit() {
-  asm volatile("cp.async.commit_group;" ::: "memory");
-}
-template <int PENDING>
-__device__ __forceinline__ void copy_async_wait() {
-  asm volatile("cp.async.wait_group %0;" ::"n"(PENDING) : "memory");
-}
-
 // grid (ceil(H / 1024), tiles, T), 128 threads, down_ring_bytes(kDownStages) of dynamic
 // shared memory.  One CTA sums up to 64 kept rows of one expert, each scaled by its
 // activation, over 1024 output columns.  A warp takes every fourth row of the
@@ -1809,7 +1136,7 @@ __device__ __forceinline__ void down_tile(const Layer& L, const Workspace& ws, i
       const __nv_bfloat16* row = base + static_cast<size_t>(tile_channel[r]) * L.H;
 #pragma unroll
       for (int j = 0; j < CHUNKS; ++j)
-        if (live[j]) copy_async16(mine + s * kDownRowBytes + 512 * j, row + 256 * j);
+        if (live[j]) copy_async16(shared_u32(mine + s * kDownRowBytes + 512 * j), row + 256 * j);
     }
     copy_async_commit();  // also when empty: the group count per iteration stays fixed
   };
@@ -1952,11 +1279,10 @@ __global__ void __launch_bounds__(kEncodeThreads) k_encode(Layer L, Workspace ws
 #pragma unroll
   for (int j = 0; j < 8; ++j) acc[j] = 0.0f;
   if (!dead) {
-    const float* pg = ws.partial + static_cast<size_t>(t) * 2 * L.N + slot * L.I;
-    const float* pu = pg + L.N;
+    const __nv_bfloat16* sketched = ws.features + static_cast<size_t>(t) * L.N + slot * L.I;
     const uint8_t* sel = ws.selected + static_cast<size_t>(t) * L.N + slot * L.I;
     for (int c = c0 + tid; c < c1; c += kEncodeThreads)
-      feature[c - c0] = sel[c] ? 0.0f : sketch_feature(pg[c], pu[c], L.activation);
+      feature[c - c0] = sel[c] ? 0.0f : __bfloat162float(sketched[c]);
     __syncthreads();
     const __nv_bfloat16* enc = L.encoder + static_cast<size_t>(e) * L.I * R + col;
     constexpr int U = 8;
@@ -2376,29 +1702,73 @@ static int launched() {
   return err == cudaSuccess ? 0 : static_cast<int>(err);
 }
 
-static int run_prepare(const Bound& b, const cfm_call* call) {
-  if (b.L.F >= b.L.N) return 0;
-  if (!call->hidden) return CFM_E_NULL;
-  k_prepare<<<dim3(b.T, b.L.B), kBlock, 0, b.stream>>>(
-      b.L, b.ws, static_cast<const __nv_bfloat16*>(call->hidden), b.padding);
+// ---- rules on sizes ----
+// Experts that can have pairs.
+static int busy_experts(const Bound& b) {
+  return static_cast<int>(std::min<int64_t>(b.L.E, static_cast<int64_t>(b.T) * b.L.K));
+}
+// Layers that have a row-major sketch screen expert-major (the kernels read it 16 bytes at a time).
+static bool screens_grouped(const Bound& b) {
+  return b.L.F < b.L.N && b.L.sketch_grouped &&
+         ((reinterpret_cast<uintptr_t>(b.L.sketch_grouped) | reinterpret_cast<uintptr_t>(b.L.statistics)) & 15) == 0;
+}
+// From 16/3 tokens per expert on average, half of the experts or more fill passes of sixteen
+// tokens, which the tcgen05 screen decodes the sketch once for.
+static bool shares_decode(const Bound& b) {
+  return 3 * static_cast<int64_t>(b.T) * b.L.K > 16 * static_cast<int64_t>(b.L.E);
+}
+// The tcgen05 screen, by rule or on request, where its tables fit shared memory.
+static bool screens_tc(const Bound& b) {
+  return (b.L.tensor_engine == CFM_ENGINE_TCGEN05 || shares_decode(b)) && b.L.B <= 512;
+}
+static int pass_pairs(const Bound& b) { return screens_tc(b) && shares_decode(b) ? 16 : 8; }
+
+static int group_smem(const Bound& b, size_t* smem) {
+  *smem = std::max<size_t>(sizeof(int) * b.L.E, sizeof(float) * kPrepareThreads * 4);
+  return *smem > 200 * 1024 ? CFM_E_SHAPE : 0;
+}
+static Routes routes_of(const Bound& b, const cfm_call* call) {
+  Routes r = {};
+  if (call) r = Routes{call->ids, call->weights, call->ids_are_int64, call->weights_are_bf16, 1, 0};
+  r.lanes = 1;
+  while (r.lanes < b.L.K) r.lanes *= 2;
+  r.pass = pass_pairs(b);
+  return r;
+}
+
+// Rotation of the input, or routing and grouping, or both in one launch.
+static int run_prepare(const Bound& b, const cfm_call* call, bool rotate, bool group) {
+  rotate = rotate && b.L.F < b.L.N;
+  if (!rotate && !group) return 0;
+  if (rotate && !call->hidden) return CFM_E_NULL;
+  if (group && (!call->ids || !call->weights)) return CFM_E_NULL;
+  size_t smem;
+  const int rc = group_smem(b, &smem);
+  if (rc) return rc;
+  if (smem > 40 * 1024) {
+    const cudaError_t err = cudaFuncSetAttribute(
+        k_prepare, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    if (err != cudaSuccess) return static_cast<int>(err);
+  }
+  constexpr int kPerCta = kPrepareThreads / 32;
+  const int64_t ctas = rotate ? (static_cast<int64_t>(b.T) * b.L.B + kPerCta - 1) / kPerCta : 0;
+  k_prepare<<<static_cast<unsigned>(ctas + group), kPrepareThreads, smem, b.stream>>>(
+      b.L, b.ws, static_cast<const __nv_bfloat16*>(call->hidden), b.padding, b.T, group,
+      routes_of(b, call));
   return launched();
 }
 
-// Batch size from which the screen runs expert-major on the tensor cores.
-constexpr int kGroupedScreenTokens = 8;
-
-static bool screens_grouped(const Bound& b) {
-  return b.L.F < b.L.N && b.L.sketch_grouped && b.T >= kGroupedScreenTokens && b.L.E <= 4096;
-}
-
-static int run_route(const Bound& b, const cfm_call* call) {
-  if (!call->ids || !call->weights) return CFM_E_NULL;
-  k_route<<<b.T, 32, 0, b.stream>>>(b.L, b.ws, call->ids, call->ids_are_int64, call->weights,
-                                    call->weights_are_bf16);
-  int rc = launched();
-  if (rc || !screens_grouped(b)) return rc;
-  // The expert-major screen reads the (token, slot) pairs grouped by expert.
-  k_group<<<1, 1024, 2 * sizeof(int) * b.L.E, b.stream>>>(b.L, b.ws, b.padding, b.T);
+// Grouping after routes that another kernel wrote.
+static int run_group(const Bound& b) {
+  size_t smem;
+  const int rc = group_smem(b, &smem);
+  if (rc) return rc;
+  if (smem > 40 * 1024) {
+    const cudaError_t err = cudaFuncSetAttribute(
+        k_group, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    if (err != cudaSuccess) return static_cast<int>(err);
+  }
+  k_group<<<1, kPrepareThreads, smem, b.stream>>>(b.L, b.ws, b.padding, b.T, routes_of(b, nullptr));
   return launched();
 }
 
@@ -2415,47 +1785,64 @@ static int launch_screen(const Bound& b, int S) {
   return launched();
 }
 
-static int run_screen_grouped(const Bound& b) {
-  int rc = 0;
-  // Experts with many tokens (few local experts under expert parallelism) spread
-  // their passes of eight tokens over grid.z.
-  const int64_t per_expert = (static_cast<int64_t>(b.T) * b.L.K + b.L.E - 1) / b.L.E;
-  const int passes = static_cast<int>(std::min<int64_t>(8, std::max<int64_t>(1, (per_expert + 7) / 8)));
-  const dim3 grid((2 * b.L.I + kGroupWarps * 16 - 1) / (kGroupWarps * 16), b.L.E, passes);
-  const size_t tc_bytes = tc::shared_bytes(b.L.B);
-  if (b.L.tensor_engine == CFM_ENGINE_TCGEN05 && tc_bytes <= 200 * 1024) {
+template <int TOKENS, bool RISK>
+static int launch_screen_tc(const Bound& b, dim3 grid, int dead) {
+  const size_t smem = Screen<TOKENS>::shared_bytes(b.L.B);
+  const cudaError_t err = cudaFuncSetAttribute(
+      k_screen_tc<TOKENS, RISK>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+  if (err != cudaSuccess) return static_cast<int>(err);
+  launch_dependent(k_screen_tc<TOKENS, RISK>, grid, dim3(kScreenThreads), smem, b.stream, b.L, b.ws,
+                   b.padding, dead);
+  return launched();
+}
+
+template <int W>
+static int launch_screen_tiles(const Bound& b, int rows, int dead) {
+  using S = ScreenTiles<W>;
+  const size_t smem = S::shared_bytes(b.L.B);
+  if (smem > 40 * 1024) {
     const cudaError_t err = cudaFuncSetAttribute(
-        k_screen_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(tc_bytes));
+        k_screen_tiles<W>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
     if (err != cudaSuccess) return static_cast<int>(err);
-    const int tc_passes = static_cast<int>(
-        std::min<int64_t>(8, std::max<int64_t>(1, (per_expert + tc::kTokens - 1) / tc::kTokens)));
-    k_screen_tc<<<dim3(grid.x, grid.y, tc_passes), tc::kThreads, tc_bytes, b.stream>>>(b.L, b.ws);
-  } else if (per_expert < 8 && (reinterpret_cast<uintptr_t>(b.L.sketch_grouped) & 15) == 0 &&
-             (reinterpret_cast<uintptr_t>(b.L.statistics) & 15) == 0) {
-    // Up to eight tokens per expert on average (one pass for most experts): two row
-    // tiles per warp share the digit fragments.  Measured on the benchmark shapes
-    // against the one-tile kernel: 61 vs 67 us (128 experts of width 768, 64 tokens),
-    // 157 vs 257 us (hidden 4096, width 1536, 32 tokens); with eight and more tokens
-    // per expert (256 experts of width 512, 256 tokens) the one-tile kernel, which
-    // has the digits of the next block in registers, is ahead (214 vs 231 us).
-    const dim3 wide((2 * b.L.I + kRows32Warps * 32 - 1) / (kRows32Warps * 32), b.L.E, passes);
-    k_screen_rows32<<<wide, kRows32Warps * 32, 0, b.stream>>>(b.L, b.ws);
-  } else {
-    k_screen_grouped<<<grid, kGroupWarps * 32, 0, b.stream>>>(b.L, b.ws);
   }
-  if ((rc = launched())) return rc;
-  if (b.padding || b.L.expert_map) {
-    k_clear_dead<<<dim3(b.T, (b.L.N + 255) / 256), 256, 0, b.stream>>>(b.L, b.ws, b.padding);
-    rc = launched();
+  const int channels = 16 * S::kTiles;
+  launch_dependent(k_screen_tiles<W>, dim3((b.L.I + channels - 1) / channels, rows),
+                   dim3(S::kThreads), smem, b.stream, b.L, b.ws, b.padding, dead);
+  return launched();
+}
+
+static int run_screen_grouped(const Bound& b) {
+  const int64_t pairs = static_cast<int64_t>(b.T) * b.L.K;
+  const int dead = b.padding || b.L.expert_map ? static_cast<int>(pairs) : 0;
+  const int pass = pass_pairs(b);
+  // Passes, at most; one more row of CTAs clears the dead pairs.
+  const int rows = static_cast<int>(pairs / pass) + busy_experts(b) + (dead > 0);
+  if (screens_tc(b)) {
+    const dim3 grid((b.L.I + kScreenChannels - 1) / kScreenChannels, rows);
+    const bool risk = b.L.score == CFM_SCORE_RECOVERY_AWARE;
+    if (pass == 16)
+      return risk ? launch_screen_tc<16, true>(b, grid, dead) : launch_screen_tc<16, false>(b, grid, dead);
+    return risk ? launch_screen_tc<8, true>(b, grid, dead) : launch_screen_tc<8, false>(b, grid, dead);
   }
-  return rc;
+  // Warps per tile: until the chip's 148 x 16 warps have a share of one of the tiles each.
+  const int64_t tiles = static_cast<int64_t>(busy_experts(b)) * (b.L.I / 16);
+  int W = 1;
+  while (W < 8 && W < b.L.B && tiles * W < 148 * 16) W *= 2;
+  if (const char* v = std::getenv("CFM_W")) W = std::atoi(v);
+  if (b.L.B > 100) W = 1;  // the products of a tile would not fit shared memory
+  switch (W) {
+    case 1: return launch_screen_tiles<1>(b, rows, dead);
+    case 2: return launch_screen_tiles<2>(b, rows, dead);
+    case 4: return launch_screen_tiles<4>(b, rows, dead);
+    default: return launch_screen_tiles<8>(b, rows, dead);
+  }
 }
 
 static int run_screen_projections(const Bound& b);
 
 static int run_screen(const Bound& b) {
   if (b.L.F >= b.L.N) return 0;
-  if (b.L.score == CFM_SCORE_RECOVERY_AWARE) {
+  if (b.L.score == CFM_SCORE_RECOVERY_AWARE && !screens_grouped(b)) {
     k_variance<<<dim3(b.T * b.L.K, (2 * b.L.I + 255) / 256), 256, 0, b.stream>>>(b.L, b.ws,
                                                                                  b.padding);
     const int rc = launched();
@@ -2519,9 +1906,10 @@ static int run_score(const Bound& b) {
   return launched();
 }
 
-// Batches whose pairs are grouped by expert also read the experts' native rows
-// expert-major (the groups come from k_group, launched by route and adopt).
-static bool pairs_grouped(const Bound& b) { return screens_grouped(b); }  // see run_select
+// Batch size from which the native rows are read in expert order (the groups come from route and
+// adopt).
+constexpr int kGroupedTokens = 8;
+static bool pairs_grouped(const Bound& b) { return b.T >= kGroupedTokens; }
 
 // Expert-major exact, down and encode: a row is read once for all the tokens of
 // its expert that kept it.  On the shapes measured so far (4 to 16 tokens per
@@ -2791,8 +2179,8 @@ int cfm_workspace_layout_for(const cfm_layer* layer, int32_t capacity,
     body                                                                           \
   }
 
-CFM_STAGE(cfm_prepare_input, return run_prepare(b, call);)
-CFM_STAGE(cfm_route, return run_route(b, call);)
+CFM_STAGE(cfm_prepare_input, return run_prepare(b, call, true, false);)
+CFM_STAGE(cfm_route, return run_prepare(b, call, false, true);)
 CFM_STAGE(cfm_screen, return run_screen(b);)
 CFM_STAGE(cfm_select, {
   // With an exchange in the call (home rank of an expert-parallel layer, plain
@@ -2861,12 +2249,10 @@ int cfm_adopt(const cfm_layer* layer, void* workspace, int32_t capacity, const c
   }
   k_adopt<<<b.T, 256, 0, b.stream>>>(b.L, b.ws, call->ids, call->ids_are_int64, call->weights,
                                      call->weights_are_bf16, b.padding, call->lists, x, peers);
-  int code = launched();
-  if (code || !pairs_grouped(b)) return code;
+  const int code = launched();
   // The exact and down kernels read the pairs grouped by expert; the down tiles are
   // listed by cfm_list_tiles, which may run beside cfm_exact.
-  k_group<<<1, 1024, 2 * sizeof(int) * b.L.E, b.stream>>>(b.L, b.ws, b.padding, b.T);
-  return launched();
+  return code || !pairs_grouped(b) ? code : run_group(b);
 }
 
 int cfm_build_sketch(const cfm_layer* layer, const void* gate_up, const int8_t* signs,
@@ -2982,17 +2368,7 @@ int cfm_reader_forward(const cfm_layer* layer, void* workspace, int32_t capacity
   };
   Bound on_side = b;
   if (have_side) on_side.stream = side.stream;
-  if (have_side && !call->input_prepared) {
-    // Routing (and the grouping by expert) does not depend on the rotated input:
-    // it runs on the side stream beside the rotation.
-    if ((rc = fork_side())) return leave(rc);
-    if ((rc = run_route(on_side, call))) return leave(rc);
-    if ((rc = run_prepare(b, call))) return leave(rc);
-    if ((rc = join_side())) return leave(rc);
-  } else {
-    if (!call->input_prepared && (rc = run_prepare(b, call))) return rc;
-    if ((rc = run_route(b, call))) return rc;
-  }
+  if ((rc = run_prepare(b, call, !call->input_prepared, true))) return rc;
   if ((rc = run_screen(b))) return rc;
   if ((rc = run_select(b, 0))) return rc;
   // The listing of the down tiles and the recovery encoder (L2-resident rows,

@@ -1,0 +1,267 @@
+// Expert-major screen: int8 tensor-core dots of sketch rows with fixed-point tokens (sm_100a).
+//
+// The (token, expert) pairs are grouped by expert into passes (k_prepare).  A pass's tokens are
+// the columns of the product, three base-256 digits each; the sketch rows' 2-bit codes are its
+// rows, as unsigned bytes 0, 1, 2 (trit + 1), so decoding is a mask and a shift per four codes,
+// and the product is corrected by the sum of the token's values.  Products are exact int32 sums;
+// each rotation block's is rescaled in FP32 and added in block order, as the reference does, so
+// results do not depend on which kernel or split computed them.  A kernel here has both
+// projections of its channels in hand at the end, so it also computes what follows from them
+// alone: the selection score and the feature the recovery encoder takes for a skipped channel
+// (one CTA per token did that in the selection: 10 us of its 25 for one token).
+// Included by cfm_reader.cu inside namespace cfm.
+#pragma once
+
+// Codes of four coordinates as bytes; m = 0 .. 3 gives coordinates {0, 2, 8, 10}, {4, 6, 12, 14},
+// {1, 3, 9, 11}, {5, 7, 13, 15} of a word of the row-major layout.  The digits of a token are
+// stored in the same order (digit_byte).
+__device__ __forceinline__ uint32_t codes_of(uint32_t word, int m) {
+  return (word >> (2 * m)) & 0x03030303u;
+}
+
+// d += (A: unsigned codes) x (B: signed digits), m16n8k32.
+__device__ __forceinline__ void mma_u8s8(int (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2,
+                                         uint32_t a3, uint32_t b0, uint32_t b1) {
+  asm("mma.sync.aligned.m16n8k32.row.col.s32.u8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
+      "{%0,%1,%2,%3};"
+      : "+r"(d[0]), "+r"(d[1]), "+r"(d[2]), "+r"(d[3])
+      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
+// Asks L2 for `bytes` (a multiple of 16) from `p` (16-byte aligned); no data returns.
+__device__ __forceinline__ void prefetch_l2(const void* p, uint32_t bytes) {
+  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
+}
+
+// 2^(e - 21): undoes the fixed point of a block.
+__device__ __forceinline__ float unscale_of(int e) {
+  return __uint_as_float(static_cast<uint32_t>(127 + e - kQuantBits) << 23);
+}
+
+// What the selection and the recovery encoder take from a live candidate's projections (and
+// their residual variances): channel c of expert e, slot `pair` = (token, slot).
+__device__ __forceinline__ void finish_candidate(const Layer& L, const Workspace& ws, int pair,
+                                                 int e, int c, float gate, float up,
+                                                 float gate_variance, float up_variance) {
+  const size_t channel = static_cast<size_t>(e) * L.I + c, at = static_cast<size_t>(pair) * L.I + c;
+  const float norm = L.norms[channel], weight = ws.weights[pair];
+  float score;
+  if (L.score == CFM_SCORE_POINT) {
+    score = point_score(gate, up, norm, weight, L.activation);
+  } else {
+    const float2 geometry = L.geometry ? reinterpret_cast<const float2*>(L.geometry)[channel]
+                                       : make_float2(0.0f, 0.0f);
+    score = risk_score(gate, up, gate_variance, up_variance, norm, geometry.x, geometry.y, weight,
+                       L.activation);
+  }
+  ws.scores[at] = score;  // N = K I: candidate slot * I + c of the token
+  ws.features[at] = __float2bfloat16_rn(sketch_feature(gate, up, L.activation));
+}
+
+// Residual variances of a channel's projections: per block, in block order, the row's FP16
+// residual variance times the energy of the token's kept coordinates.
+__device__ __forceinline__ float2 channel_variance(const Layer& L, const Workspace& ws, int t, int e,
+                                                   int c) {
+  const size_t rows = 2 * static_cast<size_t>(L.I);
+  const __half* gate = L.statistics + (static_cast<size_t>(e) * L.B * 2 + 1) * rows + c;
+  const float* energy = ws.norms + static_cast<size_t>(t) * L.B;
+  float2 sum = make_float2(0.0f, 0.0f);
+#pragma unroll 4
+  for (int b = 0; b < L.B; ++b, gate += 2 * rows) {
+    sum.x = __fadd_rn(sum.x, __fmul_rn(__half2float(gate[0]), energy[b]));
+    sum.y = __fadd_rn(sum.y, __fmul_rn(__half2float(gate[L.I]), energy[b]));
+  }
+  return sum;
+}
+
+// Stores the projections of channel c for a pair and finishes the candidate.
+__device__ __forceinline__ void store_candidate(const Layer& L, const Workspace& ws, int pair, int t,
+                                                int e, int c, float gate, float up) {
+  // Projections of a token: gate plane, up plane, N = K I each; (t K + slot) I = pair I.
+  const size_t at = static_cast<size_t>(t) * L.N + static_cast<size_t>(pair) * L.I + c;
+  ws.partial[at] = gate;
+  ws.partial[at + L.N] = up;
+  float2 variance = make_float2(0.0f, 0.0f);
+  if (L.score != CFM_SCORE_POINT) {
+    variance = channel_variance(L, ws, t, e, c);
+    ws.variances[at] = variance.x;
+    ws.variances[at + L.N] = variance.y;
+  }
+  finish_candidate(L, ws, pair, e, c, gate, up, variance.x, variance.y);
+}
+
+// Zeroes the projections of channels c0 .. c1 - 1 for every remote or padded pair of the call.
+__device__ __forceinline__ void clear_dead(const Layer& L, const Workspace& ws,
+                                           const uint8_t* padding, int pairs, int c0, int c1) {
+  for (int p = threadIdx.x; p < pairs; p += blockDim.x) {
+    const int t = p / L.K;
+    if (ws.ids[p] >= 0 && !(padding && padding[t])) continue;
+    float* gate = ws.partial + static_cast<size_t>(t) * L.N + static_cast<size_t>(p) * L.I;
+    for (int c = c0; c < c1; ++c) gate[c] = gate[L.N + c] = 0.0f;
+  }
+}
+
+// ---------------------------------------------------------------------------
+// warp-level products (mma.sync)
+// ---------------------------------------------------------------------------
+// A tile is sixteen channels of an expert, their gate and up rows, against up to eight tokens.
+// W warps share it, warp w taking rotation blocks w, w + W, ...; lane (g, tq) holds coordinates
+// 32 tq .. + 31 of rows g and g + 8 of both and of token g's digits, all straight from global
+// memory (L1/L2 resident digits, 32 contiguous bytes each), codes one block ahead.  With W = 1
+// the projections stay in registers; otherwise the blocks' products meet in shared memory and
+// are added there in block order.
+//
+// The kernel is bound by dependency latency (some 1.5 us per block and warp, whatever the load),
+// so what counts is warps in flight: calls with few tiles split a tile's blocks over up to eight
+// warps.
+template <int W>
+struct ScreenTiles {
+  static constexpr int kWarps = W > 4 ? W : 4;
+  static constexpr int kTiles = kWarps / W;
+  static constexpr int kThreads = 32 * kWarps;
+  static size_t shared_bytes(int B) {
+    return W > 1 ? static_cast<size_t>(kTiles) * B * 256 * sizeof(float) : 0;
+  }
+};
+
+// grid (ceil(I / (16 tiles)), most passes of eight tokens); with `pairs` one more row of CTAs that
+// clears the projections of the call's dead pairs.
+template <int W>
+__global__ void __launch_bounds__(ScreenTiles<W>::kThreads, 16 / ScreenTiles<W>::kWarps)
+    k_screen_tiles(Layer L, Workspace ws, const uint8_t* padding, int pairs) {
+  using S = ScreenTiles<W>;
+  extern __shared__ float products[];  // [tile][block][gate 0..3, up 0..3][lane]
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, tq = lane & 3;
+  grid_dependency_wait();     // the digits and the passes are complete
+  grid_dependency_release();  // the selection may be scheduled; it waits for this grid
+  const int I = L.I, B = L.B, rows = 2 * I;
+  if (pairs && blockIdx.y == gridDim.y - 1) {
+    const int c0 = blockIdx.x * 16 * S::kTiles;
+    clear_dead(L, ws, padding, pairs, c0, min(I, c0 + 16 * S::kTiles));
+    return;
+  }
+  if (static_cast<int>(blockIdx.y) >= ws.work_counts[kPassCount]) return;
+  const int4 pass = *reinterpret_cast<const int4*>(ws.pass_work + blockIdx.y);
+  const int e = pass.x, first = pass.y, count = pass.z;
+  const int part = warp % W, c0 = (blockIdx.x * S::kTiles + warp / W) * 16;
+  const bool inside = c0 < I;
+  if (W == 1 && !inside) return;
+
+  const size_t row_words = kBlock / 32;  // uint2 per row and block
+  const size_t block_words = static_cast<size_t>(rows) * row_words, up_words = I * row_words;
+  const uint2* codes = reinterpret_cast<const uint2*>(L.sketch_grouped) +
+                       (static_cast<size_t>(e) * B * rows + c0) * row_words;
+  const __half* scales = L.statistics + static_cast<size_t>(e) * B * 2 * rows + c0;
+  if (inside)  // the whole sketch stream of the warp, once: codes 512 bytes, scales 32 per plane
+    for (int b = part + lane * W; b < B; b += 32 * W) {
+      prefetch_l2(codes + b * block_words, 512);
+      prefetch_l2(codes + b * block_words + up_words, 512);
+      prefetch_l2(scales + static_cast<size_t>(b) * 2 * rows, 32);
+      prefetch_l2(scales + static_cast<size_t>(b) * 2 * rows + I, 32);
+    }
+  // Columns beyond the pass repeat its first token.
+  const int pair_g = ws.group_pairs[first + (g < count ? g : 0)];
+  const int token_g = pair_g / L.K;
+  const int pair_0 = __shfl_sync(kFull, pair_g, 8 * tq), pair_1 = __shfl_sync(kFull, pair_g, 8 * tq + 4);
+  const int token_0 = __shfl_sync(kFull, token_g, 8 * tq), token_1 = __shfl_sync(kFull, token_g, 8 * tq + 4);
+
+  struct Words {
+    uint2 row[4];     // 32 coordinates of gate rows g, g + 8 and up rows g, g + 8
+    __half scale[4];  // and the block scales of those rows
+  };
+  const uint2* next_codes = codes + part * block_words + g * row_words + tq;
+  const __half* next_scales = scales + static_cast<size_t>(part) * 2 * rows + g;
+  auto fetch = [&]() {
+    Words w;
+    w.row[0] = next_codes[0];
+    w.row[1] = next_codes[8 * row_words];
+    w.row[2] = next_codes[up_words];
+    w.row[3] = next_codes[up_words + 8 * row_words];
+    w.scale[0] = next_scales[0];
+    w.scale[1] = next_scales[8];
+    w.scale[2] = next_scales[I];
+    w.scale[3] = next_scales[I + 8];
+    next_codes += W * block_words;
+    next_scales += static_cast<size_t>(W) * 2 * rows;
+    return w;
+  };
+  const uint4* digits = reinterpret_cast<const uint4*>(
+      ws.limbs + (static_cast<size_t>(token_g) * B + part) * 3 * kBlock + 32 * tq);
+  const int2* factors_0 = reinterpret_cast<const int2*>(ws.exponents) + static_cast<size_t>(token_0) * B + part;
+  const int2* factors_1 = reinterpret_cast<const int2*>(ws.exponents) + static_cast<size_t>(token_1) * B + part;
+  float run[8] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
+  float* mine = products + (static_cast<size_t>(warp / W) * B + part) * 256 + lane;
+  auto compute = [&](const Words& cur) {
+    uint4 digit[3][2];
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+      digit[j][0] = digits[j * (kBlock / 16)];
+      digit[j][1] = digits[j * (kBlock / 16) + 1];
+    }
+    const int2 f0 = *factors_0, f1 = *factors_1;  // exponent, sum of the values
+    digits += W * 3 * kBlock / 16;
+    factors_0 += W;
+    factors_1 += W;
+    const float unscale[2] = {unscale_of(f0.x), unscale_of(f1.x)};
+#pragma unroll
+    for (int tile = 0; tile < 2; ++tile) {
+      const uint2 a = cur.row[2 * tile], b = cur.row[2 * tile + 1];
+      // code = trit + 1: the sum of the values is taken off where the first sum starts.
+      int acc[3][4] = {{-f0.y, -f1.y, -f0.y, -f1.y}, {0, 0, 0, 0}, {0, 0, 0, 0}};
+#pragma unroll
+      for (int m = 0; m < 4; ++m) {
+        const uint32_t a0 = codes_of(a.x, m), a1 = codes_of(b.x, m);
+        const uint32_t a2 = codes_of(a.y, m), a3 = codes_of(b.y, m);
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+          const uint4 lo = digit[j][0], hi = digit[j][1];
+          mma_u8s8(acc[j], a0, a1, a2, a3, m == 0 ? lo.x : m == 1 ? lo.y : m == 2 ? lo.z : lo.w,
+                   m == 0 ? hi.x : m == 1 ? hi.y : m == 2 ? hi.z : hi.w);
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int dot = acc[0][i] + acc[1][i] * 256 + acc[2][i] * 65536;
+        const float d = __fmul_rn(__int2float_rn(dot), unscale[i & 1]);
+        const float product = __fmul_rn(__half2float(cur.scale[2 * tile + (i >> 1)]), d);
+        if (W == 1) run[4 * tile + i] = __fadd_rn(run[4 * tile + i], product);
+        else mine[(4 * tile + i) * 32] = product;
+      }
+    }
+    if (W > 1) mine += W * 256;
+  };
+  if (inside) {
+    // Two code buffers used in turn: while one block computes, the next one's codes arrive.
+    Words even, odd;
+    if (part < B) even = fetch();
+    for (int b = part; b < B; b += 2 * W) {
+      if (b + W < B) odd = fetch();
+      compute(even);
+      if (b + 2 * W < B) even = fetch();
+      if (b + W < B) compute(odd);
+    }
+  }
+  if (W == 1) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      if (2 * tq + (i & 1) < count)
+        store_candidate(L, ws, (i & 1) ? pair_1 : pair_0, (i & 1) ? token_1 : token_0, e,
+                        c0 + g + 8 * (i >> 1), run[i], run[4 + i]);
+    return;
+  }
+  __syncthreads();
+  // Warp `part` of a tile finishes registers part, part + W of the tile's lanes.
+  if (!inside) return;
+  for (int i = part; i < 4; i += W) {
+    if (2 * tq + (i & 1) >= count) continue;
+    const float* from = products + static_cast<size_t>(warp / W) * B * 256 + i * 32 + lane;
+    float gate = 0.0f, up = 0.0f;
+#pragma unroll 8
+    for (int b = 0; b < B; ++b, from += 256) {
+      gate = __fadd_rn(gate, from[0]);
+      up = __fadd_rn(up, from[128]);
+    }
+    store_candidate(L, ws, (i & 1) ? pair_1 : pair_0, (i & 1) ? token_1 : token_0, e,
+                    c0 + g + 8 * (i >> 1), gate, up);
+  }
+}

@@ -38,9 +38,6 @@ ROW_ENGINES = {"auto": 0, "per_token": 1, "expert_major": 2}
 # path whose results do not depend on them.
 GROUPED_TOKENS = 32
 GROUPED_SCREEN_TOKENS = 64
-# Batch size from which the library screens expert-major; readers with a smaller
-# capacity do not keep the row-major sketch copy that path reads.
-GROUPED_SCREEN_MIN_TOKENS = 8
 
 
 def channel_major_down(weight: Tensor) -> Tensor:
@@ -86,7 +83,8 @@ _TORCH_TYPES = {
     "exact": torch.float32, "down_parts": torch.float32, "encoder_parts": torch.float32,
     "latent": torch.float32, "status": torch.int32, "limbs": torch.int8,
     "group_offsets": torch.int32, "group_pairs": torch.int32, "cuts": torch.int32,
-    "variances": torch.float32, "unscales": torch.float32, "zero_limbs": torch.int8,
+    "variances": torch.float32, "features": torch.bfloat16, "busy_experts": torch.int32,
+    "work_counts": torch.int32,
     "tile_list": torch.int32, "tile_count": torch.int32,
 }
 
@@ -155,7 +153,8 @@ class ReaderWorkspace:
             "encoder_parts": (c, k, layout.encoder_tiles, r), "latent": (c, r),
             "status": (4,), "limbs": (c, blocks, 3, 128),
             "group_offsets": (self.experts + 1,), "group_pairs": (c * k,), "cuts": (c, k + 1),
-            "variances": (c, 2, n), "unscales": (c, blocks), "zero_limbs": (blocks, 3, 128),
+            "variances": (c, 2, n), "features": (c, n),
+            "busy_experts": (self.experts,), "work_counts": (4,),
             "tile_list": (c * (-(-f // 64) + k), 8), "tile_count": (4,),
         }
         for name, shape in shapes.items():
@@ -348,8 +347,9 @@ class ProgressiveReader:
         blocks = h // 128
         if sketch is None and sketch_builder == "cuda":
             # One pass of the library's kernel over the weights, straight into the kernel layouts.
-            self.sketch_words, grouped, statistics = build_sketch_on_device(gate_up, self.sketch_signs)
-            self.sketch_grouped_words = grouped if max_tokens >= GROUPED_SCREEN_MIN_TOKENS else None
+            self.sketch_words, self.sketch_grouped_words, statistics = build_sketch_on_device(
+                gate_up, self.sketch_signs
+            )
             self.sketch_codes = (
                 codes_from_words(self.sketch_words, 2 * i, h) if retain_reference_sketch else None
             )
@@ -370,17 +370,14 @@ class ProgressiveReader:
                 raise ValueError("Sketch must match the local native routed experts")
             # Kernel layout: two bits per trit, [E, H, 2I/16] words.
             self.sketch_words = repack_sketch(codes, 2 * i, h)
-            # Row-major copy for the expert-major screen of batches of 8 tokens and more.
-            self.sketch_grouped_words = (
-                repack_sketch_grouped(codes, 2 * i, h)
-                if max_tokens >= GROUPED_SCREEN_MIN_TOKENS else None
-            )
+            # Row-major copy, which the expert-major screen reads.
+            self.sketch_grouped_words = repack_sketch_grouped(codes, 2 * i, h)
             self.sketch_codes = codes if retain_reference_sketch else None
         self.sketch_statistics = statistics
         self.sketch_resident_bytes = (
             self.sketch_words.numel() * 4
             + statistics.numel() * 2
-            + (self.sketch_grouped_words.numel() * 4 if self.sketch_grouped_words is not None else 0)
+            + self.sketch_grouped_words.numel() * 4
         )
 
         self.norms = down.float().square().sum(1).sqrt().contiguous()
@@ -457,9 +454,7 @@ class ProgressiveReader:
         layer.gate_up = self.native_gu.data_ptr()
         layer.down = self.down.data_ptr()
         layer.sketch = self.sketch_words.data_ptr()
-        layer.sketch_grouped = (
-            self.sketch_grouped_words.data_ptr() if self.sketch_grouped_words is not None else None
-        )
+        layer.sketch_grouped = self.sketch_grouped_words.data_ptr()
         layer.statistics = statistics.data_ptr()
         layer.norms = self.norms.data_ptr()
         layer.geometry = (

@@ -30,7 +30,7 @@
 extern "C" {
 #endif
 
-#define CFM_ABI_VERSION 10
+#define CFM_ABI_VERSION 11
 
 /* argument errors */
 #define CFM_E_NULL -1       /* a required pointer is NULL                      */
@@ -132,7 +132,8 @@ typedef struct cfm_workspace_layout {
   int64_t bytes;
   int64_t ids;            /* i32 [C, K]  experts sorted ascending, local ids    */
   int64_t weights;        /* f32 [C, K]  router weights in the same order       */
-  int64_t norms;          /* f32 [C, B]  energy of the kept rotated coordinates */
+  int64_t norms;          /* f32 [C, B]  energy of the kept rotated coordinates
+                             (recovery-aware score only)                        */
   int64_t planes;         /* f32 [C, B, KEEP] kept rotated values               */
   int64_t coordinates;    /* i32 [C, B, KEEP] their coordinates, ascending      */
   int64_t quantized;      /* i32 [C, B, KEEP] fixed-point kept values           */
@@ -153,13 +154,17 @@ typedef struct cfm_workspace_layout {
   int64_t encoder_parts;  /* f32 [C, K, encoder_tiles, R]                       */
   int64_t latent;         /* f32 [C, R]                                         */
   int64_t status;         /* i32 [4] device-side error flags (zero = healthy)   */
-  int64_t limbs;          /* i8  [C, B, 3, 128] base-256 digits of `quantized`  */
+  int64_t limbs;          /* i8  [C, B, 3, 128] base-256 digits of `quantized`, sixteen
+                             coordinates at a time in the order 0 2 8 10 4 6 12 14
+                             1 3 9 11 5 7 13 15                                 */
   int64_t group_offsets;  /* i32 [E + 1] first pair of every expert             */
   int64_t group_pairs;    /* i32 [C * K] (token, slot) pairs grouped by expert  */
   int64_t cuts;           /* i32 [C, 1 + K] score cut and per-slot tie budgets   */
   int64_t variances;      /* f32 [C, 2, N] residual variances of the projections */
-  int64_t unscales;       /* f32 [C, B] 2^(exponent - 21), undoes the fixed point */
-  int64_t zero_limbs;     /* i8  [B, 3, 128] zero digits for empty token slots    */
+  int64_t features;       /* bf16 [C, N] phi(g) u of the sketch projections     */
+  int64_t pass_work;      /* i32 [.., 4] passes of the screen over the experts   */
+  int64_t busy_experts;   /* i32 [E] experts some pair is routed to, ascending  */
+  int64_t work_counts;    /* i32 [4] passes, busy experts                       */
   int64_t tile_list;      /* i32 [C * (ceil(F / 64) + K), 8] down tiles in expert order */
   int64_t tile_count;     /* i32 [4] number of listed tiles                        */
   int32_t parts_tokens;   /* tokens the split screen can serve                  */
