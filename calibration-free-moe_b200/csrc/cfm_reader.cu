@@ -1717,9 +1717,14 @@ static bool screens_grouped(const Bound& b) {
 static bool shares_decode(const Bound& b) {
   return 3 * static_cast<int64_t>(b.T) * b.L.K > 16 * static_cast<int64_t>(b.L.E);
 }
-// The tcgen05 screen, by rule or on request, where its tables fit shared memory.
+// The tcgen05 screen on request, where it shares its decode, or where its CTAs of 64 channels fill
+// the chip (six per SM): 32 tokens of the 128-expert layer 43.7 us against 49.3 of the warp-level
+// kernel, hidden 4096 and width 1536 136.8 against 161.5; with half of that work in flight (8
+// tokens) 24.7 against 23.1.  Its tables have to fit shared memory.
 static bool screens_tc(const Bound& b) {
-  return (b.L.tensor_engine == CFM_ENGINE_TCGEN05 || shares_decode(b)) && b.L.B <= 512;
+  const int64_t ctas = static_cast<int64_t>(busy_experts(b)) * ((b.L.I + 63) / 64);
+  return (b.L.tensor_engine == CFM_ENGINE_TCGEN05 || shares_decode(b) || ctas >= 6 * 148) &&
+         b.L.B <= 512;
 }
 static int pass_pairs(const Bound& b) { return screens_tc(b) && shares_decode(b) ? 16 : 8; }
 
@@ -1824,18 +1829,12 @@ static int run_screen_grouped(const Bound& b) {
       return risk ? launch_screen_tc<16, true>(b, grid, dead) : launch_screen_tc<16, false>(b, grid, dead);
     return risk ? launch_screen_tc<8, true>(b, grid, dead) : launch_screen_tc<8, false>(b, grid, dead);
   }
-  // Warps per tile: until the chip's 148 x 16 warps have a share of one of the tiles each.
+  // Four warps per tile while one each would not give every SM its sixteen (one token of the
+  // 128-expert layer: 6.9 us against 12.3; 8 tokens 24.5 against 23.4).  The products of a tile
+  // have to fit shared memory.
   const int64_t tiles = static_cast<int64_t>(busy_experts(b)) * (b.L.I / 16);
-  int W = 1;
-  while (W < 8 && W < b.L.B && tiles * W < 148 * 16) W *= 2;
-  if (const char* v = std::getenv("CFM_W")) W = std::atoi(v);
-  if (b.L.B > 100) W = 1;  // the products of a tile would not fit shared memory
-  switch (W) {
-    case 1: return launch_screen_tiles<1>(b, rows, dead);
-    case 2: return launch_screen_tiles<2>(b, rows, dead);
-    case 4: return launch_screen_tiles<4>(b, rows, dead);
-    default: return launch_screen_tiles<8>(b, rows, dead);
-  }
+  if (tiles < 148 * 16 && b.L.B <= 128) return launch_screen_tiles<4>(b, rows, dead);
+  return launch_screen_tiles<1>(b, rows, dead);
 }
 
 static int run_screen_projections(const Bound& b);

@@ -28,11 +28,6 @@ __device__ __forceinline__ void mma_u8s8(int (&d)[4], uint32_t a0, uint32_t a1, 
       : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
-// Asks L2 for `bytes` (a multiple of 16) from `p` (16-byte aligned); no data returns.
-__device__ __forceinline__ void prefetch_l2(const void* p, uint32_t bytes) {
-  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
-}
-
 // 2^(e - 21): undoes the fixed point of a block.
 __device__ __forceinline__ float unscale_of(int e) {
   return __uint_as_float(static_cast<uint32_t>(127 + e - kQuantBits) << 23);
@@ -106,21 +101,24 @@ __device__ __forceinline__ void clear_dead(const Layer& L, const Workspace& ws,
 // ---------------------------------------------------------------------------
 // A tile is sixteen channels of an expert, their gate and up rows, against up to eight tokens.
 // W warps share it, warp w taking rotation blocks w, w + W, ...; lane (g, tq) holds coordinates
-// 32 tq .. + 31 of rows g and g + 8 of both and of token g's digits, all straight from global
-// memory (L1/L2 resident digits, 32 contiguous bytes each), codes one block ahead.  With W = 1
-// the projections stay in registers; otherwise the blocks' products meet in shared memory and
-// are added there in block order.
-//
-// The kernel is bound by dependency latency (some 1.5 us per block and warp, whatever the load),
-// so what counts is warps in flight: calls with few tiles split a tile's blocks over up to eight
-// warps.
+// 32 tq .. + 31 of rows g and g + 8 of both and of token g's digits.  Digits come straight from
+// global memory (L1 resident, 32 contiguous bytes each), codes and scales through a ring of the
+// warp's own in shared memory, four blocks deep, filled with cp.async.  (Requested from L2 with
+// bulk prefetches they cost some 25 cycles of the SM's copy engine per 512 bytes: 25 us at 8
+// tokens of the 128-expert layer.)  With W = 1 the projections stay in registers; otherwise the
+// blocks' products meet in shared memory and are added there in block order.
+// Bound by the integer ALU (58 % busy), the L1 reads of the digits and the latency between them:
+// some 160 cycles of an SM per 32 rows x 128 coordinates x 8 tokens, whatever the split.
 template <int W>
 struct ScreenTiles {
-  static constexpr int kWarps = W > 4 ? W : 4;
+  static constexpr int kWarps = 4;
   static constexpr int kTiles = kWarps / W;
   static constexpr int kThreads = 32 * kWarps;
+  static constexpr int kStages = 4;
+  static constexpr int kStageBytes = 1024 + 64;  // codes of 32 rows, their scales
+  static constexpr int kRingBytes = kWarps * kStages * kStageBytes;
   static size_t shared_bytes(int B) {
-    return W > 1 ? static_cast<size_t>(kTiles) * B * 256 * sizeof(float) : 0;
+    return kRingBytes + (W > 1 ? static_cast<size_t>(kTiles) * B * 256 * sizeof(float) : 0);
   }
 };
 
@@ -130,7 +128,8 @@ template <int W>
 __global__ void __launch_bounds__(ScreenTiles<W>::kThreads, 16 / ScreenTiles<W>::kWarps)
     k_screen_tiles(Layer L, Workspace ws, const uint8_t* padding, int pairs) {
   using S = ScreenTiles<W>;
-  extern __shared__ float products[];  // [tile][block][gate 0..3, up 0..3][lane]
+  extern __shared__ __align__(128) uint8_t tiles_shared[];
+  float* products = reinterpret_cast<float*>(tiles_shared + S::kRingBytes);  // [tile][block][8][lane]
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, tq = lane & 3;
   grid_dependency_wait();     // the digits and the passes are complete
   grid_dependency_release();  // the selection may be scheduled; it waits for this grid
@@ -147,51 +146,45 @@ __global__ void __launch_bounds__(ScreenTiles<W>::kThreads, 16 / ScreenTiles<W>:
   const bool inside = c0 < I;
   if (W == 1 && !inside) return;
 
-  const size_t row_words = kBlock / 32;  // uint2 per row and block
-  const size_t block_words = static_cast<size_t>(rows) * row_words, up_words = I * row_words;
-  const uint2* codes = reinterpret_cast<const uint2*>(L.sketch_grouped) +
-                       (static_cast<size_t>(e) * B * rows + c0) * row_words;
-  const __half* scales = L.statistics + static_cast<size_t>(e) * B * 2 * rows + c0;
-  if (inside)  // the whole sketch stream of the warp, once: codes 512 bytes, scales 32 per plane
-    for (int b = part + lane * W; b < B; b += 32 * W) {
-      prefetch_l2(codes + b * block_words, 512);
-      prefetch_l2(codes + b * block_words + up_words, 512);
-      prefetch_l2(scales + static_cast<size_t>(b) * 2 * rows, 32);
-      prefetch_l2(scales + static_cast<size_t>(b) * 2 * rows + I, 32);
+  // This lane's 16-byte pieces of a block: of the gate and the up codes (512 contiguous bytes
+  // each), and, in four lanes, of the scales.
+  const size_t code_step = static_cast<size_t>(rows) * 32, scale_step = static_cast<size_t>(rows) * 4;
+  const uint8_t* codes = reinterpret_cast<const uint8_t*>(L.sketch_grouped) +
+                         (static_cast<size_t>(e) * B + part) * code_step + c0 * 32 + lane * 16;
+  const uint8_t* scales = reinterpret_cast<const uint8_t*>(L.statistics) +
+                          (static_cast<size_t>(e) * B + part) * scale_step +
+                          ((lane & 2 ? I : 0) + c0 + 8 * (lane & 1)) * 2;
+  uint8_t* ring = tiles_shared + warp * (S::kStages * S::kStageBytes);
+  const uint32_t ring_address = shared_u32(ring) + lane * 16;
+  int fetched = part, fetch_stage = 0;
+  auto fetch = [&]() {  // the next block of this warp
+    if (inside && fetched < B) {
+      const uint32_t to = ring_address + fetch_stage * S::kStageBytes;
+      copy_async16(to, codes);
+      copy_async16(to + 512, codes + static_cast<size_t>(I) * 32);
+      if (lane < 4) copy_async16(to + 1024, scales);
+      codes += W * code_step;
+      scales += W * scale_step;
+      fetched += W;
     }
+    fetch_stage = (fetch_stage + 1) % S::kStages;
+    copy_async_commit();  // also when empty: one group per block
+  };
+#pragma unroll
+  for (int i = 0; i < S::kStages - 1; ++i) fetch();
   // Columns beyond the pass repeat its first token.
   const int pair_g = ws.group_pairs[first + (g < count ? g : 0)];
   const int token_g = pair_g / L.K;
   const int pair_0 = __shfl_sync(kFull, pair_g, 8 * tq), pair_1 = __shfl_sync(kFull, pair_g, 8 * tq + 4);
   const int token_0 = __shfl_sync(kFull, token_g, 8 * tq), token_1 = __shfl_sync(kFull, token_g, 8 * tq + 4);
 
-  struct Words {
-    uint2 row[4];     // 32 coordinates of gate rows g, g + 8 and up rows g, g + 8
-    __half scale[4];  // and the block scales of those rows
-  };
-  const uint2* next_codes = codes + part * block_words + g * row_words + tq;
-  const __half* next_scales = scales + static_cast<size_t>(part) * 2 * rows + g;
-  auto fetch = [&]() {
-    Words w;
-    w.row[0] = next_codes[0];
-    w.row[1] = next_codes[8 * row_words];
-    w.row[2] = next_codes[up_words];
-    w.row[3] = next_codes[up_words + 8 * row_words];
-    w.scale[0] = next_scales[0];
-    w.scale[1] = next_scales[8];
-    w.scale[2] = next_scales[I];
-    w.scale[3] = next_scales[I + 8];
-    next_codes += W * block_words;
-    next_scales += static_cast<size_t>(W) * 2 * rows;
-    return w;
-  };
   const uint4* digits = reinterpret_cast<const uint4*>(
       ws.limbs + (static_cast<size_t>(token_g) * B + part) * 3 * kBlock + 32 * tq);
   const int2* factors_0 = reinterpret_cast<const int2*>(ws.exponents) + static_cast<size_t>(token_0) * B + part;
   const int2* factors_1 = reinterpret_cast<const int2*>(ws.exponents) + static_cast<size_t>(token_1) * B + part;
   float run[8] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
   float* mine = products + (static_cast<size_t>(warp / W) * B + part) * 256 + lane;
-  auto compute = [&](const Words& cur) {
+  auto compute = [&](const uint8_t* stage) {
     uint4 digit[3][2];
 #pragma unroll
     for (int j = 0; j < 3; ++j) {
@@ -205,7 +198,11 @@ __global__ void __launch_bounds__(ScreenTiles<W>::kThreads, 16 / ScreenTiles<W>:
     const float unscale[2] = {unscale_of(f0.x), unscale_of(f1.x)};
 #pragma unroll
     for (int tile = 0; tile < 2; ++tile) {
-      const uint2 a = cur.row[2 * tile], b = cur.row[2 * tile + 1];
+      const uint8_t* from = stage + 512 * tile + g * 32 + tq * 8;
+      const uint2 a = *reinterpret_cast<const uint2*>(from);
+      const uint2 b = *reinterpret_cast<const uint2*>(from + 256);
+      const __half* scale = reinterpret_cast<const __half*>(stage + 1024) + 16 * tile + g;
+      const float scales[2] = {__half2float(scale[0]), __half2float(scale[8])};
       // code = trit + 1: the sum of the values is taken off where the first sum starts.
       int acc[3][4] = {{-f0.y, -f1.y, -f0.y, -f1.y}, {0, 0, 0, 0}, {0, 0, 0, 0}};
 #pragma unroll
@@ -223,7 +220,7 @@ __global__ void __launch_bounds__(ScreenTiles<W>::kThreads, 16 / ScreenTiles<W>:
       for (int i = 0; i < 4; ++i) {
         const int dot = acc[0][i] + acc[1][i] * 256 + acc[2][i] * 65536;
         const float d = __fmul_rn(__int2float_rn(dot), unscale[i & 1]);
-        const float product = __fmul_rn(__half2float(cur.scale[2 * tile + (i >> 1)]), d);
+        const float product = __fmul_rn(scales[i >> 1], d);
         if (W == 1) run[4 * tile + i] = __fadd_rn(run[4 * tile + i], product);
         else mine[(4 * tile + i) * 32] = product;
       }
@@ -231,14 +228,13 @@ __global__ void __launch_bounds__(ScreenTiles<W>::kThreads, 16 / ScreenTiles<W>:
     if (W > 1) mine += W * 256;
   };
   if (inside) {
-    // Two code buffers used in turn: while one block computes, the next one's codes arrive.
-    Words even, odd;
-    if (part < B) even = fetch();
-    for (int b = part; b < B; b += 2 * W) {
-      if (b + W < B) odd = fetch();
-      compute(even);
-      if (b + 2 * W < B) even = fetch();
-      if (b + W < B) compute(odd);
+    int stage = 0;
+    for (int b = part; b < B; b += W) {
+      copy_async_wait<S::kStages - 2>();
+      __syncwarp();  // the block has landed, for all lanes; all have read the one before it
+      fetch();       // into that one's place
+      compute(ring + stage * S::kStageBytes);
+      stage = (stage + 1) % S::kStages;
     }
   }
   if (W == 1) {
