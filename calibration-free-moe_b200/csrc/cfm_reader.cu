@@ -613,7 +613,35 @@ __device__ __forceinline__ void account_reads(const Layer& L, int lane, int loca
   }
 }
 
-// grid (T), 1024 threads, dynamic shared memory: N keys.
+// The same from one slot per lane: whether it is held here and how many channels it kept.
+__device__ __forceinline__ void account_token(const Layer& L, int lane, bool local, int count,
+                                              bool screened) {
+  const int local_slots = __popc(__ballot_sync(kFull, local));
+  const int kept_local = __reduce_add_sync(kFull, local ? count : 0);
+  account_reads(L, lane, local_slots, kept_local, screened);
+}
+
+// Sums over the warps before this one and over all of them of a warp-uniform value; `slots` holds
+// 32 values; one barrier.
+__device__ __forceinline__ uint2 warp_prefix(uint32_t mine, uint32_t* slots) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (lane == 0) slots[warp] = mine;
+  __syncthreads();
+  const uint32_t v = slots[lane];
+  return make_uint2(__reduce_add_sync(kFull, lane < warp ? v : 0u), __reduce_add_sync(kFull, v));
+}
+
+constexpr int kSelectListed = 256;  // keys that one warp finishes the search among
+
+// grid (T), 1024 threads, up to PER keys each in registers: candidate 32 (PER warp + j) + lane.
+// The F-th largest key is searched two bits at a time from the top (three counts of the whole
+// CTA per step, one barrier); once at most 256 keys are left between the bounds, they are listed
+// and one warp goes on alone, a bit at a time.  The search ends when exactly F keys reach its
+// bound.  Then ballots give every warp its keys' places in candidate order.  Bound by the latency
+// of one CTA per token: what only ties, remote slots or budgets need is branched around, and the
+// read-cost counters are left to the output kernel where one follows (`account`).  One token of
+// 6144 candidates: 8.4 us with its launch (a histogram of 2048 bins per eleven bits, built with atomics,
+// a contiguous chunk of candidates per thread and the counters: 14 us).
 // With `peers` (expert parallelism over peer memory; row_offset 0, T = x.tokens) a
 // CTA ends by storing its token's kept list into slot [rank] of every rank's exchange
 // block; the last CTA to arrive releases each destination's flag with the call's epoch.
@@ -623,18 +651,20 @@ struct NoExchange {
   int world, rank, tokens;
   char* block[1];
 };
-template <bool PEERS>
-__global__ void __launch_bounds__(kSelectThreads)
-    k_select(Layer L, Workspace ws, const uint8_t* padding, int scores_ready, int row_offset,
+template <bool PEERS, int PER>
+__global__ void __launch_bounds__(kSelectThreads, PER <= 4 ? 2 : 1)
+    k_select(Layer L, Workspace ws, const uint8_t* padding, int scores_ready, int row_offset, int account,
              typename std::conditional<PEERS, Exchange, NoExchange>::type x) {
   constexpr bool peers = PEERS;
   grid_dependency_release();  // the exact gather may be scheduled; it waits for this grid
   grid_dependency_wait();     // the screen's projections are complete
-  extern __shared__ uint32_t keys[];
-  __shared__ int hist[2048];
-  __shared__ int warp_above[33], warp_ties[32];
-  __shared__ int s_digit, s_remaining;
-  __shared__ int s_starts[33], s_tie_start[33], s_budget[32];
+  __shared__ uint2 s_counts[2][32];
+  __shared__ uint32_t s_slots[2][32], s_listed[kSelectListed];
+  __shared__ uint32_t s_cut;
+  __shared__ int s_take, s_count;
+  __shared__ int s_route[32], s_tie_start[33], s_budget[32];
+  __shared__ uint32_t s_chunk[32 * PER];   // kept candidates of every 32, as bits
+  __shared__ uint16_t s_before[32 * PER];  // kept candidates before them
   const int t = blockIdx.x + row_offset, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int N = L.N, F = L.F, K = L.K, I = L.I;
   const bool cut_given = scores_ready == 2, cut_only = scores_ready == 3;
@@ -687,77 +717,126 @@ __global__ void __launch_bounds__(kSelectThreads)
     return;
   }
   const bool screened = F < N;
-  uint32_t cut = 0;
-  int take_ties = 0;
-  if (screened) {
-    float* score = ws.scores + static_cast<size_t>(t) * N;
-    if (scores_ready) {
-      for (int i = tid; i < N; i += kSelectThreads) keys[i] = __float_as_uint(score[i]);
-    } else {
-      // The screen's scores; zero for remote slots.
-      for (int i = tid; i < N; i += kSelectThreads) {
-        const bool live = ws.ids[static_cast<size_t>(t) * K + slot_of(L, i)] >= 0;
-        keys[i] = live ? __float_as_uint(score[i]) : 0u;
-        if (!live) score[i] = 0.0f;
+  if (tid < 32) {
+    s_route[tid] = tid < K ? ws.ids[static_cast<size_t>(t) * K + tid] : -1;
+  }
+  if (tid == 0) s_count = 0;
+  const int first = 32 * PER * warp + lane;  // this thread's candidates: first, first + 32, ...
+  float* score = ws.scores + static_cast<size_t>(t) * N;
+  uint32_t key[PER];
+#pragma unroll
+  for (int j = 0; j < PER; ++j) {
+    const int i = first + 32 * j;
+    key[j] = screened && i < N ? __float_as_uint(score[i]) : 0u;
+  }
+  __syncthreads();
+  const bool remote = __any_sync(kFull, lane < K && s_route[lane] < 0);
+  if (screened && !scores_ready && remote) {
+#pragma unroll
+    for (int j = 0; j < PER; ++j) {  // the screen's scores; zero for remote slots
+      const int i = first + 32 * j;
+      if (i < N && s_route[slot_of(L, i)] < 0) {
+        key[j] = 0u;
+        score[i] = 0.0f;
       }
     }
-    // Radix search for the F-th largest key: digits of 11, 11 and 10 bits from
-    // the top.  Each pass histograms the keys that match the prefix found so far,
-    // then a block-wide scan from the highest digit down locates the digit in
-    // which the running count reaches the number still wanted.
-    uint32_t prefix = 0, mask = 0;
-    int remaining = F;
-#pragma unroll 1
-    for (int pass = 0; pass < (cut_given ? 0 : 3); ++pass) {
-      const int shift = pass == 0 ? 21 : pass == 1 ? 10 : 0;
-      const int bins = pass == 2 ? 1024 : 2048;
-      for (int i = tid; i < bins; i += kSelectThreads) hist[i] = 0;
-      __syncthreads();
-      for (int i = tid; i < N; i += kSelectThreads) {
-        const uint32_t k = keys[i];
-        if ((k & mask) == prefix) atomicAdd(&hist[(k >> shift) & (bins - 1)], 1);
+  }
+  uint32_t cut = 0;
+  int take_ties = 0;
+  if (screened && !cut_given) {
+    int reached = N, above = 0;  // keys from `cut` up, and beyond the current bounds
+    bool found = false;
+    int shift = 30;
+    for (int step = 0; shift >= 0; shift -= 2, ++step) {
+      uint32_t low = 0, high = 0;  // counts from one and two steps up, from three steps up
+#pragma unroll
+      for (int j = 0; j < PER; ++j) {
+        low += (key[j] >= (cut | (1u << shift)) ? 1u : 0u) + (key[j] >= (cut | (2u << shift)) ? 0x10000u : 0u);
+        high += key[j] >= (cut | (3u << shift)) ? 1u : 0u;
       }
+      low = __reduce_add_sync(kFull, low);
+      high = __reduce_add_sync(kFull, high);
+      if (lane == 0) s_counts[step & 1][warp] = make_uint2(low, high);
       __syncthreads();
-      // Thread tid owns digits bins-1-2*tid and bins-2-2*tid (descending order).
-      const int d0 = bins - 1 - 2 * tid;
-      const int c0 = d0 >= 0 ? hist[d0] : 0;
-      const int c1 = d0 >= 1 ? hist[d0 - 1] : 0;
-      const int total = c0 + c1;
-      int scan = total;
+      const uint2 c = s_counts[step & 1][lane];
+      low = __reduce_add_sync(kFull, c.x);
+      const int c3 = __reduce_add_sync(kFull, c.y), c2 = low >> 16, c1 = low & 0xffff;
+      if (c3 >= F) {
+        cut |= 3u << shift;
+        reached = c3;
+      } else if (c2 >= F) {
+        cut |= 2u << shift;
+        reached = c2;
+        above = c3;
+      } else if (c1 >= F) {
+        cut |= 1u << shift;
+        reached = c1;
+        above = c2;
+      } else {
+        above = c1;
+      }
+      if (reached == F) {  // exactly the keys from the cut up
+        cut -= 1;
+        found = true;
+        break;
+      }
+      if (shift > 0 && reached - above <= kSelectListed) break;
+    }
+    if (!found && shift <= 0) {
+      take_ties = F - above;  // the cut is the F-th largest key
+    } else if (!found) {
+      const uint32_t top = cut + ((1u << shift) - 1);  // largest key within the bounds
+      int inside = 0;
+#pragma unroll
+      for (int j = 0; j < PER; ++j)
+        inside += first + 32 * j < N && key[j] >= cut && key[j] <= top;
+      // Any order will do: a place for every thread's keys from one addition per warp.
+      int scan = inside;
 #pragma unroll
       for (int w = 1; w < 32; w <<= 1) {
         const int o = __shfl_up_sync(kFull, scan, w);
         if (lane >= w) scan += o;
       }
-      if (lane == 31) warp_above[warp] = scan;
+      int at = 0;
+      if (lane == 31 && scan) at = atomicAdd(&s_count, scan);
+      at = __shfl_sync(kFull, at, 31) + scan - inside;
+      if (inside) {
+#pragma unroll
+        for (int j = 0; j < PER; ++j)
+          if (first + 32 * j < N && key[j] >= cut && key[j] <= top) s_listed[at++] = key[j];
+      }
       __syncthreads();
       if (warp == 0) {
-        int totals = warp_above[lane];
+        const int listed = s_count, wanted = F - above;
+        uint32_t k[kSelectListed / 32];
 #pragma unroll
-        for (int w = 1; w < 32; w <<= 1) {
-          const int o = __shfl_up_sync(kFull, totals, w);
-          if (lane >= w) totals += o;
+        for (int j = 0; j < kSelectListed / 32; ++j) k[j] = 32 * j + lane < listed ? s_listed[32 * j + lane] : 0u;
+        auto count_from = [&](uint32_t bound) {
+          int n = 0;
+#pragma unroll
+          for (int j = 0; j < kSelectListed / 32; ++j) n += k[j] >= bound;
+          return __reduce_add_sync(kFull, n);
+        };
+        for (int bit = shift - 1; bit >= 0 && !found; --bit) {
+          const uint32_t trial = cut | (1u << bit);
+          const int n = count_from(trial);
+          if (n >= wanted) cut = trial;
+          found = n == wanted;
         }
-        warp_ties[lane] = totals;  // inclusive scan of the warp totals
+        const int ties = found ? 0 : wanted - count_from(cut + 1);
+        if (lane == 0) {
+          s_cut = found ? cut - 1 : cut;
+          s_take = ties;
+        }
       }
       __syncthreads();
-      const int before = scan - total + (warp ? warp_ties[warp - 1] : 0);
-      if (before < remaining && before + total >= remaining) {
-        const bool first = before + c0 >= remaining;
-        s_digit = first ? d0 : d0 - 1;
-        s_remaining = remaining - (first ? before : before + c0);
-      }
-      __syncthreads();
-      prefix |= static_cast<uint32_t>(s_digit) << shift;
-      mask |= static_cast<uint32_t>(bins - 1) << shift;
-      remaining = s_remaining;
+      cut = s_cut;
+      take_ties = s_take;
     }
-    cut = prefix;
-    take_ties = remaining;
-    if (L.threshold && !cut_given) {
-      // Threshold mode: every score at or above the layer threshold, at most F
-      // (best first).  When fewer than F reach it, the cut moves up to just below
-      // the threshold's key and no tie budget is needed.
+    if (L.threshold) {
+      // Threshold mode: every score at or above the layer threshold, at most F (best first).
+      // When fewer than F reach it, the cut moves up to just below the threshold's key and no
+      // tie budget is needed.
       const uint32_t floor_key = __float_as_uint(__fadd_rn(*L.threshold, 0.0f));
       if (cut < floor_key) {
         cut = floor_key - 1u;
@@ -766,37 +845,32 @@ __global__ void __launch_bounds__(kSelectThreads)
     }
   }
 
-  // Compaction in candidate order: a thread owns a contiguous chunk.  Ties at
-  // the cut are kept in candidate order; that rule is applied slot by slot with a
+  // Ties at the cut are kept in candidate order; that rule is applied slot by slot with a
   // per-slot tie budget, so that a rank holding only some of a token's slots can
   // repeat the selection from the cut and the budgets alone.
-  const int chunk = (N + kSelectThreads - 1) / kSelectThreads;
-  const int begin = min(N, tid * chunk), end = min(N, begin + chunk);
-  const int32_t* route = ws.ids + static_cast<size_t>(t) * K;
   int32_t* cuts = ws.cuts + static_cast<size_t>(t) * (K + 1);
   if (cut_given) cut = static_cast<uint32_t>(cuts[0]);
-  auto block_exclusive = [&](int value, int* total) {
-    return block_exclusive_scan(value, warp_above, total);
-  };
-  // Counts above the cut and tied with it, packed into one scan (N < 65536).
   const bool budgets = cut_given || cut_only;
-  int counted = 0;
-  if (screened)
-    for (int i = begin; i < end; ++i) {
-      const uint32_t k = keys[i];
-      counted += (k > cut ? 0x10000 : 0) + (k == cut ? 1 : 0);
-    }
-  int all_counted = 0;
-  const int counted_before = block_exclusive(counted, &all_counted);
-  const int ties_before = counted_before & 0xffff, above_before = counted_before >> 16;
+  const unsigned before = (1u << lane) - 1;
+  const bool tied_keys = screened && (budgets || take_ties > 0);
+  uint32_t mine = 0;
+  uint2 ties = make_uint2(0, 0);  // before this warp, in all
+  if (tied_keys) {
+#pragma unroll
+    for (int j = 0; j < PER; ++j)
+      mine += __popc(__ballot_sync(kFull, first + 32 * j < N && key[j] == cut));
+    ties = warp_prefix(mine, s_slots[0]);
+  }
   if (budgets) {
-    int running = ties_before;
-    for (int i = begin; i < end; ++i) {
-      const int slot = slot_of(L, i);
-      if (i == slot * I) s_tie_start[slot] = running;
-      running += screened && keys[i] == cut;
+    uint32_t running = ties.x;
+#pragma unroll
+    for (int j = 0; j < PER; ++j) {
+      const int i = first + 32 * j, slot = slot_of(L, min(i, N - 1));
+      const unsigned tied = __ballot_sync(kFull, screened && i < N && key[j] == cut);
+      if (i < N && i == slot * I) s_tie_start[slot] = running + __popc(tied & before);
+      running += __popc(tied);
     }
-    if (tid == 0) s_tie_start[K] = all_counted & 0xffff;
+    if (tid == 0) s_tie_start[K] = ties.y;
     __syncthreads();
     if (tid < K) {
       int budget;
@@ -813,47 +887,68 @@ __global__ void __launch_bounds__(kSelectThreads)
     if (cut_only) return;  // the token's home rank only publishes the cut and the budgets
     __syncthreads();
   }
-  auto keeps = [&](int i, int running) {
-    const int slot = slot_of(L, i);
-    if (cut_given && route[slot] < 0) return false;  // another rank's slot
-    if (!screened) return true;
-    const uint32_t k = keys[i];
-    if (k != cut) return k > cut;
-    return budgets ? running - s_tie_start[slot] < s_budget[slot] : running < take_ties;
-  };
-  int total_kept = screened ? (all_counted >> 16) + min(all_counted & 0xffff, take_ties) : F;
-  int position = above_before + min(ties_before, take_ties);
-  if (!screened) position = begin;
-  if (budgets) {
-    int kept = 0, running = ties_before;
-    for (int i = begin; i < end; ++i) {
-      kept += keeps(i, running);
-      running += screened && keys[i] == cut;
+  uint32_t kept = 0;  // bit j: this thread keeps its candidate j
+#pragma unroll
+  for (int j = 0; j < PER; ++j)
+    kept |= static_cast<uint32_t>(first + 32 * j < N && (!screened || key[j] > cut)) << j;
+  if (tied_keys) {
+    uint32_t running = ties.x;
+#pragma unroll
+    for (int j = 0; j < PER; ++j) {
+      const int i = first + 32 * j;
+      const bool tie = i < N && key[j] == cut;
+      const unsigned tied = __ballot_sync(kFull, tie);
+      const int tie_index = running + __popc(tied & before);
+      running += __popc(tied);
+      if (tie) {
+        const int slot = slot_of(L, i);
+        const bool keep = budgets ? tie_index - s_tie_start[slot] < s_budget[slot] : tie_index < take_ties;
+        kept |= static_cast<uint32_t>(keep) << j;
+      }
     }
-    position = block_exclusive(kept, &total_kept);
   }
+  if (cut_given && remote) {  // other ranks' slots
+#pragma unroll
+    for (int j = 0; j < PER; ++j)
+      if (first + 32 * j < N && s_route[slot_of(L, first + 32 * j)] < 0) kept &= ~(1u << j);
+  }
+  mine = 0;
+#pragma unroll
+  for (int j = 0; j < PER; ++j) mine += __popc(__ballot_sync(kFull, (kept >> j) & 1u));
+  const uint2 kept_counts = warp_prefix(mine, s_slots[1]);
+  const int total_kept = kept_counts.y;
   uint8_t* selected = ws.selected + static_cast<size_t>(t) * N;
   uint8_t* completed = ws.completed + static_cast<size_t>(t) * N;
   int32_t* list = ws.candidate_ids + static_cast<size_t>(t) * F;
   {
-    int running = ties_before;
-    for (int i = begin; i < end; ++i) {
-      const bool keep = keeps(i, running);
-      running += screened && keys[i] == cut;
-      const int slot = slot_of(L, i);
-      if (i - slot * I == 0) s_starts[slot] = position;
-      selected[i] = keep;
-      completed[i] = keep && route[slot] >= 0;
-      if (keep) list[position++] = i;
+    int running = kept_counts.x;
+#pragma unroll
+    for (int j = 0; j < PER; ++j) {
+      const int i = first + 32 * j;
+      const bool keep = (kept >> j) & 1u;
+      const unsigned ballot = __ballot_sync(kFull, keep);
+      if (lane == 0) {
+        s_chunk[warp * PER + j] = ballot;
+        s_before[warp * PER + j] = static_cast<uint16_t>(running);
+      }
+      if (i < N) {
+        selected[i] = keep;
+        completed[i] = keep && (!remote || s_route[slot_of(L, i)] >= 0);
+        if (keep) list[running + __popc(ballot & before)] = i;
+      }
+      running += __popc(ballot);
     }
   }
   for (int i = total_kept + tid; i < F; i += kSelectThreads) list[i] = -1;
-  if (tid == 0) s_starts[K] = total_kept;
   __syncthreads();
   if (warp == 0) {
     const bool live = lane < K;
-    const int count = live ? s_starts[lane + 1] - s_starts[lane] : 0;
-    const bool local = live && route[lane] >= 0;
+    const int from = min(lane, K) * I, chunk = from / 32;  // the slot's first candidate
+    int start = total_kept;
+    if (lane < K) start = s_before[chunk] + __popc(s_chunk[chunk] & ((1u << (from & 31)) - 1));
+    const int next = __shfl_down_sync(kFull, start, 1);
+    const int count = live ? (lane == 31 || lane + 1 >= K ? total_kept : next) - start : 0;
+    const bool local = live && s_route[lane] >= 0;
     const int tiles = local ? (count + kDownTileRows - 1) / kDownTileRows : 0;
     int scan = tiles;
 #pragma unroll
@@ -863,17 +958,10 @@ __global__ void __launch_bounds__(kSelectThreads)
     }
     if (live) {
       counts[lane] = count;
-      starts[lane] = s_starts[lane];
+      starts[lane] = start;
       tile_starts[lane] = scan - tiles;
     }
-    // Read-cost counters of this token (integers, so FP64 atomics are exact).
-    int local_slots = local, kept_local = local ? count : 0;
-#pragma unroll
-    for (int w = 16; w; w >>= 1) {
-      local_slots += __shfl_xor_sync(kFull, local_slots, w);
-      kept_local += __shfl_xor_sync(kFull, kept_local, w);
-    }
-    account_reads(L, lane, local_slots, kept_local, screened);
+    if (account) account_token(L, lane, local, count, screened);
   }
   if (peers) publish(true);
 }
@@ -1474,7 +1562,7 @@ __device__ __forceinline__ float4 mix_down_tiles4(const float* parts, int used, 
 // number of partial sums per local slot the expert-major down kernel wrote, or 0
 // after the per-token down kernel.
 __global__ void __launch_bounds__(128) k_output(Layer L, Workspace ws, const uint8_t* padding,
-                                                __nv_bfloat16* out, int fixed) {
+                                                __nv_bfloat16* out, int fixed, int account) {
   __shared__ float latent[256];
   __shared__ int slot_end[32];       // one past the last down tile of every slot
   __shared__ float slot_weight[32];
@@ -1484,6 +1572,12 @@ __global__ void __launch_bounds__(128) k_output(Layer L, Workspace ws, const uin
     return;
   }
   const bool recover = L.R > 0 && L.owner && L.decoder;
+  if (account && blockIdx.x == 0 && tid >= 96) {  // the token's read-cost counters
+    const int lane = tid - 96;
+    const size_t pair = static_cast<size_t>(t) * L.K + lane;
+    const bool local = lane < L.K && ws.ids[pair] >= 0;
+    account_token(L, lane, local, local ? ws.counts[pair] : 0, L.F < L.N);
+  }
   if (tid < L.K) {
     const size_t pair = static_cast<size_t>(t) * L.K + tid;
     slot_end[tid] = down_slot_end(L, ws, t, tid, fixed);
@@ -1873,23 +1967,25 @@ static int run_screen_projections(const Bound& b) {
 
 static bool pairs_grouped(const Bound& b);
 
-static int run_select(const Bound& b, int scores_ready, const Exchange* exchange = nullptr) {
-  const size_t smem = sizeof(uint32_t) * b.L.N;
-  if (smem + 10240 > 48 * 1024) {  // static shared memory counts against the default limit
-    cudaError_t err = cudaFuncSetAttribute(
-        k_select<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-    if (err == cudaSuccess)
-      err = cudaFuncSetAttribute(k_select<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 static_cast<int>(smem));
-    if (err != cudaSuccess) return static_cast<int>(err);
-  }
+template <int PER>
+static int launch_select(const Bound& b, int scores_ready, const Exchange* exchange, int account) {
   if (exchange)
-    launch_dependent(k_select<true>, dim3(b.T), dim3(kSelectThreads), smem, b.stream, b.L, b.ws,
-                     b.padding, scores_ready, b.row_offset, *exchange);
+    launch_dependent(k_select<true, PER>, dim3(b.T), dim3(kSelectThreads), 0, b.stream, b.L, b.ws,
+                     b.padding, scores_ready, b.row_offset, account, *exchange);
   else
-    launch_dependent(k_select<false>, dim3(b.T), dim3(kSelectThreads), smem, b.stream, b.L, b.ws,
-                     b.padding, scores_ready, b.row_offset, NoExchange{});
+    launch_dependent(k_select<false, PER>, dim3(b.T), dim3(kSelectThreads), 0, b.stream, b.L, b.ws,
+                     b.padding, scores_ready, b.row_offset, account, NoExchange{});
   return launched();
+}
+
+static int run_select(const Bound& b, int scores_ready, const Exchange* exchange, bool account) {
+  const int per = (b.L.N + kSelectThreads - 1) / kSelectThreads;  // keys per thread
+  if (per <= 2) return launch_select<2>(b, scores_ready, exchange, account);
+  if (per <= 4) return launch_select<4>(b, scores_ready, exchange, account);
+  if (per <= 6) return launch_select<6>(b, scores_ready, exchange, account);
+  if (per <= 8) return launch_select<8>(b, scores_ready, exchange, account);
+  if (per <= 12) return launch_select<12>(b, scores_ready, exchange, account);
+  return launch_select<32>(b, scores_ready, exchange, account);
 }
 
 // The down tiles of the call in expert order, once the selection is done.
@@ -2078,11 +2174,11 @@ static int run_encode(const Bound& b) {
   return launched();
 }
 
-static int run_output(const Bound& b, const cfm_call* call) {
+static int run_output(const Bound& b, const cfm_call* call, bool account) {
   if (!call->out) return CFM_E_NULL;
   k_output<<<dim3(b.L.H / 128, b.T), 128, 0, b.stream>>>(
       b.L, b.ws, b.padding, static_cast<__nv_bfloat16*>(call->out),
-      rows_grouped(b) ? down_grouped_parts(b) : 0);
+      rows_grouped(b) ? down_grouped_parts(b) : 0, account);
   return launched();
 }
 
@@ -2191,7 +2287,7 @@ CFM_STAGE(cfm_select, {
     if (bound) return bound;
     if (b.row_offset != 0) return CFM_E_CAPACITY;
   }
-  const int code = run_select(b, call->scores_ready, send ? &x : nullptr);
+  const int code = run_select(b, call->scores_ready, send ? &x : nullptr, true);
   // Mode 3 only publishes the cut; every other mode leaves final counts behind.
   return code || call->scores_ready == 3 ? code : run_list_tiles(b);
 })
@@ -2200,7 +2296,7 @@ CFM_STAGE(cfm_list_tiles, return run_list_tiles(b);)
 CFM_STAGE(cfm_exact, return run_exact(b, call);)
 CFM_STAGE(cfm_down, return run_down(b);)
 CFM_STAGE(cfm_encode, return run_encode(b);)
-CFM_STAGE(cfm_output, return run_output(b, call);)
+CFM_STAGE(cfm_output, return run_output(b, call, false);)
 
 int cfm_partial_output(const cfm_layer* layer, void* workspace, int32_t capacity,
                        const cfm_call* call, void* stream) {
@@ -2369,7 +2465,7 @@ int cfm_reader_forward(const cfm_layer* layer, void* workspace, int32_t capacity
   if (have_side) on_side.stream = side.stream;
   if ((rc = run_prepare(b, call, !call->input_prepared, true))) return rc;
   if ((rc = run_screen(b))) return rc;
-  if ((rc = run_select(b, 0))) return rc;
+  if ((rc = run_select(b, 0, nullptr, false))) return rc;
   // The listing of the down tiles and the recovery encoder (L2-resident rows,
   // arithmetic) run on the side stream beside the two HBM-bound gathers; the down
   // kernel waits for the list, the output mix for the encoder.
@@ -2391,7 +2487,7 @@ int cfm_reader_forward(const cfm_layer* layer, void* workspace, int32_t capacity
   } else if ((rc = run_encode(b))) {
     return rc;
   }
-  return run_output(b, call);
+  return run_output(b, call, true);
 }
 
 }  // extern "C"
