@@ -1,4 +1,4 @@
-// Expert-major exact gate/up, down and recovery-encode kernels (sm_100a).
+// Expert-major exact gate/up and down kernels (sm_100a).
 //
 // From eight tokens per call the (token, expert) pairs are grouped by expert
 // (k_group).  The kernels here walk one expert at a time: a row of the expert's
@@ -7,7 +7,6 @@
 //
 //   k_exact_grouped   gate and up rows of the union of the kept channels
 //   k_down_grouped    channel-major down rows of the same union
-//   k_encode_grouped  recovery-encoder rows, applied to every token of the expert
 //
 // Every CTA rebuilds, in shared memory, what it needs to know about its expert
 // from the kept lists of the expert's tokens (a few hundred list entries): no
@@ -21,8 +20,7 @@ constexpr int kExactGroupedThreads = 256;
 // Tokens whose dot products share one pass over a row's registers.
 constexpr int kExactTogether = 4;
 
-// Tokens of one expert whose partial sums a CTA of k_down_grouped (and of
-// k_encode_grouped) keeps in registers at a time.
+// Tokens of one expert whose partial sums a CTA of k_down_grouped keeps in registers at a time.
 constexpr int kDownChunkTokens = 8;
 constexpr int kDownGroupedColumns = 256;  // output columns per CTA: 8 per lane
 constexpr int kDownGroupedThreads = 128;
@@ -404,141 +402,6 @@ __global__ void __launch_bounds__(kDownGroupedThreads, 4)
       *reinterpret_cast<float4*>(parts_out) =
           make_float4(((a.x + b.x) + d.x) + g.x, ((a.y + b.y) + d.y) + g.y,
                       ((a.z + b.z) + d.z) + g.z, ((a.w + b.w) + d.w) + g.w);
-    }
-  }
-}
-
-// ---------------------------------------------------------------------------
-// encode, expert-major
-// ---------------------------------------------------------------------------
-// Element r of the router-weighted latent of token t from the per-(pair, tile)
-// encoder sums: per live slot the tiles are added in order, rounded to BF16 and
-// mixed by the router weight.
-__device__ __forceinline__ float mix_latent(const Layer& L, const Workspace& ws, int t, int r) {
-  float latent = 0.0f;
-  for (int s = 0; s < L.K; ++s) {
-    if (ws.ids[static_cast<size_t>(t) * L.K + s] < 0) continue;
-    const float* p =
-        ws.encoder_parts + (static_cast<size_t>(t) * L.K + s) * ws.encoder_tiles * L.R + r;
-    float sum = 0.0f;
-    for (int j = 0; j < ws.encoder_tiles; ++j) sum += __ldcg(p + static_cast<size_t>(j) * L.R);
-    latent = fmaf(bf16_round(sum), ws.weights[static_cast<size_t>(t) * L.K + s], latent);
-  }
-  return latent;
-}
-
-// grid (encoder_tiles, E), 256 threads, dynamic shared memory
-// encode_grouped_bytes(R).  A CTA owns 256 channels of one expert: it reads their
-// encoder rows once for up to eight of the expert's tokens at a time.  Features
-// of the skipped channels (zero for kept ones) go to shared memory; LPR = R / 8
-// lanes cover one encoder row (16 bytes each) and 256 / LPR row groups walk the
-// channels, every row applied to the eight tokens' sums in registers; the row
-// groups are folded as in the per-pair kernel (shuffles, then shared memory in
-// warp order), so both give the same bits.  The last CTA to arrive for a token
-// mixes its latent.  Single-device readers only: every slot of every token is
-// local, so a token expects K * encoder_tiles arrivals.
-__host__ __device__ inline size_t encode_grouped_bytes(int R) {
-  return sizeof(float) * (static_cast<size_t>(kDownChunkTokens) * kEncodeTileRows +
-                          static_cast<size_t>(kDownChunkTokens) * (kEncodeThreads / 32) * R);
-}
-
-__global__ void __launch_bounds__(kEncodeThreads)
-    k_encode_grouped(Layer L, Workspace ws) {
-  extern __shared__ float encode_smem[];
-  float (*feature)[kEncodeTileRows] = reinterpret_cast<float (*)[kEncodeTileRows]>(encode_smem);
-  float* red = encode_smem + kDownChunkTokens * kEncodeTileRows;  // [token][fold][R]
-  __shared__ int tok_t[kDownChunkTokens], tok_slot[kDownChunkTokens], tok_last[kDownChunkTokens];
-  const int tile = blockIdx.x, e = blockIdx.y, tid = threadIdx.x;
-  const int first = ws.group_offsets[e], total = ws.group_offsets[e + 1] - first;
-  if (total <= 0) return;
-  const int R = L.R, lpr = R / 8, groups = kEncodeThreads / lpr;
-  const int c0 = tile * kEncodeTileRows, c1 = min(L.I, c0 + kEncodeTileRows);
-  const int group = tid / lpr, col = (tid - group * lpr) * 8;
-  const int lane = tid & 31, warp = tid >> 5;
-  constexpr int kFolds = kEncodeThreads / 32;
-  const __nv_bfloat16* enc = L.encoder + static_cast<size_t>(e) * L.I * R + col;
-
-  for (int begin = 0; begin < total; begin += kDownChunkTokens) {
-    const int tokens = min(kDownChunkTokens, total - begin);
-    __syncthreads();
-    if (tid < tokens) {
-      const int pair = ws.group_pairs[first + begin + tid];
-      tok_t[tid] = pair / L.K;
-      tok_slot[tid] = pair - tok_t[tid] * L.K;
-    }
-    __syncthreads();
-    for (int index = tid; index < tokens * (c1 - c0); index += kEncodeThreads) {
-      const int j = index / (c1 - c0), c = c0 + index - j * (c1 - c0);
-      const size_t t = static_cast<size_t>(tok_t[j]);
-      const size_t at = t * 2 * L.N + static_cast<size_t>(tok_slot[j]) * L.I + c;
-      feature[j][c - c0] =
-          ws.selected[t * L.N + static_cast<size_t>(tok_slot[j]) * L.I + c]
-              ? 0.0f : sketch_feature(ws.partial[at], ws.partial[at + L.N], L.activation);
-    }
-    __syncthreads();
-    float acc[kDownChunkTokens][8];
-#pragma unroll
-    for (int j = 0; j < kDownChunkTokens; ++j)
-#pragma unroll
-      for (int i = 0; i < 8; ++i) acc[j][i] = 0.0f;
-    constexpr int U = 4;
-    for (int base = c0 + group; base < c1; base += groups * U) {
-      uint4 w[U];
-#pragma unroll
-      for (int u = 0; u < U; ++u) {
-        const int c = base + u * groups;
-        w[u] = c < c1 ? *reinterpret_cast<const uint4*>(enc + static_cast<size_t>(c) * R)
-                      : make_uint4(0, 0, 0, 0);
-      }
-#pragma unroll
-      for (int u = 0; u < U; ++u) {
-        const int c = min(base + u * groups, c1 - 1) - c0;
-#pragma unroll
-        for (int j = 0; j < kDownChunkTokens; ++j)
-          if (j < tokens) down_add_row(acc[j], w[u], feature[j][c]);  // uniform over the CTA
-      }
-    }
-    // Fold the row groups that share a warp (lanes lpr apart hold the same columns),
-    // then the warps (or, for rows wider than a warp, the row groups) in order.
-#pragma unroll
-    for (int j = 0; j < kDownChunkTokens; ++j) {
-      if (j < tokens) {
-        for (int w = lpr; w < 32; w <<= 1) {
-#pragma unroll
-          for (int i = 0; i < 8; ++i) acc[j][i] += __shfl_xor_sync(kFull, acc[j][i], w);
-        }
-        float* mine = red + (static_cast<size_t>(j) * kFolds + (lpr >= 32 ? group : warp)) * R + col;
-        if (lpr >= 32 || lane < lpr) {
-#pragma unroll
-          for (int i = 0; i < 8; ++i) mine[i] = acc[j][i];
-        }
-      }
-    }
-    __syncthreads();
-    const int folds = lpr >= 32 ? groups : kFolds;
-    for (int index = tid; index < tokens * R; index += kEncodeThreads) {
-      const int j = index / R, r = index - j * R;
-      float sum = 0.0f;
-      for (int f = 0; f < folds; ++f) sum += red[(static_cast<size_t>(j) * kFolds + f) * R + r];
-      const size_t pair = static_cast<size_t>(tok_t[j]) * L.K + tok_slot[j];
-      ws.encoder_parts[(pair * ws.encoder_tiles + tile) * R + r] = sum;
-    }
-    // The last CTA to arrive for a token mixes its latent.
-    __threadfence();
-    __syncthreads();
-    if (tid < tokens) {
-      uint32_t* counter = ws.counters + 2 * static_cast<size_t>(ws.capacity) * L.K + tok_t[tid];
-      const unsigned expected = static_cast<unsigned>(L.K * ws.encoder_tiles);
-      const unsigned old = atomicAdd(counter, 1u);
-      tok_last[tid] = old == expected - 1;
-      if (tok_last[tid]) *counter = 0;
-    }
-    __syncthreads();
-    for (int index = tid; index < tokens * R; index += kEncodeThreads) {
-      const int j = index / R, r = index - j * R;
-      if (!tok_last[j]) continue;
-      __threadfence();
-      ws.latent[static_cast<size_t>(tok_t[j]) * R + r] = mix_latent(L, ws, tok_t[j], r);
     }
   }
 }

@@ -1050,7 +1050,8 @@ __device__ __forceinline__ void exact_dot(const uint4* gate, const uint4* up, co
 __global__ void __launch_bounds__(kExactWarps * 32) k_exact(Layer L, Workspace ws,
                                                             const __nv_bfloat16* hidden,
                                                             const uint8_t* padding) {
-  grid_dependency_wait();  // the selection is complete
+  grid_dependency_wait();     // the selection is complete
+  grid_dependency_release();  // the down kernel may be scheduled: its encoder needs no more than that
   extern __shared__ uint4 xs[];  // H bf16 values of the token
   const int t = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   if (padding && padding[t]) return;
@@ -1152,55 +1153,164 @@ __device__ __forceinline__ void exact_pair(const Layer& L, const Workspace& ws,
   }
 }
 
+// With `list` one more CTA row, the first, lists the down tiles meanwhile.
 // STRIDED: under expert parallelism fewer CTA rows than (token, slot) pairs are launched,
 // since a rank owns few of them; row y then takes pairs y, y + gridDim.y, ...
 template <bool STRIDED>
 __global__ void __launch_bounds__(kExactWarps * 32) k_exact_pairs(Layer L, Workspace ws,
-                                                                  const __nv_bfloat16* hidden) {
-  grid_dependency_wait();  // the selection is complete
+                                                                  const __nv_bfloat16* hidden,
+                                                                  int list) {
+  grid_dependency_wait();     // the selection is complete
+  grid_dependency_release();  // the down kernel may be scheduled: its encoder needs no more than that
   extern __shared__ uint4 xs[];  // H bf16 values of the token
-  const int pairs = ws.group_offsets[L.E];
-  if (!STRIDED) {
-    if (static_cast<int>(blockIdx.y) < pairs) exact_pair(L, ws, hidden, xs, blockIdx.y);
+  __shared__ int scratch[33];
+  if (list && blockIdx.y == 0) {
+    if (blockIdx.x == 0) list_down_tiles(L, ws, scratch);
     return;
   }
-  for (int y = blockIdx.y; y < pairs; y += gridDim.y) {
+  const int pairs = ws.group_offsets[L.E], first = blockIdx.y - list;
+  if (!STRIDED) {
+    if (first < pairs) exact_pair(L, ws, hidden, xs, first);
+    return;
+  }
+  for (int y = first; y < pairs; y += gridDim.y - list) {
     exact_pair(L, ws, hidden, xs, y);
     __syncthreads();  // the staged row may be overwritten by the next pair
   }
 }
 
 // ---------------------------------------------------------------------------
+// encode: recovery encoder over skipped channels, then the latent
+// ---------------------------------------------------------------------------
+// 128 threads.  A CTA owns 256 channels of one (token, expert) pair: index = pair * tiles + tile.
+// The sketch features of the skipped channels (0 for kept ones) go to shared memory; then the
+// encoder rows stream: LPR = R / 8 lanes cover one row (16 bytes each), 128 / LPR row groups walk
+// the channels with eight rows in flight per thread; last, the row groups fold (shuffles inside a
+// warp, shared memory across warps).  L2 and latency bound, and needed by nothing before the output
+// mix, so its CTAs ride at the head of the down kernel's launch, beside the gathers (a stream of
+// its own cost two events and, for one token, 7 us at its end).  `shared`: 256 + 4 * 256 floats.
+constexpr int kEncodeThreads = 128;
+
+__device__ __forceinline__ void encode_tile(const Layer& L, const Workspace& ws,
+                                            const uint8_t* padding, int index, float* shared) {
+  float* feature = shared;
+  float(*red)[256] = reinterpret_cast<float(*)[256]>(shared + kEncodeTileRows);
+  const int pair = index / ws.encoder_tiles, tile = index - pair * ws.encoder_tiles;
+  const int tid = threadIdx.x, t = pair / L.K, slot = pair - t * L.K;
+  const int R = L.R, lpr = R / 8, groups = kEncodeThreads / lpr;
+  const int e = ws.ids[pair];
+  if ((padding && padding[t]) || e < 0) return;
+  const int c0 = tile * kEncodeTileRows, c1 = min(L.I, c0 + kEncodeTileRows);
+  const int group = tid / lpr, col = (tid - group * lpr) * 8;
+  float acc[8];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) acc[j] = 0.0f;
+  {
+    const size_t first = static_cast<size_t>(t) * L.N + slot * L.I;
+    for (int c = c0 + tid; c < c1; c += kEncodeThreads)
+      feature[c - c0] = ws.selected[first + c] ? 0.0f : __bfloat162float(ws.features[first + c]);
+    __syncthreads();
+    const __nv_bfloat16* enc = L.encoder + static_cast<size_t>(e) * L.I * R + col;
+    constexpr int U = 8;
+    for (int base = c0 + group; base < c1; base += groups * U) {
+      uint4 w[U];
+      float p[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int c = base + u * groups;
+        p[u] = 0.0f;
+        w[u] = make_uint4(0, 0, 0, 0);
+        if (c < c1) {
+          p[u] = feature[c - c0];
+          w[u] = *reinterpret_cast<const uint4*>(enc + static_cast<size_t>(c) * R);
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        acc[0] = fmaf(bf16_lo(w[u].x), p[u], acc[0]);
+        acc[1] = fmaf(bf16_hi(w[u].x), p[u], acc[1]);
+        acc[2] = fmaf(bf16_lo(w[u].y), p[u], acc[2]);
+        acc[3] = fmaf(bf16_hi(w[u].y), p[u], acc[3]);
+        acc[4] = fmaf(bf16_lo(w[u].z), p[u], acc[4]);
+        acc[5] = fmaf(bf16_hi(w[u].z), p[u], acc[5]);
+        acc[6] = fmaf(bf16_lo(w[u].w), p[u], acc[6]);
+        acc[7] = fmaf(bf16_hi(w[u].w), p[u], acc[7]);
+      }
+    }
+  }
+  // Fold the row groups that share a warp (lanes lpr apart hold the same columns).
+  for (int w = lpr; w < 32; w <<= 1) {
+#pragma unroll
+    for (int j = 0; j < 8; ++j) acc[j] += __shfl_xor_sync(kFull, acc[j], w);
+  }
+  const int lane = tid & 31, warp = tid >> 5;
+  if (lane < lpr) {
+#pragma unroll
+    for (int j = 0; j < 8; ++j) red[warp][col + j] = acc[j];
+  }
+  __syncthreads();
+  float* parts = ws.encoder_parts + static_cast<size_t>(index) * R;
+  for (int r = tid; r < R; r += kEncodeThreads)
+    parts[r] = ((red[0][r] + red[1][r]) + red[2][r]) + red[3][r];
+}
+
+// Entry r of a token's latent: per slot the encoder's sums in tile order, rounded to BF16, times the
+// router weight, in slot order.
+__device__ __forceinline__ float mix_latent(const Layer& L, const Workspace& ws, int t, int r) {
+  const size_t pair0 = static_cast<size_t>(t) * L.K;
+  const float* parts = ws.encoder_parts + pair0 * ws.encoder_tiles * L.R + r;
+  float latent = 0.0f;
+#pragma unroll 4
+  for (int s = 0; s < L.K; ++s) {
+    float sum = 0.0f;
+    for (int j = 0; j < ws.encoder_tiles; ++j)
+      sum += parts[static_cast<size_t>(s * ws.encoder_tiles + j) * L.R];
+    if (ws.ids[pair0 + s] >= 0) latent = fmaf(bf16_round(sum), ws.weights[pair0 + s], latent);
+  }
+  return latent;
+}
+
+// The encoder on its own: grid (pairs * tiles), 128 threads.
+__global__ void __launch_bounds__(kEncodeThreads) k_encode(Layer L, Workspace ws,
+                                                           const uint8_t* padding) {
+  __shared__ float shared[kEncodeTileRows + 4 * 256];
+  encode_tile(L, ws, padding, blockIdx.x, shared);
+}
+
+// grid (T), 128 threads: the latents, after an encoder run of its own (padding rows: zero).
+__global__ void k_latent(Layer L, Workspace ws, const uint8_t* padding) {
+  const int t = blockIdx.x;
+  for (int r = threadIdx.x; r < L.R; r += blockDim.x)
+    ws.latent[static_cast<size_t>(t) * L.R + r] =
+        padding && padding[t] ? 0.0f : mix_latent(L, ws, t, r);
+}
+
+// ---------------------------------------------------------------------------
 // down: gathered channel-major down rows
 // ---------------------------------------------------------------------------
-constexpr int kDownColumns = 1024;  // output columns per CTA: 32 accumulators per lane
-constexpr int kDownStages = 4;      // rows in flight per warp (3, 4 and 6 measured alike)
-constexpr int kDownRowBytes = kDownColumns * 2;  // one row's share of a CTA: 2 KiB per warp and row
-constexpr int down_ring_bytes(int stages) { return 4 * stages * kDownRowBytes; }  // per CTA
+constexpr int kDownRingBytes = 32 * 1024;  // per CTA
 
-// grid (ceil(H / 1024), tiles, T), 128 threads, down_ring_bytes(kDownStages) of dynamic
-// shared memory.  One CTA sums up to 64 kept rows of one expert, each scaled by its
-// activation, over 1024 output columns.  A warp takes every fourth row of the
-// tile.  Rows travel through a ring in shared memory, four per warp in flight:
-// per row a lane copies four 16-byte pieces 512 bytes apart (2 KiB contiguous per
-// warp and row) with cp.async and later reads back exactly the pieces it copied,
-// so a lane only ever waits for its own copy groups and the ring needs no barrier.
-// The row is accumulated into 32 FP32 registers per lane in row order; the four
-// warps' sums are added in warp order through shared memory (the ring's, once
-// all copies have landed).  Under expert parallelism (STRIDED) fewer CTAs than
-// tiles are launched per token, since a rank owns few of a token's slots; they
-// walk the tiles in strides.
+// 128 threads, kDownRingBytes of dynamic shared memory.  A CTA sums up to 64 kept rows of one
+// expert, each scaled by its activation, over 256 CHUNKS output columns.  A warp takes every fourth
+// row of the tile.  Rows travel through a ring in shared memory, 16 / CHUNKS per warp in flight:
+// per row a lane copies CHUNKS 16-byte pieces 512 bytes apart with cp.async and later reads back
+// exactly the pieces it copied, so a lane only ever waits for its own copy groups and the ring
+// needs no barrier.  The row is accumulated into 8 CHUNKS FP32 registers per lane in row order;
+// the four warps' sums are added in warp order through shared memory (the ring's, once
+// all copies have landed): same bits for every CHUNKS.  Calls with few tiles split the columns
+// finer, so that their rows come in over more SMs.
 // One tile: `rows` (at most 64) kept rows of slot `slot` of token t, an expert-e
-// slot, whose candidate ids start at `list`, summed into down tile `tile`.
+// slot, whose candidate ids start at `list`, summed into down tile `tile`, columns from `column`.
 // Called by all 128 threads of a CTA; begins and ends with the shared arrays free.
-template <int STAGES>
+template <int CHUNKS>
 __device__ __forceinline__ void down_tile(const Layer& L, const Workspace& ws, int t, int slot,
                                           int e, int rows, const int32_t* list, int tile,
-                                          int* tile_channel, float* tile_activation,
+                                          int column, int* tile_channel, float* tile_activation,
                                           uint8_t* ring) {
-  constexpr int CHUNKS = kDownColumns / 256;  // 16-byte pieces per lane and row
+  constexpr int STAGES = 16 / CHUNKS, kColumns = 256 * CHUNKS, kRowBytes = 2 * kColumns;
+  static_assert(4 * STAGES * kRowBytes == kDownRingBytes, "ring");
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int column0 = blockIdx.x * kDownColumns + lane * 8;  // this lane's first column
+  const int column0 = column + lane * 8;  // this lane's first column
   const __nv_bfloat16* act = ws.activations + static_cast<size_t>(t) * L.N;
   if (tid < rows) {
     const int cid = list[tid];
@@ -1218,13 +1328,13 @@ __device__ __forceinline__ void down_tile(const Layer& L, const Workspace& ws, i
 #pragma unroll
     for (int i = 0; i < 8; ++i) acc[j][i] = 0.0f;
   // This lane's pieces of ring slot s of its warp.
-  uint8_t* mine = ring + warp * (STAGES * kDownRowBytes) + lane * 16;
+  uint8_t* mine = ring + warp * (STAGES * kRowBytes) + lane * 16;
   auto fetch = [&](int r, int s) {  // row r of the tile into slot s; one copy group
     if (r < rows) {
       const __nv_bfloat16* row = base + static_cast<size_t>(tile_channel[r]) * L.H;
 #pragma unroll
       for (int j = 0; j < CHUNKS; ++j)
-        if (live[j]) copy_async16(shared_u32(mine + s * kDownRowBytes + 512 * j), row + 256 * j);
+        if (live[j]) copy_async16(shared_u32(mine + s * kRowBytes + 512 * j), row + 256 * j);
     }
     copy_async_commit();  // also when empty: the group count per iteration stays fixed
   };
@@ -1232,7 +1342,7 @@ __device__ __forceinline__ void down_tile(const Layer& L, const Workspace& ws, i
     const float a = tile_activation[r];
 #pragma unroll
     for (int j = 0; j < CHUNKS; ++j) {
-      const uint4 w = live[j] ? *reinterpret_cast<const uint4*>(mine + s * kDownRowBytes + 512 * j)
+      const uint4 w = live[j] ? *reinterpret_cast<const uint4*>(mine + s * kRowBytes + 512 * j)
                               : make_uint4(0, 0, 0, 0);
       acc[j][0] = fmaf(bf16_lo(w.x), a, acc[j][0]);
       acc[j][1] = fmaf(bf16_hi(w.x), a, acc[j][1]);
@@ -1255,7 +1365,7 @@ __device__ __forceinline__ void down_tile(const Layer& L, const Workspace& ws, i
   }
   copy_async_wait<0>();
   __syncthreads();  // every warp is done with the ring: it now holds the warps' sums
-  float(*red)[kDownColumns] = reinterpret_cast<float(*)[kDownColumns]>(ring);
+  float(*red)[kColumns] = reinterpret_cast<float(*)[kColumns]>(ring);
 #pragma unroll
   for (int j = 0; j < CHUNKS; ++j) {
     float4* out = reinterpret_cast<float4*>(&red[warp][256 * j + lane * 8]);
@@ -1263,10 +1373,9 @@ __device__ __forceinline__ void down_tile(const Layer& L, const Workspace& ws, i
     out[1] = make_float4(acc[j][4], acc[j][5], acc[j][6], acc[j][7]);
   }
   __syncthreads();
-  float* parts = ws.down_parts + (static_cast<size_t>(t) * ws.down_tiles + tile) * L.H +
-                 blockIdx.x * kDownColumns;
-  for (int c = tid * 4; c < kDownColumns; c += 128 * 4) {
-    if (blockIdx.x * kDownColumns + c < L.H) {
+  float* parts = ws.down_parts + (static_cast<size_t>(t) * ws.down_tiles + tile) * L.H + column;
+  for (int c = tid * 4; c < kColumns; c += 128 * 4) {
+    if (column + c < L.H) {
       const float4 a = *reinterpret_cast<const float4*>(&red[0][c]);
       const float4 b = *reinterpret_cast<const float4*>(&red[1][c]);
       const float4 d = *reinterpret_cast<const float4*>(&red[2][c]);
@@ -1279,13 +1388,34 @@ __device__ __forceinline__ void down_tile(const Layer& L, const Workspace& ws, i
   __syncthreads();  // the shared arrays may be reused
 }
 
-template <bool STRIDED, int STAGES>
-__global__ void __launch_bounds__(128, 4) k_down(Layer L, Workspace ws, const uint8_t* padding) {
+// What a launch of a down kernel does: `encode_ctas` CTAs of the recovery encoder first, then
+// `columns` CTAs per tile.
+struct DownGrid {
+  int encode_ctas, columns, tiles;
+};
+
+// The tiles of every token in turn: 1D grid of encode_ctas + T * tiles * columns CTAs.  Under expert
+// parallelism (STRIDED) fewer CTAs than tiles are launched per token, since a rank owns few of a
+// token's slots; they walk the tiles in strides.
+template <bool STRIDED, int CHUNKS>
+__global__ void __launch_bounds__(128, 4) k_down(Layer L, Workspace ws, const uint8_t* padding,
+                                                 DownGrid d) {
   extern __shared__ __align__(128) uint8_t down_ring[];
   __shared__ int tile_channel[kDownTileRows];
   __shared__ float tile_activation[kDownTileRows];
   __shared__ int s_slot, s_first;
-  const int t = blockIdx.z, tid = threadIdx.x;
+  if (static_cast<int>(blockIdx.x) < d.encode_ctas) {
+    grid_dependency_release();
+    encode_tile(L, ws, padding, blockIdx.x, reinterpret_cast<float*>(down_ring));
+    return;
+  }
+  grid_dependency_wait();     // the activations are complete
+  grid_dependency_release();  // the output may be scheduled; it waits for this grid
+  int at = blockIdx.x - d.encode_ctas;
+  const int column = at % d.columns * (256 * CHUNKS);
+  at /= d.columns;
+  const int t = at / d.tiles, tid = threadIdx.x;
+  int tile = at - t * d.tiles;
   if (padding && padding[t]) return;
   const size_t token_pairs = static_cast<size_t>(t) * L.K;
   int used;
@@ -1296,7 +1426,6 @@ __global__ void __launch_bounds__(128, 4) k_down(Layer L, Workspace ws, const ui
         ws.ids[last] >= 0 ? (ws.counts[last] + kDownTileRows - 1) / kDownTileRows : 0;
     used = ws.tile_starts[last] + tail;
   }
-  int tile = blockIdx.y;
   if (tile >= used) return;
   do {
     if (tid == 0) s_slot = -1;
@@ -1314,148 +1443,36 @@ __global__ void __launch_bounds__(128, 4) k_down(Layer L, Workspace ws, const ui
     __syncthreads();
     const int slot = s_slot, first = s_first;
     if (slot < 0) continue;  // uniform: every thread read the same slot
-    down_tile<STAGES>(L, ws, t, slot, ws.ids[token_pairs + slot],
+    down_tile<CHUNKS>(L, ws, t, slot, ws.ids[token_pairs + slot],
               min(kDownTileRows, ws.counts[token_pairs + slot] - first),
               ws.candidate_ids + static_cast<size_t>(t) * L.F + ws.starts[token_pairs + slot] + first,
-              tile, tile_channel, tile_activation, down_ring);
-  } while (STRIDED && (tile += gridDim.y) < used);
+              tile, column, tile_channel, tile_activation, down_ring);
+  } while (STRIDED && (tile += d.tiles) < used);
 }
 
 // The same tiles from the list of the call's tiles in expert order
-// (cfm_select.cuh): grid (ceil(H / 1024), most tiles a call can have), 128
-// threads.  A CTA reads its 32-byte record and goes straight to the tile's rows.
-// Same tiles, same sums, same bits as k_down.
-template <int STAGES>
-__global__ void __launch_bounds__(128, 4) k_down_tiles(Layer L, Workspace ws) {
+// (cfm_select.cuh): 1D grid of encode_ctas + tiles * columns CTAs.  A CTA reads its 32-byte record
+// and goes straight to the tile's rows.  Same tiles, same sums, same bits as k_down.
+template <int CHUNKS>
+__global__ void __launch_bounds__(128, 4) k_down_tiles(Layer L, Workspace ws, const uint8_t* padding,
+                                                       DownGrid d) {
   extern __shared__ __align__(128) uint8_t down_ring[];
   __shared__ int tile_channel[kDownTileRows];
   __shared__ float tile_activation[kDownTileRows];
-  const int tiles = ws.tile_count[0];
-  for (int y = blockIdx.y; y < tiles; y += gridDim.y) {  // strides under expert parallelism
+  if (static_cast<int>(blockIdx.x) < d.encode_ctas) {
+    grid_dependency_release();
+    encode_tile(L, ws, padding, blockIdx.x, reinterpret_cast<float*>(down_ring));
+    return;
+  }
+  grid_dependency_wait();     // the activations and the list are complete
+  grid_dependency_release();  // the output may be scheduled; it waits for this grid
+  const int at = blockIdx.x - d.encode_ctas, tiles = ws.tile_count[0];
+  const int column = at % d.columns * (256 * CHUNKS);
+  for (int y = at / d.columns; y < tiles; y += d.tiles) {  // strides under expert parallelism
     const int4* record = reinterpret_cast<const int4*>(ws.tile_list) + 2 * y;
     const int4 a = record[0], b = record[1];  // t, slot, expert, rows | list, tile
-    down_tile<STAGES>(L, ws, a.x, a.y, a.z, a.w, ws.candidate_ids + b.x, b.y, tile_channel,
+    down_tile<CHUNKS>(L, ws, a.x, a.y, a.z, a.w, ws.candidate_ids + b.x, b.y, column, tile_channel,
                       tile_activation, down_ring);
-  }
-}
-
-// ---------------------------------------------------------------------------
-// encode: recovery encoder over skipped channels, then the latent
-// ---------------------------------------------------------------------------
-// grid (encoder_tiles, T*K), 256 threads.  A CTA owns 256 channels of one
-// (token, expert) pair.  Phase 1 turns the sketch projections of the skipped
-// channels into features in shared memory (0 for kept channels); phase 2
-// streams the encoder rows: LPR = R / 8 lanes cover one row (16 bytes each),
-// 256 / LPR row groups walk the channels with eight rows in flight per thread;
-// phase 3 folds the row groups (shuffles inside a warp, shared memory across
-// warps).  The last CTA of a token to arrive mixes the latent.
-constexpr int kEncodeThreads = 256;
-
-__global__ void __launch_bounds__(kEncodeThreads) k_encode(Layer L, Workspace ws,
-                                                           const uint8_t* padding) {
-  __shared__ float feature[kEncodeTileRows];
-  __shared__ float red[kEncodeThreads / 32][256];
-  __shared__ int s_last;
-  const int tile = blockIdx.x, pair = blockIdx.y, tid = threadIdx.x;
-  const int t = pair / L.K, slot = pair - t * L.K;
-  const int R = L.R, lpr = R / 8, groups = kEncodeThreads / lpr;
-  const int e = ws.ids[pair];
-  const bool dead = (padding && padding[t]) || e < 0;
-  const int c0 = tile * kEncodeTileRows, c1 = min(L.I, c0 + kEncodeTileRows);
-  const int group = tid / lpr, col = (tid - group * lpr) * 8;
-  float acc[8];
-#pragma unroll
-  for (int j = 0; j < 8; ++j) acc[j] = 0.0f;
-  if (!dead) {
-    const __nv_bfloat16* sketched = ws.features + static_cast<size_t>(t) * L.N + slot * L.I;
-    const uint8_t* sel = ws.selected + static_cast<size_t>(t) * L.N + slot * L.I;
-    for (int c = c0 + tid; c < c1; c += kEncodeThreads)
-      feature[c - c0] = sel[c] ? 0.0f : __bfloat162float(sketched[c]);
-    __syncthreads();
-    const __nv_bfloat16* enc = L.encoder + static_cast<size_t>(e) * L.I * R + col;
-    constexpr int U = 8;
-    for (int base = c0 + group; base < c1; base += groups * U) {
-      uint4 w[U];
-      float p[U];
-      if (base + (U - 1) * groups < c1) {
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-          const int c = base + u * groups;
-          p[u] = feature[c - c0];
-          w[u] = *reinterpret_cast<const uint4*>(enc + static_cast<size_t>(c) * R);
-        }
-      } else {
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-          const int c = base + u * groups;
-          p[u] = 0.0f;
-          w[u] = make_uint4(0, 0, 0, 0);
-          if (c < c1) {
-            p[u] = feature[c - c0];
-            w[u] = *reinterpret_cast<const uint4*>(enc + static_cast<size_t>(c) * R);
-          }
-        }
-      }
-#pragma unroll
-      for (int u = 0; u < U; ++u) {
-        acc[0] = fmaf(bf16_lo(w[u].x), p[u], acc[0]);
-        acc[1] = fmaf(bf16_hi(w[u].x), p[u], acc[1]);
-        acc[2] = fmaf(bf16_lo(w[u].y), p[u], acc[2]);
-        acc[3] = fmaf(bf16_hi(w[u].y), p[u], acc[3]);
-        acc[4] = fmaf(bf16_lo(w[u].z), p[u], acc[4]);
-        acc[5] = fmaf(bf16_hi(w[u].z), p[u], acc[5]);
-        acc[6] = fmaf(bf16_lo(w[u].w), p[u], acc[6]);
-        acc[7] = fmaf(bf16_hi(w[u].w), p[u], acc[7]);
-      }
-    }
-  }
-  // Fold the row groups that share a warp (lanes lpr apart hold the same columns).
-  for (int w = lpr; w < 32; w <<= 1) {
-#pragma unroll
-    for (int j = 0; j < 8; ++j) acc[j] += __shfl_xor_sync(kFull, acc[j], w);
-  }
-  const int lane = tid & 31, warp = tid >> 5;
-  if (lpr >= 32) {
-    // One row spans the whole warp or more: lane owns columns (tid % lpr) * 8.
-#pragma unroll
-    for (int j = 0; j < 8; ++j) red[group][col + j] = acc[j];
-  } else if (lane < lpr) {
-#pragma unroll
-    for (int j = 0; j < 8; ++j) red[warp][col + j] = acc[j];
-  }
-  __syncthreads();
-  const int folds = lpr >= 32 ? groups : kEncodeThreads / 32;
-  float* parts = ws.encoder_parts + (static_cast<size_t>(pair) * ws.encoder_tiles + tile) * R;
-  for (int r = tid; r < R; r += kEncodeThreads) {
-    float sum = 0.0f;
-    for (int f = 0; f < folds; ++f) sum += red[f][r];
-    parts[r] = sum;
-  }
-  // Last CTA of the token mixes the latent.
-  __threadfence();
-  __syncthreads();
-  uint32_t* counter = ws.counters + 2 * static_cast<size_t>(ws.capacity) * L.K + t;
-  if (tid == 0) {
-    const unsigned total = static_cast<unsigned>(L.K * ws.encoder_tiles);
-    const unsigned old = atomicAdd(counter, 1u);
-    s_last = (old == total - 1);
-    if (s_last) *counter = 0;
-  }
-  __syncthreads();
-  if (!s_last) return;
-  __threadfence();
-  for (int r = tid; r < R; r += kEncodeThreads) {
-    float latent = 0.0f;
-    for (int s2 = 0; s2 < L.K; ++s2) {
-      const int pe = ws.ids[static_cast<size_t>(t) * L.K + s2];
-      if (pe < 0 || (padding && padding[t])) continue;
-      const float* p = ws.encoder_parts +
-                       (static_cast<size_t>(t) * L.K + s2) * ws.encoder_tiles * R + r;
-      float sum = 0.0f;
-      for (int j = 0; j < ws.encoder_tiles; ++j) sum += __ldcg(p + static_cast<size_t>(j) * R);
-      latent = fmaf(bf16_round(sum), ws.weights[static_cast<size_t>(t) * L.K + s2], latent);
-    }
-    ws.latent[static_cast<size_t>(t) * R + r] = latent;
   }
 }
 
@@ -1558,36 +1575,40 @@ __device__ __forceinline__ float4 mix_down_tiles4(const float* parts, int used, 
   return routed;
 }
 
-// grid (H / 128, T), 128 threads, one output column per thread.  `fixed` is the
+// grid (H / 128, T), 128 threads, one output column per thread; with one more column of CTAs that
+// add the tokens' read-cost counters.  `fixed` is the
 // number of partial sums per local slot the expert-major down kernel wrote, or 0
 // after the per-token down kernel.
-__global__ void __launch_bounds__(128) k_output(Layer L, Workspace ws, const uint8_t* padding,
-                                                __nv_bfloat16* out, int fixed, int account) {
+// Where the output kernel finds a token's latent: in the workspace, in the encoder's sums (it then
+// also leaves it in the workspace), or nowhere (zero).
+constexpr int kLatentGiven = 0, kLatentMix = 1, kLatentZero = 2;
+
+__global__ void __launch_bounds__(128, 6) k_output(Layer L, Workspace ws, const uint8_t* padding,
+                                                __nv_bfloat16* out, int fixed, int latents,
+                                                int early) {
   __shared__ float latent[256];
   __shared__ int slot_end[32];       // one past the last down tile of every slot
   __shared__ float slot_weight[32];
   const int t = blockIdx.y, tid = threadIdx.x, h = blockIdx.x * 128 + tid;
+  if (!early) grid_dependency_wait();
+  if (h >= L.H) {  // the token's read-cost counters
+    if (tid < 32 && !(padding && padding[t])) {
+      const size_t pair = static_cast<size_t>(t) * L.K + tid;
+      const bool local = tid < L.K && ws.ids[pair] >= 0;
+      account_token(L, tid, local, local ? ws.counts[pair] : 0, L.F < L.N);
+    }
+    return;
+  }
   if (padding && padding[t]) {
+    if (early) grid_dependency_wait();
     out[static_cast<size_t>(t) * L.H + h] = __float2bfloat16_rn(0.0f);
+    if (latents != kLatentGiven && blockIdx.x == 0)
+      for (int r = tid; r < L.R; r += 128) ws.latent[static_cast<size_t>(t) * L.R + r] = 0.0f;
     return;
   }
   const bool recover = L.R > 0 && L.owner && L.decoder;
-  if (account && blockIdx.x == 0 && tid >= 96) {  // the token's read-cost counters
-    const int lane = tid - 96;
-    const size_t pair = static_cast<size_t>(t) * L.K + lane;
-    const bool local = lane < L.K && ws.ids[pair] >= 0;
-    account_token(L, lane, local, local ? ws.counts[pair] : 0, L.F < L.N);
-  }
-  if (tid < L.K) {
-    const size_t pair = static_cast<size_t>(t) * L.K + tid;
-    slot_end[tid] = down_slot_end(L, ws, t, tid, fixed);
-    slot_weight[tid] = ws.weights[pair];
-  }
-  if (recover)
-    for (int r = tid; r < L.R; r += 128)
-      latent[r] = bf16_round(ws.latent[static_cast<size_t>(t) * L.R + r]);
-  // The decoder row does not depend on the slot table: its first chunks are on their
-  // way before the barrier.
+  // With `early` the down kernel is the launch before this one, so the selection is complete when
+  // this grid starts; the decoder row and the slot table are read while the last tiles are summed.
   constexpr int kAhead = 8;  // 16-byte chunks of the decoder row fetched ahead (R <= 64: all)
   float correction = 0.0f;
   const uint4* decoder_row = reinterpret_cast<const uint4*>(L.decoder + static_cast<size_t>(h) * L.R);
@@ -1596,6 +1617,18 @@ __global__ void __launch_bounds__(128) k_output(Layer L, Workspace ws, const uin
 #pragma unroll
     for (int i = 0; i < kAhead; ++i)
       ahead[i] = i < L.R / 8 ? decoder_row[i] : make_uint4(0, 0, 0, 0);
+  }
+  if (tid < L.K) {
+    const size_t pair = static_cast<size_t>(t) * L.K + tid;
+    slot_end[tid] = down_slot_end(L, ws, t, tid, fixed);
+    slot_weight[tid] = ws.weights[pair];
+  }
+  if (early) grid_dependency_wait();  // the sums are complete
+  for (int r = tid; r < L.R; r += 128) {
+    float* kept = ws.latent + static_cast<size_t>(t) * L.R + r;
+    const float z = latents == kLatentGiven ? *kept : latents == kLatentMix ? mix_latent(L, ws, t, r) : 0.0f;
+    if (latents != kLatentGiven && blockIdx.x == 0) *kept = z;
+    latent[r] = bf16_round(z);
   }
   __syncthreads();
   const int used = slot_end[L.K - 1];  // tiles are laid out slot after slot
@@ -2044,7 +2077,8 @@ static int run_exact_grouped(const Bound& b, const cfm_call* call) {
   return launched();
 }
 
-static int run_exact(const Bound& b, const cfm_call* call) {
+// `list`: list the down tiles too.
+static int run_exact(const Bound& b, const cfm_call* call, bool list) {
   if (!call->hidden || !b.L.gate_up) return CFM_E_NULL;
   if (rows_grouped(b)) return run_exact_grouped(b, call);
   const size_t smem = static_cast<size_t>(b.L.H) * 2;
@@ -2070,13 +2104,15 @@ static int run_exact(const Bound& b, const cfm_call* call) {
                                       rows, (2 * rows * b.L.E + b.L.global_experts - 1) /
                                                 b.L.global_experts));
     if (rows < static_cast<int64_t>(b.T) * b.L.K)
-      launch_dependent(k_exact_pairs<true>, dim3(ctas, static_cast<unsigned>(rows)),
+      launch_dependent(k_exact_pairs<true>, dim3(ctas, static_cast<unsigned>(rows + list)),
                        dim3(kExactWarps * 32), smem, b.stream, b.L, b.ws,
-                       static_cast<const __nv_bfloat16*>(call->hidden));
+                       static_cast<const __nv_bfloat16*>(call->hidden),
+                       static_cast<int>(list));
     else
-      launch_dependent(k_exact_pairs<false>, dim3(ctas, static_cast<unsigned>(rows)),
+      launch_dependent(k_exact_pairs<false>, dim3(ctas, static_cast<unsigned>(rows + list)),
                        dim3(kExactWarps * 32), smem, b.stream, b.L, b.ws,
-                       static_cast<const __nv_bfloat16*>(call->hidden));
+                       static_cast<const __nv_bfloat16*>(call->hidden),
+                       static_cast<int>(list));
     return launched();
   }
   int ctas = (b.L.F + kExactWarps - 1) / kExactWarps;
@@ -2092,13 +2128,8 @@ static int run_exact(const Bound& b, const cfm_call* call) {
   return launched();
 }
 
-// Passes the ring depth of the down kernels to `launch` as a compile-time constant.
-template <typename Launch>
-static int launch_down(Launch launch) {
-  return launch(std::integral_constant<int, kDownStages>{});
-}
-
-static int run_down(const Bound& b) {
+// `encode`: run the recovery encoder too.
+static int run_down(const Bound& b, bool encode) {
   if (!b.L.down) return CFM_E_NULL;
   if (rows_grouped(b)) {
     const size_t smem = down_grouped_bytes(b.L.I);
@@ -2112,47 +2143,45 @@ static int run_down(const Bound& b) {
     k_down_grouped<<<grid, kDownGroupedThreads, smem, b.stream>>>(b.L, b.ws, parts);
     return launched();
   }
-  if (pairs_grouped(b)) {
-    // The call's tiles were listed in expert order after the selection.
-    int64_t most = static_cast<int64_t>(b.T) * ((b.L.F + kDownTileRows - 1) / kDownTileRows + b.L.K);
-    if (b.L.expert_map && b.L.global_experts > 0)  // twice the expected share of the tiles
-      most = std::max<int64_t>(8, std::min<int64_t>(
-                                      most, (2 * most * b.L.E + b.L.global_experts - 1) /
-                                                b.L.global_experts));
-    const dim3 grid((b.L.H + kDownColumns - 1) / kDownColumns, static_cast<unsigned>(most));
-    return launch_down([&](auto stages) {
-      constexpr int S = decltype(stages)::value;
-      cudaError_t err = cudaFuncSetAttribute(
-          k_down_tiles<S>, cudaFuncAttributeMaxDynamicSharedMemorySize, down_ring_bytes(S));
-      if (err != cudaSuccess) return static_cast<int>(err);
-      k_down_tiles<S><<<grid, 128, down_ring_bytes(S), b.stream>>>(b.L, b.ws);
-      return launched();
-    });
-  }
-  int tiles = b.ws.down_tiles;
-  if (b.L.expert_map && b.L.global_experts > 0) {
-    // Expert parallel: about E / global of a token's tiles are local; twice that
-    // share of CTAs is launched per token and walks the tiles in strides.
-    const int64_t share = (2LL * tiles * b.L.E + b.L.global_experts - 1) / b.L.global_experts;
-    tiles = static_cast<int>(std::max<int64_t>(2, std::min<int64_t>(tiles, share)));
-  }
-  const dim3 grid((b.L.H + kDownColumns - 1) / kDownColumns, tiles, b.T);
-  return launch_down([&](auto stages) {
-    constexpr int S = decltype(stages)::value;
-    cudaError_t err = cudaFuncSetAttribute(
-        k_down<true, S>, cudaFuncAttributeMaxDynamicSharedMemorySize, down_ring_bytes(S));
-    if (err == cudaSuccess)
-      err = cudaFuncSetAttribute(k_down<false, S>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 down_ring_bytes(S));
-    if (err != cudaSuccess) return static_cast<int>(err);
-    if (tiles < b.ws.down_tiles)
-      k_down<true, S><<<grid, 128, down_ring_bytes(S), b.stream>>>(b.L, b.ws, b.padding);
+  // Tiles per token (T < 8) or of the call, at most; twice the expected share under expert
+  // parallelism, walked in strides.
+  const bool listed = pairs_grouped(b);
+  int64_t tiles = listed ? static_cast<int64_t>(b.T) * ((b.L.F + kDownTileRows - 1) / kDownTileRows + b.L.K)
+                         : (b.L.F + kDownTileRows - 1) / kDownTileRows + b.L.K - 1;
+  const int64_t all = tiles;
+  if (b.L.expert_map && b.L.global_experts > 0)
+    tiles = std::max<int64_t>(listed ? 8 : 2, std::min<int64_t>(
+        tiles, (2 * tiles * b.L.E + b.L.global_experts - 1) / b.L.global_experts));
+  // Columns per CTA: finer until every SM has two CTAs of the tiles there will be about.
+  const int64_t expected = static_cast<int64_t>(b.T) * (b.L.F / kDownTileRows + b.L.K / 2 + 1);
+  int chunks = 4;
+  while (chunks > 1 && expected * ((b.L.H + 256 * chunks - 1) / (256 * chunks)) < 2 * 148) chunks /= 2;
+  DownGrid d;
+  d.encode_ctas = encode ? b.T * b.L.K * b.ws.encoder_tiles : 0;
+  d.columns = (b.L.H + 256 * chunks - 1) / (256 * chunks);
+  d.tiles = static_cast<int>(tiles);
+  const unsigned ctas = static_cast<unsigned>(d.encode_ctas + tiles * d.columns * (listed ? 1 : b.T));
+  auto launch = [&](auto chunk) {
+    constexpr int C = decltype(chunk)::value;
+    if (listed)
+      launch_dependent(k_down_tiles<C>, dim3(ctas), dim3(128), kDownRingBytes, b.stream, b.L, b.ws,
+                       b.padding, d);
+    else if (tiles < all)
+      launch_dependent(k_down<true, C>, dim3(ctas), dim3(128), kDownRingBytes, b.stream, b.L, b.ws,
+                       b.padding, d);
     else
-      k_down<false, S><<<grid, 128, down_ring_bytes(S), b.stream>>>(b.L, b.ws, b.padding);
+      launch_dependent(k_down<false, C>, dim3(ctas), dim3(128), kDownRingBytes, b.stream, b.L, b.ws,
+                       b.padding, d);
     return launched();
-  });
-
+  };
+  switch (chunks) {
+    case 1: return launch(std::integral_constant<int, 1>{});
+    case 2: return launch(std::integral_constant<int, 2>{});
+    default: return launch(std::integral_constant<int, 4>{});
+  }
 }
+
+static bool encodes(const Bound& b) { return b.L.R > 0 && b.L.F < b.L.N; }
 
 static int run_encode(const Bound& b) {
   if (b.L.R == 0) return 0;
@@ -2160,63 +2189,20 @@ static int run_encode(const Bound& b) {
     k_zero_latent<<<b.T, 128, 0, b.stream>>>(b.L, b.ws);
     return launched();
   }
-  if (rows_grouped(b) && !b.L.expert_map) {
-    const size_t smem = encode_grouped_bytes(b.L.R);
-    if (smem > 48 * 1024) {
-      const cudaError_t err = cudaFuncSetAttribute(
-          k_encode_grouped, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-      if (err != cudaSuccess) return static_cast<int>(err);
-    }
-    k_encode_grouped<<<dim3(b.ws.encoder_tiles, b.L.E), kEncodeThreads, smem, b.stream>>>(b.L, b.ws);
-    return launched();
-  }
-  k_encode<<<dim3(b.ws.encoder_tiles, b.T * b.L.K), kEncodeThreads, 0, b.stream>>>(b.L, b.ws, b.padding);
+  k_encode<<<b.T * b.L.K * b.ws.encoder_tiles, kEncodeThreads, 0, b.stream>>>(b.L, b.ws, b.padding);
+  k_latent<<<b.T, 128, 0, b.stream>>>(b.L, b.ws, b.padding);
   return launched();
 }
 
-static int run_output(const Bound& b, const cfm_call* call, bool account) {
+// `whole`: the last launch of a whole call.
+static int run_output(const Bound& b, const cfm_call* call, bool whole) {
   if (!call->out) return CFM_E_NULL;
-  k_output<<<dim3(b.L.H / 128, b.T), 128, 0, b.stream>>>(
-      b.L, b.ws, b.padding, static_cast<__nv_bfloat16*>(call->out),
-      rows_grouped(b) ? down_grouped_parts(b) : 0, account);
+  const int latents = !whole || rows_grouped(b) ? kLatentGiven : encodes(b) ? kLatentMix : kLatentZero;
+  launch_dependent(k_output, dim3(b.L.H / 128 + whole, b.T), dim3(128), 0, b.stream, b.L, b.ws, b.padding,
+                   static_cast<__nv_bfloat16*>(call->out),
+                   rows_grouped(b) ? down_grouped_parts(b) : 0, latents,
+                   static_cast<int>(whole && !rows_grouped(b)));
   return launched();
-}
-
-// One side stream and two events per device, created on the first whole-layer
-// call on that device (make that call outside stream capture).
-struct SideStream {
-  cudaStream_t stream;
-  cudaEvent_t fork, join, tiles;
-  std::mutex* sequence;  // held while a whole-layer call enqueues its fork .. join sequence
-  bool ready;
-};
-static SideStream g_side[64];
-static std::mutex g_side_sequence[64];
-static std::mutex g_side_lock;
-
-static int side_stream(SideStream* out) {
-  int device = 0;
-  if (cudaGetDevice(&device) != cudaSuccess || device < 0 || device >= 64) return -1;
-  std::lock_guard<std::mutex> guard(g_side_lock);
-  SideStream& slot = g_side[device];
-  if (!slot.ready) {
-    int low = 0, high = 0;
-    if (cudaDeviceGetStreamPriorityRange(&low, &high) != cudaSuccess) return -1;
-    if (cudaStreamCreateWithPriority(&slot.stream, cudaStreamNonBlocking, high) != cudaSuccess) {
-      (void)cudaGetLastError();
-      return -1;
-    }
-    if (cudaEventCreateWithFlags(&slot.fork, cudaEventDisableTiming) != cudaSuccess ||
-        cudaEventCreateWithFlags(&slot.join, cudaEventDisableTiming) != cudaSuccess ||
-        cudaEventCreateWithFlags(&slot.tiles, cudaEventDisableTiming) != cudaSuccess) {
-      (void)cudaGetLastError();
-      return -1;
-    }
-    slot.sequence = &g_side_sequence[device];
-    slot.ready = true;
-  }
-  *out = slot;
-  return 0;
 }
 
 // Checks an exchange description against the layer and the call (`rows` = tokens
@@ -2293,8 +2279,8 @@ CFM_STAGE(cfm_select, {
 })
 CFM_STAGE(cfm_score, return run_score(b);)
 CFM_STAGE(cfm_list_tiles, return run_list_tiles(b);)
-CFM_STAGE(cfm_exact, return run_exact(b, call);)
-CFM_STAGE(cfm_down, return run_down(b);)
+CFM_STAGE(cfm_exact, return run_exact(b, call, false);)
+CFM_STAGE(cfm_down, return run_down(b, false);)
 CFM_STAGE(cfm_encode, return run_encode(b);)
 CFM_STAGE(cfm_output, return run_output(b, call, false);)
 
@@ -2431,62 +2417,12 @@ int cfm_reader_forward(const cfm_layer* layer, void* workspace, int32_t capacity
   int rc = bind_call(layer, workspace, capacity, call, stream, &b);
   if (rc) return rc;
   if (!layer->gate_up || !layer->down) return CFM_E_NULL;
-  SideStream side;
-  const bool have_side = b.L.F < b.L.N && side_stream(&side) == 0;
-  // The side stream and its two events are shared by every whole-layer call on the
-  // device: the enqueue sequence below runs under the device's lock, so calls from
-  // several host threads do not interleave their fork and join points.
-  std::unique_lock<std::mutex> sequence;
-  if (have_side) sequence = std::unique_lock<std::mutex>(*side.sequence);
-  // After a fork the caller's stream must wait for the side stream again whatever
-  // happens, or a capture of the caller's stream would be left with an unjoined branch.
-  bool forked = false;
-  auto leave = [&](int code) {
-    if (forked) {
-      (void)cudaEventRecord(side.join, side.stream);
-      (void)cudaStreamWaitEvent(b.stream, side.join, 0);
-      forked = false;
-    }
-    return code;
-  };
-  auto fork_side = [&]() {
-    cudaError_t err = cudaEventRecord(side.fork, b.stream);
-    if (err == cudaSuccess) err = cudaStreamWaitEvent(side.stream, side.fork, 0);
-    if (err == cudaSuccess) forked = true;
-    return static_cast<int>(err);
-  };
-  auto join_side = [&]() {
-    cudaError_t err = cudaEventRecord(side.join, side.stream);
-    if (err == cudaSuccess) err = cudaStreamWaitEvent(b.stream, side.join, 0);
-    forked = false;
-    return static_cast<int>(err);
-  };
-  Bound on_side = b;
-  if (have_side) on_side.stream = side.stream;
   if ((rc = run_prepare(b, call, !call->input_prepared, true))) return rc;
   if ((rc = run_screen(b))) return rc;
   if ((rc = run_select(b, 0, nullptr, false))) return rc;
-  // The listing of the down tiles and the recovery encoder (L2-resident rows,
-  // arithmetic) run on the side stream beside the two HBM-bound gathers; the down
-  // kernel waits for the list, the output mix for the encoder.
-  const bool fork = have_side && (b.L.R > 0 || pairs_grouped(b));
-  if (fork) {
-    if ((rc = fork_side())) return leave(rc);
-    if ((rc = run_list_tiles(on_side))) return leave(rc);
-    if (cudaEventRecord(side.tiles, side.stream) != cudaSuccess) return leave(static_cast<int>(cudaGetLastError()));
-    if ((rc = run_encode(on_side))) return leave(rc);
-  } else if ((rc = run_list_tiles(b))) {
-    return rc;
-  }
-  if ((rc = run_exact(b, call))) return leave(rc);
-  if (fork && cudaStreamWaitEvent(b.stream, side.tiles, 0) != cudaSuccess)
-    return leave(static_cast<int>(cudaGetLastError()));
-  if ((rc = run_down(b))) return leave(rc);
-  if (fork) {
-    if ((rc = join_side())) return leave(rc);
-  } else if ((rc = run_encode(b))) {
-    return rc;
-  }
+  if ((rc = run_exact(b, call, !rows_grouped(b)))) return rc;
+  if ((rc = run_down(b, encodes(b) && !rows_grouped(b)))) return rc;
+  if (rows_grouped(b) && (rc = run_encode(b))) return rc;
   return run_output(b, call, true);
 }
 
