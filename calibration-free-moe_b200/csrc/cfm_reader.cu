@@ -1188,7 +1188,9 @@ __global__ void __launch_bounds__(kExactWarps * 32) k_exact_pairs(Layer L, Works
 // the channels with eight rows in flight per thread; last, the row groups fold (shuffles inside a
 // warp, shared memory across warps).  L2 and latency bound, and needed by nothing before the output
 // mix, so its CTAs ride at the head of the down kernel's launch, beside the gathers (a stream of
-// its own cost two events and, for one token, 7 us at its end).  `shared`: 256 + 4 * 256 floats.
+// its own cost two events and, for one token, 7 us at its end).  The last CTA of a token to arrive
+// mixes the latent, hidden there as well (in every CTA of the output it took 4 us for one token and
+// 13 us for 64).  `shared`: 256 + 4 * 256 floats.
 constexpr int kEncodeThreads = 128;
 
 __device__ __forceinline__ void encode_tile(const Layer& L, const Workspace& ws,
@@ -1199,8 +1201,12 @@ __device__ __forceinline__ void encode_tile(const Layer& L, const Workspace& ws,
   const int tid = threadIdx.x, t = pair / L.K, slot = pair - t * L.K;
   const int R = L.R, lpr = R / 8, groups = kEncodeThreads / lpr;
   const int e = ws.ids[pair];
-  if ((padding && padding[t]) || e < 0) return;
-  const int c0 = tile * kEncodeTileRows, c1 = min(L.I, c0 + kEncodeTileRows);
+  if (padding && padding[t]) {
+    if (slot == 0 && tile == 0)
+      for (int r = tid; r < R; r += kEncodeThreads) ws.latent[static_cast<size_t>(t) * R + r] = 0.0f;
+    return;
+  }
+  const int c0 = tile * kEncodeTileRows, c1 = e < 0 ? c0 : min(L.I, c0 + kEncodeTileRows);
   const int group = tid / lpr, col = (tid - group * lpr) * 8;
   float acc[8];
 #pragma unroll
@@ -1252,22 +1258,30 @@ __device__ __forceinline__ void encode_tile(const Layer& L, const Workspace& ws,
   float* parts = ws.encoder_parts + static_cast<size_t>(index) * R;
   for (int r = tid; r < R; r += kEncodeThreads)
     parts[r] = ((red[0][r] + red[1][r]) + red[2][r]) + red[3][r];
-}
-
-// Entry r of a token's latent: per slot the encoder's sums in tile order, rounded to BF16, times the
-// router weight, in slot order.
-__device__ __forceinline__ float mix_latent(const Layer& L, const Workspace& ws, int t, int r) {
-  const size_t pair0 = static_cast<size_t>(t) * L.K;
-  const float* parts = ws.encoder_parts + pair0 * ws.encoder_tiles * L.R + r;
-  float latent = 0.0f;
-#pragma unroll 4
-  for (int s = 0; s < L.K; ++s) {
-    float sum = 0.0f;
-    for (int j = 0; j < ws.encoder_tiles; ++j)
-      sum += parts[static_cast<size_t>(s * ws.encoder_tiles + j) * L.R];
-    if (ws.ids[pair0 + s] >= 0) latent = fmaf(bf16_round(sum), ws.weights[pair0 + s], latent);
+  __threadfence();
+  __syncthreads();
+  uint32_t* counter = ws.counters + 2 * static_cast<size_t>(ws.capacity) * L.K + t;
+  if (tid == 0) {
+    const bool last = atomicAdd(counter, 1u) == static_cast<unsigned>(L.K * ws.encoder_tiles - 1);
+    if (last) *counter = 0;
+    shared[0] = last ? 1.0f : 0.0f;
   }
-  return latent;
+  __syncthreads();
+  if (shared[0] == 0.0f) return;
+  __threadfence();
+  // Per slot the sums in tile order, rounded to BF16, times the router weight, in slot order.
+  for (int r = tid; r < R; r += kEncodeThreads) {
+    float latent = 0.0f;
+    for (int s2 = 0; s2 < L.K; ++s2) {
+      const size_t other = static_cast<size_t>(t) * L.K + s2;
+      if (ws.ids[other] < 0) continue;
+      const float* p = ws.encoder_parts + other * ws.encoder_tiles * R + r;
+      float sum = 0.0f;
+      for (int j = 0; j < ws.encoder_tiles; ++j) sum += __ldcg(p + static_cast<size_t>(j) * R);
+      latent = fmaf(bf16_round(sum), ws.weights[other], latent);
+    }
+    ws.latent[static_cast<size_t>(t) * R + r] = latent;
+  }
 }
 
 // The encoder on its own: grid (pairs * tiles), 128 threads.
@@ -1275,14 +1289,6 @@ __global__ void __launch_bounds__(kEncodeThreads) k_encode(Layer L, Workspace ws
                                                            const uint8_t* padding) {
   __shared__ float shared[kEncodeTileRows + 4 * 256];
   encode_tile(L, ws, padding, blockIdx.x, shared);
-}
-
-// grid (T), 128 threads: the latents, after an encoder run of its own (padding rows: zero).
-__global__ void k_latent(Layer L, Workspace ws, const uint8_t* padding) {
-  const int t = blockIdx.x;
-  for (int r = threadIdx.x; r < L.R; r += blockDim.x)
-    ws.latent[static_cast<size_t>(t) * L.R + r] =
-        padding && padding[t] ? 0.0f : mix_latent(L, ws, t, r);
 }
 
 // ---------------------------------------------------------------------------
@@ -1579,11 +1585,8 @@ __device__ __forceinline__ float4 mix_down_tiles4(const float* parts, int used, 
 // add the tokens' read-cost counters.  `fixed` is the
 // number of partial sums per local slot the expert-major down kernel wrote, or 0
 // after the per-token down kernel.
-// Where the output kernel finds a token's latent: in the workspace, in the encoder's sums (it then
-// also leaves it in the workspace), or nowhere (zero).
-constexpr int kLatentGiven = 0, kLatentMix = 1, kLatentZero = 2;
-
-__global__ void __launch_bounds__(128, 6) k_output(Layer L, Workspace ws, const uint8_t* padding,
+// `latents` false: there are none (the workspace's are set to zero).
+__global__ void __launch_bounds__(128) k_output(Layer L, Workspace ws, const uint8_t* padding,
                                                 __nv_bfloat16* out, int fixed, int latents,
                                                 int early) {
   __shared__ float latent[256];
@@ -1602,8 +1605,6 @@ __global__ void __launch_bounds__(128, 6) k_output(Layer L, Workspace ws, const 
   if (padding && padding[t]) {
     if (early) grid_dependency_wait();
     out[static_cast<size_t>(t) * L.H + h] = __float2bfloat16_rn(0.0f);
-    if (latents != kLatentGiven && blockIdx.x == 0)
-      for (int r = tid; r < L.R; r += 128) ws.latent[static_cast<size_t>(t) * L.R + r] = 0.0f;
     return;
   }
   const bool recover = L.R > 0 && L.owner && L.decoder;
@@ -1626,9 +1627,8 @@ __global__ void __launch_bounds__(128, 6) k_output(Layer L, Workspace ws, const 
   if (early) grid_dependency_wait();  // the sums are complete
   for (int r = tid; r < L.R; r += 128) {
     float* kept = ws.latent + static_cast<size_t>(t) * L.R + r;
-    const float z = latents == kLatentGiven ? *kept : latents == kLatentMix ? mix_latent(L, ws, t, r) : 0.0f;
-    if (latents != kLatentGiven && blockIdx.x == 0) *kept = z;
-    latent[r] = bf16_round(z);
+    if (!latents && blockIdx.x == 0) *kept = 0.0f;
+    latent[r] = latents ? bf16_round(*kept) : 0.0f;
   }
   __syncthreads();
   const int used = slot_end[L.K - 1];  // tiles are laid out slot after slot
@@ -2190,17 +2190,15 @@ static int run_encode(const Bound& b) {
     return launched();
   }
   k_encode<<<b.T * b.L.K * b.ws.encoder_tiles, kEncodeThreads, 0, b.stream>>>(b.L, b.ws, b.padding);
-  k_latent<<<b.T, 128, 0, b.stream>>>(b.L, b.ws, b.padding);
   return launched();
 }
 
 // `whole`: the last launch of a whole call.
 static int run_output(const Bound& b, const cfm_call* call, bool whole) {
   if (!call->out) return CFM_E_NULL;
-  const int latents = !whole || rows_grouped(b) ? kLatentGiven : encodes(b) ? kLatentMix : kLatentZero;
   launch_dependent(k_output, dim3(b.L.H / 128 + whole, b.T), dim3(128), 0, b.stream, b.L, b.ws, b.padding,
                    static_cast<__nv_bfloat16*>(call->out),
-                   rows_grouped(b) ? down_grouped_parts(b) : 0, latents,
+                   rows_grouped(b) ? down_grouped_parts(b) : 0, static_cast<int>(!whole || encodes(b)),
                    static_cast<int>(whole && !rows_grouped(b)));
   return launched();
 }
