@@ -275,6 +275,7 @@ __global__ void __launch_bounds__(kPrepareThreads)
     k_prepare(Layer L, Workspace ws, const __nv_bfloat16* hidden, const uint8_t* padding, int T,
               int group, Routes r) {
   extern __shared__ __align__(16) uint8_t prepare_shared[];  // E counters | 16 x 128 squares
+  grid_dependency_wait();     // the workspace and the inputs may still be in use, or in the making
   grid_dependency_release();  // the screen may be scheduled; it waits for this grid
   if (group && blockIdx.x == 0) {
     group_pairs(L, ws, r, true, padding, T, reinterpret_cast<int*>(prepare_shared));

@@ -1270,15 +1270,29 @@ __device__ __forceinline__ void encode_tile(const Layer& L, const Workspace& ws,
   if (shared[0] == 0.0f) return;
   __threadfence();
   // Per slot the sums in tile order, rounded to BF16, times the router weight, in slot order.
+  const int parts_of_slot = ws.encoder_tiles, all_parts = L.K * parts_of_slot;
+  const size_t pair0 = static_cast<size_t>(t) * L.K;
   for (int r = tid; r < R; r += kEncodeThreads) {
-    float latent = 0.0f;
-    for (int s2 = 0; s2 < L.K; ++s2) {
-      const size_t other = static_cast<size_t>(t) * L.K + s2;
-      if (ws.ids[other] < 0) continue;
-      const float* p = ws.encoder_parts + other * ws.encoder_tiles * R + r;
-      float sum = 0.0f;
-      for (int j = 0; j < ws.encoder_tiles; ++j) sum += __ldcg(p + static_cast<size_t>(j) * R);
-      latent = fmaf(bf16_round(sum), ws.weights[other], latent);
+    const float* p = ws.encoder_parts + pair0 * parts_of_slot * R + r;
+    float latent = 0.0f, sum = 0.0f;
+    int slot2 = 0, left = parts_of_slot;
+    for (int n0 = 0; n0 < all_parts; n0 += 8) {
+      float v[8];  // on their way together
+#pragma unroll
+      for (int n = 0; n < 8; ++n)
+        v[n] = n0 + n < all_parts ? __ldcg(p + static_cast<size_t>(n0 + n) * R) : 0.0f;
+#pragma unroll
+      for (int n = 0; n < 8; ++n) {
+        if (n0 + n >= all_parts) break;
+        sum += v[n];
+        if (--left == 0) {
+          if (ws.ids[pair0 + slot2] >= 0)
+            latent = fmaf(bf16_round(sum), ws.weights[pair0 + slot2], latent);
+          sum = 0.0f;
+          left = parts_of_slot;
+          ++slot2;
+        }
+      }
     }
     ws.latent[static_cast<size_t>(t) * R + r] = latent;
   }
@@ -1884,9 +1898,9 @@ static int run_prepare(const Bound& b, const cfm_call* call, bool rotate, bool g
   }
   constexpr int kPerCta = kPrepareThreads / 32;
   const int64_t ctas = rotate ? (static_cast<int64_t>(b.T) * b.L.B + kPerCta - 1) / kPerCta : 0;
-  k_prepare<<<static_cast<unsigned>(ctas + group), kPrepareThreads, smem, b.stream>>>(
-      b.L, b.ws, static_cast<const __nv_bfloat16*>(call->hidden), b.padding, b.T, group,
-      routes_of(b, call));
+  launch_dependent(k_prepare, dim3(static_cast<unsigned>(ctas + group)), dim3(kPrepareThreads), smem,
+                   b.stream, b.L, b.ws, static_cast<const __nv_bfloat16*>(call->hidden), b.padding, b.T,
+                   static_cast<int>(group), routes_of(b, call));
   return launched();
 }
 

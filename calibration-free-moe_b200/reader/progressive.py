@@ -471,6 +471,12 @@ class ProgressiveReader:
         self._layer = layer
         self._library = _native.load()
         self._device = device
+        # What a call needs again and again.
+        self._device_index = device.index if device.index is not None else torch.cuda.current_device()
+        self._layer_ref = ctypes.byref(layer)
+        self._workspace_pointer = ctypes.c_void_p(self.workspace.buffer.data_ptr())
+        self._workspace_capacity = self.workspace.capacity
+        self._forward = self._library.cfm_reader_forward
 
     # ------------------------------------------------------------------
     def _validate_input(self, hidden: Tensor, padding: Tensor | None) -> int:
@@ -502,30 +508,29 @@ class ProgressiveReader:
         out: Tensor | None,
         input_prepared: bool,
     ) -> _native.Call:
-        call = _native.Call()
-        call.tokens = tokens
-        call.ids_are_int64 = int(ids is not None and ids.dtype == torch.int64)
-        call.weights_are_bf16 = int(weights is not None and weights.dtype == torch.bfloat16)
-        call.input_prepared = int(input_prepared)
-        call.hidden = hidden.data_ptr()
-        call.ids = ids.data_ptr() if ids is not None else None
-        call.weights = weights.data_ptr() if weights is not None else None
-        call.padding = padding.data_ptr() if padding is not None else None
-        call.out = out.data_ptr() if out is not None else None
-        return call
+        return _native.Call(
+            tokens,
+            ids is not None and ids.dtype == torch.int64,
+            weights is not None and weights.dtype == torch.bfloat16,
+            input_prepared, 0, 0,
+            hidden.data_ptr(),
+            ids.data_ptr() if ids is not None else None,
+            weights.data_ptr() if weights is not None else None,
+            padding.data_ptr() if padding is not None else None,
+            out.data_ptr() if out is not None else None,
+        )
 
     def _stage(self, name: str, call: _native.Call) -> None:
-        stream = torch.cuda.current_stream(self._device).cuda_stream
-        code = getattr(self._library, name)(
-            ctypes.byref(self._layer),
-            self.workspace.buffer.data_ptr(),
-            self.workspace.capacity,
-            ctypes.byref(call),
-            ctypes.c_void_p(stream),
-        )
-        _native.check(code, name)
+        self._enqueue(getattr(self._library, name), name, call)
 
-    @torch.no_grad()
+    def _enqueue(self, function, name: str, call: _native.Call) -> None:
+        code = function(
+            self._layer_ref, self._workspace_pointer, self._workspace_capacity,
+            ctypes.byref(call), torch._C._cuda_getCurrentRawStream(self._device_index),
+        )
+        if code:
+            _native.check(code, name)
+
     def prepare_input(self, hidden: Tensor, padding: Tensor | None = None) -> bool:
         """Run the routing-independent input rotation ahead of the router.
 
@@ -539,14 +544,14 @@ class ProgressiveReader:
         if self.expert_map is not None or p.completion_count == p.candidate_count:
             return False
         tokens = self._validate_input(hidden, padding)
-        with torch.cuda.device(self._device):
-            self._stage(
-                "cfm_prepare_input",
-                self._call_struct(tokens, hidden, None, None, padding, None, False),
-            )
+        call = self._call_struct(tokens, hidden, None, None, padding, None, False)
+        if torch.cuda.current_device() == self._device_index:
+            self._stage("cfm_prepare_input", call)
+        else:
+            with torch.cuda.device(self._device):
+                self._stage("cfm_prepare_input", call)
         return True
 
-    @torch.no_grad()
     def __call__(
         self,
         hidden: Tensor,
@@ -590,10 +595,14 @@ class ProgressiveReader:
         if out is None:
             out = torch.empty_like(hidden)
         call = self._call_struct(tokens, hidden, ids, weights, padding, out, input_prepared)
-        with torch.cuda.device(self._device):
-            if self.expert_map is None:
-                self._stage("cfm_reader_forward", call)
-                return out
+        if self.expert_map is None:
+            if torch.cuda.current_device() == self._device_index:
+                self._enqueue(self._forward, "cfm_reader_forward", call)
+            else:
+                with torch.cuda.device(self._device):
+                    self._enqueue(self._forward, "cfm_reader_forward", call)
+            return out
+        with torch.no_grad(), torch.cuda.device(self._device):
             # Expert parallel, replicated tokens: every rank screens its local
             # experts, the scores are summed across ranks so all ranks keep the
             # same channels, and the latent is summed before the owner decodes
