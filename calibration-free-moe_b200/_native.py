@@ -15,13 +15,13 @@ from pathlib import Path
 
 PACKAGE = Path(__file__).resolve().parent
 SOURCES = [PACKAGE / "csrc" / "cfm_reader.cu"]
-HEADERS = [PACKAGE / "csrc" / "cfm_device.cuh", PACKAGE / "csrc" / "cfm_grouped.cuh",
+HEADERS = [PACKAGE / "csrc" / "cfm_device.cuh", PACKAGE / "csrc" / "cfm_union.cuh",
            PACKAGE / "csrc" / "cfm_exchange.cuh", PACKAGE / "csrc" / "cfm_select.cuh",
            PACKAGE / "csrc" / "cfm_build.cuh", PACKAGE / "csrc" / "cfm_screen.cuh",
            PACKAGE / "csrc" / "cfm_screen_tc.cuh", PACKAGE / "csrc" / "cfm_prepare.cuh",
            PACKAGE.parent / "include" / "cfm_b200.h"]
 LIBRARY = PACKAGE / "libcfm_b200.so"
-ABI_VERSION = 11
+ABI_VERSION = 12
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
@@ -113,7 +113,8 @@ _LAYOUT_ARRAYS = (
     "counters", "partial", "scores", "selected", "completed", "candidate_ids", "counts",
     "starts", "tile_starts", "activations", "exact", "down_parts", "encoder_parts", "latent",
     "status", "limbs", "group_offsets", "group_pairs", "cuts", "variances", "features", "pass_work", "busy_experts", "work_counts",
-    "tile_list", "tile_count",
+    "tile_list", "tile_count", "kept_bits", "kept_before", "union_channels", "union_activations",
+    "exact_work", "down_work",
 )
 
 

@@ -33,6 +33,7 @@ namespace cfm {
 // Workspace binding
 // ---------------------------------------------------------------------------
 struct Pass;
+struct UnionWork;
 struct Workspace {
   int32_t* ids;
   float* weights;
@@ -68,6 +69,12 @@ struct Workspace {
   int32_t* work_counts;
   int32_t* tile_list;
   int32_t* tile_count;
+  uint32_t* kept_bits;
+  uint16_t* kept_before;
+  uint16_t* union_channels;
+  __nv_bfloat16* union_activations;
+  UnionWork* exact_work;
+  UnionWork* down_work;
   int32_t parts_tokens;
   int32_t down_tiles;
   int32_t encoder_tiles;
@@ -101,8 +108,8 @@ __device__ __forceinline__ int slot_of(const Layer& L, int i) {
 
 static int64_t align256(int64_t v) { return (v + 255) / 256 * 256; }
 
-// Most partial sums per (token, slot) the expert-major down kernel writes.
-constexpr int64_t kDownGroupedMaxParts = 8;
+// 32-bit words of a token's kept candidates as bits; one more, so that two in a row can be read.
+__host__ __device__ inline int kept_words(int N) { return (N + 31) / 32 + 1; }
 
 // Most candidates per token (N = K * I) the selection kernels take: their scans pack two
 // counts of at most N into the halves of one 32-bit integer.
@@ -125,8 +132,7 @@ static int make_layout(const cfm_layer* l, int32_t capacity, cfm_workspace_layou
     return here;
   };
   o->parts_tokens = static_cast<int32_t>(C < 16 ? C : 16);
-  o->down_tiles = static_cast<int32_t>(std::max<int64_t>(
-      (F + kDownTileRows - 1) / kDownTileRows + K - 1, kDownGroupedMaxParts * K));
+  o->down_tiles = static_cast<int32_t>((F + kDownTileRows - 1) / kDownTileRows + K - 1);
   o->encoder_tiles = static_cast<int32_t>((I + kEncodeTileRows - 1) / kEncodeTileRows);
   o->reserved = 0;
   o->ids = take(4 * C * K);
@@ -164,6 +170,13 @@ static int make_layout(const cfm_layer* l, int32_t capacity, cfm_workspace_layou
   o->work_counts = take(16);
   o->tile_list = take(32 * C * ((F + kDownTileRows - 1) / kDownTileRows + K));
   o->tile_count = take(16);
+  o->kept_bits = take(4 * C * kept_words(static_cast<int>(N)));
+  o->kept_before = take(2 * C * kept_words(static_cast<int>(N)));
+  o->union_channels = take(2 * E * I);
+  o->union_activations = take(2 * C * N);
+  const int64_t passes = C * K / 8 + std::min(E, C * K);  // of at least eight pairs
+  o->exact_work = take(32 * passes * ((I + 15) / 16));
+  o->down_work = take(32 * passes);
   o->bytes = at;
   return 0;
 }
@@ -205,6 +218,12 @@ static Workspace bind(const cfm_workspace_layout& o, void* base, int32_t capacit
   w.work_counts = reinterpret_cast<int32_t*>(p + o.work_counts);
   w.tile_list = reinterpret_cast<int32_t*>(p + o.tile_list);
   w.tile_count = reinterpret_cast<int32_t*>(p + o.tile_count);
+  w.kept_bits = reinterpret_cast<uint32_t*>(p + o.kept_bits);
+  w.kept_before = reinterpret_cast<uint16_t*>(p + o.kept_before);
+  w.union_channels = reinterpret_cast<uint16_t*>(p + o.union_channels);
+  w.union_activations = reinterpret_cast<__nv_bfloat16*>(p + o.union_activations);
+  w.exact_work = reinterpret_cast<UnionWork*>(p + o.exact_work);
+  w.down_work = reinterpret_cast<UnionWork*>(p + o.down_work);
   w.parts_tokens = o.parts_tokens;
   w.down_tiles = o.down_tiles;
   w.encoder_tiles = o.encoder_tiles;
@@ -340,6 +359,20 @@ __global__ void __launch_bounds__(256) k_adopt(Layer L, Workspace ws, const void
     __syncthreads();
   }
   for (int i = kept + tid; i < L.F; i += 256) out[i] = -1;
+  {  // the same channels as bits, with the number of them before every word
+    const int words = kept_words(L.N);
+    uint32_t* bits = ws.kept_bits + static_cast<size_t>(t) * words;
+    for (int w = tid; w < words; w += 256) bits[w] = 0;
+    __syncthreads();
+    for (int i = tid; i < kept; i += 256) {
+      const int w = out[i] >> 5;
+      if (i > 0 && out[i - 1] >> 5 == w) continue;  // the word's first entry writes it
+      uint32_t word = 0;
+      for (int j = i; j < kept && out[j] >> 5 == w; ++j) word |= 1u << (out[j] & 31);
+      bits[w] = word;
+      ws.kept_before[static_cast<size_t>(t) * words + w] = static_cast<uint16_t>(i);
+    }
+  }
   if (warp == 0) {
     const bool live = lane < L.K;
     const int mine = live ? count[lane] : 0;
@@ -654,7 +687,7 @@ struct NoExchange {
 template <bool PEERS, int PER>
 __global__ void __launch_bounds__(kSelectThreads, PER <= 4 ? 2 : 1)
     k_select(Layer L, Workspace ws, const uint8_t* padding, int scores_ready, int row_offset, int account,
-             typename std::conditional<PEERS, Exchange, NoExchange>::type x) {
+             int clear, typename std::conditional<PEERS, Exchange, NoExchange>::type x) {
   constexpr bool peers = PEERS;
   grid_dependency_release();  // the exact gather may be scheduled; it waits for this grid
   grid_dependency_wait();     // the screen's projections are complete
@@ -928,13 +961,21 @@ __global__ void __launch_bounds__(kSelectThreads, PER <= 4 ? 2 : 1)
       const bool keep = (kept >> j) & 1u;
       const unsigned ballot = __ballot_sync(kFull, keep);
       if (lane == 0) {
-        s_chunk[warp * PER + j] = ballot;
-        s_before[warp * PER + j] = static_cast<uint16_t>(running);
+        const int word = warp * PER + j;
+        s_chunk[word] = ballot;
+        s_before[word] = static_cast<uint16_t>(running);
+        if (32 * word < N) {
+          ws.kept_bits[static_cast<size_t>(t) * kept_words(N) + word] = ballot;
+          ws.kept_before[static_cast<size_t>(t) * kept_words(N) + word] = static_cast<uint16_t>(running);
+        }
       }
       if (i < N) {
         selected[i] = keep;
         completed[i] = keep && (!remote || s_route[slot_of(L, i)] >= 0);
-        if (keep) list[running + __popc(ballot & before)] = i;
+        if (keep) {
+          list[running + __popc(ballot & before)] = i;
+          if (clear) ws.features[static_cast<size_t>(t) * N + i] = __float2bfloat16_rn(0.0f);
+        }
       }
       running += __popc(ballot);
     }
@@ -1502,23 +1543,14 @@ __global__ void k_zero_latent(Layer L, Workspace ws) {
     ws.latent[static_cast<size_t>(blockIdx.x) * L.R + r] = 0.0f;
 }
 
-#include "cfm_grouped.cuh"
+#include "cfm_union.cuh"
 
-// One past the last down tile of slot `slot` of token t.  The per-token down
-// kernel lays a token's tiles out slot after slot, ceil(count / 64) tiles per
-// local slot, starting at `tile_starts`; the expert-major one writes `fixed`
-// partial sums for every local slot, slot after slot.
-__device__ __forceinline__ int down_slot_end(const Layer& L, const Workspace& ws, int t, int slot,
-                                             int fixed) {
-  const size_t pairs = static_cast<size_t>(t) * L.K;
-  if (fixed == 0) {
-    const int tiles = ws.ids[pairs + slot] >= 0
-                          ? (ws.counts[pairs + slot] + kDownTileRows - 1) / kDownTileRows : 0;
-    return ws.tile_starts[pairs + slot] + tiles;
-  }
-  int local = 0;
-  for (int s = 0; s <= slot; ++s) local += ws.ids[pairs + s] >= 0;
-  return local * fixed;
+// One past the last down tile of slot `slot` of token t: a token's tiles lie slot after slot,
+// ceil(count / 64) per local slot, from `tile_starts`.
+__device__ __forceinline__ int down_slot_end(const Layer& L, const Workspace& ws, int t, int slot) {
+  const size_t pair = static_cast<size_t>(t) * L.K + slot;
+  const int tiles = ws.ids[pair] >= 0 ? (ws.counts[pair] + kDownTileRows - 1) / kDownTileRows : 0;
+  return ws.tile_starts[pair] + tiles;
 }
 
 // ---------------------------------------------------------------------------
@@ -1596,13 +1628,10 @@ __device__ __forceinline__ float4 mix_down_tiles4(const float* parts, int used, 
 }
 
 // grid (H / 128, T), 128 threads, one output column per thread; with one more column of CTAs that
-// add the tokens' read-cost counters.  `fixed` is the
-// number of partial sums per local slot the expert-major down kernel wrote, or 0
-// after the per-token down kernel.
+// add the tokens' read-cost counters.
 // `latents` false: there are none (the workspace's are set to zero).
 __global__ void __launch_bounds__(128) k_output(Layer L, Workspace ws, const uint8_t* padding,
-                                                __nv_bfloat16* out, int fixed, int latents,
-                                                int early) {
+                                                __nv_bfloat16* out, int latents, int early) {
   __shared__ float latent[256];
   __shared__ int slot_end[32];       // one past the last down tile of every slot
   __shared__ float slot_weight[32];
@@ -1635,7 +1664,7 @@ __global__ void __launch_bounds__(128) k_output(Layer L, Workspace ws, const uin
   }
   if (tid < L.K) {
     const size_t pair = static_cast<size_t>(t) * L.K + tid;
-    slot_end[tid] = down_slot_end(L, ws, t, tid, fixed);
+    slot_end[tid] = down_slot_end(L, ws, t, tid);
     slot_weight[tid] = ws.weights[pair];
   }
   if (early) grid_dependency_wait();  // the sums are complete
@@ -1689,7 +1718,7 @@ __global__ void __launch_bounds__(128) k_output(Layer L, Workspace ws, const uin
 // CTA of a home rank's rows announces the epoch there.
 __global__ void __launch_bounds__(128) k_partial_output(Layer L, Workspace ws,
                                                         const uint8_t* padding, float* combined,
-                                                        int fixed, Exchange x, int peers) {
+                                                        int by_union, Exchange x, int peers) {
   __shared__ int slot_end[32];
   __shared__ float slot_weight[32];
   const int t = blockIdx.y, tid = threadIdx.x, h = blockIdx.x * 128 + tid;
@@ -1704,9 +1733,13 @@ __global__ void __launch_bounds__(128) k_partial_output(Layer L, Workspace ws,
                                           exchange_rows_offset(x.world, x.tokens, L.F)) +
                  (static_cast<size_t>(x.rank) * x.tokens + row) * L.H;
     float4 routed = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    if (!padded) {
+    if (!padded && by_union) {
+      if (h4 < L.H)
+        routed = make_float4(mix_sums(L, ws, t, h4), mix_sums(L, ws, t, h4 + 1),
+                             mix_sums(L, ws, t, h4 + 2), mix_sums(L, ws, t, h4 + 3));
+    } else if (!padded) {
       if (tid < L.K) {
-        slot_end[tid] = down_slot_end(L, ws, t, tid, fixed);
+        slot_end[tid] = down_slot_end(L, ws, t, tid);
         slot_weight[tid] = ws.weights[static_cast<size_t>(t) * L.K + tid];
       }
       __syncthreads();
@@ -1729,9 +1762,13 @@ __global__ void __launch_bounds__(128) k_partial_output(Layer L, Workspace ws,
     routed_out[h] = 0.0f;
     return;
   }
+  if (by_union) {
+    routed_out[h] = mix_sums(L, ws, t, h);
+    return;
+  }
   if (tid < L.K) {
     const size_t pair = static_cast<size_t>(t) * L.K + tid;
-    slot_end[tid] = down_slot_end(L, ws, t, tid, fixed);
+    slot_end[tid] = down_slot_end(L, ws, t, tid);
     slot_weight[tid] = ws.weights[pair];
   }
   __syncthreads();
@@ -2013,15 +2050,16 @@ static int run_screen_projections(const Bound& b) {
 }
 
 static bool pairs_grouped(const Bound& b);
+static bool encodes_by_union(const Bound& b);
 
 template <int PER>
 static int launch_select(const Bound& b, int scores_ready, const Exchange* exchange, int account) {
   if (exchange)
     launch_dependent(k_select<true, PER>, dim3(b.T), dim3(kSelectThreads), 0, b.stream, b.L, b.ws,
-                     b.padding, scores_ready, b.row_offset, account, *exchange);
+                     b.padding, scores_ready, b.row_offset, account, static_cast<int>(encodes_by_union(b)), *exchange);
   else
     launch_dependent(k_select<false, PER>, dim3(b.T), dim3(kSelectThreads), 0, b.stream, b.L, b.ws,
-                     b.padding, scores_ready, b.row_offset, account, NoExchange{});
+                     b.padding, scores_ready, b.row_offset, account, static_cast<int>(encodes_by_union(b)), NoExchange{});
   return launched();
 }
 
@@ -2053,48 +2091,96 @@ static int run_score(const Bound& b) {
 constexpr int kGroupedTokens = 8;
 static bool pairs_grouped(const Bound& b) { return b.T >= kGroupedTokens; }
 
-// Expert-major exact, down and encode: a row is read once for all the tokens of
-// its expert that kept it.  On the shapes measured so far (4 to 16 tokens per
-// expert) the per-token kernels walking the pairs in expert order are faster: the
-// rows several tokens share come from HBM once either way (from L2 after the
-// first), and the per-token kernels keep more loads in flight.  So the automatic
-// choice is per-token; the expert-major kernels run on request.
-static bool rows_grouped(const Bound& b) {
-  return pairs_grouped(b) && b.L.row_engine == CFM_ROWS_EXPERT_MAJOR;
-}
+static bool encodes(const Bound& b) { return b.L.R > 0 && b.L.F < b.L.N; }
 
-// Partial sums per (token, local slot) of the expert-major down kernel: enough
-// CTAs to fill the device, at most what the workspace has room for.
-static int down_grouped_parts(const Bound& b) {
-  const int64_t column_blocks = (b.L.H + kDownGroupedColumns - 1) / kDownGroupedColumns;
-  const int64_t wanted = (8 * 148 + column_blocks * b.L.E - 1) / (column_blocks * b.L.E);
-  const int64_t room = std::min<int64_t>(kDownGroupedMaxParts, b.ws.down_tiles / b.L.K);
-  return static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(std::max<int64_t>(2, wanted), room)));
+// The expert-major exact kernel, on request and from three tokens per expert and sixteen tokens on:
+// below that the unions of an expert's kept channels are little smaller than their sum.  64 tokens of
+// the 128-expert layer 60 us with the unions against 69 of the gathers, 256 of the 256-expert layer
+// 83 against 155; 32 tokens of the 128-expert layer 39 against 35.  Under expert parallelism the
+// gathers per token stay, so that a token's bits do not depend on how the experts are spread.
+static bool exact_by_union(const Bound& b) {
+  if (!pairs_grouped(b) || b.L.expert_map || b.L.row_engine == CFM_ROWS_PER_TOKEN) return false;
+  return b.L.row_engine == CFM_ROWS_EXPERT_MAJOR ||
+         (b.T >= 16 && static_cast<int64_t>(b.T) * b.L.K >= 3 * static_cast<int64_t>(b.L.E));
 }
+// The expert-major down kernel, on request and where most experts have more than a pass of eight
+// tokens: 64 tokens of the 128-expert layer 38 us and 6 in the output against 35 and 7 of the tiles
+// per token, 100 of the 64-expert layer 46 and 7 against 65 and 15.
+static bool down_by_union(const Bound& b) {
+  return exact_by_union(b) && (b.L.row_engine == CFM_ROWS_EXPERT_MAJOR || shares_decode(b));
+}
+// The recovery encoder in the expert-major down launch.  By size alone: a latent does not depend on
+// the row engine.
+static bool encodes_by_union(const Bound& b) {
+  return down_by_union(b) && shares_decode(b) && encodes(b);
+}
+// Tokens per pass of the expert-major kernels, in eights: the next size up while the mean load is
+// more than two thirds of the one before.
+static int union_tiles(const Bound& b, int most) {
+  int tiles = 1;
+  while (tiles < most && 3 * static_cast<int64_t>(b.T) * b.L.K > 16 * tiles * static_cast<int64_t>(b.L.E)) tiles *= 2;
+  return tiles;
+}
+static int exact_union_tiles(const Bound& b) { return union_tiles(b, 4); }
+static int down_union_tiles(const Bound& b) { return union_tiles(b, 2); }
 
-static int run_exact_grouped(const Bound& b, const cfm_call* call) {
-  // Entries of the per-channel token table: four times the mean number of kept
-  // channels per expert, at least one expert's width (the largest one token can need).
-  const int64_t mean = (static_cast<int64_t>(b.T) * b.L.F + b.L.E - 1) / b.L.E;
-  const int entries = static_cast<int>(
-      std::min<int64_t>(16384, std::max<int64_t>(b.L.I, 4 * mean)));
-  const size_t smem = exact_grouped_bytes(b.L.I, entries);
-  if (smem > 48 * 1024) {
-    const cudaError_t err = cudaFuncSetAttribute(
-        k_exact_grouped, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-    if (err != cudaSuccess) return static_cast<int>(err);
-  }
-  const int parts = static_cast<int>(
-      std::max<int64_t>(1, std::min<int64_t>(32, (4 * 148 + b.L.E - 1) / b.L.E)));
-  k_exact_grouped<<<dim3(parts, b.L.E), kExactGroupedThreads, smem, b.stream>>>(
-      b.L, b.ws, static_cast<const __nv_bfloat16*>(call->hidden), entries);
+// As many CTAs as run at a time, at most `work` of them.
+template <typename... Params, typename... Args>
+static int launch_persistent(void (*kernel)(Params...), int64_t work, int per_sm, int threads, size_t smem,
+                             cudaStream_t stream, Args... args) {
+  const cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               static_cast<int>(smem));
+  if (err != cudaSuccess) return static_cast<int>(err);
+  const unsigned ctas = static_cast<unsigned>(std::max<int64_t>(1, std::min<int64_t>(work, 148 * per_sm)));
+  launch_dependent(kernel, dim3(ctas), dim3(threads), smem, stream, args...);
   return launched();
 }
 
-// `list`: list the down tiles too.
-static int run_exact(const Bound& b, const cfm_call* call, bool list) {
+// `whole`: part of a whole call, which grouped the pairs and cleared the lists' lengths.
+static int run_exact_union(const Bound& b, const cfm_call* call, bool whole) {
+  if (!whole) {
+    const cudaError_t err = cudaMemsetAsync(b.ws.work_counts + kExactCount, 0, 2 * sizeof(int32_t), b.stream);
+    if (err != cudaSuccess) return static_cast<int>(err);
+  }
+  const int tiles = exact_union_tiles(b);
+  launch_dependent(k_union, dim3(busy_experts(b)), dim3(kUnionThreads), 0, b.stream, b.L, b.ws, 8 * tiles,
+                   8 * down_union_tiles(b), static_cast<int>(whole));
+  const int rc = launched();
+  if (rc) return rc;
+  const int64_t pairs = static_cast<int64_t>(b.T) * b.L.K;
+  const int64_t work = (pairs / 8 + busy_experts(b)) * ((b.L.I + 15) / 16);
+  const int by_union = down_by_union(b), list = whole && !by_union;
+  const auto* hidden = static_cast<const __nv_bfloat16*>(call->hidden);
+  auto launch = [&](auto tile) {
+    constexpr int NT = decltype(tile)::value;
+    using X = ExactUnion<NT>;
+    return launch_persistent(k_exact_union<NT>, work + list, X::kPerSm, X::kThreads, X::kSharedBytes, b.stream,
+                             b.L, b.ws, hidden, by_union, list);
+  };
+  switch (tiles) {
+    case 1: return launch(std::integral_constant<int, 1>{});
+    case 2: return launch(std::integral_constant<int, 2>{});
+    default: return launch(std::integral_constant<int, 4>{});
+  }
+}
+
+static int run_down_union(const Bound& b, bool encode) {
+  const int encoder_blocks = encode && encodes_by_union(b) ? (b.L.R + 63) / 64 : 0;
+  const int64_t passes = static_cast<int64_t>(b.T) * b.L.K / 8 + busy_experts(b);
+  const int64_t ctas = (passes * (b.L.H / 64 + encoder_blocks) + 3) / 4;
+  auto launch = [&](auto tile) {
+    using X = DownUnion<decltype(tile)::value>;
+    return launch_persistent(k_down_union<decltype(tile)::value>, ctas, X::kPerSm, X::kThreads, X::kSharedBytes,
+                             b.stream, b.L, b.ws, encoder_blocks);
+  };
+  return down_union_tiles(b) == 1 ? launch(std::integral_constant<int, 1>{})
+                                  : launch(std::integral_constant<int, 2>{});
+}
+
+// `whole`: part of a whole call; the down tiles are listed too where the down kernel needs them.
+static int run_exact(const Bound& b, const cfm_call* call, bool whole) {
   if (!call->hidden || !b.L.gate_up) return CFM_E_NULL;
-  if (rows_grouped(b)) return run_exact_grouped(b, call);
+  if (exact_by_union(b)) return run_exact_union(b, call, whole);
   const size_t smem = static_cast<size_t>(b.L.H) * 2;
   if (smem > 48 * 1024) {
     cudaError_t err = cudaFuncSetAttribute(
@@ -2109,6 +2195,7 @@ static int run_exact(const Bound& b, const cfm_call* call, bool list) {
     if (err != cudaSuccess) return static_cast<int>(err);
   }
   if (pairs_grouped(b)) {
+    const bool list = whole;
     // One warp per kept row of a pair when the pair keeps the mean number of rows.
     const int per_pair = (b.L.F + b.L.K - 1) / b.L.K;
     const int ctas = std::max(1, (per_pair + kExactWarps - 1) / kExactWarps);
@@ -2145,18 +2232,7 @@ static int run_exact(const Bound& b, const cfm_call* call, bool list) {
 // `encode`: run the recovery encoder too.
 static int run_down(const Bound& b, bool encode) {
   if (!b.L.down) return CFM_E_NULL;
-  if (rows_grouped(b)) {
-    const size_t smem = down_grouped_bytes(b.L.I);
-    if (smem > 48 * 1024) {
-      const cudaError_t err = cudaFuncSetAttribute(
-          k_down_grouped, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-      if (err != cudaSuccess) return static_cast<int>(err);
-    }
-    const int parts = down_grouped_parts(b);
-    const dim3 grid((b.L.H + kDownGroupedColumns - 1) / kDownGroupedColumns, b.L.E, parts);
-    k_down_grouped<<<grid, kDownGroupedThreads, smem, b.stream>>>(b.L, b.ws, parts);
-    return launched();
-  }
+  if (down_by_union(b)) return run_down_union(b, encode);
   // Tiles per token (T < 8) or of the call, at most; twice the expected share under expert
   // parallelism, walked in strides.
   const bool listed = pairs_grouped(b);
@@ -2195,8 +2271,6 @@ static int run_down(const Bound& b, bool encode) {
   }
 }
 
-static bool encodes(const Bound& b) { return b.L.R > 0 && b.L.F < b.L.N; }
-
 static int run_encode(const Bound& b) {
   if (b.L.R == 0) return 0;
   if (b.L.F >= b.L.N) {
@@ -2210,11 +2284,25 @@ static int run_encode(const Bound& b) {
 // `whole`: the last launch of a whole call.
 static int run_output(const Bound& b, const cfm_call* call, bool whole) {
   if (!call->out) return CFM_E_NULL;
-  launch_dependent(k_output, dim3(b.L.H / 128 + whole, b.T), dim3(128), 0, b.stream, b.L, b.ws, b.padding,
-                   static_cast<__nv_bfloat16*>(call->out),
-                   rows_grouped(b) ? down_grouped_parts(b) : 0, static_cast<int>(!whole || encodes(b)),
-                   static_cast<int>(whole && !rows_grouped(b)));
-  return launched();
+  const int latents = !whole || encodes(b);
+  auto* out = static_cast<__nv_bfloat16*>(call->out);
+  if (!down_by_union(b)) {
+    launch_dependent(k_output, dim3(b.L.H / 128 + whole, b.T), dim3(128), 0, b.stream, b.L, b.ws, b.padding,
+                     out, latents, static_cast<int>(whole));
+    return launched();
+  }
+  // Tokens per CTA: enough CTAs for two per SM, and no more.
+  const int early = whole && (!encodes(b) || encodes_by_union(b));
+  auto launch = [&](auto tokens) {
+    constexpr int TOKENS = decltype(tokens)::value;
+    launch_dependent(k_mix<TOKENS>, dim3(b.L.H / 128 + whole, (b.T + TOKENS - 1) / TOKENS), dim3(128), 0, b.stream,
+                     b.L, b.ws, b.padding, b.T, out, latents, early);
+    return launched();
+  };
+  if (b.T <= 16) return launch(std::integral_constant<int, 1>{});
+  if (b.T <= 64) return launch(std::integral_constant<int, 2>{});
+  if (b.T <= 128) return launch(std::integral_constant<int, 4>{});
+  return launch(std::integral_constant<int, 8>{});
 }
 
 // Checks an exchange description against the layer and the call (`rows` = tokens
@@ -2311,7 +2399,7 @@ int cfm_partial_output(const cfm_layer* layer, void* workspace, int32_t capacity
   }
   k_partial_output<<<dim3(peers ? (b.L.H + 511) / 512 : b.L.H / 128, b.T), 128, 0, b.stream>>>(
       b.L, b.ws, b.padding, static_cast<float*>(call->out),
-      rows_grouped(b) ? down_grouped_parts(b) : 0, x, peers);
+      static_cast<int>(down_by_union(b)), x, peers);
   return launched();
 }
 
@@ -2432,9 +2520,9 @@ int cfm_reader_forward(const cfm_layer* layer, void* workspace, int32_t capacity
   if ((rc = run_prepare(b, call, !call->input_prepared, true))) return rc;
   if ((rc = run_screen(b))) return rc;
   if ((rc = run_select(b, 0, nullptr, false))) return rc;
-  if ((rc = run_exact(b, call, !rows_grouped(b)))) return rc;
-  if ((rc = run_down(b, encodes(b) && !rows_grouped(b)))) return rc;
-  if (rows_grouped(b) && (rc = run_encode(b))) return rc;
+  if ((rc = run_exact(b, call, true))) return rc;
+  if ((rc = run_down(b, encodes(b)))) return rc;
+  if (down_by_union(b) && encodes(b) && !encodes_by_union(b) && (rc = run_encode(b))) return rc;
   return run_output(b, call, true);
 }
 

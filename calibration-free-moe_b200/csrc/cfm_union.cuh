@@ -170,17 +170,23 @@ struct ExactSource {
   const char *a, *b, *x[NT];
 };
 
-// `by_candidate`: activations go to their candidates' places, for the tile-wise down kernel.
+// `by_union`: activations also go to their union rows, for k_down_union.  With `list` one more CTA,
+// the first, lists the down tiles for the tile-wise down kernel.
 template <int NT>
 __global__ void __launch_bounds__(ExactUnion<NT>::kThreads, ExactUnion<NT>::kPerSm)
-    k_exact_union(Layer L, Workspace ws, const __nv_bfloat16* hidden, int by_candidate) {
+    k_exact_union(Layer L, Workspace ws, const __nv_bfloat16* hidden, int by_union, int list) {
   using X = ExactUnion<NT>;
   constexpr int kSlots = X::kSlots;
   extern __shared__ __align__(1024) uint8_t union_shared[];
+  __shared__ int scratch[33];
   grid_dependency_wait();     // the work list is complete
-  grid_dependency_release();  // the down kernel may be scheduled: it reads the lists at once
-  const int work_count = ws.work_counts[kExactCount];
-  int index = blockIdx.x;
+  grid_dependency_release();  // the down kernel may be scheduled: its encoder needs no more than that
+  if (list && blockIdx.x == 0) {
+    list_down_tiles(L, ws, scratch);
+    return;
+  }
+  const int work_count = ws.work_counts[kExactCount], stride = gridDim.x - list;
+  int index = blockIdx.x - list;
   if (index >= work_count) return;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, tq = lane & 3;
   const int column = warp * (L.H / 4) + 8 * tq;
@@ -219,7 +225,7 @@ __global__ void __launch_bounds__(ExactUnion<NT>::kThreads, ExactUnion<NT>::kPer
     for (int n = 0; n < NT; ++n) copy_async16(to + 512 * (4 + n), s.x[n] + offset);
   };
 
-  UnionWork work = read_work(index), next = read_work(index + gridDim.x);
+  UnionWork work = read_work(index), next = read_work(index + stride);
   ExactSource<NT> source = locate(work);
 #pragma unroll
   for (int j = 0; j < kSlots - 1; ++j) {
@@ -227,28 +233,31 @@ __global__ void __launch_bounds__(ExactUnion<NT>::kThreads, ExactUnion<NT>::kPer
     copy_async_commit();  // also when empty: the group count per step stays fixed
   }
   for (;;) {
-    const bool more = index + static_cast<int>(gridDim.x) < work_count;
+    const bool more = index + stride < work_count;
     // What the end of the tile needs, and where the next one's rows are, on their way early.
     const int at = work.tile * 16 + g + 8 * (warp >> 1);
     const bool finishes = at < work.rows;
     const int channel =
         finishes ? ws.union_channels[static_cast<size_t>(work.e) * L.I + at] : 0;
     uint32_t bits[NT];
-    int pairs[NT];
+    int pairs[NT], places[NT];  // where the kept channels of the candidate's word begin in its list
 #pragma unroll
     for (int n = 0; n < NT; ++n) {
       const int token = 8 * n + 2 * tq + (warp & 1);
       bits[n] = 0;
-      pairs[n] = 0;
+      pairs[n] = places[n] = 0;
       if (finishes && token < work.count) {
         pairs[n] = ws.group_pairs[work.first + token];
         const int t = pairs[n] / L.K, candidate = (pairs[n] - t * L.K) * L.I + channel;
-        bits[n] = ws.kept_bits[static_cast<size_t>(t) * token_words + (candidate >> 5)] >> (candidate & 31);
+        const size_t word = static_cast<size_t>(t) * token_words + (candidate >> 5);
+        const uint32_t kept = ws.kept_bits[word];
+        bits[n] = kept >> (candidate & 31);
+        places[n] = ws.kept_before[word] + __popc(kept & ((1u << (candidate & 31)) - 1));
       }
     }
     ExactSource<NT> next_source = source;
     if (more) next_source = locate(next);
-    const UnionWork after = read_work(index + 2 * gridDim.x);
+    const UnionWork after = read_work(index + 2 * stride);
 
     float acc[NT][2][4];
 #pragma unroll
@@ -306,9 +315,8 @@ __global__ void __launch_bounds__(ExactUnion<NT>::kThreads, ExactUnion<NT>::kPer
     for (int n = 0; n < NT; ++n) {
       const int token = 8 * n + 2 * tq + (warp & 1);
       if (!finishes || token >= work.count) continue;
-      const bool kept = bits[n] & 1u;
-      float feature = 0.0f;
-      if (kept) {
+      __nv_bfloat16 feature = __float2bfloat16_rn(0.0f);
+      if (bits[n] & 1u) {
         float gate = 0.0f, up = 0.0f;
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
@@ -316,18 +324,365 @@ __global__ void __launch_bounds__(ExactUnion<NT>::kThreads, ExactUnion<NT>::kPer
           gate += sums[(n * 8 + warp) * 32];
           up += sums[(n * 8 + 4 + warp) * 32];
         }
-        feature = exact_feature(gate, up, L.activation);
+        feature = __float2bfloat16_rn(exact_feature(gate, up, L.activation));
+        ws.activations[static_cast<size_t>(pairs[n]) * L.I + channel] = feature;
+        float* exact = ws.exact + static_cast<size_t>(pairs[n] / L.K) * 2 * L.F + places[n];
+        exact[0] = gate;
+        exact[L.F] = up;
       }
-      if (!by_candidate)
-        ws.activations[static_cast<size_t>(work.first + token) * L.I + at] = __float2bfloat16_rn(feature);
-      else if (kept)
-        ws.activations[static_cast<size_t>(pairs[n]) * L.I + channel] = __float2bfloat16_rn(feature);
+      if (by_union) ws.union_activations[static_cast<size_t>(work.first + token) * L.I + at] = feature;
     }
     if (!more) break;
     __syncthreads();  // the sums may be overwritten
-    index += gridDim.x;
+    index += stride;
     work = next;
     next = after;
     source = next_source;
+  }
+}
+
+// ---------------------------------------------------------------------------
+// down, and the recovery encoder
+// ---------------------------------------------------------------------------
+// D[column][token] = sum over union rows: sixteen rows and sixteen columns of weights are the
+// instruction's first operand, sixteen rows of NT x 8 tokens' activations (zero where a token did
+// not keep the row) the second.  A warp takes one piece of work on its own: 64 columns of one pass
+// over one expert, all the union's rows, sixteen (a unit) at a time through a ring of cp.async
+// copies that runs on into its next piece.  ldmatrix transposes the weights on their way to
+// registers; rows lie 144 bytes apart, which keeps its eight addresses in different banks.  Union
+// row 4 a + 2 b + i of a unit is the instruction's row 8 b + 2 a + i, so that a lane's four
+// activations are adjacent in memory.  Rows beyond the union repeat its last one and meet zeros.
+// The recovery encoder is the same product with an expert's whole width as its rows and the sketch
+// features (zero for kept channels, k_select) as activations; its pieces come first, and the last
+// of a token's to arrive mixes its latent.  Bound by the weights' way from L2 and HBM to the SMs.
+template <int NT>
+struct DownUnion {
+  static constexpr int kThreads = 128;
+  static constexpr int kPass = 8 * NT;
+  static constexpr int kColumns = 64;
+  static constexpr int kPerSm = 4;
+  static constexpr int kSlots = NT == 1 ? 5 : 4;
+  static constexpr int kRowBytes = 144;
+  static constexpr int kUnitBytes = 16 * kRowBytes;
+  static constexpr int kSlotBytes = kUnitBytes + 256 * NT;
+  static constexpr int kSharedBytes = 4 * kSlots * kSlotBytes;
+};
+
+
+// `encoder_blocks`: column blocks of the recovery encoder, or 0 without it.
+template <int NT>
+__global__ void __launch_bounds__(DownUnion<NT>::kThreads, DownUnion<NT>::kPerSm)
+    k_down_union(Layer L, Workspace ws, int encoder_blocks) {
+  using X = DownUnion<NT>;
+  constexpr int kSlots = X::kSlots;
+  extern __shared__ __align__(128) uint8_t union_shared[];
+  grid_dependency_wait();     // the activations are complete
+  grid_dependency_release();  // the output may be scheduled; it waits for this grid
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, tq = lane & 3;
+  const int passes = ws.work_counts[kDownCount], blocks = L.H / X::kColumns;
+  const int encoder_pieces = passes * encoder_blocks, pieces = encoder_pieces + passes * blocks;
+  const int stride = gridDim.x * 4;
+  const uint32_t ring = shared_u32(union_shared) + warp * (kSlots * X::kSlotBytes);
+  const int copy_row = lane >> 3, copy_column = (lane & 7) * 8;
+  const uint32_t copy_to = ring + ((copy_row >> 1) * 8 + (copy_row & 1)) * X::kRowBytes + (lane & 7) * 16;
+  int index = blockIdx.x * 4 + warp;
+  if (index >= pieces) return;
+
+  auto encodes = [&](int i) { return i < encoder_pieces; };
+  auto block_of = [&](int i) { return encodes(i) ? i % encoder_blocks : (i - encoder_pieces) % blocks; };
+  auto read_work = [&](int i) {
+    if (i >= pieces) return UnionWork{0, 0, 0, 0, 0};
+    UnionWork w = load_work(ws.down_work +
+                            (encodes(i) ? i / encoder_blocks : (i - encoder_pieces) / blocks));
+    if (encodes(i)) w.rows = L.I;
+    return w;
+  };
+  // Channels of union rows 32 `window` .. of the piece, one per lane.
+  auto channel_window = [&](const UnionWork& w, bool encoder, int window) -> int {
+    const int row = max(0, min(32 * window + lane, w.rows - 1));
+    return encoder ? row : ws.union_channels[static_cast<size_t>(w.e) * L.I + row];
+  };
+
+  // ---- the copies, some units ahead of the sums ----
+  int ahead = index, unit = 0, units = 0, channels = 0, more_channels = 0;
+  bool live = false, encoder = false;
+  size_t row_bytes = 0;
+  const char* rows = nullptr;
+  const __nv_bfloat16* values[NT];
+  UnionWork source = read_work(ahead), source_next = read_work(ahead + stride);
+  int first_channels = channel_window(source, encodes(ahead), 0);
+  auto start_piece = [&]() {
+    encoder = encodes(ahead);
+    const int width = encoder ? L.R : L.H, column = block_of(ahead) * X::kColumns + copy_column;
+    live = column < width;
+    row_bytes = static_cast<size_t>(width) * 2;
+    rows = reinterpret_cast<const char*>((encoder ? L.encoder : L.down) +
+                                         static_cast<size_t>(source.e) * L.I * width + column);
+#pragma unroll
+    for (int n = 0; n < NT; ++n) {  // columns beyond the pass repeat its last token
+      const int at = source.first + min(8 * n + g, source.count - 1);
+      values[n] = (encoder ? ws.features + static_cast<size_t>(ws.group_pairs[at]) * L.I
+                           : ws.union_activations + static_cast<size_t>(at) * L.I) + 4 * tq;
+    }
+    unit = 0;
+    units = max(1, (source.rows + 15) / 16);
+    channels = first_channels;
+    more_channels = units > 2 ? channel_window(source, encoder, 1) : 0;
+    first_channels = ahead + stride < pieces ? channel_window(source_next, encodes(ahead + stride), 0) : 0;
+  };
+  auto fetch = [&](int slot) {
+    if (unit < units) {
+      const uint32_t to = copy_to + slot * X::kSlotBytes;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int channel = __shfl_sync(kFull, channels, 16 * (unit & 1) + copy_row + 4 * i);
+        if (live) copy_async16(to + 2 * i * X::kRowBytes, rows + channel * row_bytes);
+      }
+#pragma unroll
+      for (int n = 0; n < NT; ++n)
+        copy_async8(ring + slot * X::kSlotBytes + X::kUnitBytes + 256 * n + 8 * lane,
+                    values[n] + 16 * unit);
+      if (++unit == units) {
+        ahead += stride;
+        units = 0;
+        if (ahead < pieces) {
+          source = source_next;
+          source_next = read_work(ahead + stride);
+          start_piece();
+        }
+      } else if ((unit & 1) == 0) {
+        channels = more_channels;
+        if (unit + 2 < units) more_channels = channel_window(source, encoder, unit / 2 + 1);
+      }
+    }
+    copy_async_commit();  // also when empty: the group count per step stays fixed
+  };
+  start_piece();
+#pragma unroll
+  for (int s = 0; s < kSlots - 1; ++s) fetch(s);
+
+  // ---- the sums ----
+  const int k = ((lane >> 4) << 3) + (lane & 7);  // the row whose address this lane gives to ldmatrix
+  const uint32_t load_from = ring + k * X::kRowBytes + ((lane >> 3) & 1) * 16;
+  int slot = 0;
+  UnionWork work = read_work(index);
+  for (; index < pieces; index += stride) {
+    const UnionWork next = read_work(index + stride);
+    const bool is_encoder = encodes(index);
+    const int steps = max(1, (work.rows + 15) / 16);
+    int pairs[NT][2];
+#pragma unroll
+    for (int n = 0; n < NT; ++n)
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        const int token = 8 * n + 2 * tq + i;
+        pairs[n][i] = token < work.count ? ws.group_pairs[work.first + token] : -1;
+      }
+    float acc[NT][4][4];
+#pragma unroll
+    for (int n = 0; n < NT; ++n)
+#pragma unroll
+      for (int m = 0; m < 4; ++m)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) acc[n][m][i] = 0.0f;
+    for (int step = 0; step < steps; ++step) {
+      copy_async_wait<kSlots - 2>();
+      __syncwarp();  // every lane's copies of the unit have landed; the unit before is in registers
+      fetch(slot == 0 ? kSlots - 1 : slot - 1);
+      uint2 b[NT];
+#pragma unroll
+      for (int n = 0; n < NT; ++n)
+        b[n] = load_shared8(ring + slot * X::kSlotBytes + X::kUnitBytes + 256 * n + 8 * lane);
+      const int left = work.rows - 16 * step;
+      if (left < 16) {  // rows beyond the union weigh nothing
+        const int mine = left - 4 * tq;
+        const uint32_t x = mine > 1 ? ~0u : mine > 0 ? 0xffffu : 0u;
+        const uint32_t y = mine > 3 ? ~0u : mine > 2 ? 0xffffu : 0u;
+#pragma unroll
+        for (int n = 0; n < NT; ++n) {
+          b[n].x &= x;
+          b[n].y &= y;
+        }
+      }
+#pragma unroll
+      for (int m = 0; m < 4; ++m) {
+        uint32_t a[4];
+        load_matrices_transposed(a, load_from + slot * X::kSlotBytes + 32 * m);
+#pragma unroll
+        for (int n = 0; n < NT; ++n) mma_bf16(acc[n][m], a[0], a[1], a[2], a[3], b[n].x, b[n].y);
+      }
+      slot = slot + 1 == kSlots ? 0 : slot + 1;
+    }
+    // A token's sum over the expert, rounded to BF16 as the mix takes it.
+    __nv_bfloat16* out = reinterpret_cast<__nv_bfloat16*>(is_encoder ? ws.encoder_parts : ws.down_parts);
+    const int width = is_encoder ? L.R : L.H, column = block_of(index) * X::kColumns + g;
+#pragma unroll
+    for (int n = 0; n < NT; ++n)
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        if (pairs[n][i] < 0) continue;
+        __nv_bfloat16* row = out + static_cast<size_t>(pairs[n][i]) * width;
+#pragma unroll
+        for (int m = 0; m < 4; ++m) {
+          const int c = column + 16 * m;
+          if (c < width) row[c] = __float2bfloat16_rn(acc[n][m][i]);
+          if (c + 8 < width) row[c + 8] = __float2bfloat16_rn(acc[n][m][2 + i]);
+        }
+      }
+    if (is_encoder) {
+      __threadfence();
+      __syncwarp();
+      bool last = false;
+      int t = 0;
+      if (lane < work.count) {
+        t = ws.group_pairs[work.first + lane] / L.K;
+        int local = 0;
+        for (int s = 0; s < L.K; ++s) local += ws.ids[static_cast<size_t>(t) * L.K + s] >= 0;
+        uint32_t* counter = ws.counters + 2 * static_cast<size_t>(ws.capacity) * L.K + t;
+        last = atomicAdd(counter, 1u) == static_cast<unsigned>(local * encoder_blocks - 1);
+        if (last) *counter = 0;
+      }
+      unsigned finished = __ballot_sync(kFull, last);
+      if (finished) __threadfence();
+      for (; finished; finished &= finished - 1) {
+        const size_t pair0 = static_cast<size_t>(__shfl_sync(kFull, t, __ffs(finished) - 1)) * L.K;
+        const unsigned short* parts = reinterpret_cast<const unsigned short*>(ws.encoder_parts) + pair0 * L.R;
+        for (int r = lane; r < L.R; r += 32) {
+          float latent = 0.0f;
+#pragma unroll 8
+          for (int s = 0; s < L.K; ++s)
+            if (ws.ids[pair0 + s] >= 0)
+              latent = fmaf(__bfloat162float(__ushort_as_bfloat16(__ldcg(parts + static_cast<size_t>(s) * L.R + r))),
+                            ws.weights[pair0 + s], latent);
+          ws.latent[pair0 / L.K * L.R + r] = latent;
+        }
+      }
+    }
+    work = next;
+  }
+}
+
+// ---------------------------------------------------------------------------
+// output after k_down_union
+// ---------------------------------------------------------------------------
+// Router mix of the BF16 expert sums of token t at column h, in slot order.
+__device__ __forceinline__ float mix_sums(const Layer& L, const Workspace& ws, int t, int h) {
+  const unsigned short* sums = reinterpret_cast<const unsigned short*>(ws.down_parts) +
+                               static_cast<size_t>(t) * L.K * L.H + h;
+  float routed = 0.0f;
+#pragma unroll 8
+  for (int s = 0; s < L.K; ++s) {
+    const size_t pair = static_cast<size_t>(t) * L.K + s;
+    if (ws.ids[pair] >= 0)
+      routed = fmaf(__bfloat162float(__ushort_as_bfloat16(__ldcg(sums + static_cast<size_t>(s) * L.H))),
+                    ws.weights[pair], routed);
+  }
+  return routed;
+}
+
+// grid (H / 128, or one more for the tokens' read-cost counters; ceil(T / TOKENS)), 128 threads, one
+// output column of TOKENS tokens per thread.  The decoder row is read once for them; their dot
+// products with it run side by side, each in the order k_output takes, and their expert sums are on
+// their way meanwhile.  Bound by latency (and by instructions from some 128 tokens on).
+template <int TOKENS>
+__global__ void __launch_bounds__(128) k_mix(Layer L, Workspace ws, const uint8_t* padding, int tokens,
+                                             __nv_bfloat16* out, int latents, int early) {
+  __shared__ __align__(16) float latent[TOKENS][256];
+  __shared__ float weight[TOKENS][32];
+  __shared__ uint32_t valid[TOKENS];
+  const int t0 = blockIdx.y * TOKENS, count = min(TOKENS, tokens - t0);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, h = blockIdx.x * 128 + tid;
+  if (!early) grid_dependency_wait();
+  if (static_cast<int>(blockIdx.x) * 128 >= L.H) {  // the read-cost counters
+    for (int j = warp; j < count; j += 4) {
+      const int t = t0 + j;
+      if (padding && padding[t]) continue;
+      const size_t pair = static_cast<size_t>(t) * L.K + lane;
+      const bool local = lane < L.K && ws.ids[pair] >= 0;
+      account_token(L, lane, local, local ? ws.counts[pair] : 0, L.F < L.N);
+    }
+    return;
+  }
+  const bool recover = L.R > 0 && L.owner && L.decoder;
+  constexpr int kAhead = 8;
+  const int chunks = recover ? L.R / 8 : 0;
+  const uint4* decoder_row = reinterpret_cast<const uint4*>(L.decoder + static_cast<size_t>(h) * L.R);
+  uint4 decoder[kAhead];
+#pragma unroll
+  for (int i = 0; i < kAhead; ++i) decoder[i] = i < chunks ? decoder_row[i] : make_uint4(0, 0, 0, 0);
+  for (int j = warp; j < TOKENS; j += 4) {  // the slots that have sums, and their weights
+    bool here = false;
+    if (j < count && lane < L.K) {
+      const size_t pair = static_cast<size_t>(t0 + j) * L.K + lane;
+      here = ws.ids[pair] >= 0 && !(padding && padding[t0 + j]);
+      weight[j][lane] = ws.weights[pair];
+    }
+    const unsigned slots = __ballot_sync(kFull, here);
+    if (lane == 0) valid[j] = slots;
+  }
+  if (early) grid_dependency_wait();
+  __syncthreads();
+  constexpr int kSums = 8;  // of each token on their way at a time
+  unsigned short sums[TOKENS][kSums];
+  const unsigned short* from = reinterpret_cast<const unsigned short*>(ws.down_parts) +
+                               static_cast<size_t>(t0) * L.K * L.H + h;
+#pragma unroll
+  for (int j = 0; j < TOKENS; ++j)
+#pragma unroll
+    for (int s = 0; s < kSums; ++s)
+      sums[j][s] = (valid[j] >> s) & 1u ? __ldcg(from + static_cast<size_t>(j * L.K + s) * L.H) : 0;
+  if (L.R > 0) {
+    for (int i = tid; i < count * L.R; i += 128) {
+      const int j = i / L.R, r = i - j * L.R;
+      float* kept = ws.latent + static_cast<size_t>(t0 + j) * L.R + r;
+      const bool given = latents && valid[j];
+      if (!given && blockIdx.x == 0) *kept = 0.0f;
+      latent[j][r] = given ? bf16_round(*kept) : 0.0f;
+    }
+    __syncthreads();
+  }
+  float dot[TOKENS];
+#pragma unroll
+  for (int j = 0; j < TOKENS; ++j) dot[j] = 0.0f;
+  auto fold = [&](const uint4& w, int i) {
+#pragma unroll
+    for (int j = 0; j < TOKENS; ++j) {
+      const float4 a = *reinterpret_cast<const float4*>(&latent[j][8 * i]);
+      const float4 b = *reinterpret_cast<const float4*>(&latent[j][8 * i + 4]);
+      dot[j] = fmaf(bf16_lo(w.x), a.x, dot[j]);
+      dot[j] = fmaf(bf16_hi(w.x), a.y, dot[j]);
+      dot[j] = fmaf(bf16_lo(w.y), a.z, dot[j]);
+      dot[j] = fmaf(bf16_hi(w.y), a.w, dot[j]);
+      dot[j] = fmaf(bf16_lo(w.z), b.x, dot[j]);
+      dot[j] = fmaf(bf16_hi(w.z), b.y, dot[j]);
+      dot[j] = fmaf(bf16_lo(w.w), b.z, dot[j]);
+      dot[j] = fmaf(bf16_hi(w.w), b.w, dot[j]);
+    }
+  };
+#pragma unroll
+  for (int i = 0; i < kAhead; ++i)
+    if (i < chunks) fold(decoder[i], i);
+  for (int i0 = kAhead; i0 < chunks; i0 += kAhead) {
+#pragma unroll
+    for (int i = 0; i < kAhead; ++i)
+      decoder[i] = i0 + i < chunks ? decoder_row[i0 + i] : make_uint4(0, 0, 0, 0);
+#pragma unroll
+    for (int i = 0; i < kAhead; ++i)
+      if (i0 + i < chunks) fold(decoder[i], i0 + i);
+  }
+#pragma unroll
+  for (int j = 0; j < TOKENS; ++j) {
+    if (j >= count) break;
+    float routed = 0.0f;
+#pragma unroll
+    for (int s = 0; s < kSums; ++s)
+      if ((valid[j] >> s) & 1u)
+        routed = fmaf(__bfloat162float(__ushort_as_bfloat16(sums[j][s])), weight[j][s], routed);
+#pragma unroll 4
+    for (int s = kSums; s < L.K; ++s)
+      if ((valid[j] >> s) & 1u)
+        routed = fmaf(__bfloat162float(__ushort_as_bfloat16(__ldcg(from + static_cast<size_t>(j * L.K + s) * L.H))),
+                      weight[j][s], routed);
+    out[static_cast<size_t>(t0 + j) * L.H + h] = __float2bfloat16_rn(routed + bf16_round(dot[j]));
   }
 }

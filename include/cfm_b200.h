@@ -30,7 +30,7 @@
 extern "C" {
 #endif
 
-#define CFM_ABI_VERSION 11
+#define CFM_ABI_VERSION 12
 
 /* argument errors */
 #define CFM_E_NULL -1       /* a required pointer is NULL                      */
@@ -150,8 +150,8 @@ typedef struct cfm_workspace_layout {
   int64_t tile_starts;    /* i32 [C, K]                                         */
   int64_t activations;    /* bf16 [C, N] exact phi(g) u of kept candidates      */
   int64_t exact;          /* f32 [C, 2, F] exact gate and up projections        */
-  int64_t down_parts;     /* f32 [C, down_tiles, H]                             */
-  int64_t encoder_parts;  /* f32 [C, K, encoder_tiles, R]                       */
+  int64_t down_parts;     /* f32 [C, down_tiles, H]; expert-major bf16 [C, K, H] */
+  int64_t encoder_parts;  /* f32 [C, K, encoder_tiles, R]; expert-major bf16 [C, K, R] */
   int64_t latent;         /* f32 [C, R]                                         */
   int64_t status;         /* i32 [4] device-side error flags (zero = healthy)   */
   int64_t limbs;          /* i8  [C, B, 3, 128] base-256 digits of `quantized`, sixteen
@@ -164,11 +164,17 @@ typedef struct cfm_workspace_layout {
   int64_t features;       /* bf16 [C, N] phi(g) u of the sketch projections     */
   int64_t pass_work;      /* i32 [.., 4] passes of the screen over the experts   */
   int64_t busy_experts;   /* i32 [E] experts some pair is routed to, ascending  */
-  int64_t work_counts;    /* i32 [4] passes, busy experts                       */
+  int64_t work_counts;    /* i32 [4] passes, busy experts, lengths of the two work lists */
   int64_t tile_list;      /* i32 [C * (ceil(F / 64) + K), 8] down tiles in expert order */
   int64_t tile_count;     /* i32 [4] number of listed tiles                        */
+  int64_t kept_bits;      /* u32 [C, ceil(N / 32) + 1] kept candidates as bits     */
+  int64_t kept_before;    /* u16 [C, ceil(N / 32) + 1] kept candidates before a word */
+  int64_t union_channels; /* u16 [E, I] channels some token of an expert kept      */
+  int64_t union_activations; /* bf16 [C * K, I] activations by row of the union    */
+  int64_t exact_work;     /* i32 [.., 8] work of the expert-major exact kernel     */
+  int64_t down_work;      /* i32 [.., 8] work of the expert-major down kernel      */
   int32_t parts_tokens;   /* tokens the split screen can serve                  */
-  int32_t down_tiles;     /* max(ceil(F / 64) + K - 1, 8 K) partial sums per token */
+  int32_t down_tiles;     /* ceil(F / 64) + K - 1 partial sums per token         */
   int32_t encoder_tiles;  /* ceil(I / 256)                                      */
   int32_t reserved;
 } cfm_workspace_layout;
