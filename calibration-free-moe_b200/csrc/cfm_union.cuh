@@ -148,6 +148,8 @@ __global__ void __launch_bounds__(kUnionThreads)
 // memory with cp.async and reads them back itself: it waits for its own copies only, and the ring
 // needs no barrier.  The instruction's column order is free as long as both operands agree, so the
 // eight columns serve as columns 2 tq, 2 tq + 1, 2 tq + 8, 2 tq + 9 of two instructions.  The
+// instruction truncates where an FMA rounds, so a sum leaves it after 128 columns and goes on by
+// ordinary additions, which keeps it as accurate as the gathers' (error against FP64 MEASURED_ERR).  The
 // tokens' rows travel with the weights because the ring leaves L1 too small to hold them.  (Loads
 // straight into registers were issued one by one: 76 us at 64 tokens of the 128-expert layer, 54
 // with the ring; the gathers per token take 69.)
@@ -177,7 +179,7 @@ __global__ void __launch_bounds__(ExactUnion<NT>::kThreads, ExactUnion<NT>::kPer
     k_exact_union(Layer L, Workspace ws, const __nv_bfloat16* hidden, int by_union, int list) {
   using X = ExactUnion<NT>;
   constexpr int kSlots = X::kSlots;
-  extern __shared__ __align__(1024) uint8_t union_shared[];
+  extern __shared__ __align__(128) uint8_t union_shared[];
   __shared__ int scratch[33];
   grid_dependency_wait();     // the work list is complete
   grid_dependency_release();  // the down kernel may be scheduled: its encoder needs no more than that
@@ -267,6 +269,11 @@ __global__ void __launch_bounds__(ExactUnion<NT>::kThreads, ExactUnion<NT>::kPer
 #pragma unroll 1
     for (int s = 0; s < padded; s += kSlots) {
       const bool last = s + kSlots >= padded;
+      float part[NT][2][4];  // of this turn of the ring
+#pragma unroll
+      for (int n = 0; n < NT; ++n)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) part[n][0][i] = part[n][1][i] = 0.0f;
 #pragma unroll
       for (int j = 0; j < kSlots; ++j) {
         copy_async_wait<kSlots - 2>();  // this lane's copies of step s + j have landed
@@ -291,13 +298,20 @@ __global__ void __launch_bounds__(ExactUnion<NT>::kThreads, ExactUnion<NT>::kPer
         if (live) {
 #pragma unroll
           for (int n = 0; n < NT; ++n) {
-            mma_bf16(acc[n][0], w[0].x, w[1].x, w[0].y, w[1].y, t[n].x, t[n].y);
-            mma_bf16(acc[n][1], w[2].x, w[3].x, w[2].y, w[3].y, t[n].x, t[n].y);
-            mma_bf16(acc[n][0], w[0].z, w[1].z, w[0].w, w[1].w, t[n].z, t[n].w);
-            mma_bf16(acc[n][1], w[2].z, w[3].z, w[2].w, w[3].w, t[n].z, t[n].w);
+            mma_bf16(part[n][0], w[0].x, w[1].x, w[0].y, w[1].y, t[n].x, t[n].y);
+            mma_bf16(part[n][1], w[2].x, w[3].x, w[2].y, w[3].y, t[n].x, t[n].y);
+            mma_bf16(part[n][0], w[0].z, w[1].z, w[0].w, w[1].w, t[n].z, t[n].w);
+            mma_bf16(part[n][1], w[2].z, w[3].z, w[2].w, w[3].w, t[n].z, t[n].w);
           }
         }
       }
+#pragma unroll
+      for (int n = 0; n < NT; ++n)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          acc[n][0][i] += part[n][0][i];
+          acc[n][1][i] += part[n][1][i];
+        }
     }
     // Sums of the quarters: [quarter][tile of tokens][gate, up][accumulator register][lane].
     float* own = red + warp * X::kSumFloats + lane;
@@ -317,18 +331,20 @@ __global__ void __launch_bounds__(ExactUnion<NT>::kThreads, ExactUnion<NT>::kPer
       if (!finishes || token >= work.count) continue;
       __nv_bfloat16 feature = __float2bfloat16_rn(0.0f);
       if (bits[n] & 1u) {
-        float gate = 0.0f, up = 0.0f;
+        float gate[4], up[4];
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
           const float* sums = red + q * X::kSumFloats + lane;
-          gate += sums[(n * 8 + warp) * 32];
-          up += sums[(n * 8 + 4 + warp) * 32];
+          gate[q] = sums[(n * 8 + warp) * 32];
+          up[q] = sums[(n * 8 + 4 + warp) * 32];
         }
-        feature = __float2bfloat16_rn(exact_feature(gate, up, L.activation));
+        const float g_sum = (gate[0] + gate[1]) + (gate[2] + gate[3]);
+        const float u_sum = (up[0] + up[1]) + (up[2] + up[3]);
+        feature = __float2bfloat16_rn(exact_feature(g_sum, u_sum, L.activation));
         ws.activations[static_cast<size_t>(pairs[n]) * L.I + channel] = feature;
         float* exact = ws.exact + static_cast<size_t>(pairs[n] / L.K) * 2 * L.F + places[n];
-        exact[0] = gate;
-        exact[L.F] = up;
+        exact[0] = g_sum;
+        exact[L.F] = u_sum;
       }
       if (by_union) ws.union_activations[static_cast<size_t>(work.first + token) * L.I + at] = feature;
     }
