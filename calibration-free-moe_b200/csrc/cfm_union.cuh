@@ -21,6 +21,14 @@
 // the next.  Included by cfm_reader.cu inside namespace cfm.
 #pragma once
 
+// d = a b, without a sum to add to.
+__device__ __forceinline__ void mma_bf16_first(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2,
+                                               uint32_t a3, uint32_t b0, uint32_t b1) {
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, "
+      "{%8,%9}, {%10,%10,%10,%10};"
+      : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(0.0f));
+}
 __device__ __forceinline__ void mma_bf16(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2,
                                          uint32_t a3, uint32_t b0, uint32_t b1) {
   asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, "
@@ -49,7 +57,7 @@ __device__ __forceinline__ void load_matrices_transposed(uint32_t (&a)[4], uint3
 // unions and work lists
 // ---------------------------------------------------------------------------
 constexpr int kUnionThreads = 128;
-constexpr int kUnionStagedPairs = 128;  // pairs of an expert whose numbers a CTA stages
+constexpr int kUnionStagedPairs = 512;  // pairs of an expert whose numbers a CTA stages
 
 // One piece of work of the exact kernel (tile `tile` of expert e's union for `count` pairs from
 // `first` of the grouped list) or of the down kernel (`tile` unused).  The union has `rows`
@@ -83,6 +91,7 @@ __global__ void __launch_bounds__(kUnionThreads)
     k_union(Layer L, Workspace ws, int exact_pass, int down_pass, int early) {
   __shared__ int scratch[33];
   __shared__ int staged[kUnionStagedPairs];
+  __shared__ uint32_t masks[kUnionThreads];
   __shared__ int s_base[2];
   const int tid = threadIdx.x, words = (L.I + 31) / 32, token_words = kept_words(L.N);
   if (!early) grid_dependency_wait();
@@ -104,15 +113,27 @@ __global__ void __launch_bounds__(kUnionThreads)
     return slot_word(ws.kept_bits + static_cast<size_t>(t) * token_words, L.I, pair - t * L.K, w);
   };
   uint16_t* channels = ws.union_channels + static_cast<size_t>(e) * L.I;
+  // Few words leave threads over: groups of them share the pairs.
+  int lanes = 32;
+  while (lanes < words && lanes < kUnionThreads) lanes *= 2;
+  const int groups = kUnionThreads / lanes, group = tid / lanes;
   int rows = 0;
   for (int w0 = 0; w0 < words; w0 += kUnionThreads) {
-    const int w = w0 + tid;
+    const int w = w0 + tid - group * lanes;
     uint32_t mask = 0;
     if (w < words) {
       const int quick = min(total, kUnionStagedPairs);
+      int j = group;
 #pragma unroll 8
-      for (int j = 0; j < quick; ++j) mask |= word_of(staged[j], w);
-      for (int j = quick; j < total; ++j) mask |= word_of(ws.group_pairs[first + j], w);
+      for (; j < quick; j += groups) mask |= word_of(staged[j], w);
+      for (; j < total; j += groups) mask |= word_of(ws.group_pairs[first + j], w);
+    }
+    if (groups > 1) {
+      masks[tid] = mask;
+      __syncthreads();
+      mask = 0;
+      if (group == 0)
+        for (int i = 0; i < groups; ++i) mask |= masks[i * lanes + tid];
     }
     int all = 0;
     int at = rows + block_exclusive_scan(__popc(mask), scratch, &all);
@@ -271,13 +292,9 @@ __global__ void __launch_bounds__(ExactUnion<NT>::kThreads, ExactUnion<NT>::kPer
       const bool last = s + kSlots >= padded;
       float part[NT][2][4];  // of this turn of the ring
 #pragma unroll
-      for (int n = 0; n < NT; ++n)
-#pragma unroll
-        for (int i = 0; i < 4; ++i) part[n][0][i] = part[n][1][i] = 0.0f;
-#pragma unroll
       for (int j = 0; j < kSlots; ++j) {
         copy_async_wait<kSlots - 2>();  // this lane's copies of step s + j have landed
-        const bool live = s + j < steps;
+        const bool live = j == 0 || s + j < steps;
         uint4 w[4], t[NT];
         if (live) {
           const uint32_t from = mine + j * X::kStepBytes;
@@ -298,8 +315,13 @@ __global__ void __launch_bounds__(ExactUnion<NT>::kThreads, ExactUnion<NT>::kPer
         if (live) {
 #pragma unroll
           for (int n = 0; n < NT; ++n) {
-            mma_bf16(part[n][0], w[0].x, w[1].x, w[0].y, w[1].y, t[n].x, t[n].y);
-            mma_bf16(part[n][1], w[2].x, w[3].x, w[2].y, w[3].y, t[n].x, t[n].y);
+            if (j == 0) {
+              mma_bf16_first(part[n][0], w[0].x, w[1].x, w[0].y, w[1].y, t[n].x, t[n].y);
+              mma_bf16_first(part[n][1], w[2].x, w[3].x, w[2].y, w[3].y, t[n].x, t[n].y);
+            } else {
+              mma_bf16(part[n][0], w[0].x, w[1].x, w[0].y, w[1].y, t[n].x, t[n].y);
+              mma_bf16(part[n][1], w[2].x, w[3].x, w[2].y, w[3].y, t[n].x, t[n].y);
+            }
             mma_bf16(part[n][0], w[0].z, w[1].z, w[0].w, w[1].w, t[n].z, t[n].w);
             mma_bf16(part[n][1], w[2].z, w[3].z, w[2].w, w[3].w, t[n].z, t[n].w);
           }
@@ -426,6 +448,7 @@ __global__ void __launch_bounds__(DownUnion<NT>::kThreads, DownUnion<NT>::kPerSm
   const char* rows = nullptr;
   const __nv_bfloat16* values[NT];
   UnionWork source = read_work(ahead), source_next = read_work(ahead + stride);
+  UnionWork source_after = read_work(ahead + 2 * stride);
   int first_channels = channel_window(source, encodes(ahead), 0);
   auto start_piece = [&]() {
     encoder = encodes(ahead);
@@ -463,7 +486,8 @@ __global__ void __launch_bounds__(DownUnion<NT>::kThreads, DownUnion<NT>::kPerSm
         units = 0;
         if (ahead < pieces) {
           source = source_next;
-          source_next = read_work(ahead + stride);
+          source_next = source_after;
+          source_after = read_work(ahead + 2 * stride);
           start_piece();
         }
       } else if ((unit & 1) == 0) {
@@ -646,7 +670,7 @@ __global__ void __launch_bounds__(128) k_mix(Layer L, Workspace ws, const uint8_
   for (int j = 0; j < TOKENS; ++j)
 #pragma unroll
     for (int s = 0; s < kSums; ++s)
-      sums[j][s] = (valid[j] >> s) & 1u ? __ldcg(from + static_cast<size_t>(j * L.K + s) * L.H) : 0;
+      sums[j][s] = s < L.K && j < count ? __ldcg(from + static_cast<size_t>(j * L.K + s) * L.H) : 0;
   if (L.R > 0) {
     for (int i = tid; i < count * L.R; i += 128) {
       const int j = i / L.R, r = i - j * L.R;
