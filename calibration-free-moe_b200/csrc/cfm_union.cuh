@@ -21,36 +21,68 @@
 // the next.  Included by cfm_reader.cu inside namespace cfm.
 #pragma once
 
-// d = a b, without a sum to add to.
-__device__ __forceinline__ void mma_bf16_first(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2,
-                                               uint32_t a3, uint32_t b0, uint32_t b1) {
-  asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, "
-      "{%8,%9}, {%10,%10,%10,%10};"
-      : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
-      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(0.0f));
+// d = a b, and d += a b.
+__device__ __forceinline__ void mma_bf16_first(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, "
+               "{%8,%9}, {%10,%10,%10,%10};"
+               : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+               : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(0.0f));
 }
-__device__ __forceinline__ void mma_bf16(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2,
-                                         uint32_t a3, uint32_t b0, uint32_t b1) {
-  asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, "
-      "{%8,%9}, {%0,%1,%2,%3};"
-      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+__device__ __forceinline__ void mma_bf16(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, "
+               "{%8,%9}, {%0,%1,%2,%3};"
+               : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+               : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
-// 8 bytes global -> shared memory in the thread's current cp.async group.
-__device__ __forceinline__ void copy_async8(uint32_t shared, const void* global) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(shared), "l"(global) : "memory");
+// Copies and loads at a fixed distance from a shared-memory address, which the instruction adds.
+// (With `bytes` 0 instead of 16 nothing is read and zeros are written.)
+template <int AT, int FROM>
+__device__ __forceinline__ void copy_async16_at(uint32_t shared, const void* global, int bytes) {
+  asm volatile("cp.async.cg.shared.global [%0+%2], [%1+%3], 16, %4;" ::"r"(shared), "l"(global), "n"(AT), "n"(FROM),
+               "r"(bytes)
+               : "memory");
 }
-__device__ __forceinline__ uint2 load_shared8(uint32_t address) {
+template <int AT>
+__device__ __forceinline__ void copy_async16_at(uint32_t shared, const void* global) {
+  asm volatile("cp.async.cg.shared.global [%0+%2], [%1], 16;" ::"r"(shared), "l"(global), "n"(AT) : "memory");
+}
+template <int AT>
+__device__ __forceinline__ void copy_async8_at(uint32_t shared, const void* global) {
+  asm volatile("cp.async.ca.shared.global [%0+%2], [%1], 8;" ::"r"(shared), "l"(global), "n"(AT) : "memory");
+}
+template <int AT>
+__device__ __forceinline__ uint2 load_shared8_at(uint32_t address) {
   uint2 v;
-  asm volatile("ld.shared.v2.u32 {%0,%1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(address) : "memory");
+  asm volatile("ld.shared.v2.u32 {%0,%1}, [%2+%3];" : "=r"(v.x), "=r"(v.y) : "r"(address), "n"(AT) : "memory");
   return v;
 }
-__device__ __forceinline__ void load_matrices_transposed(uint32_t (&a)[4], uint32_t address) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+template <int AT>
+__device__ __forceinline__ void load_matrices_at(uint32_t (&a)[4], uint32_t address) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4+%5];"
                : "=r"(a[0]), "=r"(a[1]), "=r"(a[2]), "=r"(a[3])
-               : "r"(address)
+               : "r"(address), "n"(AT)
                : "memory");
+}
+template <int AT>
+__device__ __forceinline__ void load_matrices_transposed_at(uint32_t (&a)[4], uint32_t address) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4+%5];"
+               : "=r"(a[0]), "=r"(a[1]), "=r"(a[2]), "=r"(a[3])
+               : "r"(address), "n"(AT)
+               : "memory");
+}
+template <int I>
+struct Index {
+  static constexpr int value = I;
+  __host__ __device__ constexpr operator int() const { return I; }
+};
+// f(0), f(1), ... f(N - 1) with the index as a constant.
+template <int N, int I = 0, typename F>
+__device__ __forceinline__ void repeat(F&& f) {
+  if constexpr (I < N) {
+    f(Index<I>{});
+    repeat<N, I + 1>(f);
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -164,16 +196,15 @@ __global__ void __launch_bounds__(kUnionThreads)
 // exact
 // ---------------------------------------------------------------------------
 // A tile is sixteen union rows of gate and up against NT x 8 tokens; its columns are cut into
-// quarters of H, one per warp.  Per step of 32 columns lane (g, tq) takes 16 bytes (eight columns)
-// of rows g and g + 8, gate and up, and of its tokens' rows, copies them into a ring in shared
-// memory with cp.async and reads them back itself: it waits for its own copies only, and the ring
-// needs no barrier.  The instruction's column order is free as long as both operands agree, so the
-// eight columns serve as columns 2 tq, 2 tq + 1, 2 tq + 8, 2 tq + 9 of two instructions.  The
+// quarters of H, one per warp.  Per step of 32 columns lane (g, tq) copies 16 bytes (eight columns)
+// of rows g and g + 8, gate and up, and of its tokens' rows into a ring of the warp's own with
+// cp.async; the matrix loads read them from there as the instruction wants them.  A row's four
+// pieces are permuted by the row, so that the eight rows of a matrix lie in different banks.  The
+// tokens' rows travel with the weights because the ring leaves L1 too small to hold them.  The
 // instruction truncates where an FMA rounds, so a sum leaves it after 128 columns and goes on by
-// ordinary additions, which keeps it as accurate as the gathers' (error against FP64 MEASURED_ERR).  The
-// tokens' rows travel with the weights because the ring leaves L1 too small to hold them.  (Loads
-// straight into registers were issued one by one: 76 us at 64 tokens of the 128-expert layer, 54
-// with the ring; the gathers per token take 69.)
+// ordinary additions (RMS error of a gate sum of 2048 columns against FP64: 8.0e-7 without, 4.1e-7
+// with, 2.1e-7 the gathers'; it is rounded to BF16 next).  Loads straight into registers were issued
+// one by one: 76 us at 64 tokens of the 128-expert layer.  MEASURED_EXACT
 template <int NT>
 struct ExactUnion {
   static constexpr int kThreads = 128;
@@ -187,10 +218,14 @@ struct ExactUnion {
   static constexpr int kPerSm = NT == 1 ? 5 : NT == 2 ? 3 : 2;
 };
 
-// Where a lane's pieces of a tile come from.
+// Where a lane's pieces of a tile come from: row and token numbers, and pointers.
+template <int NT>
+struct ExactRows {
+  int e, channel[2], token[NT];
+};
 template <int NT>
 struct ExactSource {
-  const char *a, *b, *x[NT];
+  const char *row[4], *x[NT];  // gate of rows g and g + 8, up of the same
 };
 
 // `by_union`: activations also go to their union rows, for k_down_union.  With `list` one more CTA,
@@ -217,69 +252,84 @@ __global__ void __launch_bounds__(ExactUnion<NT>::kThreads, ExactUnion<NT>::kPer
   const int padded = (steps + kSlots - 1) / kSlots * kSlots;
   const size_t up_bytes = static_cast<size_t>(L.I) * L.H * 2;
   const int token_words = kept_words(L.N);
-  const uint32_t mine = shared_u32(union_shared) + warp * (kSlots * X::kStepBytes) + lane * 16;
+  const uint32_t ring = shared_u32(union_shared) + warp * (kSlots * X::kStepBytes);
+  const uint32_t mine = ring + 64 * g + 16 * (tq ^ ((g >> 1) & 3));
+  // Where this lane's row of a matrix lies: of the first operand (rows 0 to 7 and 8 to 15 of the
+  // first eight columns, then of the next; the other sixteen columns 32 bytes away by xor), and of
+  // the second (a token's four pieces).
+  const int r = lane & 7, matrix = lane >> 3;
+  const uint32_t weights_at = ring + (matrix & 1) * 512 + 64 * r + 16 * ((matrix >> 1) ^ ((r >> 1) & 3));
+  const uint32_t weights_at2 = weights_at ^ 32;
+  const uint32_t tokens_at = ring + 64 * r + 16 * (matrix ^ ((r >> 1) & 3));
   float* red = reinterpret_cast<float*>(union_shared + X::kRingBytes);
 
   auto read_work = [&](int i) {
     return i < work_count ? load_work(ws.exact_work + i) : UnionWork{0, 0, 0, 0, 0};
   };
   auto locate = [&](const UnionWork& w) {  // rows beyond the union repeat its last one
-    ExactSource<NT> s;
+    ExactRows<NT> at;
     const uint16_t* channels = ws.union_channels + static_cast<size_t>(w.e) * L.I;
     const int last = w.rows - 1, row = w.tile * 16 + g;
-    const char* weights = reinterpret_cast<const char*>(
-        L.gate_up + static_cast<size_t>(w.e) * 2 * L.I * L.H + column);
-    s.a = weights + static_cast<size_t>(channels[min(row, last)]) * L.H * 2;
-    s.b = weights + static_cast<size_t>(channels[min(row + 8, last)]) * L.H * 2;
+    at.e = w.e;
+    at.channel[0] = channels[min(row, last)];
+    at.channel[1] = channels[min(row + 8, last)];
 #pragma unroll
-    for (int n = 0; n < NT; ++n) {  // columns beyond the pass repeat its last token
-      const int pair = ws.group_pairs[w.first + min(8 * n + g, w.count - 1)];
-      s.x[n] = reinterpret_cast<const char*>(hidden + static_cast<size_t>(pair / L.K) * L.H + column);
+    for (int n = 0; n < NT; ++n)  // columns beyond the pass repeat its last token
+      at.token[n] = ws.group_pairs[w.first + min(8 * n + g, w.count - 1)];
+    return at;
+  };
+  auto point = [&](const ExactRows<NT>& at) {
+    ExactSource<NT> s;
+    const char* weights = reinterpret_cast<const char*>(
+        L.gate_up + static_cast<size_t>(at.e) * 2 * L.I * L.H + column);
+    const uint32_t row_bytes = 2 * L.H;
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      s.row[i] = weights + static_cast<uint64_t>(static_cast<uint32_t>(at.channel[i])) * row_bytes;
+      s.row[2 + i] = s.row[i] + up_bytes;
     }
+#pragma unroll
+    for (int n = 0; n < NT; ++n)
+      s.x[n] = reinterpret_cast<const char*>(hidden + column) +
+               static_cast<uint64_t>(static_cast<uint32_t>(at.token[n]) / static_cast<uint32_t>(L.K)) * row_bytes;
     return s;
   };
-  auto copy = [&](int slot, const ExactSource<NT>& s, int offset) {
-    const uint32_t to = mine + slot * X::kStepBytes;
-    copy_async16(to, s.a + offset);
-    copy_async16(to + 512, s.b + offset);
-    copy_async16(to + 1024, s.a + up_bytes + offset);
-    copy_async16(to + 1536, s.b + up_bytes + offset);
-#pragma unroll
-    for (int n = 0; n < NT; ++n) copy_async16(to + 512 * (4 + n), s.x[n] + offset);
+  // Step `step` from where the source's pointers stand, into place `slot` of the ring
+  // (zeros where the quarter has no such step).
+  auto copy = [&](auto slot, const ExactSource<NT>& s, auto step, bool there) {
+    const int bytes = there ? 16 : 0;
+    constexpr int kTo = decltype(slot)::value * X::kStepBytes, kFrom = 64 * decltype(step)::value;
+    repeat<4>([&](auto i) { copy_async16_at<kTo + 512 * decltype(i)::value, kFrom>(mine, s.row[i], bytes); });
+    repeat<NT>([&](auto n) { copy_async16_at<kTo + 512 * (4 + decltype(n)::value), kFrom>(mine, s.x[n], bytes); });
   };
 
   UnionWork work = read_work(index), next = read_work(index + stride);
-  ExactSource<NT> source = locate(work);
-#pragma unroll
-  for (int j = 0; j < kSlots - 1; ++j) {
-    if (j < steps) copy(j, source, 64 * j);
-    copy_async_commit();  // also when empty: the group count per step stays fixed
-  }
+  ExactRows<NT> rows = locate(work);
+  ExactSource<NT> source = point(rows);
+  repeat<kSlots - 1>([&](auto j) {
+    copy(j, source, j, j < steps);
+    copy_async_commit();
+  });
   for (;;) {
     const bool more = index + stride < work_count;
-    // What the end of the tile needs, and where the next one's rows are, on their way early.
+    // What the end of the tile needs, and where the next one's rows are, on their way early.  There
+    // this thread has row g or g + 8 and a token that another lane has located.
     const int at = work.tile * 16 + g + 8 * (warp >> 1);
     const bool finishes = at < work.rows;
-    const int channel =
-        finishes ? ws.union_channels[static_cast<size_t>(work.e) * L.I + at] : 0;
-    uint32_t bits[NT];
-    int pairs[NT], places[NT];  // where the kept channels of the candidate's word begin in its list
+    const int channel = warp < 2 ? rows.channel[0] : rows.channel[1];
+    int pairs[NT];
+    uint32_t bits[NT];     // the kept bits of the candidate's word
+    uint16_t before[NT];   // kept channels of the token before the word
 #pragma unroll
     for (int n = 0; n < NT; ++n) {
-      const int token = 8 * n + 2 * tq + (warp & 1);
-      bits[n] = 0;
-      pairs[n] = places[n] = 0;
-      if (finishes && token < work.count) {
-        pairs[n] = ws.group_pairs[work.first + token];
-        const int t = pairs[n] / L.K, candidate = (pairs[n] - t * L.K) * L.I + channel;
-        const size_t word = static_cast<size_t>(t) * token_words + (candidate >> 5);
-        const uint32_t kept = ws.kept_bits[word];
-        bits[n] = kept >> (candidate & 31);
-        places[n] = ws.kept_before[word] + __popc(kept & ((1u << (candidate & 31)) - 1));
-      }
+      pairs[n] = __shfl_sync(kFull, rows.token[n], 4 * (2 * tq + (warp & 1)));
+      const int t = pairs[n] / L.K, candidate = (pairs[n] - t * L.K) * L.I + channel;
+      const size_t word = static_cast<size_t>(t) * token_words + (candidate >> 5);
+      bits[n] = ws.kept_bits[word];
+      before[n] = ws.kept_before[word];
     }
-    ExactSource<NT> next_source = source;
-    if (more) next_source = locate(next);
+    ExactRows<NT> next_rows = {};
+    if (more) next_rows = locate(next);
     const UnionWork after = read_work(index + 2 * stride);
 
     float acc[NT][2][4];
@@ -291,41 +341,45 @@ __global__ void __launch_bounds__(ExactUnion<NT>::kThreads, ExactUnion<NT>::kPer
     for (int s = 0; s < padded; s += kSlots) {
       const bool last = s + kSlots >= padded;
       float part[NT][2][4];  // of this turn of the ring
-#pragma unroll
-      for (int j = 0; j < kSlots; ++j) {
-        copy_async_wait<kSlots - 2>();  // this lane's copies of step s + j have landed
-        const bool live = j == 0 || s + j < steps;
-        uint4 w[4], t[NT];
-        if (live) {
-          const uint32_t from = mine + j * X::kStepBytes;
-#pragma unroll
-          for (int i = 0; i < 4; ++i) w[i] = load_shared16(from + 512 * i);
-#pragma unroll
-          for (int n = 0; n < NT; ++n) t[n] = load_shared16(from + 512 * (4 + n));
-        }
+      // The last turn's copies, but for its first, are the next tile's: the pointers go on there.
+      repeat<kSlots>([&](auto turn) {
+        constexpr int j = decltype(turn)::value;
+        constexpr Index<(j + kSlots - 1) % kSlots> free{};
+        copy_async_wait<kSlots - 2>();
+        __syncwarp();  // every lane's copies of step s + j have landed; the step before has been read
+        uint32_t w[4][4], t[NT][4];
+        constexpr int kFrom = j * X::kStepBytes;
+        load_matrices_at<kFrom>(w[0], weights_at);
+        load_matrices_at<kFrom + 1024>(w[1], weights_at);
+        repeat<NT>([&](auto n) { load_matrices_at<kFrom + 512 * (4 + decltype(n)::value)>(t[n], tokens_at); });
+        load_matrices_at<kFrom>(w[2], weights_at2);
+        load_matrices_at<kFrom + 1024>(w[3], weights_at2);
         // Refill the place read one step ago.
-        if (j == 0) {
-          if (s + kSlots - 1 < steps) copy(kSlots - 1, source, 64 * (s + kSlots - 1));
-        } else if (!last) {
-          if (s + kSlots + j - 1 < steps) copy(j - 1, source, 64 * (s + kSlots + j - 1));
-        } else if (more && j - 1 < steps) {
-          copy(j - 1, next_source, 64 * (j - 1));
+        if (j == 1 && last && more) source = point(next_rows);
+        if (j == 0 || !last) {
+          copy(free, source, Index<kSlots + j - 1>{}, s + kSlots + j - 1 < steps);
+        } else if (more) {
+          copy(free, source, Index<(j > 0 ? j - 1 : 0)>{}, j - 1 < steps);
         }
         copy_async_commit();
-        if (live) {
 #pragma unroll
-          for (int n = 0; n < NT; ++n) {
-            if (j == 0) {
-              mma_bf16_first(part[n][0], w[0].x, w[1].x, w[0].y, w[1].y, t[n].x, t[n].y);
-              mma_bf16_first(part[n][1], w[2].x, w[3].x, w[2].y, w[3].y, t[n].x, t[n].y);
-            } else {
-              mma_bf16(part[n][0], w[0].x, w[1].x, w[0].y, w[1].y, t[n].x, t[n].y);
-              mma_bf16(part[n][1], w[2].x, w[3].x, w[2].y, w[3].y, t[n].x, t[n].y);
-            }
-            mma_bf16(part[n][0], w[0].z, w[1].z, w[0].w, w[1].w, t[n].z, t[n].w);
-            mma_bf16(part[n][1], w[2].z, w[3].z, w[2].w, w[3].w, t[n].z, t[n].w);
+        for (int n = 0; n < NT; ++n) {
+          if (j == 0) {
+            mma_bf16_first(part[n][0], w[0], t[n][0], t[n][1]);
+            mma_bf16_first(part[n][1], w[1], t[n][0], t[n][1]);
+          } else {
+            mma_bf16(part[n][0], w[0], t[n][0], t[n][1]);
+            mma_bf16(part[n][1], w[1], t[n][0], t[n][1]);
           }
+          mma_bf16(part[n][0], w[2], t[n][2], t[n][3]);
+          mma_bf16(part[n][1], w[3], t[n][2], t[n][3]);
         }
+      });
+      if (!last) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) source.row[i] += 64 * kSlots;
+#pragma unroll
+        for (int n = 0; n < NT; ++n) source.x[n] += 64 * kSlots;
       }
 #pragma unroll
       for (int n = 0; n < NT; ++n)
@@ -352,7 +406,8 @@ __global__ void __launch_bounds__(ExactUnion<NT>::kThreads, ExactUnion<NT>::kPer
       const int token = 8 * n + 2 * tq + (warp & 1);
       if (!finishes || token >= work.count) continue;
       __nv_bfloat16 feature = __float2bfloat16_rn(0.0f);
-      if (bits[n] & 1u) {
+      const int t = pairs[n] / L.K, bit = ((pairs[n] - t * L.K) * L.I + channel) & 31;
+      if ((bits[n] >> bit) & 1u) {
         float gate[4], up[4];
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
@@ -364,7 +419,8 @@ __global__ void __launch_bounds__(ExactUnion<NT>::kThreads, ExactUnion<NT>::kPer
         const float u_sum = (up[0] + up[1]) + (up[2] + up[3]);
         feature = __float2bfloat16_rn(exact_feature(g_sum, u_sum, L.activation));
         ws.activations[static_cast<size_t>(pairs[n]) * L.I + channel] = feature;
-        float* exact = ws.exact + static_cast<size_t>(pairs[n] / L.K) * 2 * L.F + places[n];
+        float* exact = ws.exact + static_cast<size_t>(t) * 2 * L.F + before[n] +
+                       __popc(bits[n] & ((1u << bit) - 1));
         exact[0] = g_sum;
         exact[L.F] = u_sum;
       }
@@ -375,7 +431,7 @@ __global__ void __launch_bounds__(ExactUnion<NT>::kThreads, ExactUnion<NT>::kPer
     index += stride;
     work = next;
     next = after;
-    source = next_source;
+    rows = next_rows;
   }
 }
 
@@ -423,6 +479,7 @@ __global__ void __launch_bounds__(DownUnion<NT>::kThreads, DownUnion<NT>::kPerSm
   const uint32_t ring = shared_u32(union_shared) + warp * (kSlots * X::kSlotBytes);
   const int copy_row = lane >> 3, copy_column = (lane & 7) * 8;
   const uint32_t copy_to = ring + ((copy_row >> 1) * 8 + (copy_row & 1)) * X::kRowBytes + (lane & 7) * 16;
+  const uint32_t values_at = ring + X::kUnitBytes + 8 * lane;
   int index = blockIdx.x * 4 + warp;
   if (index >= pieces) return;
 
@@ -435,26 +492,27 @@ __global__ void __launch_bounds__(DownUnion<NT>::kThreads, DownUnion<NT>::kPerSm
     if (encodes(i)) w.rows = L.I;
     return w;
   };
-  // Channels of union rows 32 `window` .. of the piece, one per lane.
-  auto channel_window = [&](const UnionWork& w, bool encoder, int window) -> int {
-    const int row = max(0, min(32 * window + lane, w.rows - 1));
-    return encoder ? row : ws.union_channels[static_cast<size_t>(w.e) * L.I + row];
+  // Channels of union rows 32 `window` .. of a piece, one per lane; any for rows beyond the last.
+  auto channel_window = [&](const UnionWork& w, bool encoder, int window) -> uint32_t {
+    const int row = 32 * window + lane;
+    if (encoder) return row;
+    return row < w.rows ? ws.union_channels[static_cast<size_t>(w.e) * L.I + row] : 0;
   };
 
   // ---- the copies, some units ahead of the sums ----
-  int ahead = index, unit = 0, units = 0, channels = 0, more_channels = 0;
+  int ahead = index, unit = 0, units = 0;
+  uint32_t channels = 0, more_channels = 0, row_bytes = 0;
   bool live = false, encoder = false;
-  size_t row_bytes = 0;
   const char* rows = nullptr;
   const __nv_bfloat16* values[NT];
   UnionWork source = read_work(ahead), source_next = read_work(ahead + stride);
   UnionWork source_after = read_work(ahead + 2 * stride);
-  int first_channels = channel_window(source, encodes(ahead), 0);
+  uint32_t first_channels = channel_window(source, encodes(ahead), 0);
   auto start_piece = [&]() {
     encoder = encodes(ahead);
     const int width = encoder ? L.R : L.H, column = block_of(ahead) * X::kColumns + copy_column;
     live = column < width;
-    row_bytes = static_cast<size_t>(width) * 2;
+    row_bytes = 2 * width;
     rows = reinterpret_cast<const char*>((encoder ? L.encoder : L.down) +
                                          static_cast<size_t>(source.e) * L.I * width + column);
 #pragma unroll
@@ -469,18 +527,20 @@ __global__ void __launch_bounds__(DownUnion<NT>::kThreads, DownUnion<NT>::kPerSm
     more_channels = units > 2 ? channel_window(source, encoder, 1) : 0;
     first_channels = ahead + stride < pieces ? channel_window(source_next, encodes(ahead + stride), 0) : 0;
   };
-  auto fetch = [&](int slot) {
+  uint32_t put = 0;  // where the next unit goes in the ring
+  auto fetch = [&]() {
     if (unit < units) {
-      const uint32_t to = copy_to + slot * X::kSlotBytes;
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const int channel = __shfl_sync(kFull, channels, 16 * (unit & 1) + copy_row + 4 * i);
-        if (live) copy_async16(to + 2 * i * X::kRowBytes, rows + channel * row_bytes);
-      }
-#pragma unroll
-      for (int n = 0; n < NT; ++n)
-        copy_async8(ring + slot * X::kSlotBytes + X::kUnitBytes + 256 * n + 8 * lane,
-                    values[n] + 16 * unit);
+      const uint32_t to = copy_to + put;
+      const int from = 16 * (unit & 1) + copy_row;
+      repeat<4>([&](auto i) {
+        const uint32_t channel = __shfl_sync(kFull, channels, from + 4 * i);
+        if (live)
+          copy_async16_at<2 * i * X::kRowBytes>(to, rows + static_cast<uint64_t>(channel) * row_bytes);
+      });
+      repeat<NT>([&](auto n) {
+        copy_async8_at<256 * n>(values_at + put, values[n]);
+        values[n] += 16;
+      });
       if (++unit == units) {
         ahead += stride;
         units = 0;
@@ -496,15 +556,16 @@ __global__ void __launch_bounds__(DownUnion<NT>::kThreads, DownUnion<NT>::kPerSm
       }
     }
     copy_async_commit();  // also when empty: the group count per step stays fixed
+    put = put == (kSlots - 1) * X::kSlotBytes ? 0 : put + X::kSlotBytes;
   };
   start_piece();
-#pragma unroll
-  for (int s = 0; s < kSlots - 1; ++s) fetch(s);
+#pragma unroll 1
+  for (int s = 0; s < kSlots - 1; ++s) fetch();
 
   // ---- the sums ----
   const int k = ((lane >> 4) << 3) + (lane & 7);  // the row whose address this lane gives to ldmatrix
   const uint32_t load_from = ring + k * X::kRowBytes + ((lane >> 3) & 1) * 16;
-  int slot = 0;
+  uint32_t get = 0;  // where the next unit lies in the ring
   UnionWork work = read_work(index);
   for (; index < pieces; index += stride) {
     const UnionWork next = read_work(index + stride);
@@ -528,11 +589,9 @@ __global__ void __launch_bounds__(DownUnion<NT>::kThreads, DownUnion<NT>::kPerSm
     for (int step = 0; step < steps; ++step) {
       copy_async_wait<kSlots - 2>();
       __syncwarp();  // every lane's copies of the unit have landed; the unit before is in registers
-      fetch(slot == 0 ? kSlots - 1 : slot - 1);
+      fetch();
       uint2 b[NT];
-#pragma unroll
-      for (int n = 0; n < NT; ++n)
-        b[n] = load_shared8(ring + slot * X::kSlotBytes + X::kUnitBytes + 256 * n + 8 * lane);
+      repeat<NT>([&](auto n) { b[n] = load_shared8_at<256 * n>(values_at + get); });
       const int left = work.rows - 16 * step;
       if (left < 16) {  // rows beyond the union weigh nothing
         const int mine = left - 4 * tq;
@@ -544,14 +603,13 @@ __global__ void __launch_bounds__(DownUnion<NT>::kThreads, DownUnion<NT>::kPerSm
           b[n].y &= y;
         }
       }
-#pragma unroll
-      for (int m = 0; m < 4; ++m) {
+      repeat<4>([&](auto m) {
         uint32_t a[4];
-        load_matrices_transposed(a, load_from + slot * X::kSlotBytes + 32 * m);
+        load_matrices_transposed_at<32 * m>(a, load_from + get);
 #pragma unroll
-        for (int n = 0; n < NT; ++n) mma_bf16(acc[n][m], a[0], a[1], a[2], a[3], b[n].x, b[n].y);
-      }
-      slot = slot + 1 == kSlots ? 0 : slot + 1;
+        for (int n = 0; n < NT; ++n) mma_bf16(acc[n][m], a, b[n].x, b[n].y);
+      });
+      get = get == (kSlots - 1) * X::kSlotBytes ? 0 : get + X::kSlotBytes;
     }
     // A token's sum over the expert, rounded to BF16 as the mix takes it.
     __nv_bfloat16* out = reinterpret_cast<__nv_bfloat16*>(is_encoder ? ws.encoder_parts : ws.down_parts);
