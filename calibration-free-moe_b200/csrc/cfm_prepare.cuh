@@ -6,6 +6,8 @@ constexpr int kPrepareThreads = 512;
 
 // Lengths of the work lists.
 constexpr int kPassCount = 0, kBusyCount = 1, kExactCount = 2, kDownCount = 3;
+// Pieces of the expert-major down kernel claimed so far.
+constexpr int kDownNext = 4;
 
 // Up to `pass` pairs of one expert, `first .. first + count - 1` of the grouped list.
 struct __align__(16) Pass {
@@ -261,7 +263,7 @@ __device__ __forceinline__ void group_pairs(const Layer& L, const Workspace& ws,
     ws.group_offsets[L.E] = static_cast<int>(base & 0xffffff);
     ws.work_counts[kPassCount] = static_cast<int>(base >> 44);
     ws.work_counts[kBusyCount] = static_cast<int>((base >> 24) & 0xfffff);
-    ws.work_counts[kExactCount] = ws.work_counts[kDownCount] = 0;
+    ws.work_counts[kExactCount] = ws.work_counts[kDownCount] = ws.work_counts[kDownNext] = 0;
   }
   __syncthreads();
   for (int p = tid; p < pairs; p += threads) {

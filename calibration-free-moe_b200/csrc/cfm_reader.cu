@@ -167,7 +167,7 @@ static int make_layout(const cfm_layer* l, int32_t capacity, cfm_workspace_layou
   o->features = take(2 * C * N);
   o->pass_work = take(16 * (C * K / 8 + std::min(E, C * K)));  // of at least eight pairs
   o->busy_experts = take(4 * E);
-  o->work_counts = take(16);
+  o->work_counts = take(32);
   o->tile_list = take(32 * C * ((F + kDownTileRows - 1) / kDownTileRows + K));
   o->tile_count = take(16);
   o->kept_bits = take(4 * C * kept_words(static_cast<int>(N)));
@@ -2114,15 +2114,13 @@ static bool down_by_union(const Bound& b) {
 static bool encodes_by_union(const Bound& b) {
   return down_by_union(b) && shares_decode(b) && encodes(b);
 }
-// Tokens per pass of the expert-major kernels, in eights: the next size up while the mean load is
-// more than two thirds of the one before.
-static int union_tiles(const Bound& b, int most) {
+// Tokens per pass of the expert-major exact kernel, in eights: the next size up while the mean load
+// is more than two thirds of the one before.
+static int exact_union_tiles(const Bound& b) {
   int tiles = 1;
-  while (tiles < most && 3 * static_cast<int64_t>(b.T) * b.L.K > 16 * tiles * static_cast<int64_t>(b.L.E)) tiles *= 2;
+  while (tiles < 4 && 3 * static_cast<int64_t>(b.T) * b.L.K > 16 * tiles * static_cast<int64_t>(b.L.E)) tiles *= 2;
   return tiles;
 }
-static int exact_union_tiles(const Bound& b) { return union_tiles(b, 4); }
-static int down_union_tiles(const Bound& b) { return union_tiles(b, 2); }
 
 // As many CTAs as run at a time, at most `work` of them.
 template <typename... Params, typename... Args>
@@ -2144,7 +2142,7 @@ static int run_exact_union(const Bound& b, const cfm_call* call, bool whole) {
   }
   const int tiles = exact_union_tiles(b);
   launch_dependent(k_union, dim3(busy_experts(b)), dim3(kUnionThreads), 0, b.stream, b.L, b.ws, 8 * tiles,
-                   8 * down_union_tiles(b), static_cast<int>(whole));
+                   DownUnion::kPass, static_cast<int>(whole));
   const int rc = launched();
   if (rc) return rc;
   const int64_t pairs = static_cast<int64_t>(b.T) * b.L.K;
@@ -2164,17 +2162,17 @@ static int run_exact_union(const Bound& b, const cfm_call* call, bool whole) {
   }
 }
 
-static int run_down_union(const Bound& b, bool encode) {
-  const int encoder_blocks = encode && encodes_by_union(b) ? (b.L.R + 63) / 64 : 0;
-  const int64_t passes = static_cast<int64_t>(b.T) * b.L.K / 8 + busy_experts(b);
-  const int64_t ctas = (passes * (b.L.H / 64 + encoder_blocks) + 3) / 4;
-  auto launch = [&](auto tile) {
-    using X = DownUnion<decltype(tile)::value>;
-    return launch_persistent(k_down_union<decltype(tile)::value>, ctas, X::kPerSm, X::kThreads, X::kSharedBytes,
-                             b.stream, b.L, b.ws, encoder_blocks);
-  };
-  return down_union_tiles(b) == 1 ? launch(std::integral_constant<int, 1>{})
-                                  : launch(std::integral_constant<int, 2>{});
+static int run_down_union(const Bound& b, bool encode, bool whole) {
+  using X = DownUnion;
+  if (!whole) {
+    const cudaError_t err = cudaMemsetAsync(b.ws.work_counts + kDownNext, 0, sizeof(int32_t), b.stream);
+    if (err != cudaSuccess) return static_cast<int>(err);
+  }
+  const int encoder_blocks = encode && encodes_by_union(b) ? (b.L.R + X::kColumns - 1) / X::kColumns : 0;
+  const int64_t passes = static_cast<int64_t>(b.T) * b.L.K / X::kPass + busy_experts(b);
+  return launch_persistent(k_down_union, (passes * (b.L.H / X::kColumns + encoder_blocks) + 3) / 4, X::kPerSm,
+                           X::kThreads, X::kSharedBytes, b.stream, b.L, b.ws, encoder_blocks,
+                           static_cast<uint32_t>((1ull << 32) / (b.L.H / X::kColumns) + 1));
 }
 
 // `whole`: part of a whole call; the down tiles are listed too where the down kernel needs them.
@@ -2229,10 +2227,10 @@ static int run_exact(const Bound& b, const cfm_call* call, bool whole) {
   return launched();
 }
 
-// `encode`: run the recovery encoder too.
-static int run_down(const Bound& b, bool encode) {
+// `encode`: run the recovery encoder too.  `whole`: part of a whole call.
+static int run_down(const Bound& b, bool encode, bool whole) {
   if (!b.L.down) return CFM_E_NULL;
-  if (down_by_union(b)) return run_down_union(b, encode);
+  if (down_by_union(b)) return run_down_union(b, encode, whole);
   // Tiles per token (T < 8) or of the call, at most; twice the expected share under expert
   // parallelism, walked in strides.
   const bool listed = pairs_grouped(b);
@@ -2293,10 +2291,11 @@ static int run_output(const Bound& b, const cfm_call* call, bool whole) {
   }
   // Tokens per CTA: enough CTAs for two per SM, and no more.
   const int early = whole && (!encodes(b) || encodes_by_union(b));
+  const int mixed = whole && encodes_by_union(b) ? kLatentsFromSums : latents ? kLatentsGiven : kLatentsNone;
   auto launch = [&](auto tokens) {
     constexpr int TOKENS = decltype(tokens)::value;
     launch_dependent(k_mix<TOKENS>, dim3(b.L.H / 128 + whole, (b.T + TOKENS - 1) / TOKENS), dim3(128), 0, b.stream,
-                     b.L, b.ws, b.padding, b.T, out, latents, early);
+                     b.L, b.ws, b.padding, b.T, out, mixed, early);
     return launched();
   };
   if (b.T <= 16) return launch(std::integral_constant<int, 1>{});
@@ -2380,7 +2379,7 @@ CFM_STAGE(cfm_select, {
 CFM_STAGE(cfm_score, return run_score(b);)
 CFM_STAGE(cfm_list_tiles, return run_list_tiles(b);)
 CFM_STAGE(cfm_exact, return run_exact(b, call, false);)
-CFM_STAGE(cfm_down, return run_down(b, false);)
+CFM_STAGE(cfm_down, return run_down(b, false, false);)
 CFM_STAGE(cfm_encode, return run_encode(b);)
 CFM_STAGE(cfm_output, return run_output(b, call, false);)
 
@@ -2521,7 +2520,7 @@ int cfm_reader_forward(const cfm_layer* layer, void* workspace, int32_t capacity
   if ((rc = run_screen(b))) return rc;
   if ((rc = run_select(b, 0, nullptr, false))) return rc;
   if ((rc = run_exact(b, call, true))) return rc;
-  if ((rc = run_down(b, encodes(b)))) return rc;
+  if ((rc = run_down(b, encodes(b), true))) return rc;
   if (down_by_union(b) && encodes(b) && !encodes_by_union(b) && (rc = run_encode(b))) return rc;
   return run_output(b, call, true);
 }

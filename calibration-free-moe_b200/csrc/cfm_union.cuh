@@ -438,59 +438,73 @@ __global__ void __launch_bounds__(ExactUnion<NT>::kThreads, ExactUnion<NT>::kPer
 // ---------------------------------------------------------------------------
 // down, and the recovery encoder
 // ---------------------------------------------------------------------------
-// D[column][token] = sum over union rows: sixteen rows and sixteen columns of weights are the
-// instruction's first operand, sixteen rows of NT x 8 tokens' activations (zero where a token did
-// not keep the row) the second.  A warp takes one piece of work on its own: 64 columns of one pass
-// over one expert, all the union's rows, sixteen (a unit) at a time through a ring of cp.async
-// copies that runs on into its next piece.  ldmatrix transposes the weights on their way to
-// registers; rows lie 144 bytes apart, which keeps its eight addresses in different banks.  Union
-// row 4 a + 2 b + i of a unit is the instruction's row 8 b + 2 a + i, so that a lane's four
-// activations are adjacent in memory.  Rows beyond the union repeat its last one and meet zeros.
+// D[token][column] = sum over union rows: sixteen tokens' activations (zero where a token did not
+// keep the row) of sixteen rows are the instruction's first operand, the rows' weights of eight
+// columns the second.  A warp takes one piece of work on its own: 64 columns of one pass over one
+// expert, all the union's rows, sixteen (a unit) at a time through a ring of cp.async copies that
+// runs on into its next piece.  The matrix loads transpose the weights on their way to registers;
+// rows lie 144 bytes apart, which keeps the eight of a matrix in different banks.  Union row
+// 4 a + 2 b + i of a unit is the instruction's row 8 b + 2 a + i, so that a lane's four activations
+// are adjacent in memory.  Rows beyond the union are another row's weights and meet zeros.
 // The recovery encoder is the same product with an expert's whole width as its rows and the sketch
-// features (zero for kept channels, k_select) as activations; its pieces come first, and the last
-// of a token's to arrive mixes its latent.  Bound by the weights' way from L2 and HBM to the SMs.
-template <int NT>
+// features (zero for kept channels, k_select) as activations; its pieces, the longest, come first.
+// Pieces differ in length with the unions and the number of passes, so warps claim them one at a
+// time (the next one while the current one's copies run).  MEASURED_DOWN
 struct DownUnion {
   static constexpr int kThreads = 128;
-  static constexpr int kPass = 8 * NT;
+  static constexpr int kPass = 16;
   static constexpr int kColumns = 64;
   static constexpr int kPerSm = 4;
-  static constexpr int kSlots = NT == 1 ? 5 : 4;
+  static constexpr int kSlots = 5;
   static constexpr int kRowBytes = 144;
   static constexpr int kUnitBytes = 16 * kRowBytes;
-  static constexpr int kSlotBytes = kUnitBytes + 256 * NT;
+  static constexpr int kSlotBytes = kUnitBytes + 512;
   static constexpr int kSharedBytes = 4 * kSlots * kSlotBytes;
 };
 
-
-// `encoder_blocks`: column blocks of the recovery encoder, or 0 without it.
-template <int NT>
-__global__ void __launch_bounds__(DownUnion<NT>::kThreads, DownUnion<NT>::kPerSm)
-    k_down_union(Layer L, Workspace ws, int encoder_blocks) {
-  using X = DownUnion<NT>;
+// `encoder_blocks`: column blocks of the recovery encoder, or 0 without it; `blocks_magic`:
+// floor(2^32 / (H / 64)) + 1, which divides piece numbers exactly.
+__global__ void __launch_bounds__(DownUnion::kThreads, DownUnion::kPerSm)
+    k_down_union(Layer L, Workspace ws, int encoder_blocks, uint32_t blocks_magic) {
+  using X = DownUnion;
   constexpr int kSlots = X::kSlots;
   extern __shared__ __align__(128) uint8_t union_shared[];
   grid_dependency_wait();     // the activations are complete
   grid_dependency_release();  // the output may be scheduled; it waits for this grid
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, tq = lane & 3;
-  const int passes = ws.work_counts[kDownCount], blocks = L.H / X::kColumns;
+  const int blocks = L.H / X::kColumns, passes = ws.work_counts[kDownCount];
   const int encoder_pieces = passes * encoder_blocks, pieces = encoder_pieces + passes * blocks;
-  const int stride = gridDim.x * 4;
   const uint32_t ring = shared_u32(union_shared) + warp * (kSlots * X::kSlotBytes);
   const int copy_row = lane >> 3, copy_column = (lane & 7) * 8;
   const uint32_t copy_to = ring + ((copy_row >> 1) * 8 + (copy_row & 1)) * X::kRowBytes + (lane & 7) * 16;
   const uint32_t values_at = ring + X::kUnitBytes + 8 * lane;
-  int index = blockIdx.x * 4 + warp;
-  if (index >= pieces) return;
+  int ahead = blockIdx.x * 4 + warp;
+  if (ahead >= pieces) return;
 
-  auto encodes = [&](int i) { return i < encoder_pieces; };
-  auto block_of = [&](int i) { return encodes(i) ? i % encoder_blocks : (i - encoder_pieces) % blocks; };
-  auto read_work = [&](int i) {
-    if (i >= pieces) return UnionWork{0, 0, 0, 0, 0};
-    UnionWork w = load_work(ws.down_work +
-                            (encodes(i) ? i / encoder_blocks : (i - encoder_pieces) / blocks));
-    if (encodes(i)) w.rows = L.I;
-    return w;
+  // ---- the copies, some units ahead of the sums ----
+  // Piece `ahead` is block `block` of `source`; the piece after it is claimed when this one's copies
+  // begin, its record read after two units and its first channels after four.
+  int claimed = 0, block = 0, next_block = 0, next_piece = 0, stage = 0, unit = 0, units = 0;
+  uint32_t channels = 0, more_channels = 0, first_channels = 0, row_bytes = 0;
+  bool live = false;
+  const char* rows = nullptr;
+  const __nv_bfloat16* values[2];
+  UnionWork source = {}, next = {};
+  // Lane i has what the sums need to know of pieces i, 32 + i, ... of this warp.
+  int piece_of = 0, first_of = 0, count_of = 0, rows_of = 0, started = 0;
+
+  auto read_piece = [&](int piece) {
+    int pass = piece;
+    next_piece = piece;
+    next_block = 0;  // blocks of the encoder come before those of the down rows
+    if (piece < encoder_pieces) {
+      for (; pass >= passes; pass -= passes) ++next_block;
+    } else {
+      const int at = piece - encoder_pieces;
+      pass = __umulhi(static_cast<uint32_t>(at), blocks_magic);
+      next_block = encoder_blocks + at - pass * blocks;
+    }
+    if (piece < pieces) next = load_work(ws.down_work + pass);
   };
   // Channels of union rows 32 `window` .. of a piece, one per lane; any for rows beyond the last.
   auto channel_window = [&](const UnionWork& w, bool encoder, int window) -> uint32_t {
@@ -498,34 +512,38 @@ __global__ void __launch_bounds__(DownUnion<NT>::kThreads, DownUnion<NT>::kPerSm
     if (encoder) return row;
     return row < w.rows ? ws.union_channels[static_cast<size_t>(w.e) * L.I + row] : 0;
   };
-
-  // ---- the copies, some units ahead of the sums ----
-  int ahead = index, unit = 0, units = 0;
-  uint32_t channels = 0, more_channels = 0, row_bytes = 0;
-  bool live = false, encoder = false;
-  const char* rows = nullptr;
-  const __nv_bfloat16* values[NT];
-  UnionWork source = read_work(ahead), source_next = read_work(ahead + stride);
-  UnionWork source_after = read_work(ahead + 2 * stride);
-  uint32_t first_channels = channel_window(source, encodes(ahead), 0);
   auto start_piece = [&]() {
-    encoder = encodes(ahead);
-    const int width = encoder ? L.R : L.H, column = block_of(ahead) * X::kColumns + copy_column;
+    ahead = next_piece;
+    block = next_block;
+    source = next;
+    const bool encoder = block < encoder_blocks;
+    if (encoder) source.rows = L.I;
+    if (lane == (started & 31)) {
+      piece_of = ahead < pieces ? block : -1;
+      first_of = source.first;
+      count_of = source.count;
+      rows_of = source.rows;
+    }
+    ++started;
+    unit = units = 0;
+    if (ahead >= pieces) return;
+    if (lane == 0) claimed = atomicAdd(ws.work_counts + kDownNext, 1) + gridDim.x * 4;
+    stage = 0;
+    const int width = encoder ? L.R : L.H;
+    const int column = (encoder ? block : block - encoder_blocks) * X::kColumns + copy_column;
     live = column < width;
     row_bytes = 2 * width;
     rows = reinterpret_cast<const char*>((encoder ? L.encoder : L.down) +
                                          static_cast<size_t>(source.e) * L.I * width + column);
 #pragma unroll
-    for (int n = 0; n < NT; ++n) {  // columns beyond the pass repeat its last token
+    for (int n = 0; n < 2; ++n) {  // tokens beyond the pass repeat its last one
       const int at = source.first + min(8 * n + g, source.count - 1);
       values[n] = (encoder ? ws.features + static_cast<size_t>(ws.group_pairs[at]) * L.I
                            : ws.union_activations + static_cast<size_t>(at) * L.I) + 4 * tq;
     }
-    unit = 0;
     units = max(1, (source.rows + 15) / 16);
     channels = first_channels;
     more_channels = units > 2 ? channel_window(source, encoder, 1) : 0;
-    first_channels = ahead + stride < pieces ? channel_window(source_next, encodes(ahead + stride), 0) : 0;
   };
   uint32_t put = 0;  // where the next unit goes in the ring
   auto fetch = [&]() {
@@ -533,130 +551,101 @@ __global__ void __launch_bounds__(DownUnion<NT>::kThreads, DownUnion<NT>::kPerSm
       const uint32_t to = copy_to + put;
       const int from = 16 * (unit & 1) + copy_row;
       repeat<4>([&](auto i) {
-        const uint32_t channel = __shfl_sync(kFull, channels, from + 4 * i);
+        constexpr int kRow = decltype(i)::value;
+        const uint32_t channel = __shfl_sync(kFull, channels, from + 4 * kRow);
         if (live)
-          copy_async16_at<2 * i * X::kRowBytes>(to, rows + static_cast<uint64_t>(channel) * row_bytes);
+          copy_async16_at<2 * kRow * X::kRowBytes>(to, rows + static_cast<uint64_t>(channel) * row_bytes);
       });
-      repeat<NT>([&](auto n) {
-        copy_async8_at<256 * n>(values_at + put, values[n]);
-        values[n] += 16;
-      });
-      if (++unit == units) {
-        ahead += stride;
-        units = 0;
-        if (ahead < pieces) {
-          source = source_next;
-          source_next = source_after;
-          source_after = read_work(ahead + 2 * stride);
-          start_piece();
-        }
+      copy_async8_at<0>(values_at + put, values[0]);
+      copy_async8_at<256>(values_at + put, values[1]);
+      values[0] += 16;
+      values[1] += 16;
+      ++unit;
+      const bool done = unit == units;
+      if (stage == 0 && (done || unit == 2)) {
+        read_piece(__shfl_sync(kFull, claimed, 0));
+        stage = 1;
+      }
+      if (stage == 1 && (done || unit == 4)) {
+        if (next_piece < pieces) first_channels = channel_window(next, next_block < encoder_blocks, 0);
+        stage = 2;
+      }
+      if (done) {
+        start_piece();
       } else if ((unit & 1) == 0) {
         channels = more_channels;
-        if (unit + 2 < units) more_channels = channel_window(source, encoder, unit / 2 + 1);
+        if (unit + 2 < units) more_channels = channel_window(source, block < encoder_blocks, unit / 2 + 1);
       }
     }
     copy_async_commit();  // also when empty: the group count per step stays fixed
     put = put == (kSlots - 1) * X::kSlotBytes ? 0 : put + X::kSlotBytes;
   };
+  read_piece(ahead);
+  first_channels = channel_window(next, next_block < encoder_blocks, 0);
   start_piece();
 #pragma unroll 1
   for (int s = 0; s < kSlots - 1; ++s) fetch();
 
   // ---- the sums ----
-  const int k = ((lane >> 4) << 3) + (lane & 7);  // the row whose address this lane gives to ldmatrix
-  const uint32_t load_from = ring + k * X::kRowBytes + ((lane >> 3) & 1) * 16;
+  // The row whose address this lane gives to the matrix loads: rows 0 to 7 and 8 to 15 of eight
+  // columns, then of the next eight.
+  const uint32_t load_from = ring + (((lane >> 3) & 1) * 8 + (lane & 7)) * X::kRowBytes + (lane >> 4) * 16;
   uint32_t get = 0;  // where the next unit lies in the ring
-  UnionWork work = read_work(index);
-  for (; index < pieces; index += stride) {
-    const UnionWork next = read_work(index + stride);
-    const bool is_encoder = encodes(index);
-    const int steps = max(1, (work.rows + 15) / 16);
-    int pairs[NT][2];
+  for (int done = 0;; ++done) {
+    const int piece = __shfl_sync(kFull, piece_of, done & 31);
+    if (piece < 0) break;
+    const int first = __shfl_sync(kFull, first_of, done & 31), count = __shfl_sync(kFull, count_of, done & 31);
+    int left = __shfl_sync(kFull, rows_of, done & 31);
+    int pairs[2];
 #pragma unroll
-    for (int n = 0; n < NT; ++n)
+    for (int n = 0; n < 2; ++n) pairs[n] = 8 * n + g < count ? ws.group_pairs[first + 8 * n + g] : -1;
+    float acc[8][4];
 #pragma unroll
-      for (int i = 0; i < 2; ++i) {
-        const int token = 8 * n + 2 * tq + i;
-        pairs[n][i] = token < work.count ? ws.group_pairs[work.first + token] : -1;
-      }
-    float acc[NT][4][4];
+    for (int n = 0; n < 8; ++n)
 #pragma unroll
-    for (int n = 0; n < NT; ++n)
-#pragma unroll
-      for (int m = 0; m < 4; ++m)
-#pragma unroll
-        for (int i = 0; i < 4; ++i) acc[n][m][i] = 0.0f;
-    for (int step = 0; step < steps; ++step) {
+      for (int i = 0; i < 4; ++i) acc[n][i] = 0.0f;
+    do {
       copy_async_wait<kSlots - 2>();
-      __syncwarp();  // every lane's copies of the unit have landed; the unit before is in registers
+      __syncwarp();  // every lane's copies of the unit have landed; the unit before has been read
       fetch();
-      uint2 b[NT];
-      repeat<NT>([&](auto n) { b[n] = load_shared8_at<256 * n>(values_at + get); });
-      const int left = work.rows - 16 * step;
+      uint2 v[2];
+      v[0] = load_shared8_at<0>(values_at + get);
+      v[1] = load_shared8_at<256>(values_at + get);
       if (left < 16) {  // rows beyond the union weigh nothing
         const int mine = left - 4 * tq;
         const uint32_t x = mine > 1 ? ~0u : mine > 0 ? 0xffffu : 0u;
         const uint32_t y = mine > 3 ? ~0u : mine > 2 ? 0xffffu : 0u;
 #pragma unroll
-        for (int n = 0; n < NT; ++n) {
-          b[n].x &= x;
-          b[n].y &= y;
+        for (int n = 0; n < 2; ++n) {
+          v[n].x &= x;
+          v[n].y &= y;
         }
       }
+      const uint32_t a[4] = {v[0].x, v[1].x, v[0].y, v[1].y};
       repeat<4>([&](auto m) {
-        uint32_t a[4];
-        load_matrices_transposed_at<32 * m>(a, load_from + get);
-#pragma unroll
-        for (int n = 0; n < NT; ++n) mma_bf16(acc[n][m], a, b[n].x, b[n].y);
+        constexpr int kPart = decltype(m)::value;
+        uint32_t w[4];
+        load_matrices_transposed_at<32 * kPart>(w, load_from + get);
+        mma_bf16(acc[2 * kPart], a, w[0], w[1]);
+        mma_bf16(acc[2 * kPart + 1], a, w[2], w[3]);
       });
       get = get == (kSlots - 1) * X::kSlotBytes ? 0 : get + X::kSlotBytes;
-    }
+      left -= 16;
+    } while (left > 0);
     // A token's sum over the expert, rounded to BF16 as the mix takes it.
-    __nv_bfloat16* out = reinterpret_cast<__nv_bfloat16*>(is_encoder ? ws.encoder_parts : ws.down_parts);
-    const int width = is_encoder ? L.R : L.H, column = block_of(index) * X::kColumns + g;
+    const bool encoder = piece < encoder_blocks;
+    const int width = encoder ? L.R : L.H;
+    const int column = (encoder ? piece : piece - encoder_blocks) * X::kColumns;
+    __nv_bfloat16* out = reinterpret_cast<__nv_bfloat16*>(encoder ? ws.encoder_parts : ws.down_parts) + column + 2 * tq;
 #pragma unroll
-    for (int n = 0; n < NT; ++n)
+    for (int n = 0; n < 2; ++n) {
+      if (pairs[n] < 0) continue;
+      __nv_bfloat16* row = out + static_cast<size_t>(pairs[n]) * width;
 #pragma unroll
-      for (int i = 0; i < 2; ++i) {
-        if (pairs[n][i] < 0) continue;
-        __nv_bfloat16* row = out + static_cast<size_t>(pairs[n][i]) * width;
-#pragma unroll
-        for (int m = 0; m < 4; ++m) {
-          const int c = column + 16 * m;
-          if (c < width) row[c] = __float2bfloat16_rn(acc[n][m][i]);
-          if (c + 8 < width) row[c + 8] = __float2bfloat16_rn(acc[n][m][2 + i]);
-        }
-      }
-    if (is_encoder) {
-      __threadfence();
-      __syncwarp();
-      bool last = false;
-      int t = 0;
-      if (lane < work.count) {
-        t = ws.group_pairs[work.first + lane] / L.K;
-        int local = 0;
-        for (int s = 0; s < L.K; ++s) local += ws.ids[static_cast<size_t>(t) * L.K + s] >= 0;
-        uint32_t* counter = ws.counters + 2 * static_cast<size_t>(ws.capacity) * L.K + t;
-        last = atomicAdd(counter, 1u) == static_cast<unsigned>(local * encoder_blocks - 1);
-        if (last) *counter = 0;
-      }
-      unsigned finished = __ballot_sync(kFull, last);
-      if (finished) __threadfence();
-      for (; finished; finished &= finished - 1) {
-        const size_t pair0 = static_cast<size_t>(__shfl_sync(kFull, t, __ffs(finished) - 1)) * L.K;
-        const unsigned short* parts = reinterpret_cast<const unsigned short*>(ws.encoder_parts) + pair0 * L.R;
-        for (int r = lane; r < L.R; r += 32) {
-          float latent = 0.0f;
-#pragma unroll 8
-          for (int s = 0; s < L.K; ++s)
-            if (ws.ids[pair0 + s] >= 0)
-              latent = fmaf(__bfloat162float(__ushort_as_bfloat16(__ldcg(parts + static_cast<size_t>(s) * L.R + r))),
-                            ws.weights[pair0 + s], latent);
-          ws.latent[pair0 / L.K * L.R + r] = latent;
-        }
-      }
+      for (int c = 0; c < 8; ++c)
+        if (column + 8 * c < width)
+          *reinterpret_cast<__nv_bfloat162*>(row + 8 * c) = __floats2bfloat162_rn(acc[c][2 * n], acc[c][2 * n + 1]);
     }
-    work = next;
   }
 }
 
@@ -682,6 +671,9 @@ __device__ __forceinline__ float mix_sums(const Layer& L, const Workspace& ws, i
 // output column of TOKENS tokens per thread.  The decoder row is read once for them; their dot
 // products with it run side by side, each in the order k_output takes, and their expert sums are on
 // their way meanwhile.  Bound by latency (and by instructions from some 128 tokens on).
+// `latents`: none, the workspace's, or to be mixed here from the encoder's sums.
+constexpr int kLatentsNone = 0, kLatentsGiven = 1, kLatentsFromSums = 2;
+
 template <int TOKENS>
 __global__ void __launch_bounds__(128) k_mix(Layer L, Workspace ws, const uint8_t* padding, int tokens,
                                              __nv_bfloat16* out, int latents, int early) {
@@ -730,12 +722,47 @@ __global__ void __launch_bounds__(128) k_mix(Layer L, Workspace ws, const uint8_
     for (int s = 0; s < kSums; ++s)
       sums[j][s] = s < L.K && j < count ? __ldcg(from + static_cast<size_t>(j * L.K + s) * L.H) : 0;
   if (L.R > 0) {
-    for (int i = tid; i < count * L.R; i += 128) {
-      const int j = i / L.R, r = i - j * L.R;
-      float* kept = ws.latent + static_cast<size_t>(t0 + j) * L.R + r;
-      const bool given = latents && valid[j];
-      if (!given && blockIdx.x == 0) *kept = 0.0f;
-      latent[j][r] = given ? bf16_round(*kept) : 0.0f;
+    if (latents == kLatentsFromSums) {
+      // A thread mixes eight columns of a token's latent from the encoder's sums of its slots.
+      const int pieces = L.R / 8;
+      for (int i = tid; i < count * pieces; i += 128) {
+        const int j = i / pieces, r = 8 * (i - j * pieces);
+        const uint4* from = reinterpret_cast<const uint4*>(
+            reinterpret_cast<const __nv_bfloat16*>(ws.encoder_parts) + static_cast<size_t>(t0 + j) * L.K * L.R + r);
+        float z[8] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
+        for (int s0 = 0; s0 < L.K; s0 += kSums) {
+          uint4 part[kSums];
+#pragma unroll
+          for (int s = 0; s < kSums; ++s)
+            part[s] = s0 + s < L.K ? __ldcg(from + (s0 + s) * pieces) : make_uint4(0, 0, 0, 0);
+#pragma unroll
+          for (int s = 0; s < kSums; ++s) {
+            if (!((valid[j] >> (s0 + s)) & 1u)) continue;
+            const float w = weight[j][s0 + s];
+            z[0] = fmaf(bf16_lo(part[s].x), w, z[0]);
+            z[1] = fmaf(bf16_hi(part[s].x), w, z[1]);
+            z[2] = fmaf(bf16_lo(part[s].y), w, z[2]);
+            z[3] = fmaf(bf16_hi(part[s].y), w, z[3]);
+            z[4] = fmaf(bf16_lo(part[s].z), w, z[4]);
+            z[5] = fmaf(bf16_hi(part[s].z), w, z[5]);
+            z[6] = fmaf(bf16_lo(part[s].w), w, z[6]);
+            z[7] = fmaf(bf16_hi(part[s].w), w, z[7]);
+          }
+        }
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+          latent[j][r + k] = bf16_round(z[k]);
+          if (blockIdx.x == 0) ws.latent[static_cast<size_t>(t0 + j) * L.R + r + k] = z[k];
+        }
+      }
+    } else {
+      for (int i = tid; i < count * L.R; i += 128) {
+        const int j = i / L.R, r = i - j * L.R;
+        float* kept = ws.latent + static_cast<size_t>(t0 + j) * L.R + r;
+        const bool given = latents == kLatentsGiven && valid[j];
+        if (!given && blockIdx.x == 0) *kept = 0.0f;
+        latent[j][r] = given ? bf16_round(*kept) : 0.0f;
+      }
     }
     __syncthreads();
   }

@@ -154,7 +154,7 @@ class ReaderWorkspace:
             "status": (4,), "limbs": (c, blocks, 3, 128),
             "group_offsets": (self.experts + 1,), "group_pairs": (c * k,), "cuts": (c, k + 1),
             "variances": (c, 2, n), "features": (c, n),
-            "busy_experts": (self.experts,), "work_counts": (4,),
+            "busy_experts": (self.experts,), "work_counts": (8,),
             "tile_list": (c * (-(-f // 64) + k), 8), "tile_count": (4,),
         }
         for name, shape in shapes.items():

@@ -164,7 +164,7 @@ typedef struct cfm_workspace_layout {
   int64_t features;       /* bf16 [C, N] phi(g) u of the sketch projections     */
   int64_t pass_work;      /* i32 [.., 4] passes of the screen over the experts   */
   int64_t busy_experts;   /* i32 [E] experts some pair is routed to, ascending  */
-  int64_t work_counts;    /* i32 [4] passes, busy experts, lengths of the two work lists */
+  int64_t work_counts;    /* i32 [8] passes, busy experts, lengths of the two work lists, claims */
   int64_t tile_list;      /* i32 [C * (ceil(F / 64) + K), 8] down tiles in expert order */
   int64_t tile_count;     /* i32 [4] number of listed tiles                        */
   int64_t kept_bits;      /* u32 [C, ceil(N / 32) + 1] kept candidates as bits     */
