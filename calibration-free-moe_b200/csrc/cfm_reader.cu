@@ -2289,19 +2289,11 @@ static int run_output(const Bound& b, const cfm_call* call, bool whole) {
                      out, latents, static_cast<int>(whole));
     return launched();
   }
-  // Tokens per CTA: enough CTAs for two per SM, and no more.
   const int early = whole && (!encodes(b) || encodes_by_union(b));
   const int mixed = whole && encodes_by_union(b) ? kLatentsFromSums : latents ? kLatentsGiven : kLatentsNone;
-  auto launch = [&](auto tokens) {
-    constexpr int TOKENS = decltype(tokens)::value;
-    launch_dependent(k_mix<TOKENS>, dim3(b.L.H / 128 + whole, (b.T + TOKENS - 1) / TOKENS), dim3(128), 0, b.stream,
-                     b.L, b.ws, b.padding, b.T, out, mixed, early);
-    return launched();
-  };
-  if (b.T <= 16) return launch(std::integral_constant<int, 1>{});
-  if (b.T <= 64) return launch(std::integral_constant<int, 2>{});
-  if (b.T <= 128) return launch(std::integral_constant<int, 4>{});
-  return launch(std::integral_constant<int, 8>{});
+  launch_dependent(k_mix, dim3(b.L.H / 128 + whole, (b.T + kMixTokens - 1) / kMixTokens), dim3(128), 0, b.stream,
+                   b.L, b.ws, b.padding, b.T, out, mixed, early);
+  return launched();
 }
 
 // Checks an exchange description against the layer and the call (`rows` = tokens

@@ -667,21 +667,47 @@ __device__ __forceinline__ float mix_sums(const Layer& L, const Workspace& ws, i
   return routed;
 }
 
-// grid (H / 128, or one more for the tokens' read-cost counters; ceil(T / TOKENS)), 128 threads, one
-// output column of TOKENS tokens per thread.  The decoder row is read once for them; their dot
-// products with it run side by side, each in the order k_output takes, and their expert sums are on
-// their way meanwhile.  Bound by latency (and by instructions from some 128 tokens on).
+// grid (H / 128, or one more for the tokens' read-cost counters; ceil(T / 16)), 128 threads: sixteen
+// tokens, 32 output columns per warp.  The decoder term is a product of the tokens' latents (BF16)
+// with decoder rows, done by the tensor cores; a sum leaves them after 32 columns of the latent and
+// goes on by ordinary additions.  Columns are dealt to the instruction so that a thread ends up with
+// eight adjacent ones of two tokens, and the order inside sixteen latent columns so that it loads
+// eight adjacent ones of a decoder row.  The expert sums of the first slots are on their way
+// meanwhile.  Bound by latency.  (One column of up to eight tokens per thread, dot products by FMAs:
+// MEASURED_MIX)
 // `latents`: none, the workspace's, or to be mixed here from the encoder's sums.
 constexpr int kLatentsNone = 0, kLatentsGiven = 1, kLatentsFromSums = 2;
+constexpr int kMixTokens = 16;
 
-template <int TOKENS>
-__global__ void __launch_bounds__(128) k_mix(Layer L, Workspace ws, const uint8_t* padding, int tokens,
-                                             __nv_bfloat16* out, int latents, int early) {
-  __shared__ __align__(16) float latent[TOKENS][256];
-  __shared__ float weight[TOKENS][32];
-  __shared__ uint32_t valid[TOKENS];
-  const int t0 = blockIdx.y * TOKENS, count = min(TOKENS, tokens - t0);
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, h = blockIdx.x * 128 + tid;
+// z += w * (the eight BF16 values of v).
+__device__ __forceinline__ void add_scaled8(float (&z)[8], const uint4& v, float w) {
+  z[0] = fmaf(bf16_lo(v.x), w, z[0]);
+  z[1] = fmaf(bf16_hi(v.x), w, z[1]);
+  z[2] = fmaf(bf16_lo(v.y), w, z[2]);
+  z[3] = fmaf(bf16_hi(v.y), w, z[3]);
+  z[4] = fmaf(bf16_lo(v.z), w, z[4]);
+  z[5] = fmaf(bf16_hi(v.z), w, z[5]);
+  z[6] = fmaf(bf16_lo(v.w), w, z[6]);
+  z[7] = fmaf(bf16_hi(v.w), w, z[7]);
+}
+__device__ __forceinline__ uint4 pack_bf16x8(const float (&z)[8]) {
+  uint4 v;
+  uint32_t* out = reinterpret_cast<uint32_t*>(&v);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const __nv_bfloat162 two = __floats2bfloat162_rn(z[2 * i], z[2 * i + 1]);
+    out[i] = *reinterpret_cast<const uint32_t*>(&two);
+  }
+  return v;
+}
+
+__global__ void __launch_bounds__(128, 3) k_mix(Layer L, Workspace ws, const uint8_t* padding, int tokens,
+                                                __nv_bfloat16* out, int latents, int early) {
+  __shared__ __align__(16) __nv_bfloat16 latent[kMixTokens][256 + 32];
+  __shared__ float weight[kMixTokens][32];
+  __shared__ uint32_t valid[kMixTokens];  // the slots that have sums
+  const int t0 = blockIdx.y * kMixTokens, count = min(kMixTokens, tokens - t0);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, tq = lane & 3;
   if (!early) grid_dependency_wait();
   if (static_cast<int>(blockIdx.x) * 128 >= L.H) {  // the read-cost counters
     for (int j = warp; j < count; j += 4) {
@@ -693,14 +719,21 @@ __global__ void __launch_bounds__(128) k_mix(Layer L, Workspace ws, const uint8_
     }
     return;
   }
+  const int pieces = L.R / 8;  // of a latent
   const bool recover = L.R > 0 && L.owner && L.decoder;
-  constexpr int kAhead = 8;
-  const int chunks = recover ? L.R / 8 : 0;
-  const uint4* decoder_row = reinterpret_cast<const uint4*>(L.decoder + static_cast<size_t>(h) * L.R);
-  uint4 decoder[kAhead];
+  // The instruction's column g of tile n is this warp's column 8 (g / 2) + 2 n + g % 2; a decoder
+  // row is loaded 64 columns ahead.
+  const uint4* rows = reinterpret_cast<const uint4*>(
+      L.decoder + static_cast<size_t>(blockIdx.x * 128 + 32 * warp + 8 * (g >> 1) + (g & 1)) * L.R);
+  uint4 decoder[2][4];
+  auto load_decoder = [&](uint4 (&d)[4], int k) {
 #pragma unroll
-  for (int i = 0; i < kAhead; ++i) decoder[i] = i < chunks ? decoder_row[i] : make_uint4(0, 0, 0, 0);
-  for (int j = warp; j < TOKENS; j += 4) {  // the slots that have sums, and their weights
+    for (int n = 0; n < 4; ++n)
+      d[n] = recover && k + tq < pieces ? rows[2 * n * pieces + k + tq] : make_uint4(0, 0, 0, 0);
+  };
+  load_decoder(decoder[0], 0);
+  load_decoder(decoder[1], 4);
+  for (int j = warp; j < kMixTokens; j += 4) {
     bool here = false;
     if (j < count && lane < L.K) {
       const size_t pair = static_cast<size_t>(t0 + j) * L.K + lane;
@@ -712,102 +745,104 @@ __global__ void __launch_bounds__(128) k_mix(Layer L, Workspace ws, const uint8_
   }
   if (early) grid_dependency_wait();
   __syncthreads();
-  constexpr int kSums = 8;  // of each token on their way at a time
-  unsigned short sums[TOKENS][kSums];
-  const unsigned short* from = reinterpret_cast<const unsigned short*>(ws.down_parts) +
-                               static_cast<size_t>(t0) * L.K * L.H + h;
+  // This thread's columns h .. h + 7 of tokens g and g + 8.
+  const int h = blockIdx.x * 128 + 32 * warp + 8 * tq;
+  constexpr int kSums = 8;  // slots on their way at a time
+  uint4 sums[2][kSums];
+  const uint4* from[2];
 #pragma unroll
-  for (int j = 0; j < TOKENS; ++j)
+  for (int i = 0; i < 2; ++i) {
+    from[i] = reinterpret_cast<const uint4*>(reinterpret_cast<const __nv_bfloat16*>(ws.down_parts) +
+                                             static_cast<size_t>(t0 + min(8 * i + g, count - 1)) * L.K * L.H + h);
 #pragma unroll
     for (int s = 0; s < kSums; ++s)
-      sums[j][s] = s < L.K && j < count ? __ldcg(from + static_cast<size_t>(j * L.K + s) * L.H) : 0;
+      sums[i][s] = s < L.K ? __ldcg(from[i] + static_cast<size_t>(s) * (L.H / 8)) : make_uint4(0, 0, 0, 0);
+  }
   if (L.R > 0) {
-    if (latents == kLatentsFromSums) {
-      // A thread mixes eight columns of a token's latent from the encoder's sums of its slots.
-      const int pieces = L.R / 8;
-      for (int i = tid; i < count * pieces; i += 128) {
-        const int j = i / pieces, r = 8 * (i - j * pieces);
-        const uint4* from = reinterpret_cast<const uint4*>(
-            reinterpret_cast<const __nv_bfloat16*>(ws.encoder_parts) + static_cast<size_t>(t0 + j) * L.K * L.R + r);
-        float z[8] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
+    const int padded = (pieces + 3) & ~3;
+    for (int i = tid; i < kMixTokens * padded; i += 128) {
+      const int j = i / padded, piece = i - j * padded;
+      const bool live = j < count && piece < pieces;
+      float z[8] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
+      const size_t at = static_cast<size_t>(t0 + j) * L.R + 8 * piece;
+      if (live && valid[j] && latents == kLatentsFromSums) {
+        const uint4* parts = reinterpret_cast<const uint4*>(ws.encoder_parts) +
+                             static_cast<size_t>(t0 + j) * L.K * pieces + piece;
         for (int s0 = 0; s0 < L.K; s0 += kSums) {
           uint4 part[kSums];
 #pragma unroll
           for (int s = 0; s < kSums; ++s)
-            part[s] = s0 + s < L.K ? __ldcg(from + (s0 + s) * pieces) : make_uint4(0, 0, 0, 0);
+            part[s] = s0 + s < L.K ? __ldcg(parts + (s0 + s) * pieces) : make_uint4(0, 0, 0, 0);
 #pragma unroll
-          for (int s = 0; s < kSums; ++s) {
-            if (!((valid[j] >> (s0 + s)) & 1u)) continue;
-            const float w = weight[j][s0 + s];
-            z[0] = fmaf(bf16_lo(part[s].x), w, z[0]);
-            z[1] = fmaf(bf16_hi(part[s].x), w, z[1]);
-            z[2] = fmaf(bf16_lo(part[s].y), w, z[2]);
-            z[3] = fmaf(bf16_hi(part[s].y), w, z[3]);
-            z[4] = fmaf(bf16_lo(part[s].z), w, z[4]);
-            z[5] = fmaf(bf16_hi(part[s].z), w, z[5]);
-            z[6] = fmaf(bf16_lo(part[s].w), w, z[6]);
-            z[7] = fmaf(bf16_hi(part[s].w), w, z[7]);
-          }
+          for (int s = 0; s < kSums; ++s)
+            if ((valid[j] >> (s0 + s)) & 1u) add_scaled8(z, part[s], weight[j][s0 + s]);
         }
+      } else if (live && valid[j] && latents == kLatentsGiven) {
 #pragma unroll
-        for (int k = 0; k < 8; ++k) {
-          latent[j][r + k] = bf16_round(z[k]);
-          if (blockIdx.x == 0) ws.latent[static_cast<size_t>(t0 + j) * L.R + r + k] = z[k];
-        }
+        for (int k = 0; k < 8; ++k) z[k] = ws.latent[at + k];
       }
-    } else {
-      for (int i = tid; i < count * L.R; i += 128) {
-        const int j = i / L.R, r = i - j * L.R;
-        float* kept = ws.latent + static_cast<size_t>(t0 + j) * L.R + r;
-        const bool given = latents == kLatentsGiven && valid[j];
-        if (!given && blockIdx.x == 0) *kept = 0.0f;
-        latent[j][r] = given ? bf16_round(*kept) : 0.0f;
+      *reinterpret_cast<uint4*>(&latent[j][8 * piece]) = pack_bf16x8(z);
+      if (live && blockIdx.x == 0) {
+#pragma unroll
+        for (int k = 0; k < 8; ++k) ws.latent[at + k] = z[k];
       }
     }
     __syncthreads();
   }
-  float dot[TOKENS];
+  float dot[4][4];  // [n][token g, g + 8][columns 2 n, 2 n + 1 of this thread's eight]
 #pragma unroll
-  for (int j = 0; j < TOKENS; ++j) dot[j] = 0.0f;
-  auto fold = [&](const uint4& w, int i) {
+  for (int n = 0; n < 4; ++n)
 #pragma unroll
-    for (int j = 0; j < TOKENS; ++j) {
-      const float4 a = *reinterpret_cast<const float4*>(&latent[j][8 * i]);
-      const float4 b = *reinterpret_cast<const float4*>(&latent[j][8 * i + 4]);
-      dot[j] = fmaf(bf16_lo(w.x), a.x, dot[j]);
-      dot[j] = fmaf(bf16_hi(w.x), a.y, dot[j]);
-      dot[j] = fmaf(bf16_lo(w.y), a.z, dot[j]);
-      dot[j] = fmaf(bf16_hi(w.y), a.w, dot[j]);
-      dot[j] = fmaf(bf16_lo(w.z), b.x, dot[j]);
-      dot[j] = fmaf(bf16_hi(w.z), b.y, dot[j]);
-      dot[j] = fmaf(bf16_lo(w.w), b.z, dot[j]);
-      dot[j] = fmaf(bf16_hi(w.w), b.w, dot[j]);
+    for (int i = 0; i < 4; ++i) dot[n][i] = 0.0f;
+  if (recover) {
+    auto fold = [&](const uint4 (&d)[4], int k) {
+      const uint4 lo = *reinterpret_cast<const uint4*>(&latent[g][8 * (k + tq)]);
+      const uint4 hi = *reinterpret_cast<const uint4*>(&latent[g + 8][8 * (k + tq)]);
+      const uint32_t a[2][4] = {{lo.x, hi.x, lo.y, hi.y}, {lo.z, hi.z, lo.w, hi.w}};
+#pragma unroll
+      for (int n = 0; n < 4; ++n) {
+        float part[4];
+        mma_bf16_first(part, a[0], d[n].x, d[n].y);
+        mma_bf16(part, a[1], d[n].z, d[n].w);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) dot[n][i] += part[i];
+      }
+    };
+    for (int k = 0; k < pieces; k += 8) {
+      fold(decoder[0], k);
+      load_decoder(decoder[0], k + 8);
+      if (k + 4 < pieces) fold(decoder[1], k + 4);
+      load_decoder(decoder[1], k + 12);
     }
-  };
-#pragma unroll
-  for (int i = 0; i < kAhead; ++i)
-    if (i < chunks) fold(decoder[i], i);
-  for (int i0 = kAhead; i0 < chunks; i0 += kAhead) {
-#pragma unroll
-    for (int i = 0; i < kAhead; ++i)
-      decoder[i] = i0 + i < chunks ? decoder_row[i0 + i] : make_uint4(0, 0, 0, 0);
-#pragma unroll
-    for (int i = 0; i < kAhead; ++i)
-      if (i0 + i < chunks) fold(decoder[i], i0 + i);
   }
+  const bool aligned = (reinterpret_cast<uintptr_t>(out) & 15) == 0;
 #pragma unroll
-  for (int j = 0; j < TOKENS; ++j) {
-    if (j >= count) break;
-    float routed = 0.0f;
+  for (int i = 0; i < 2; ++i) {
+    const int j = 8 * i + g;
+    if (j >= count) continue;
+    float routed[8] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
 #pragma unroll
     for (int s = 0; s < kSums; ++s)
-      if ((valid[j] >> s) & 1u)
-        routed = fmaf(__bfloat162float(__ushort_as_bfloat16(sums[j][s])), weight[j][s], routed);
-#pragma unroll 4
-    for (int s = kSums; s < L.K; ++s)
-      if ((valid[j] >> s) & 1u)
-        routed = fmaf(__bfloat162float(__ushort_as_bfloat16(__ldcg(from + static_cast<size_t>(j * L.K + s) * L.H))),
-                      weight[j][s], routed);
-    out[static_cast<size_t>(t0 + j) * L.H + h] = __float2bfloat16_rn(routed + bf16_round(dot[j]));
+      if ((valid[j] >> s) & 1u) add_scaled8(routed, sums[i][s], weight[j][s]);
+    for (int s0 = kSums; s0 < L.K; s0 += kSums) {
+#pragma unroll
+      for (int s = 0; s < kSums; ++s)
+        if (s0 + s < L.K) sums[i][s] = __ldcg(from[i] + static_cast<size_t>(s0 + s) * (L.H / 8));
+#pragma unroll
+      for (int s = 0; s < kSums; ++s)
+        if (s0 + s < L.K && ((valid[j] >> (s0 + s)) & 1u)) add_scaled8(routed, sums[i][s], weight[j][s0 + s]);
+    }
+#pragma unroll
+    for (int n = 0; n < 4; ++n) {
+      routed[2 * n] += bf16_round(dot[n][2 * i]);
+      routed[2 * n + 1] += bf16_round(dot[n][2 * i + 1]);
+    }
+    __nv_bfloat16* to = out + static_cast<size_t>(t0 + j) * L.H + h;
+    if (aligned) {
+      *reinterpret_cast<uint4*>(to) = pack_bf16x8(routed);
+    } else {
+#pragma unroll
+      for (int c = 0; c < 8; ++c) to[c] = __float2bfloat16_rn(routed[c]);
+    }
   }
 }
