@@ -175,7 +175,7 @@ static int make_layout(const cfm_layer* l, int32_t capacity, cfm_workspace_layou
   o->union_channels = take(2 * E * I);
   o->union_activations = take(2 * C * N);
   const int64_t passes = C * K / 8 + std::min(E, C * K);  // of at least eight pairs
-  o->exact_work = take(32 * passes * ((I + 15) / 16));
+  o->exact_work = take(32 * passes * ((I + 31) / 32));  // tiles of 32 channels
   o->down_work = take(32 * passes);
   o->bytes = at;
   return 0;
@@ -2146,7 +2146,7 @@ static int run_exact_union(const Bound& b, const cfm_call* call, bool whole) {
   const int rc = launched();
   if (rc) return rc;
   const int64_t pairs = static_cast<int64_t>(b.T) * b.L.K;
-  const int64_t work = (pairs / 8 + busy_experts(b)) * ((b.L.I + 15) / 16);
+  const int64_t work = (pairs / (8 * tiles) + busy_experts(b)) * ((b.L.I + kUnionTile - 1) / kUnionTile);
   const int by_union = down_by_union(b), list = whole && !by_union;
   const auto* hidden = static_cast<const __nv_bfloat16*>(call->hidden);
   auto launch = [&](auto tile) {

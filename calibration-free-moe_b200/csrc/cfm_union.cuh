@@ -88,6 +88,7 @@ __device__ __forceinline__ void repeat(F&& f) {
 // ---------------------------------------------------------------------------
 // unions and work lists
 // ---------------------------------------------------------------------------
+constexpr int kUnionTile = 32;  // rows of a tile of the exact kernel
 constexpr int kUnionThreads = 128;
 constexpr int kUnionStagedPairs = 512;  // pairs of an expert whose numbers a CTA stages
 
@@ -114,7 +115,7 @@ __device__ __forceinline__ uint32_t slot_word(const uint32_t* bits, int I, int s
 
 // grid (busy experts), 128 threads.  A CTA makes the union of its expert's kept channels from the
 // tokens' masks (one OR and one scan over I / 32 words), leaves the channels behind and appends the
-// expert's tiles of sixteen channels x passes of `exact_pass` tokens and its passes of `down_pass`
+// expert's tiles of 32 channels x passes of `exact_pass` tokens and its passes of `down_pass`
 // tokens to the work lists.  With `early` the grouping is known to be complete when this grid can
 // start at all, and is read while the selection still runs.  (When every exact CTA made its
 // expert's union itself, the dependent loads and the scan cost each of them some 5 us, a third of
@@ -173,7 +174,7 @@ __global__ void __launch_bounds__(kUnionThreads)
       channels[at] = static_cast<uint16_t>(32 * w + __ffs(mask) - 1);
     rows += all;
   }
-  const int tiles = (rows + 15) / 16;
+  const int tiles = (rows + kUnionTile - 1) / kUnionTile;
   const int exact_passes = (total + exact_pass - 1) / exact_pass;
   const int down_passes = (total + down_pass - 1) / down_pass;
   if (tid == 0) {
@@ -195,9 +196,9 @@ __global__ void __launch_bounds__(kUnionThreads)
 // ---------------------------------------------------------------------------
 // exact
 // ---------------------------------------------------------------------------
-// A tile is sixteen union rows of gate and up against NT x 8 tokens; its columns are cut into
+// A tile is 32 union rows of gate and up against NT x 8 tokens; its columns are cut into
 // quarters of H, one per warp.  Per step of 32 columns lane (g, tq) copies 16 bytes (eight columns)
-// of rows g and g + 8, gate and up, and of its tokens' rows into a ring of the warp's own with
+// of rows g, g + 8, g + 16 and g + 24, gate and up, and of its tokens' rows into a ring of the warp's own with
 // cp.async; the matrix loads read them from there as the instruction wants them.  A row's four
 // pieces are permuted by the row, so that the eight rows of a matrix lie in different banks.  The
 // tokens' rows travel with the weights because the ring leaves L1 too small to hold them.  The
@@ -210,22 +211,22 @@ struct ExactUnion {
   static constexpr int kThreads = 128;
   static constexpr int kPass = 8 * NT;
   static constexpr int kSlots = 4;    // steps in the ring
-  static constexpr int kStepBytes = (4 + NT) * 512;
+  static constexpr int kStepBytes = (8 + NT) * 512;
   static constexpr int kRingBytes = 4 * kSlots * kStepBytes;
-  static constexpr int kSumFloats = NT * 2 * 4 * 32;  // of a quarter
+  static constexpr int kSumFloats = NT * 2 * 4 * 32;  // of a quarter, for half of the rows
   static constexpr int kSharedBytes = kRingBytes + 4 * kSumFloats * 4;
-  // CTAs per SM: bound by shared memory (227 KB, 1 KB of it per CTA) and registers.
-  static constexpr int kPerSm = NT == 1 ? 5 : NT == 2 ? 3 : 2;
+  static constexpr int kPerSm = 2;  // CTAs per SM: bound by shared memory (227 KB, 1 KB of it per CTA)
 };
 
-// Where a lane's pieces of a tile come from: row and token numbers, and pointers.
+// Where a lane's pieces of a tile come from: rows g, g + 8, g + 16, g + 24 and the tokens, as
+// numbers and as pointers.
 template <int NT>
 struct ExactRows {
-  int e, channel[2], token[NT];
+  int e, channel[4], token[NT];
 };
 template <int NT>
 struct ExactSource {
-  const char *row[4], *x[NT];  // gate of rows g and g + 8, up of the same
+  const char *gate[4], *x[NT];
 };
 
 // `by_union`: activations also go to their union rows, for k_down_union.  With `list` one more CTA,
@@ -269,10 +270,9 @@ __global__ void __launch_bounds__(ExactUnion<NT>::kThreads, ExactUnion<NT>::kPer
   auto locate = [&](const UnionWork& w) {  // rows beyond the union repeat its last one
     ExactRows<NT> at;
     const uint16_t* channels = ws.union_channels + static_cast<size_t>(w.e) * L.I;
-    const int last = w.rows - 1, row = w.tile * 16 + g;
     at.e = w.e;
-    at.channel[0] = channels[min(row, last)];
-    at.channel[1] = channels[min(row + 8, last)];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) at.channel[i] = channels[min(w.tile * kUnionTile + 8 * i + g, w.rows - 1)];
 #pragma unroll
     for (int n = 0; n < NT; ++n)  // columns beyond the pass repeat its last token
       at.token[n] = ws.group_pairs[w.first + min(8 * n + g, w.count - 1)];
@@ -284,10 +284,8 @@ __global__ void __launch_bounds__(ExactUnion<NT>::kThreads, ExactUnion<NT>::kPer
         L.gate_up + static_cast<size_t>(at.e) * 2 * L.I * L.H + column);
     const uint32_t row_bytes = 2 * L.H;
 #pragma unroll
-    for (int i = 0; i < 2; ++i) {
-      s.row[i] = weights + static_cast<uint64_t>(static_cast<uint32_t>(at.channel[i])) * row_bytes;
-      s.row[2 + i] = s.row[i] + up_bytes;
-    }
+    for (int i = 0; i < 4; ++i)
+      s.gate[i] = weights + static_cast<uint64_t>(static_cast<uint32_t>(at.channel[i])) * row_bytes;
 #pragma unroll
     for (int n = 0; n < NT; ++n)
       s.x[n] = reinterpret_cast<const char*>(hidden + column) +
@@ -299,8 +297,12 @@ __global__ void __launch_bounds__(ExactUnion<NT>::kThreads, ExactUnion<NT>::kPer
   auto copy = [&](auto slot, const ExactSource<NT>& s, auto step, bool there) {
     const int bytes = there ? 16 : 0;
     constexpr int kTo = decltype(slot)::value * X::kStepBytes, kFrom = 64 * decltype(step)::value;
-    repeat<4>([&](auto i) { copy_async16_at<kTo + 512 * decltype(i)::value, kFrom>(mine, s.row[i], bytes); });
-    repeat<NT>([&](auto n) { copy_async16_at<kTo + 512 * (4 + decltype(n)::value), kFrom>(mine, s.x[n], bytes); });
+    repeat<4>([&](auto i) {
+      constexpr int kPlace = kTo + 512 * ((decltype(i)::value >> 1) * 4 + (decltype(i)::value & 1));
+      copy_async16_at<kPlace, kFrom>(mine, s.gate[i], bytes);
+      copy_async16_at<kPlace + 1024, kFrom>(mine, s.gate[i] + up_bytes, bytes);
+    });
+    repeat<NT>([&](auto n) { copy_async16_at<kTo + 512 * (8 + decltype(n)::value), kFrom>(mine, s.x[n], bytes); });
   };
 
   UnionWork work = read_work(index), next = read_work(index + stride);
@@ -314,46 +316,43 @@ __global__ void __launch_bounds__(ExactUnion<NT>::kThreads, ExactUnion<NT>::kPer
     const bool more = index + stride < work_count;
     // What the end of the tile needs, and where the next one's rows are, on their way early.  There
     // this thread has row g or g + 8 and a token that another lane has located.
-    const int at = work.tile * 16 + g + 8 * (warp >> 1);
-    const bool finishes = at < work.rows;
-    const int channel = warp < 2 ? rows.channel[0] : rows.channel[1];
     int pairs[NT];
-    uint32_t bits[NT];     // the kept bits of the candidate's word
-    uint16_t before[NT];   // kept channels of the token before the word
+    uint32_t bits[2][NT];    // the kept bits of the candidate's word
+    uint16_t before[2][NT];  // kept channels of the token before the word
 #pragma unroll
     for (int n = 0; n < NT; ++n) {
       pairs[n] = __shfl_sync(kFull, rows.token[n], 4 * (2 * tq + (warp & 1)));
-      const int t = pairs[n] / L.K, candidate = (pairs[n] - t * L.K) * L.I + channel;
-      const size_t word = static_cast<size_t>(t) * token_words + (candidate >> 5);
-      bits[n] = ws.kept_bits[word];
-      before[n] = ws.kept_before[word];
+      const int t = pairs[n] / L.K;
+#pragma unroll
+      for (int half = 0; half < 2; ++half) {
+        const int channel = warp < 2 ? rows.channel[2 * half] : rows.channel[2 * half + 1];
+        const int candidate = (pairs[n] - t * L.K) * L.I + channel;
+        const size_t word = static_cast<size_t>(t) * token_words + (candidate >> 5);
+        bits[half][n] = ws.kept_bits[word];
+        before[half][n] = ws.kept_before[word];
+      }
     }
     ExactRows<NT> next_rows = {};
     if (more) next_rows = locate(next);
     const UnionWork after = read_work(index + 2 * stride);
 
-    float acc[NT][2][4];
+    float acc[2][NT][2][4];  // [rows][tokens][gate, up]
 #pragma unroll
-    for (int n = 0; n < NT; ++n)
+    for (int half = 0; half < 2; ++half)
 #pragma unroll
-      for (int i = 0; i < 4; ++i) acc[n][0][i] = acc[n][1][i] = 0.0f;
+      for (int n = 0; n < NT; ++n)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) acc[half][n][0][i] = acc[half][n][1][i] = 0.0f;
 #pragma unroll 1
     for (int s = 0; s < padded; s += kSlots) {
       const bool last = s + kSlots >= padded;
-      float part[NT][2][4];  // of this turn of the ring
+      float part[2][NT][2][4];  // of this turn of the ring
       // The last turn's copies, but for its first, are the next tile's: the pointers go on there.
       repeat<kSlots>([&](auto turn) {
         constexpr int j = decltype(turn)::value;
         constexpr Index<(j + kSlots - 1) % kSlots> free{};
         copy_async_wait<kSlots - 2>();
         __syncwarp();  // every lane's copies of step s + j have landed; the step before has been read
-        uint32_t w[4][4], t[NT][4];
-        constexpr int kFrom = j * X::kStepBytes;
-        load_matrices_at<kFrom>(w[0], weights_at);
-        load_matrices_at<kFrom + 1024>(w[1], weights_at);
-        repeat<NT>([&](auto n) { load_matrices_at<kFrom + 512 * (4 + decltype(n)::value)>(t[n], tokens_at); });
-        load_matrices_at<kFrom>(w[2], weights_at2);
-        load_matrices_at<kFrom + 1024>(w[3], weights_at2);
         // Refill the place read one step ago.
         if (j == 1 && last && more) source = point(next_rows);
         if (j == 0 || !last) {
@@ -362,69 +361,88 @@ __global__ void __launch_bounds__(ExactUnion<NT>::kThreads, ExactUnion<NT>::kPer
           copy(free, source, Index<(j > 0 ? j - 1 : 0)>{}, j - 1 < steps);
         }
         copy_async_commit();
+        constexpr int kFrom = j * X::kStepBytes;
+        uint32_t t[NT][4];
+        repeat<NT>([&](auto n) { load_matrices_at<kFrom + 512 * (8 + decltype(n)::value)>(t[n], tokens_at); });
+        repeat<2>([&](auto h) {
+          constexpr int half = decltype(h)::value, kRows = kFrom + 2048 * half;
+          uint32_t w[4][4];
+          load_matrices_at<kRows>(w[0], weights_at);
+          load_matrices_at<kRows + 1024>(w[1], weights_at);
+          load_matrices_at<kRows>(w[2], weights_at2);
+          load_matrices_at<kRows + 1024>(w[3], weights_at2);
 #pragma unroll
-        for (int n = 0; n < NT; ++n) {
-          if (j == 0) {
-            mma_bf16_first(part[n][0], w[0], t[n][0], t[n][1]);
-            mma_bf16_first(part[n][1], w[1], t[n][0], t[n][1]);
-          } else {
-            mma_bf16(part[n][0], w[0], t[n][0], t[n][1]);
-            mma_bf16(part[n][1], w[1], t[n][0], t[n][1]);
+          for (int n = 0; n < NT; ++n) {
+            if (j == 0) {
+              mma_bf16_first(part[half][n][0], w[0], t[n][0], t[n][1]);
+              mma_bf16_first(part[half][n][1], w[1], t[n][0], t[n][1]);
+            } else {
+              mma_bf16(part[half][n][0], w[0], t[n][0], t[n][1]);
+              mma_bf16(part[half][n][1], w[1], t[n][0], t[n][1]);
+            }
+            mma_bf16(part[half][n][0], w[2], t[n][2], t[n][3]);
+            mma_bf16(part[half][n][1], w[3], t[n][2], t[n][3]);
           }
-          mma_bf16(part[n][0], w[2], t[n][2], t[n][3]);
-          mma_bf16(part[n][1], w[3], t[n][2], t[n][3]);
-        }
+        });
       });
       if (!last) {
 #pragma unroll
-        for (int i = 0; i < 4; ++i) source.row[i] += 64 * kSlots;
+        for (int i = 0; i < 4; ++i) source.gate[i] += 64 * kSlots;
 #pragma unroll
         for (int n = 0; n < NT; ++n) source.x[n] += 64 * kSlots;
       }
 #pragma unroll
+      for (int half = 0; half < 2; ++half)
+#pragma unroll
+        for (int n = 0; n < NT; ++n)
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            acc[half][n][0][i] += part[half][n][0][i];
+            acc[half][n][1][i] += part[half][n][1][i];
+          }
+    }
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+      // Sums of the quarters: [quarter][tile of tokens][gate, up][accumulator register][lane].
+      float* own = red + warp * X::kSumFloats + lane;
+#pragma unroll
       for (int n = 0; n < NT; ++n)
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-          acc[n][0][i] += part[n][0][i];
-          acc[n][1][i] += part[n][1][i];
+          own[(n * 8 + i) * 32] = acc[half][n][0][i];
+          own[(n * 8 + 4 + i) * 32] = acc[half][n][1][i];
         }
-    }
-    // Sums of the quarters: [quarter][tile of tokens][gate, up][accumulator register][lane].
-    float* own = red + warp * X::kSumFloats + lane;
+      __syncthreads();
+      // Thread (register, lane): the quarters in order, then the feature, or zero for a channel the
+      // token did not keep.
+      const int at = work.tile * kUnionTile + 16 * half + g + 8 * (warp >> 1);
+      const int channel = warp < 2 ? rows.channel[2 * half] : rows.channel[2 * half + 1];
 #pragma unroll
-    for (int n = 0; n < NT; ++n)
+      for (int n = 0; n < NT; ++n) {
+        const int token = 8 * n + 2 * tq + (warp & 1);
+        if (at >= work.rows || token >= work.count) continue;
+        __nv_bfloat16 feature = __float2bfloat16_rn(0.0f);
+        const int t = pairs[n] / L.K, bit = ((pairs[n] - t * L.K) * L.I + channel) & 31;
+        if ((bits[half][n] >> bit) & 1u) {
+          float gate[4], up[4];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        own[(n * 8 + i) * 32] = acc[n][0][i];
-        own[(n * 8 + 4 + i) * 32] = acc[n][1][i];
-      }
-    __syncthreads();
-    // Thread (register, lane): the quarters in order, then the feature, or zero for a channel the
-    // token did not keep.
-#pragma unroll
-    for (int n = 0; n < NT; ++n) {
-      const int token = 8 * n + 2 * tq + (warp & 1);
-      if (!finishes || token >= work.count) continue;
-      __nv_bfloat16 feature = __float2bfloat16_rn(0.0f);
-      const int t = pairs[n] / L.K, bit = ((pairs[n] - t * L.K) * L.I + channel) & 31;
-      if ((bits[n] >> bit) & 1u) {
-        float gate[4], up[4];
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          const float* sums = red + q * X::kSumFloats + lane;
-          gate[q] = sums[(n * 8 + warp) * 32];
-          up[q] = sums[(n * 8 + 4 + warp) * 32];
+          for (int q = 0; q < 4; ++q) {
+            const float* sums = red + q * X::kSumFloats + lane;
+            gate[q] = sums[(n * 8 + warp) * 32];
+            up[q] = sums[(n * 8 + 4 + warp) * 32];
+          }
+          const float g_sum = (gate[0] + gate[1]) + (gate[2] + gate[3]);
+          const float u_sum = (up[0] + up[1]) + (up[2] + up[3]);
+          feature = __float2bfloat16_rn(exact_feature(g_sum, u_sum, L.activation));
+          ws.activations[static_cast<size_t>(pairs[n]) * L.I + channel] = feature;
+          float* exact = ws.exact + static_cast<size_t>(t) * 2 * L.F + before[half][n] +
+                         __popc(bits[half][n] & ((1u << bit) - 1));
+          exact[0] = g_sum;
+          exact[L.F] = u_sum;
         }
-        const float g_sum = (gate[0] + gate[1]) + (gate[2] + gate[3]);
-        const float u_sum = (up[0] + up[1]) + (up[2] + up[3]);
-        feature = __float2bfloat16_rn(exact_feature(g_sum, u_sum, L.activation));
-        ws.activations[static_cast<size_t>(pairs[n]) * L.I + channel] = feature;
-        float* exact = ws.exact + static_cast<size_t>(t) * 2 * L.F + before[n] +
-                       __popc(bits[n] & ((1u << bit) - 1));
-        exact[0] = g_sum;
-        exact[L.F] = u_sum;
+        if (by_union) ws.union_activations[static_cast<size_t>(work.first + token) * L.I + at] = feature;
       }
-      if (by_union) ws.union_activations[static_cast<size_t>(work.first + token) * L.I + at] = feature;
+      if (half == 0) __syncthreads();  // the sums may be overwritten
     }
     if (!more) break;
     __syncthreads();  // the sums may be overwritten
