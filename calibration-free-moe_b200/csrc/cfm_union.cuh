@@ -719,7 +719,7 @@ __device__ __forceinline__ uint4 pack_bf16x8(const float (&z)[8]) {
   return v;
 }
 
-__global__ void __launch_bounds__(128, 3) k_mix(Layer L, Workspace ws, const uint8_t* padding, int tokens,
+__global__ void __launch_bounds__(128, 4) k_mix(Layer L, Workspace ws, const uint8_t* padding, int tokens,
                                                 __nv_bfloat16* out, int latents, int early) {
   __shared__ __align__(16) __nv_bfloat16 latent[kMixTokens][256 + 32];
   __shared__ float weight[kMixTokens][32];
@@ -765,7 +765,7 @@ __global__ void __launch_bounds__(128, 3) k_mix(Layer L, Workspace ws, const uin
   __syncthreads();
   // This thread's columns h .. h + 7 of tokens g and g + 8.
   const int h = blockIdx.x * 128 + 32 * warp + 8 * tq;
-  constexpr int kSums = 8;  // slots on their way at a time
+  constexpr int kSums = 4;  // slots on their way at a time
   uint4 sums[2][kSums];
   const uint4* from[2];
 #pragma unroll
@@ -786,13 +786,13 @@ __global__ void __launch_bounds__(128, 3) k_mix(Layer L, Workspace ws, const uin
       if (live && valid[j] && latents == kLatentsFromSums) {
         const uint4* parts = reinterpret_cast<const uint4*>(ws.encoder_parts) +
                              static_cast<size_t>(t0 + j) * L.K * pieces + piece;
-        for (int s0 = 0; s0 < L.K; s0 += kSums) {
-          uint4 part[kSums];
+        for (int s0 = 0; s0 < L.K; s0 += 8) {
+          uint4 part[8];
 #pragma unroll
-          for (int s = 0; s < kSums; ++s)
+          for (int s = 0; s < 8; ++s)
             part[s] = s0 + s < L.K ? __ldcg(parts + (s0 + s) * pieces) : make_uint4(0, 0, 0, 0);
 #pragma unroll
-          for (int s = 0; s < kSums; ++s)
+          for (int s = 0; s < 8; ++s)
             if ((valid[j] >> (s0 + s)) & 1u) add_scaled8(z, part[s], weight[j][s0 + s]);
         }
       } else if (live && valid[j] && latents == kLatentsGiven) {
