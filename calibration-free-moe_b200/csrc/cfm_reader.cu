@@ -2103,17 +2103,16 @@ static bool exact_by_union(const Bound& b) {
   return b.L.row_engine == CFM_ROWS_EXPERT_MAJOR ||
          (b.T >= 16 && static_cast<int64_t>(b.T) * b.L.K >= 3 * static_cast<int64_t>(b.L.E));
 }
-// The expert-major down kernel, on request and where most experts have more than a pass of eight
-// tokens: 64 tokens of the 128-expert layer 38 us and 6 in the output against 35 and 7 of the tiles
-// per token, 100 of the 64-expert layer 46 and 7 against 65 and 15.
+// The expert-major down kernel where most experts have more than half a pass of sixteen tokens and
+// there is a piece for every second warp: 64 tokens of the 128-expert layer 38 us and 7 in the output
+// against 30 and 7 of the tiles per token, 100 of the 64-expert layer 49 and 8 against 65 and 15, 256
+// of the 256-expert layer 56 and 9 against 79 and 28.
 static bool down_by_union(const Bound& b) {
-  return exact_by_union(b) && (b.L.row_engine == CFM_ROWS_EXPERT_MAJOR || shares_decode(b));
+  return exact_by_union(b) && shares_decode(b) &&
+         static_cast<int64_t>(busy_experts(b)) * (b.L.H / DownUnion::kColumns) >= 148 * 8;
 }
-// The recovery encoder in the expert-major down launch.  By size alone: a latent does not depend on
-// the row engine.
-static bool encodes_by_union(const Bound& b) {
-  return down_by_union(b) && shares_decode(b) && encodes(b);
-}
+// The recovery encoder in the expert-major down launch.
+static bool encodes_by_union(const Bound& b) { return down_by_union(b) && encodes(b); }
 // Tokens per pass of the expert-major exact kernel, in eights: the next size up while the mean load
 // is more than two thirds of the one before.
 static int exact_union_tiles(const Bound& b) {
@@ -2289,10 +2288,9 @@ static int run_output(const Bound& b, const cfm_call* call, bool whole) {
                      out, latents, static_cast<int>(whole));
     return launched();
   }
-  const int early = whole && (!encodes(b) || encodes_by_union(b));
   const int mixed = whole && encodes_by_union(b) ? kLatentsFromSums : latents ? kLatentsGiven : kLatentsNone;
   launch_dependent(k_mix, dim3(b.L.H / 128 + whole, (b.T + kMixTokens - 1) / kMixTokens), dim3(128), 0, b.stream,
-                   b.L, b.ws, b.padding, b.T, out, mixed, early);
+                   b.L, b.ws, b.padding, b.T, out, mixed, static_cast<int>(whole));
   return launched();
 }
 
@@ -2513,7 +2511,6 @@ int cfm_reader_forward(const cfm_layer* layer, void* workspace, int32_t capacity
   if ((rc = run_select(b, 0, nullptr, false))) return rc;
   if ((rc = run_exact(b, call, true))) return rc;
   if ((rc = run_down(b, encodes(b), true))) return rc;
-  if (down_by_union(b) && encodes(b) && !encodes_by_union(b) && (rc = run_encode(b))) return rc;
   return run_output(b, call, true);
 }
 

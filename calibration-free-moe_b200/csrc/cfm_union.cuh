@@ -204,8 +204,10 @@ __global__ void __launch_bounds__(kUnionThreads)
 // tokens' rows travel with the weights because the ring leaves L1 too small to hold them.  The
 // instruction truncates where an FMA rounds, so a sum leaves it after 128 columns and goes on by
 // ordinary additions (RMS error of a gate sum of 2048 columns against FP64: 8.0e-7 without, 4.1e-7
-// with, 2.1e-7 the gathers'; it is rounded to BF16 next).  Loads straight into registers were issued
-// one by one: 76 us at 64 tokens of the 128-expert layer.  MEASURED_EXACT
+// with, 2.1e-7 the gathers').  The sums are rounded to BF16 next; where an error of that size could
+// change a rounding (some two in a thousand), the CTA puts the row down and at its end repeats the
+// product as the gathers do it, so that the activations are those of the gathers.
+// MEASURED_EXACT
 template <int NT>
 struct ExactUnion {
   static constexpr int kThreads = 128;
@@ -229,6 +231,14 @@ struct ExactSource {
   const char *gate[4], *x[NT];
 };
 
+// Sums to be repeated that a CTA has room for; any beyond them stay as they are.
+constexpr int kRepeats = 40;
+
+// Whether an error of `margin` could round v to another BF16 value.
+__device__ __forceinline__ bool rounds_either_way(float v, float margin) {
+  return bf16_round(v - margin) != bf16_round(v + margin);
+}
+
 // `by_union`: activations also go to their union rows, for k_down_union.  With `list` one more CTA,
 // the first, lists the down tiles for the tile-wise down kernel.
 template <int NT>
@@ -237,11 +247,13 @@ __global__ void __launch_bounds__(ExactUnion<NT>::kThreads, ExactUnion<NT>::kPer
   using X = ExactUnion<NT>;
   constexpr int kSlots = X::kSlots;
   extern __shared__ __align__(128) uint8_t union_shared[];
-  __shared__ int scratch[33];
+  __shared__ int4 repeats[kRepeats];  // pair, expert, channel, place among the union's activations
+  __shared__ int repeat_count;
+  static_assert(sizeof(repeats) >= 33 * sizeof(int), "scratch of the listing");
   grid_dependency_wait();     // the work list is complete
   grid_dependency_release();  // the down kernel may be scheduled: its encoder needs no more than that
   if (list && blockIdx.x == 0) {
-    list_down_tiles(L, ws, scratch);
+    list_down_tiles(L, ws, reinterpret_cast<int*>(repeats));
     return;
   }
   const int work_count = ws.work_counts[kExactCount], stride = gridDim.x - list;
@@ -305,6 +317,7 @@ __global__ void __launch_bounds__(ExactUnion<NT>::kThreads, ExactUnion<NT>::kPer
     repeat<NT>([&](auto n) { copy_async16_at<kTo + 512 * (8 + decltype(n)::value), kFrom>(mine, s.x[n], bytes); });
   };
 
+  if (tid == 0) repeat_count = 0;  // ordered by the barriers of the first tile
   UnionWork work = read_work(index), next = read_work(index + stride);
   ExactRows<NT> rows = locate(work);
   ExactSource<NT> source = point(rows);
@@ -439,6 +452,15 @@ __global__ void __launch_bounds__(ExactUnion<NT>::kThreads, ExactUnion<NT>::kPer
                          __popc(bits[half][n] & ((1u << bit) - 1));
           exact[0] = g_sum;
           exact[L.F] = u_sum;
+          const float g_size = (fabsf(gate[0]) + fabsf(gate[1])) + (fabsf(gate[2]) + fabsf(gate[3]));
+          const float u_size = (fabsf(up[0]) + fabsf(up[1])) + (fabsf(up[2]) + fabsf(up[3]));
+          constexpr float kError = 1.0f / (1 << 21);
+          if (rounds_either_way(g_sum, kError * g_size) || rounds_either_way(u_sum, kError * u_size)) {
+            const int place = atomicAdd(&repeat_count, 1);
+            if (place < kRepeats)
+              repeats[place] = make_int4(pairs[n], work.e, channel,
+                                         by_union ? (work.first + token) * L.I + at : -1);
+          }
         }
         if (by_union) ws.union_activations[static_cast<size_t>(work.first + token) * L.I + at] = feature;
       }
@@ -450,6 +472,30 @@ __global__ void __launch_bounds__(ExactUnion<NT>::kThreads, ExactUnion<NT>::kPer
     work = next;
     next = after;
     rows = next_rows;
+  }
+  __syncthreads();  // the list is complete, the activations of the rows on it are written
+  for (int i = warp; i < min(repeat_count, kRepeats); i += 4) {
+    const int4 r = repeats[i];
+    const int t = r.x / L.K, candidate = (r.x - t * L.K) * L.I + r.z;
+    const size_t word = static_cast<size_t>(t) * token_words + (candidate >> 5);
+    const uint32_t kept = ws.kept_bits[word];
+    const int place = ws.kept_before[word] + __popc(kept & ((1u << (candidate & 31)) - 1));
+    const int chunks = L.H / 8;
+    const uint4* gate = reinterpret_cast<const uint4*>(L.gate_up) +
+                        (static_cast<size_t>(r.y) * 2 * L.I + r.z) * chunks;
+    uint4 gw[kExactSweep], uw[kExactSweep];
+    float g_sum, u_sum;
+    exact_dot(gate, gate + static_cast<size_t>(L.I) * chunks,
+              reinterpret_cast<const uint4*>(hidden) + static_cast<size_t>(t) * chunks, chunks, lane, false, gw, uw,
+              g_sum, u_sum);
+    if (lane == 0) {
+      const __nv_bfloat16 feature = __float2bfloat16_rn(exact_feature(g_sum, u_sum, L.activation));
+      ws.activations[static_cast<size_t>(r.x) * L.I + r.z] = feature;
+      if (r.w >= 0) ws.union_activations[r.w] = feature;
+      float* exact = ws.exact + static_cast<size_t>(t) * 2 * L.F + place;
+      exact[0] = g_sum;
+      exact[L.F] = u_sum;
+    }
   }
 }
 

@@ -3,10 +3,13 @@
 import pytest
 import torch
 
+import cases
 from cfm_b200.reader.sketch import (
     block_hadamard_signs, build_sketch, build_sketch_on_device, repack_sketch,
     repack_sketch_grouped,
 )
+from helpers import prepared_case, relative_l2, run_oracle
+from test_gpu_parity import make_reader, run_reader
 
 pytestmark = pytest.mark.gpu
 
@@ -25,3 +28,106 @@ def test_sketch_builder_with_partial_row_tiles(experts, width, hidden):
     assert torch.equal(words, repack_sketch(codes, 2 * width, hidden))
     assert torch.equal(grouped, repack_sketch_grouped(codes, 2 * width, hidden))
     torch.testing.assert_close(fast.float(), statistics.float(), rtol=2e-3, atol=1e-7)
+
+
+# hidden, width, experts, top_k, rank, tokens, retention, screen keep, activation, score, options
+LAYERS = {
+    # One warp of a tile per split of the blocks, an odd top_k, one block.
+    "screen-one-block": (128, 48, 8, 3, 8, 1, 0.25, 0.5, "silu", "point", {}),
+    # The tcgen05 screen at the edge of its 64 channels, passes of eight with a remainder.
+    "tcgen05-ragged": (384, 80, 16, 2, 8, 9, 0.25, 0.5, "silu", "point", {"tensor_engine": "tcgen05"}),
+    "tcgen05-risk-sixteen": (256, 80, 4, 2, 16, 35, 0.25, 1.0, "silu", "recovery-aware", {}),
+    # Down columns: H not a multiple of 256, tiles per token and listed ones.
+    "down-columns": (1152, 64, 8, 2, 32, 3, 0.5, 0.625, "silu", "point", {}),
+    "down-listed": (1152, 208, 32, 3, 64, 8, 0.5, 0.625, "gelu_tanh", "point", {}),
+    # Expert-major exact with the tiles per token: three tokens per expert and more, up to 16 / 3.
+    "union-exact-only": (640, 112, 12, 3, 16, 18, 0.25, 0.625, "silu", "point", {}),
+    # One step per quarter of the columns, fewer rows than a tile; a quarter that is no whole turn.
+    "union-one-step": (128, 16, 4, 2, 8, 16, 0.25, 1.0, "silu", "point", {}),
+    "union-part-turn": (640, 176, 6, 5, 128, 33, 0.3, 0.625, "gelu_tanh", "point", {}),
+    # Several passes per expert.
+    "union-risk": (512, 80, 4, 3, 256, 70, 0.2, 0.5, "silu", "recovery-aware", {}),
+    # Expert-major down too: two column blocks of the encoder, an odd top_k, remainders everywhere.
+    "union-down": (1280, 48, 64, 5, 128, 90, 0.3, 0.625, "gelu_tanh", "point", {}),
+    # An eighth of a column block of the encoder.
+    "union-down-risk": (1280, 80, 60, 3, 8, 110, 0.2, 0.5, "silu", "recovery-aware", {}),
+    # More than eight slots, no recovery map, few rows.
+    "union-down-many-slots": (1280, 16, 64, 12, 0, 64, 0.25, 0.625, "silu", "point", {}),
+    # Requested below the sizes of the rule.
+    "union-requested": (384, 96, 16, 2, 32, 8, 0.25, 0.625, "silu", "point",
+                        {"row_engine": "expert_major"}),
+}
+
+
+@pytest.mark.parametrize("padded", [False, True])
+@pytest.mark.parametrize("name", LAYERS)
+def test_layer_at_the_edges(oracle, name, padded):
+    h, i, e, k, rank, tokens, retention, keep, activation, score, options = LAYERS[name]
+    padding = [t % 5 == 1 for t in range(tokens)] if padded else None
+    case = cases._random(name, h + i + tokens, h, i, e, k, rank, tokens, retention, keep, activation,
+                         padding=padding, score=score)
+    item = prepared_case(case)
+    reader = make_reader(item, capacity=tokens + 3, **options)
+    out = run_reader(reader, case).cpu()
+    assert int(reader.workspace.status.abs().sum()) == 0
+    own = dict(norms=reader.norms.cpu())
+    if reader.recovery_geometry is not None:
+        own["geometry"] = reader.recovery_geometry.cpu()
+    want = run_oracle(oracle, item, **own)
+    active = torch.ones(tokens, dtype=torch.bool) if case.padding is None else ~case.padding
+    assert torch.equal(reader.partial[:tokens].cpu()[active], want["partial"][active])
+    assert torch.equal(reader.scores[0][:tokens].cpu()[active], want["scores"][active])
+    assert torch.equal(reader.candidate_ids[-1][:tokens].cpu()[active], want["candidate_ids"][active])
+    torch.testing.assert_close(out.float()[active], want["output"][active], rtol=0.025, atol=0.02)
+    exact = run_oracle(oracle, item, fp32=True, **own)
+    assert relative_l2(out[active], exact["output"][active]) < 1e-2
+    assert not out[~active].any()
+    if rank:
+        torch.testing.assert_close(reader.latent[:tokens].cpu()[active], want["latent"][active],
+                                   rtol=0.015, atol=0.01)
+        assert not reader.latent[:tokens].cpu()[~active].any()
+    # Exact projections and activations of the kept channels, where the kernels leave them.
+    lists = want["candidate_ids"].long()
+    gathered = reader.activations[:tokens].cpu().reshape(tokens, -1).gather(1, lists.clamp_min(0))
+    sums = reader.workspace.exact[:tokens].cpu()
+    phi = torch.nn.functional.silu if activation == "silu" else (
+        lambda x: torch.nn.functional.gelu(x, approximate="tanh"))
+    feature = phi(sums[:, 0].bfloat16().float()).bfloat16().float() * sums[:, 1].bfloat16().float()
+    mask = active[:, None] & (lists >= 0)
+    torch.testing.assert_close(gathered.float()[mask], feature[mask], rtol=0.02, atol=1e-3)
+
+
+def test_expert_major_stages_repeat_and_misaligned_output():
+    """The stages on their own, twice, and an output that 16-byte stores cannot take."""
+    case = cases._random("stages", 5, 1280, 48, 60, 3, 16, 112, 0.25, 0.625)
+    reader = make_reader(prepared_case(case))
+    whole = run_reader(reader, case).clone()
+    device = whole.device
+    hidden, ids, weights = (t.to(device) for t in (case.hidden, case.ids, case.weights))
+    room = torch.zeros(whole.numel() + 1, dtype=whole.dtype, device=device)
+    out = room[1:].view_as(whole)
+    call = reader._call_struct(112, hidden, ids, weights, None, out, False)
+    for stage in ("cfm_prepare_input", "cfm_route", "cfm_screen", "cfm_select", "cfm_exact", "cfm_exact",
+                  "cfm_down", "cfm_down", "cfm_encode", "cfm_output"):
+        reader._stage(stage, call)
+    torch.cuda.synchronize()
+    torch.testing.assert_close(out.float(), whole.float(), rtol=0.016, atol=2e-3)
+
+
+@pytest.mark.parametrize("width", [256, 512, 768, 1024, 1536, 2048])
+def test_selection_at_every_number_of_keys_per_thread(width):
+    """Largest sizes of the selection's six variants, with and without ties at the cut."""
+    case = cases._random("select", width, 128, width, 8, 8, 0, 2, 0.125, 0.5)
+    reader = make_reader(prepared_case(case))
+    for levels in (0, 7):
+        run_reader(reader, case)
+        scores = reader.scores[0][:2]
+        if levels:  # few distinct scores: most of the cut's are ties, kept in candidate order
+            call = reader._call_struct(2, *(t.cuda() for t in (case.hidden, case.ids, case.weights)),
+                                       None, torch.empty(2, 128, dtype=torch.bfloat16, device="cuda"), False)
+            scores.copy_(torch.randint(1, levels, scores.shape, device="cuda").float())
+            call.scores_ready = 1
+            reader._stage("cfm_select", call)
+        torch.cuda.synchronize()
+        order = scores.sort(dim=1, descending=True, stable=True).indices[:, : case.plan.final_count]
+        assert torch.equal(reader.candidate_ids[-1][:2].long(), order.sort(dim=1).values)
