@@ -6,12 +6,11 @@
 //   route    sort each token's K experts ascending, map to local ids
 //   screen   exact integer dot products of the 2-bit ternary sketch with the
 //            fixed-point rotated input -> projections -> selection scores
-//   select   per token the F best scores (radix select), ties to the lower
-//            candidate index; read-cost counters
+//   select   per token the F best scores, ties to the lower candidate index
 //   exact    gathered BF16 gate/up rows of the kept channels, phi(g) * u
-//   down     gathered channel-major down rows of the kept channels
-//   encode   low-rank recovery encoder over the skipped channels
-//   output   router-weighted mix + decoder term, BF16 store
+//   down     gathered channel-major down rows of the kept channels, and in the
+//            same launch the low-rank recovery encoder over the skipped ones
+//   output   router-weighted mix + decoder term, BF16 store, read-cost counters
 //
 // Selection depends only on integer dot products and pinned FP32 operations
 // (see cfm_device.cuh), so it does not change with batch size, split count or
@@ -1852,8 +1851,7 @@ static int bind_call(const cfm_layer* layer, void* workspace, int32_t capacity,
 
 // Launch with programmatic stream serialisation: the kernel may be scheduled while its
 // predecessor in the stream is finishing and waits for it at grid_dependency_wait().
-// Used for the selection after the screen and for the exact gather after the selection
-// (measured: 0.6 to 1.3 us per call).  CFM_PDL=0 in the environment makes these ordinary
+// Used for every launch of a whole call (measured for two of them: 0.6 to 1.3 us per call).  CFM_PDL=0 in the environment makes these ordinary
 // launches.
 template <typename... Params, typename... Args>
 static void launch_dependent(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem,
@@ -2095,8 +2093,8 @@ static bool encodes(const Bound& b) { return b.L.R > 0 && b.L.F < b.L.N; }
 
 // The expert-major exact kernel, on request and from three tokens per expert and sixteen tokens on:
 // below that the unions of an expert's kept channels are little smaller than their sum.  64 tokens of
-// the 128-expert layer 60 us with the unions against 69 of the gathers, 256 of the 256-expert layer
-// 83 against 155; 32 tokens of the 128-expert layer 39 against 35.  Under expert parallelism the
+// the 128-expert layer 65 us with the unions against 69 of the gathers, 100 of the 64-expert layer 95
+// against 132, 256 of the 256-expert layer 91 against 155.  Under expert parallelism the
 // gathers per token stay, so that a token's bits do not depend on how the experts are spread.
 static bool exact_by_union(const Bound& b) {
   if (!pairs_grouped(b) || b.L.expert_map || b.L.row_engine == CFM_ROWS_PER_TOKEN) return false;
@@ -2104,9 +2102,9 @@ static bool exact_by_union(const Bound& b) {
          (b.T >= 16 && static_cast<int64_t>(b.T) * b.L.K >= 3 * static_cast<int64_t>(b.L.E));
 }
 // The expert-major down kernel where most experts have more than half a pass of sixteen tokens and
-// there is a piece for every second warp: 64 tokens of the 128-expert layer 38 us and 7 in the output
-// against 30 and 7 of the tiles per token, 100 of the 64-expert layer 49 and 8 against 65 and 15, 256
-// of the 256-expert layer 56 and 9 against 79 and 28.
+// there is a piece for every second warp: 64 tokens of the 128-expert layer 45 us in all against 37 of
+// the tiles per token and their output, 100 of the 64-expert layer 57 against 80, 256 of the 256-expert
+// layer 65 against 107.
 static bool down_by_union(const Bound& b) {
   return exact_by_union(b) && shares_decode(b) &&
          static_cast<int64_t>(busy_experts(b)) * (b.L.H / DownUnion::kColumns) >= 148 * 8;
@@ -2114,7 +2112,8 @@ static bool down_by_union(const Bound& b) {
 // The recovery encoder in the expert-major down launch.
 static bool encodes_by_union(const Bound& b) { return down_by_union(b) && encodes(b); }
 // Tokens per pass of the expert-major exact kernel, in eights: the next size up while the mean load
-// is more than two thirds of the one before.
+// is more than two thirds of the one before.  (The largest for all, leaving out tiles without tokens,
+// spilled: 256 tokens of the 256-expert layer 97 us against 80, 64 of the 128-expert one 62 against 60.)
 static int exact_union_tiles(const Bound& b) {
   int tiles = 1;
   while (tiles < 4 && 3 * static_cast<int64_t>(b.T) * b.L.K > 16 * tiles * static_cast<int64_t>(b.L.E)) tiles *= 2;

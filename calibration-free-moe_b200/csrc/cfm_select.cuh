@@ -7,8 +7,8 @@
 // read their record and go straight to the rows.  Tiles of one expert run next to
 // each other in time, so a down row several tokens kept comes from HBM once and
 // from L2 after that, and every CTA has one tile however unevenly a token's kept
-// channels spread over its experts.  The whole-layer call runs the listing on its
-// side stream beside the exact gate/up gather, so it costs the layer nothing.
+// channels spread over its experts.  In a whole call one CTA of the exact kernel's
+// launch makes the list beside the gather, so it costs the layer nothing.
 // Included by cfm_reader.cu inside namespace cfm.
 #pragma once
 

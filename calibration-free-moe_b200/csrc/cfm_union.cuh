@@ -8,7 +8,7 @@
 //   k_union         per expert the union of its tokens' kept channels; work lists
 //   k_exact_union   gate and up rows of the unions
 //   k_down_union    channel-major down rows of the unions; recovery-encoder rows
-//   k_mix           router mix of the expert sums, latent, decoder term, BF16 store
+//   k_mix           router mix of the expert sums, latent, decoder term, BF16 store, counters
 //
 // The tensor cores are not there for their rate (they idle nine tenths of the time) but for their
 // instruction count: per row and eight tokens a matrix instruction replaces some fifty loads,
@@ -207,7 +207,10 @@ __global__ void __launch_bounds__(kUnionThreads)
 // with, 2.1e-7 the gathers').  The sums are rounded to BF16 next; where an error of that size could
 // change a rounding (some two in a thousand), the CTA puts the row down and at its end repeats the
 // product as the gathers do it, so that the activations are those of the gathers.
-// MEASURED_EXACT
+// Bound by the way from L2 to the SMs (9 to 11 TB/s, the tokens' rows included; tiles of sixteen rows
+// carried them twice as often): 100 tokens of the 64-expert layer 89 us (132 the gathers per token),
+// 256 of the 256-expert layer 80 (155), 256 of hidden 4096 and width 1536 580 at 5.3 TB/s of HBM
+// (1431).
 template <int NT>
 struct ExactUnion {
   static constexpr int kThreads = 128;
@@ -513,7 +516,10 @@ __global__ void __launch_bounds__(ExactUnion<NT>::kThreads, ExactUnion<NT>::kPer
 // The recovery encoder is the same product with an expert's whole width as its rows and the sketch
 // features (zero for kept channels, k_select) as activations; its pieces, the longest, come first.
 // Pieces differ in length with the unions and the number of passes, so warps claim them one at a
-// time (the next one while the current one's copies run).  MEASURED_DOWN
+// time (the next one while the current one's copies run): with fixed strides half of the SMs were
+// idle while the longest pieces ended (85 us at 256 tokens of the 256-expert layer, 55 with claims;
+// the tiles per token take 79).  Bound by latency and instruction issue: 126 instructions per unit of
+// 2 KB.  256 tokens of hidden 4096 and width 1536 373 us at 4.7 TB/s of HBM (651 the tiles per token).
 struct DownUnion {
   static constexpr int kThreads = 128;
   static constexpr int kPass = 16;
@@ -737,8 +743,8 @@ __device__ __forceinline__ float mix_sums(const Layer& L, const Workspace& ws, i
 // goes on by ordinary additions.  Columns are dealt to the instruction so that a thread ends up with
 // eight adjacent ones of two tokens, and the order inside sixteen latent columns so that it loads
 // eight adjacent ones of a decoder row.  The expert sums of the first slots are on their way
-// meanwhile.  Bound by latency.  (One column of up to eight tokens per thread, dot products by FMAs:
-// MEASURED_MIX)
+// meanwhile.  Bound by latency.  256 tokens of the 256-expert layer 9.2 us, of hidden 4096 and rank 128
+// 13.8 (one column of up to eight tokens per thread and dot products by FMAs: 20 and 44).
 // `latents`: none, the workspace's, or to be mixed here from the encoder's sums.
 constexpr int kLatentsNone = 0, kLatentsGiven = 1, kLatentsFromSums = 2;
 constexpr int kMixTokens = 16;

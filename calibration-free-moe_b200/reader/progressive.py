@@ -249,14 +249,15 @@ class ProgressiveReader:
         `recovery_owner` (the rank that adds the decoder term; defaults to rank 0
         of the group) and `retain_reference_sketch` (keep the reference-layout
         codes resident beside the kernel layout) and `tensor_engine`, the
-        tensor-core path of the expert-major screen: "mma_sync" (default, measured
-        faster) or "tcgen05" (tensor-memory accumulators); both give the same bits;
-        and `row_engine`, how batches of eight tokens and more read the native
-        rows: "expert_major" (a row several tokens of one expert kept is read once
-        for all of them), "per_token" (one gather per token, tokens of one expert
+        tensor-core path of the expert-major screen: "mma_sync" (default: chosen by
+        size) or "tcgen05" (tensor-memory accumulators at every size); both give the
+        same bits; and `row_engine`, how batches of eight tokens and more read the
+        native rows: "expert_major" (a row several tokens of one expert kept is read
+        once for all of them), "per_token" (one gather per token, tokens of one expert
         next to each other in time so that shared rows meet in L2) or "auto"
-        (the faster one on the shapes measured so far: per token).  The kept channels
-        do not depend on it; outputs differ by FP32 summation order only.
+        (expert-major from three tokens per expert on, the faster one on the shapes
+        measured).  The kept channels do not depend on it; outputs differ by FP32
+        summation order only.
         `sketch_builder` picks who builds the sketch when none is given: "torch"
         (tensor operations, byte-identical to the reference builder on the same
         device) or "cuda" (the library's kernel, straight into the kernel layouts,

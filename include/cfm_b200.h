@@ -46,7 +46,7 @@ extern "C" {
 #define CFM_ENGINE_TCGEN05 1  /* tcgen05.mma kind::i8, accumulators in tensor memory     */
 #define CFM_ROWS_AUTO 0        /* the library's choice (per token, pairs in expert order) */
 #define CFM_ROWS_PER_TOKEN 1   /* native rows always gathered per token                 */
-#define CFM_ROWS_EXPERT_MAJOR 2 /* expert-major whenever the pairs are grouped (T >= 8) */
+#define CFM_ROWS_EXPERT_MAJOR 2 /* expert-major whenever the pairs are grouped (T >= 8) and no expert_map */
 #define CFM_READ_WORK_SLOTS 20
 
 /* One MoE layer: dimensions and resident tensors.  Mirrors the state
@@ -210,20 +210,18 @@ int cfm_prepare_input(const cfm_layer* layer, void* workspace, int32_t capacity,
                       const cfm_call* call, void* stream);
 
 /* Route: per token, sort the K expert ids ascending (stable), carry the
- * weights, map global to local ids; for batches the screen runs expert-major
- * (8 tokens and more, row-major sketch present) also group the (token, slot)
- * pairs by expert.  Independent of cfm_prepare_input: the two may run on
- * different streams.  Replaces: _prepare / _route (progressive.py:143-239,
+ * weights, map global to local ids, group the (token, slot) pairs by expert.
+ * Independent of cfm_prepare_input: the two may run on different streams.  Replaces: _prepare / _route (progressive.py:143-239,
  * 349-386), _group_sort (:2329-2382). */
 int cfm_route(const cfm_layer* layer, void* workspace, int32_t capacity,
               const cfm_call* call, void* stream);
 
 /* Screen: sketch projections of every candidate channel of every routed local
- * expert.  Writes `partial`; rows of remote or padded slots are zero.  Small
- * batches run one GEMV per (token, expert) over the coordinate-major sketch;
- * from 8 tokens the pairs, grouped by expert by cfm_route, run on the tensor
- * cores over the row-major sketch (when the layer has one).  Both give the same
- * bits.  Needs cfm_prepare_input and cfm_route of the same rows.
+ * expert.  Writes `partial`; rows of remote or padded slots are zero.  The
+ * pairs, grouped by expert by cfm_route, run on the tensor cores over the
+ * row-major sketch, which also leaves the scores and features; a layer without
+ * one runs a GEMV per (token, expert) over the coordinate-major sketch.  All
+ * give the same bits.  Needs cfm_prepare_input and cfm_route of the same rows.
  * Replaces: _sketch_screen and its helpers (progressive.py:478-1066),
  * _group_screen (:2428-2606). */
 int cfm_screen(const cfm_layer* layer, void* workspace, int32_t capacity,
@@ -241,7 +239,7 @@ int cfm_score(const cfm_layer* layer, void* workspace, int32_t capacity,
  * call's read-cost counters.  When the pairs are grouped by expert (cfm_route of
  * a batch of eight tokens and more) it also leaves the list of the call's down
  * tiles in expert order that cfm_down then reads (cfm_reader_forward builds that
- * list on its side stream beside the exact gather).  Replaces: _select
+ * list beside the exact gather, where the down kernel needs it).  Replaces: _select
  * (progressive.py:1584-1775), _account_fixed (:242-276), _count_reads
  * (:2114-2317). */
 int cfm_select(const cfm_layer* layer, void* workspace, int32_t capacity,
@@ -252,7 +250,9 @@ int cfm_select(const cfm_layer* layer, void* workspace, int32_t capacity,
  * the pairs grouped by expert, the (token, expert) pairs are walked in expert
  * order, so a row several tokens of one expert kept is fetched from HBM once
  * (row engine "per token"), or each expert's union of kept rows is read once and
- * applied to all its tokens (row engine "expert major").  Same bits either way.
+ * applied to all its tokens on the tensor cores (row engine "expert major", and
+ * batches of many tokens per expert).  The activations are the same: sums whose
+ * rounding the order of summation could change are repeated in the gathers' order.
  * Replaces: _acquire with END == H (progressive.py:1372-1581), _group_union
  * (:2609-2652), _group_complete (:2655-2718). */
 int cfm_exact(const cfm_layer* layer, void* workspace, int32_t capacity,
@@ -260,8 +260,8 @@ int cfm_exact(const cfm_layer* layer, void* workspace, int32_t capacity,
 
 /* Down: channel-major down rows of the kept candidates, weighted by their
  * activations, FP32 partial sums per tile of 64 kept rows (per token, tiles in
- * expert order when the pairs are grouped) or per (token, slot, channel range)
- * with the expert's union of kept rows read once (row engine "expert major").
+ * expert order when the pairs are grouped), or one BF16 sum per (token, slot) with
+ * the expert's union of kept rows read once (many tokens per expert).
  * Replaces: _down (progressive.py:1778-1856), _group_down (:2721-2801). */
 int cfm_down(const cfm_layer* layer, void* workspace, int32_t capacity,
              const cfm_call* call, void* stream);
