@@ -89,7 +89,7 @@ __device__ __forceinline__ void repeat(F&& f) {
 // unions and work lists
 // ---------------------------------------------------------------------------
 constexpr int kUnionTile = 32;  // rows of a tile of the exact kernel
-constexpr int kUnionThreads = 128;
+constexpr int kUnionThreads = 512;
 constexpr int kUnionStagedPairs = 512;  // pairs of an expert whose numbers a CTA stages
 
 // One piece of work of the exact kernel (tile `tile` of expert e's union for `count` pairs from
@@ -113,7 +113,7 @@ __device__ __forceinline__ uint32_t slot_word(const uint32_t* bits, int I, int s
   return 32 * w + 32 > I ? word & 0xffffu : word;
 }
 
-// grid (busy experts), 128 threads.  A CTA makes the union of its expert's kept channels from the
+// grid (busy experts), 512 threads.  A CTA makes the union of its expert's kept channels from the
 // tokens' masks (one OR and one scan over I / 32 words), leaves the channels behind and appends the
 // expert's tiles of 32 channels x passes of `exact_pass` tokens and its passes of `down_pass`
 // tokens to the work lists.  With `early` the grouping is known to be complete when this grid can
