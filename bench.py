@@ -862,7 +862,11 @@ def measure(args, shape, plan, tokens, readers, sharded, batches, stream, rank, 
     h2d = host_in[0].numel() * host_in[0].element_size()
     d2h = host_out[0].numel() * host_out[0].element_size()
     grouped = tokens >= 8 and plan.final_count < plan.candidate_count
-    launches = (10 if distributed else len(STAGES)) + int(grouped) * (2 if distributed else 1)
+    # A whole call: prepare, screen, select, exact, down, output; one more where the exact rows are
+    # read expert-major.
+    unions = tokens >= 16 and tokens * shape.top_k >= 3 * shape.experts if args.row_engine == "auto" \
+        else args.row_engine == "expert_major" and tokens >= 8
+    launches = 10 + 2 * int(grouped) if distributed else 6 + int(unions)
     return {
         "metric": METRIC, "value": tokens * world / (step_ms * 1e-3), "unit": UNIT,
         "n_gpus": world, "steps": args.steps, "warmup": args.warmup,
