@@ -2140,8 +2140,9 @@ static int run_exact_union(const Bound& b, const cfm_call* call, bool whole) {
     if (err != cudaSuccess) return static_cast<int>(err);
   }
   const int tiles = exact_union_tiles(b);
+  const bool early = whole && b.L.F < b.L.N;  // a screen stands between the grouping and the selection
   launch_dependent(k_union, dim3(busy_experts(b)), dim3(kUnionThreads), 0, b.stream, b.L, b.ws, 8 * tiles,
-                   DownUnion::kPass, static_cast<int>(whole));
+                   DownUnion::kPass, static_cast<int>(early));
   const int rc = launched();
   if (rc) return rc;
   const int64_t pairs = static_cast<int64_t>(b.T) * b.L.K;

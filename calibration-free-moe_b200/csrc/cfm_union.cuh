@@ -116,8 +116,11 @@ __device__ __forceinline__ uint32_t slot_word(const uint32_t* bits, int I, int s
 // grid (busy experts), 512 threads.  A CTA makes the union of its expert's kept channels from the
 // tokens' masks (one OR and one scan over I / 32 words), leaves the channels behind and appends the
 // expert's tiles of 32 channels x passes of `exact_pass` tokens and its passes of `down_pass`
-// tokens to the work lists.  With `early` the grouping is known to be complete when this grid can
-// start at all, and is read while the selection still runs.  (When every exact CTA made its
+// tokens to the work lists.  With `early`, in whole calls with a screen, the grouping is read while
+// the selection still runs: this grid cannot start before every CTA of the selection has, those not
+// before every CTA of the screen has released them, and the screen's CTAs release after their wait
+// for k_prepare.  The selection itself releases before it waits, so without a screen nothing orders
+// this grid's start behind the grouping, and the wait comes first.  (When every exact CTA made its
 // expert's union itself, the dependent loads and the scan cost each of them some 5 us, a third of
 // its life at 64 tokens of the 128-expert layer.)
 __global__ void __launch_bounds__(kUnionThreads)
