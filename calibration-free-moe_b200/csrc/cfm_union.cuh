@@ -207,9 +207,10 @@ __global__ void __launch_bounds__(kUnionThreads)
 // tokens' rows travel with the weights because the ring leaves L1 too small to hold them.  The
 // instruction truncates where an FMA rounds, so a sum leaves it after 128 columns and goes on by
 // ordinary additions (RMS error of a gate sum of 2048 columns against FP64: 8.0e-7 without, 4.1e-7
-// with, 2.1e-7 the gathers').  The sums are rounded to BF16 next; where an error of that size could
-// change a rounding (some two in a thousand), the CTA puts the row down and at its end repeats the
-// product as the gathers do it, so that the activations are those of the gathers.
+// with, 2.1e-7 the gathers').  The sums are rounded to BF16 next; where the distance between the two
+// ways of summing could change a rounding (kExactMargin), the CTA lists the row and repeats the
+// product as the gathers do it when the list is full and at its end, so that the activations are
+// those of the gathers.
 // Bound by the way from L2 to the SMs (9 to 11 TB/s, the tokens' rows included; tiles of sixteen rows
 // carried them twice as often): 100 tokens of the 64-expert layer 89 us (132 the gathers per token),
 // 256 of the 256-expert layer 80 (155), 256 of hidden 4096 and width 1536 580 at 5.3 TB/s of HBM
@@ -237,8 +238,17 @@ struct ExactSource {
   const char *gate[4], *x[NT];
 };
 
-// Sums to be repeated that a CTA has room for; any beyond them stay as they are.
-constexpr int kRepeats = 40;
+// Rows to be repeated that a CTA lists before it repeats them.
+constexpr int kRepeats = 64;
+
+// Largest distance of the two ways of summing a gate or up row that is provided for, in units of the
+// row sums' size: per token the largest sum, over eight rows and both matrices, of the quarters'
+// magnitudes.  Other rows than the sum's own count because a quarter whose large terms cancel would
+// say nothing about the roundings inside it.  A measured margin, not a bound: over hidden sizes of
+// 1024 to 4096 the distance was 0.04 of it RMS and 0.37 at most in seven million sums of normal, outlier
+// and Student-t inputs, 0.94 where 98 % of every two adjacent terms of all rows cancel.  One row in a
+// hundred is repeated for it.
+constexpr float kExactMargin = 1.0f / (1 << 19);
 
 // Whether an error of `margin` could round v to another BF16 value.
 __device__ __forceinline__ bool rounds_either_way(float v, float margin) {
@@ -253,7 +263,7 @@ __global__ void __launch_bounds__(ExactUnion<NT>::kThreads, ExactUnion<NT>::kPer
   using X = ExactUnion<NT>;
   constexpr int kSlots = X::kSlots;
   extern __shared__ __align__(128) uint8_t union_shared[];
-  __shared__ int4 repeats[kRepeats];  // pair, expert, channel, place among the union's activations
+  __shared__ int2 repeats[kRepeats];  // place in the grouped list; channel, and row of the union above it
   __shared__ int repeat_count;
   static_assert(sizeof(repeats) >= 33 * sizeof(int), "scratch of the listing");
   grid_dependency_wait();     // the work list is complete
@@ -323,6 +333,32 @@ __global__ void __launch_bounds__(ExactUnion<NT>::kThreads, ExactUnion<NT>::kPer
     repeat<NT>([&](auto n) { copy_async16_at<kTo + 512 * (8 + decltype(n)::value), kFrom>(mine, s.x[n], bytes); });
   };
 
+  // The first `count` rows on the list, one per warp at a time, as the gathers do them.
+  auto repeat_listed = [&](int count) {
+    for (int i = warp; i < count; i += 4) {
+      const int position = repeats[i].x, channel = repeats[i].y & 0xffff, at = repeats[i].y >> 16;
+      const int pair = ws.group_pairs[position], t = pair / L.K;
+      const int candidate = (pair - t * L.K) * L.I + channel;
+      const size_t word = static_cast<size_t>(t) * token_words + (candidate >> 5);
+      const int place = ws.kept_before[word] + __popc(ws.kept_bits[word] & ((1u << (candidate & 31)) - 1));
+      const int chunks = L.H / 8;
+      const uint4* gate = reinterpret_cast<const uint4*>(L.gate_up) +
+                          (static_cast<size_t>(ws.ids[pair]) * 2 * L.I + channel) * chunks;
+      uint4 gw[kExactSweep], uw[kExactSweep];
+      float g_sum, u_sum;
+      exact_dot(gate, gate + static_cast<size_t>(L.I) * chunks,
+                reinterpret_cast<const uint4*>(hidden) + static_cast<size_t>(t) * chunks, chunks, lane, false, gw,
+                uw, g_sum, u_sum);
+      if (lane == 0) {
+        const __nv_bfloat16 feature = __float2bfloat16_rn(exact_feature(g_sum, u_sum, L.activation));
+        ws.activations[static_cast<size_t>(pair) * L.I + channel] = feature;
+        if (by_union) ws.union_activations[static_cast<size_t>(position) * L.I + at] = feature;
+        float* exact = ws.exact + static_cast<size_t>(t) * 2 * L.F + place;
+        exact[0] = g_sum;
+        exact[L.F] = u_sum;
+      }
+    }
+  };
   if (tid == 0) repeat_count = 0;  // ordered by the barriers of the first tile
   UnionWork work = read_work(index), next = read_work(index + stride);
   ExactRows<NT> rows = locate(work);
@@ -355,6 +391,7 @@ __global__ void __launch_bounds__(ExactUnion<NT>::kThreads, ExactUnion<NT>::kPer
     if (more) next_rows = locate(next);
     const UnionWork after = read_work(index + 2 * stride);
 
+    uint32_t doubt = 0;  // of this thread's sums: bit half * NT + n
     float acc[2][NT][2][4];  // [rows][tokens][gate, up]
 #pragma unroll
     for (int half = 0; half < 2; ++half)
@@ -439,17 +476,21 @@ __global__ void __launch_bounds__(ExactUnion<NT>::kThreads, ExactUnion<NT>::kPer
 #pragma unroll
       for (int n = 0; n < NT; ++n) {
         const int token = 8 * n + 2 * tq + (warp & 1);
+        float gate[4], up[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          const float* sums = red + q * X::kSumFloats + lane;
+          gate[q] = sums[(n * 8 + warp) * 32];
+          up[q] = sums[(n * 8 + 4 + warp) * 32];
+        }
+        float size = fmaxf((fabsf(gate[0]) + fabsf(gate[1])) + (fabsf(gate[2]) + fabsf(gate[3])),
+                           (fabsf(up[0]) + fabsf(up[1])) + (fabsf(up[2]) + fabsf(up[3])));
+#pragma unroll
+        for (int w = 4; w < 32; w <<= 1) size = fmaxf(size, __shfl_xor_sync(kFull, size, w));
         if (at >= work.rows || token >= work.count) continue;
         __nv_bfloat16 feature = __float2bfloat16_rn(0.0f);
         const int t = pairs[n] / L.K, bit = ((pairs[n] - t * L.K) * L.I + channel) & 31;
         if ((bits[half][n] >> bit) & 1u) {
-          float gate[4], up[4];
-#pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            const float* sums = red + q * X::kSumFloats + lane;
-            gate[q] = sums[(n * 8 + warp) * 32];
-            up[q] = sums[(n * 8 + 4 + warp) * 32];
-          }
           const float g_sum = (gate[0] + gate[1]) + (gate[2] + gate[3]);
           const float u_sum = (up[0] + up[1]) + (up[2] + up[3]);
           feature = __float2bfloat16_rn(exact_feature(g_sum, u_sum, L.activation));
@@ -458,50 +499,38 @@ __global__ void __launch_bounds__(ExactUnion<NT>::kThreads, ExactUnion<NT>::kPer
                          __popc(bits[half][n] & ((1u << bit) - 1));
           exact[0] = g_sum;
           exact[L.F] = u_sum;
-          const float g_size = (fabsf(gate[0]) + fabsf(gate[1])) + (fabsf(gate[2]) + fabsf(gate[3]));
-          const float u_size = (fabsf(up[0]) + fabsf(up[1])) + (fabsf(up[2]) + fabsf(up[3]));
-          constexpr float kError = 1.0f / (1 << 21);
-          if (rounds_either_way(g_sum, kError * g_size) || rounds_either_way(u_sum, kError * u_size)) {
-            const int place = atomicAdd(&repeat_count, 1);
-            if (place < kRepeats)
-              repeats[place] = make_int4(pairs[n], work.e, channel,
-                                         by_union ? (work.first + token) * L.I + at : -1);
-          }
+          const float margin = kExactMargin * size;
+          if (rounds_either_way(g_sum, margin) || rounds_either_way(u_sum, margin))
+            doubt |= 1u << (half * NT + n);
         }
         if (by_union) ws.union_activations[static_cast<size_t>(work.first + token) * L.I + at] = feature;
       }
       if (half == 0) __syncthreads();  // the sums may be overwritten
     }
-    if (!more) break;
-    __syncthreads();  // the sums may be overwritten
+    for (;;) {
+      for (; doubt; doubt &= doubt - 1) {
+        const int place = atomicAdd(&repeat_count, 1);
+        if (place >= kRepeats) break;
+        const int bit = __ffs(doubt) - 1, half = bit / NT, n = bit - half * NT;
+        const int channel = warp < 2 ? (half ? rows.channel[2] : rows.channel[0])
+                                     : (half ? rows.channel[3] : rows.channel[1]);
+        repeats[place] = make_int2(work.first + 8 * n + 2 * tq + (warp & 1),
+                                   channel | (work.tile * kUnionTile + 16 * half + g + 8 * (warp >> 1)) << 16);
+      }
+      // The sums may be overwritten, the list is complete, what the tile left for its rows is written.
+      __syncthreads();
+      const int listed = repeat_count;
+      if (more && listed <= kRepeats) break;
+      repeat_listed(min(listed, kRepeats));
+      if (listed <= kRepeats) return;
+      __syncthreads();
+      if (tid == 0) repeat_count = 0;
+      __syncthreads();
+    }
     index += stride;
     work = next;
     next = after;
     rows = next_rows;
-  }
-  __syncthreads();  // the list is complete, the activations of the rows on it are written
-  for (int i = warp; i < min(repeat_count, kRepeats); i += 4) {
-    const int4 r = repeats[i];
-    const int t = r.x / L.K, candidate = (r.x - t * L.K) * L.I + r.z;
-    const size_t word = static_cast<size_t>(t) * token_words + (candidate >> 5);
-    const uint32_t kept = ws.kept_bits[word];
-    const int place = ws.kept_before[word] + __popc(kept & ((1u << (candidate & 31)) - 1));
-    const int chunks = L.H / 8;
-    const uint4* gate = reinterpret_cast<const uint4*>(L.gate_up) +
-                        (static_cast<size_t>(r.y) * 2 * L.I + r.z) * chunks;
-    uint4 gw[kExactSweep], uw[kExactSweep];
-    float g_sum, u_sum;
-    exact_dot(gate, gate + static_cast<size_t>(L.I) * chunks,
-              reinterpret_cast<const uint4*>(hidden) + static_cast<size_t>(t) * chunks, chunks, lane, false, gw, uw,
-              g_sum, u_sum);
-    if (lane == 0) {
-      const __nv_bfloat16 feature = __float2bfloat16_rn(exact_feature(g_sum, u_sum, L.activation));
-      ws.activations[static_cast<size_t>(r.x) * L.I + r.z] = feature;
-      if (r.w >= 0) ws.union_activations[r.w] = feature;
-      float* exact = ws.exact + static_cast<size_t>(t) * 2 * L.F + place;
-      exact[0] = g_sum;
-      exact[L.F] = u_sum;
-    }
   }
 }
 

@@ -6,6 +6,8 @@ import pytest
 import torch
 
 import cases
+from cfm_b200.reader.budget import compile_budget
+from cfm_b200.reader.progressive import ProgressiveReader
 from helpers import prepared_case, run_oracle
 from test_gpu_parity import make_reader
 
@@ -46,3 +48,69 @@ def test_unscreened_calls_that_change_their_routes(oracle, shape):
     case.hidden, case.ids, case.weights, case.padding = hidden, ids, weights, padding
     want = run_oracle(oracle, item, norms=reader.norms.cpu())
     torch.testing.assert_close(outs[1].cpu().float(), want["output"], rtol=0.025, atol=0.02)
+
+
+def _layer(experts, hidden, width, top_k, rank, seed=3):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    gate_up = torch.empty(experts, 2 * width, hidden, device="cuda", dtype=torch.bfloat16).normal_(0, 0.02, generator=g)
+    down = torch.empty(experts, width, hidden, device="cuda", dtype=torch.bfloat16).normal_(0, 0.02, generator=g)
+    down = down.transpose(1, 2)
+    if not rank:
+        return gate_up, down, None, None
+    decoder = torch.linalg.qr(torch.randn(hidden, rank, device="cuda", generator=g)).Q.bfloat16()
+    return gate_up, down, torch.matmul(decoder.T, down), decoder
+
+
+def _inputs(kind, tokens, hidden, experts, top_k, seed):
+    """Hidden rows and routes; outliers: one column in a hundred is twenty times as large."""
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    x = torch.randn(tokens, hidden, device="cuda", generator=g)
+    if kind == "outliers":
+        x[:, torch.randperm(hidden, device="cuda", generator=g)[: hidden // 100]] *= 20
+    elif kind == "student_t":
+        x /= (torch.randn(tokens, hidden, 3, device="cuda", generator=g).square().sum(-1) / 3).sqrt()
+    ids = torch.rand(tokens, experts, device="cuda", generator=g).topk(top_k, dim=1).indices.int().contiguous()
+    weights = torch.rand(tokens, top_k, device="cuda", generator=g) * 0.6 + 0.2
+    return x.bfloat16(), ids, weights
+
+
+def _readers(layer, plan, tokens, **options):
+    return [ProgressiveReader(*layer, plan, tokens, selection_score="point", sketch_builder="cuda",
+                              retain_reference_sketch=False, row_engine=engine, **options)
+            for engine in ("auto", "per_token")]
+
+
+# hidden, width, experts, top_k, rank, tokens, retention
+WIDE = {
+    "kept-256": (2048, 768, 40, 8, 64, 256, 1.0),
+    "kept-1024": (2048, 768, 40, 8, 64, 1024, 1.0),
+    "screened-96": (2048, 512, 40, 8, 64, 96, 0.125),
+    "screened-200": (4096, 320, 24, 6, 128, 200, 0.25),
+    "screened-130": (1152, 208, 66, 5, 16, 130, 0.2),
+}
+
+
+@pytest.mark.parametrize("inputs", ["normal", "outliers", "student_t"])
+@pytest.mark.parametrize("name", WIDE)
+def test_activations_are_those_of_the_gathers(name, inputs):
+    """Bit by bit, however many sums of a CTA are in doubt, and again in every call."""
+    h, i, e, k, rank, tokens, retention = WIDE[name]
+    plan = compile_budget(hidden_size=h, expert_width=i, top_k=k, retention=retention,
+                          screen_keep=1.0 if retention == 1.0 else 0.625)
+    reader, plain = _readers(_layer(e, h, i, k, rank), plan, tokens)
+    call = _inputs(inputs, tokens, h, e, k, 7)
+
+    def kept(r):
+        lists = r.candidate_ids[-1][:tokens].long()
+        return r.activations[:tokens].view(tokens, -1).gather(1, lists.clamp_min(0)).view(torch.int16)
+
+    plain(*call)
+    want = kept(plain)
+    first = reader(*call)
+    assert torch.equal(reader.candidate_ids[-1][:tokens], plain.candidate_ids[-1][:tokens])
+    sums = reader.workspace.exact.clone()
+    for _ in range(10):
+        assert torch.equal(kept(reader), want)
+        reader.activations.zero_()
+        assert torch.equal(reader(*call), first)
+    assert torch.equal(reader.workspace.exact, sums)
