@@ -545,6 +545,9 @@ __global__ void __launch_bounds__(ExactUnion<NT>::kThreads, ExactUnion<NT>::kPer
 // rows lie 144 bytes apart, which keeps the eight of a matrix in different banks.  Union row
 // 4 a + 2 b + i of a unit is the instruction's row 8 b + 2 a + i, so that a lane's four activations
 // are adjacent in memory.  Rows beyond the union are another row's weights and meet zeros.
+// The instruction truncates, so a sum leaves it after four units and goes on by ordinary additions
+// (of 786,432 sums over 1536 rows 92 round to another BF16 value than the sum in 64 bits does, 90 of
+// the gathers' and 819 of one chain).
 // The recovery encoder is the same product with an expert's whole width as its rows and the sketch
 // features (zero for kept channels, k_select) as activations; its pieces, the longest, come first.
 // Pieces differ in length with the unions and the number of passes, so warps claim them one at a
@@ -560,6 +563,7 @@ struct DownUnion {
   static constexpr int kSlots = 5;
   static constexpr int kRowBytes = 144;
   static constexpr int kUnitBytes = 16 * kRowBytes;
+  static constexpr int kFold = 4;  // units after which a sum leaves the tensor cores
   static constexpr int kSlotBytes = kUnitBytes + 512;
   static constexpr int kSharedBytes = 4 * kSlots * kSlotBytes;
 };
@@ -701,11 +705,12 @@ __global__ void __launch_bounds__(DownUnion::kThreads, DownUnion::kPerSm)
     int pairs[2];
 #pragma unroll
     for (int n = 0; n < 2; ++n) pairs[n] = 8 * n + g < count ? ws.group_pairs[first + 8 * n + g] : -1;
-    float acc[8][4];
+    float acc[8][4], part[8][4];  // of all the rows, of the last few units
 #pragma unroll
     for (int n = 0; n < 8; ++n)
 #pragma unroll
-      for (int i = 0; i < 4; ++i) acc[n][i] = 0.0f;
+      for (int i = 0; i < 4; ++i) acc[n][i] = part[n][i] = 0.0f;
+    int turn = 0;
     do {
       copy_async_wait<kSlots - 2>();
       __syncwarp();  // every lane's copies of the unit have landed; the unit before has been read
@@ -728,11 +733,21 @@ __global__ void __launch_bounds__(DownUnion::kThreads, DownUnion::kPerSm)
         constexpr int kPart = decltype(m)::value;
         uint32_t w[4];
         load_matrices_transposed_at<32 * kPart>(w, load_from + get);
-        mma_bf16(acc[2 * kPart], a, w[0], w[1]);
-        mma_bf16(acc[2 * kPart + 1], a, w[2], w[3]);
+        mma_bf16(part[2 * kPart], a, w[0], w[1]);
+        mma_bf16(part[2 * kPart + 1], a, w[2], w[3]);
       });
       get = get == (kSlots - 1) * X::kSlotBytes ? 0 : get + X::kSlotBytes;
       left -= 16;
+      if (++turn == X::kFold || left <= 0) {
+        turn = 0;
+#pragma unroll
+        for (int n = 0; n < 8; ++n)
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            acc[n][i] += part[n][i];
+            part[n][i] = 0.0f;
+          }
+      }
     } while (left > 0);
     // A token's sum over the expert, rounded to BF16 as the mix takes it.
     const bool encoder = piece < encoder_blocks;
