@@ -2102,12 +2102,15 @@ static bool exact_by_union(const Bound& b) {
   return b.L.row_engine == CFM_ROWS_EXPERT_MAJOR ||
          (b.T >= 16 && static_cast<int64_t>(b.T) * b.L.K >= 3 * static_cast<int64_t>(b.L.E));
 }
-// The expert-major down kernel where most experts have more than half a pass of sixteen tokens and
-// there is a piece for every second warp: 64 tokens of the 128-expert layer 45 us in all against 37 of
-// the tiles per token and their output, 100 of the 64-expert layer 57 against 80, 256 of the 256-expert
-// layer 65 against 107.
+// The expert-major down kernel, on request only: its sums depend in their last FP32 bits on what the
+// other tokens of an expert kept, while the tiles give a token the same bits in every batch.  Where
+// most experts have more than half a pass of sixteen tokens and there is a piece for every second
+// warp: 64 tokens of the 128-expert layer 45 us in all against 37 of the tiles per token and their
+// output, whole calls of 256 tokens 280 against 310 (256-expert layer) and 1494 against 1830 (hidden
+// 4096, width 1536).  (Repeating the sums that the distance could round otherwise, one in a hundred,
+// costs more than the tiles: 3390 us there, most of it for single columns of rows that have left L2.)
 static bool down_by_union(const Bound& b) {
-  return exact_by_union(b) && shares_decode(b) &&
+  return exact_by_union(b) && b.L.row_engine == CFM_ROWS_EXPERT_MAJOR && shares_decode(b) &&
          static_cast<int64_t>(busy_experts(b)) * (b.L.H / DownUnion::kColumns) >= 148 * 8;
 }
 // The recovery encoder in the expert-major down launch.

@@ -14,8 +14,9 @@
 // instruction count: per row and eight tokens a matrix instruction replaces some fifty loads,
 // conversions and FMAs, which is what gathers per token are bound by once tokens share experts.
 // A token's gate and up sums depend on its own row and the weights only, in an order fixed by H
-// (quarters of H, columns ascending inside a quarter); its down sums go sixteen union rows at a
-// time and depend in their last FP32 bits on the channels the other tokens of an expert kept.
+// (quarters of H, columns ascending inside a quarter), and round as the gathers' do; its down and
+// encoder sums go sixteen union rows at a time and depend in their last FP32 bits on the channels
+// the other tokens of an expert kept, which is why the last two kernels run on request only.
 // The exact and down kernels are persistent and take their work from flat lists, so experts of
 // very different load keep all SMs busy, and their copies run ahead from one piece of work into
 // the next.  Included by cfm_reader.cu inside namespace cfm.

@@ -252,12 +252,17 @@ class ProgressiveReader:
         tensor-core path of the expert-major screen: "mma_sync" (default: chosen by
         size) or "tcgen05" (tensor-memory accumulators at every size); both give the
         same bits; and `row_engine`, how batches of eight tokens and more read the
-        native rows: "expert_major" (a row several tokens of one expert kept is read
-        once for all of them), "per_token" (one gather per token, tokens of one expert
-        next to each other in time so that shared rows meet in L2) or "auto"
-        (expert-major from three tokens per expert on, the faster one on the shapes
-        measured).  The kept channels do not depend on it; outputs differ by FP32
-        summation order only.
+        native rows: "per_token" (one gather per token, tokens of one expert next to
+        each other in time so that shared rows meet in L2), "auto" (from three tokens
+        per expert on a gate/up row that several tokens of one expert kept is read
+        once for all of them) or "expert_major" (the same in every batch of eight
+        tokens and more, and in batches of many tokens per expert the down and encoder
+        rows too).  The kept channels and the activations do not depend on it.
+        "per_token" and "auto" give a token the same output bits in every batch;
+        with "expert_major" the FP32 order of a token's down and encoder sums depends
+        on which channels the other tokens of its experts kept, so its last BF16 bits
+        can change with the batch (256 tokens of the largest layers measured take a
+        tenth to a fifth less time for it).
         `sketch_builder` picks who builds the sketch when none is given: "torch"
         (tensor operations, byte-identical to the reference builder on the same
         device) or "cuda" (the library's kernel, straight into the kernel layouts,

@@ -44,9 +44,12 @@ extern "C" {
 #define CFM_SCORE_RECOVERY_AWARE 1
 #define CFM_ENGINE_MMA_SYNC 0 /* warp-level mma.sync.m16n8k32 (default: measured faster) */
 #define CFM_ENGINE_TCGEN05 1  /* tcgen05.mma kind::i8, accumulators in tensor memory     */
-#define CFM_ROWS_AUTO 0        /* the library's choice (per token, pairs in expert order) */
+#define CFM_ROWS_AUTO 0        /* the library's choice; a token's output bits do not depend on it
+                                  or on the batch                                         */
 #define CFM_ROWS_PER_TOKEN 1   /* native rows always gathered per token                 */
-#define CFM_ROWS_EXPERT_MAJOR 2 /* expert-major whenever the pairs are grouped (T >= 8) and no expert_map */
+#define CFM_ROWS_EXPERT_MAJOR 2 /* expert-major whenever the pairs are grouped (T >= 8) and no expert_map,
+                                  down and encode too in batches of many tokens per expert:
+                                  last FP32 bits of a token's sums then depend on its batch */
 #define CFM_READ_WORK_SLOTS 20
 
 /* One MoE layer: dimensions and resident tensors.  Mirrors the state
@@ -251,7 +254,7 @@ int cfm_select(const cfm_layer* layer, void* workspace, int32_t capacity,
  * order, so a row several tokens of one expert kept is fetched from HBM once
  * (row engine "per token"), or each expert's union of kept rows is read once and
  * applied to all its tokens on the tensor cores (row engine "expert major", and
- * batches of many tokens per expert).  The activations are the same: sums whose
+ * batches of many tokens per expert).  The activations are the same bits: sums whose
  * rounding the order of summation could change are repeated in the gathers' order.
  * Replaces: _acquire with END == H (progressive.py:1372-1581), _group_union
  * (:2609-2652), _group_complete (:2655-2718). */
@@ -261,7 +264,8 @@ int cfm_exact(const cfm_layer* layer, void* workspace, int32_t capacity,
 /* Down: channel-major down rows of the kept candidates, weighted by their
  * activations, FP32 partial sums per tile of 64 kept rows (per token, tiles in
  * expert order when the pairs are grouped), or one BF16 sum per (token, slot) with
- * the expert's union of kept rows read once (many tokens per expert).
+ * the expert's union of kept rows read once (row engine "expert major" and many
+ * tokens per expert; the order of a sum then depends on the expert's other tokens).
  * Replaces: _down (progressive.py:1778-1856), _group_down (:2721-2801). */
 int cfm_down(const cfm_layer* layer, void* workspace, int32_t capacity,
              const cfm_call* call, void* stream);
@@ -269,7 +273,7 @@ int cfm_down(const cfm_layer* layer, void* workspace, int32_t capacity,
 /* Recovery encode: sketch features of the skipped channels through the
  * encoder rows, then the router-weighted latent; per (token, expert) pair, or
  * with an expert's encoder rows read once for all its tokens (row engine "expert
- * major"; same bits).  Replaces: _encode and _latent (progressive.py:1859-2016),
+ * major" and many tokens per expert: another order of the sums).  Replaces: _encode and _latent (progressive.py:1859-2016),
  * _group_encode (:2804-2865). */
 int cfm_encode(const cfm_layer* layer, void* workspace, int32_t capacity,
                const cfm_call* call, void* stream);

@@ -125,11 +125,12 @@ def test_results_do_not_depend_on_batch_or_capacity(oracle):
     """Each token's selection is the same alone, in a batch, or in a larger workspace; so is its
     output within one kind of kernels.
 
-    Batches of eight tokens and more read the experts' rows expert-major, smaller ones per
-    token: between the two the FP32 sums are associated differently, and the outputs agree
-    within the tolerance the reference allows between its own two paths (rtol 0.016, atol
-    2e-3, tests/test_progressive_reader.py:875-978 of the reference).  Inside the
-    expert-major path a token's sums do not depend on which other tokens share its experts.
+    On request batches of eight tokens and more read the experts' rows expert-major.  Its
+    outputs agree with those per token within the tolerance the reference allows between its
+    own two paths (rtol 0.016, atol 2e-3, tests/test_progressive_reader.py:875-978 of the
+    reference).  This layer stays below the sizes from which the down rows are read
+    expert-major too, so here a token's sums do not depend on which other tokens share its
+    experts; above them they do (tests/test_gpu_row_engines.py).
     """
     item = prepared("qwen3-e16-t8")
     case = item["case"]

@@ -9,7 +9,8 @@ import cases
 from cfm_b200.reader.budget import compile_budget
 from cfm_b200.reader.progressive import ProgressiveReader
 from helpers import prepared_case, run_oracle
-from test_gpu_parity import make_reader
+from test_gpu_edges import LAYERS
+from test_gpu_parity import make_reader, run_reader
 
 pytestmark = pytest.mark.gpu
 
@@ -74,10 +75,15 @@ def _inputs(kind, tokens, hidden, experts, top_k, seed):
     return x.bfloat16(), ids, weights
 
 
-def _readers(layer, plan, tokens, **options):
+def _readers(layer, plan, tokens, engine="auto"):
     return [ProgressiveReader(*layer, plan, tokens, selection_score="point", sketch_builder="cuda",
-                              retain_reference_sketch=False, row_engine=engine, **options)
-            for engine in ("auto", "per_token")]
+                              retain_reference_sketch=False, row_engine=which) for which in (engine, "per_token")]
+
+
+def _plan(name):
+    h, i, e, k, _, _, retention = WIDE[name]
+    return compile_budget(hidden_size=h, expert_width=i, top_k=k, retention=retention,
+                          screen_keep=1.0 if retention == 1.0 else 0.625)
 
 
 # hidden, width, experts, top_k, rank, tokens, retention
@@ -94,10 +100,8 @@ WIDE = {
 @pytest.mark.parametrize("name", WIDE)
 def test_activations_are_those_of_the_gathers(name, inputs):
     """Bit by bit, however many sums of a CTA are in doubt, and again in every call."""
-    h, i, e, k, rank, tokens, retention = WIDE[name]
-    plan = compile_budget(hidden_size=h, expert_width=i, top_k=k, retention=retention,
-                          screen_keep=1.0 if retention == 1.0 else 0.625)
-    reader, plain = _readers(_layer(e, h, i, k, rank), plan, tokens)
+    h, i, e, k, rank, tokens, _ = WIDE[name]
+    reader, plain = _readers(_layer(e, h, i, k, rank), _plan(name), tokens)
     call = _inputs(inputs, tokens, h, e, k, 7)
 
     def kept(r):
@@ -123,7 +127,7 @@ def test_down_sums_are_as_near_to_64_bits_as_the_gathers():
     h, i, e, k, tokens = 2048, 1536, 40, 4, 96
     plan = compile_budget(hidden_size=h, expert_width=i, top_k=k, retention=1.0, screen_keep=1.0)
     layer = _layer(e, h, i, k, 0)
-    reader, plain = _readers(layer, plan, tokens)
+    reader, plain = _readers(layer, plan, tokens, "expert_major")
     call = _inputs("normal", tokens, h, e, k, 11)
     reader(*call)
     plain(*call)
@@ -140,3 +144,74 @@ def test_down_sums_are_as_near_to_64_bits_as_the_gathers():
         wrong += torch.stack([(sums[t].bfloat16() != want).sum(), (union[t] != want).sum()])
     gathers, unions = wrong.tolist()
     assert 0 < gathers and unions <= 2 * gathers
+
+
+@pytest.mark.parametrize("inputs", ["normal", "outliers", "student_t"])
+@pytest.mark.parametrize("name", WIDE)
+def test_outputs_do_not_depend_on_the_batch(name, inputs):
+    """Bit by bit: the gathers per token, the unions of the whole batch, and tokens on their own."""
+    h, i, e, k, rank, tokens, _ = WIDE[name]
+    reader, plain = _readers(_layer(e, h, i, k, rank), _plan(name), tokens)
+    call = _inputs(inputs, tokens, h, e, k, 13)
+    want, latent = plain(*call), plain.latent[:tokens].clone()
+    out = reader(*call)
+    assert torch.equal(out, want)
+    if rank:
+        assert torch.equal(reader.latent[:tokens], latent)
+    for first, count in ((0, 1), (tokens - 1, 1), (tokens // 3, 9), (5, tokens // 2), (tokens // 2, tokens // 3)):
+        part = reader(*(x[first : first + count] for x in call))
+        assert torch.equal(part, want[first : first + count])
+
+
+@pytest.mark.parametrize("padded", [False, True])
+@pytest.mark.parametrize("name", [n for n in LAYERS if n.startswith("union")])
+def test_outputs_at_the_edges_are_those_of_the_gathers(name, padded):
+    h, i, e, k, rank, tokens, retention, keep, activation, score, _ = LAYERS[name]
+    padding = [t % 5 == 1 for t in range(tokens)] if padded else None
+    item = prepared_case(cases._random(name, h + i + tokens, h, i, e, k, rank, tokens, retention, keep, activation,
+                                       padding=padding, score=score))
+    unions, plain = (make_reader(item, row_engine=engine) for engine in ("auto", "per_token"))
+    want, out = run_reader(plain, item["case"]), run_reader(unions, item["case"])
+    assert torch.equal(out, want)
+    if rank:
+        assert torch.equal(unions.latent[:tokens], plain.latent[:tokens])
+
+
+@pytest.mark.parametrize("name", ["kept-256", "screened-96"])
+def test_expert_major_down_sums(name):
+    """On request the down and encoder rows are read expert-major too: the same bits in every call, those
+    of the gathers but for roundings that the order of summation turns."""
+    h, i, e, k, rank, tokens, _ = WIDE[name]
+    reader, plain = _readers(_layer(e, h, i, k, rank), _plan(name), tokens, "expert_major")
+    call = _inputs("outliers", tokens, h, e, k, 19)
+    claims = 4  # of `work_counts`: pieces the expert-major down kernel has claimed
+    want = plain(*call)
+    assert plain.workspace.work_counts[claims] == 0
+    first = reader(*call)
+    assert reader.workspace.work_counts[claims] > 0
+    torch.testing.assert_close(first.float(), want.float(), rtol=0.016, atol=2e-3)
+    for _ in range(10):
+        assert torch.equal(reader(*call), first)
+
+
+@pytest.mark.parametrize("padded", [False, True])
+@pytest.mark.parametrize("name", [n for n in LAYERS if n.startswith("union-down")])
+def test_expert_major_down_at_the_edges(name, padded):
+    """The whole call, and its stages on their own, twice where they claim their work."""
+    h, i, e, k, rank, tokens, retention, keep, activation, score, _ = LAYERS[name]
+    padding = [t % 5 == 1 for t in range(tokens)] if padded else None
+    item = prepared_case(cases._random(name, h + i + tokens, h, i, e, k, rank, tokens, retention, keep, activation,
+                                       padding=padding, score=score))
+    case = item["case"]
+    unions, plain = (make_reader(item, row_engine=engine) for engine in ("expert_major", "per_token"))
+    want, out = run_reader(plain, case), run_reader(unions, case).clone()
+    assert unions.workspace.work_counts[4] > 0
+    torch.testing.assert_close(out.float(), want.float(), rtol=0.016, atol=2e-3)
+    device = [x.cuda() if x is not None else None for x in (case.hidden, case.ids, case.weights, case.padding)]
+    again = torch.empty_like(out)
+    call = unions._call_struct(tokens, *device, again, False)
+    for stage in ("cfm_prepare_input", "cfm_route", "cfm_screen", "cfm_select", "cfm_exact", "cfm_down", "cfm_down",
+                  "cfm_encode", "cfm_output"):
+        unions._stage(stage, call)
+    torch.cuda.synchronize()
+    torch.testing.assert_close(again.float(), want.float(), rtol=0.016, atol=2e-3)
