@@ -556,11 +556,13 @@ __global__ void __launch_bounds__(ExactUnion<NT>::kThreads, ExactUnion<NT>::kPer
 // idle while the longest pieces ended (85 us at 256 tokens of the 256-expert layer, 55 with claims;
 // the tiles per token take 79).  Bound by latency and instruction issue: 126 instructions per unit of
 // 2 KB.  256 tokens of hidden 4096 and width 1536 373 us at 4.7 TB/s of HBM (651 the tiles per token).
+// A row with a weight that is not finite would meet the zeros of tokens that did not keep it and leave
+// them NaN: sums that are NaN are repeated over the token's own rows, as the tiles add them.
 struct DownUnion {
   static constexpr int kThreads = 128;
   static constexpr int kPass = 16;
   static constexpr int kColumns = 64;
-  static constexpr int kPerSm = 4;
+  static constexpr int kPerSm = 3;  // four would spill in the loop: 1577 us for 1525 at the widest, 297 for 285
   static constexpr int kSlots = 5;
   static constexpr int kRowBytes = 144;
   static constexpr int kUnitBytes = 16 * kRowBytes;
@@ -568,6 +570,36 @@ struct DownUnion {
   static constexpr int kSlotBytes = kUnitBytes + 512;
   static constexpr int kSharedBytes = 4 * kSlots * kSlotBytes;
 };
+
+// The lane with the `index`-th of the bits, or -1.
+__device__ __forceinline__ int lane_of_bit(unsigned bits, int index) {
+  for (; index > 0; --index) bits &= bits - 1;
+  return __ffs(bits) - 1;
+}
+
+// One column of a pair's down sum as down_tile and the output add it: tiles of 64 of the `rows` kept
+// candidates of `list`, four chains of every fourth row in a tile.  Four adjacent lanes per sum, one
+// chain each; all lanes of the warp call it (with no rows: for nothing).  `weights`: the column in the
+// row of candidate 0.
+__device__ __forceinline__ float repeat_down_sum(const int32_t* list, const __nv_bfloat16* values,
+                                              const __nv_bfloat16* weights, int H, int rows) {
+  const int lane = threadIdx.x & 31, base = lane & ~3;
+  const int most = __reduce_max_sync(kFull, rows);
+  float sum = 0.0f;
+  for (int r0 = 0; r0 < most; r0 += kDownTileRows) {
+    float chain = 0.0f;
+    for (int r = r0 + (lane & 3); r < min(rows, r0 + kDownTileRows); r += 4) {
+      const int candidate = list[r];
+      chain = fmaf(__bfloat162float(weights[static_cast<int64_t>(candidate) * H]), __bfloat162float(values[candidate]),
+                   chain);
+    }
+    __syncwarp();
+    const float c0 = __shfl_sync(kFull, chain, base), c1 = __shfl_sync(kFull, chain, base + 1);
+    const float c2 = __shfl_sync(kFull, chain, base + 2), c3 = __shfl_sync(kFull, chain, base + 3);
+    if (r0 < rows) sum += ((c0 + c1) + c2) + c3;
+  }
+  return sum;
+}
 
 // `encoder_blocks`: column blocks of the recovery encoder, or 0 without it; `blocks_magic`:
 // floor(2^32 / (H / 64)) + 1, which divides piece numbers exactly.
@@ -754,15 +786,38 @@ __global__ void __launch_bounds__(DownUnion::kThreads, DownUnion::kPerSm)
     const bool encoder = piece < encoder_blocks;
     const int width = encoder ? L.R : L.H;
     const int column = (encoder ? piece : piece - encoder_blocks) * X::kColumns;
-    __nv_bfloat16* out = reinterpret_cast<__nv_bfloat16*>(encoder ? ws.encoder_parts : ws.down_parts) + column + 2 * tq;
+    __nv_bfloat16* out = reinterpret_cast<__nv_bfloat16*>(encoder ? ws.encoder_parts : ws.down_parts) + column;
+    uint32_t repeat = 0;  // bit 16 n + 2 c + b: column 8 c + 2 tq + b of token 8 n + g
 #pragma unroll
     for (int n = 0; n < 2; ++n) {
       if (pairs[n] < 0) continue;
-      __nv_bfloat16* row = out + static_cast<size_t>(pairs[n]) * width;
+      __nv_bfloat16* row = out + static_cast<size_t>(pairs[n]) * width + 2 * tq;
 #pragma unroll
       for (int c = 0; c < 8; ++c)
-        if (column + 8 * c < width)
+        if (column + 8 * c < width) {
           *reinterpret_cast<__nv_bfloat162*>(row + 8 * c) = __floats2bfloat162_rn(acc[c][2 * n], acc[c][2 * n + 1]);
+          repeat |= static_cast<uint32_t>(isnan(acc[c][2 * n])) << (16 * n + 2 * c);
+          repeat |= static_cast<uint32_t>(isnan(acc[c][2 * n + 1])) << (16 * n + 2 * c + 1);
+        }
+    }
+    if (encoder) continue;  // the encoder rows meet every token's zeros in encode_tile too
+    __syncwarp();           // the sums stored above may be replaced
+    for (;;) {
+      const unsigned any = __ballot_sync(kFull, repeat != 0);
+      if (!any) break;
+      // The first of the sums of up to eight lanes, each for four lanes.
+      const int source = lane_of_bit(any, lane >> 2), from = max(source, 0);
+      const uint32_t bits = __shfl_sync(kFull, repeat, from);
+      const int low = __shfl_sync(kFull, pairs[0], from), high = __shfl_sync(kFull, pairs[1], from);
+      const int bit = __ffs(bits) - 1, pair = source < 0 ? -1 : bit & 16 ? high : low;
+      const int of = column + 8 * ((bit >> 1) & 7) + 2 * (from & 3) + (bit & 1);
+      const int p = max(pair, 0), t = p / L.K;
+      const float sum = repeat_down_sum(
+          ws.candidate_ids + static_cast<size_t>(t) * L.F + ws.starts[p], ws.activations + static_cast<size_t>(t) * L.N,
+          L.down + (static_cast<int64_t>(ws.ids[p]) - (p - t * L.K)) * L.I * L.H + of, L.H, pair < 0 ? 0 : ws.counts[p]);
+      if (pair >= 0 && (lane & 3) == 0)
+        out[static_cast<size_t>(pair) * width + of - column] = __float2bfloat16_rn(sum);
+      if (__popc(any & ((1u << lane) - 1)) < 8) repeat &= repeat - 1;
     }
   }
 }

@@ -215,3 +215,21 @@ def test_expert_major_down_at_the_edges(name, padded):
         unions._stage(stage, call)
     torch.cuda.synchronize()
     torch.testing.assert_close(again.float(), want.float(), rtol=0.016, atol=2e-3)
+
+
+@pytest.mark.parametrize("engine", ["auto", "expert_major"])
+def test_a_row_that_is_not_finite_reaches_only_tokens_that_kept_it(engine):
+    h, i, e, k, rank, tokens, _ = WIDE["screened-96"]
+    layer = _layer(e, h, i, k, rank)
+    reader, plain = _readers(layer, _plan("screened-96"), tokens, engine)
+    call = _inputs("normal", tokens, h, e, k, 17)
+    reader(*call)
+    chosen = reader.candidate_ids[-1][0, 0].item()  # a channel the first token keeps
+    expert, channel = reader.ids[0, chosen // i].item(), chosen % i
+    layer[1][expert, :, channel] = float("inf")  # the native weights are read in place
+    out, want = reader(*call), plain(*call)
+    keeps = ((reader.ids[:tokens] == expert)[:, :, None] & reader.selected[:tokens].view(tokens, k, i))[:, :, channel]
+    assert keeps.any() and not keeps.any(1).all()
+    assert out[~keeps.any(1)].isfinite().all() and not out[keeps.any(1)].isfinite().any()
+    assert torch.equal(out.isnan(), want.isnan())
+    torch.testing.assert_close(out.float().nan_to_num(), want.float().nan_to_num(), rtol=0.016, atol=2e-3)
