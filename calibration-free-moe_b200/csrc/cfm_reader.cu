@@ -1821,6 +1821,8 @@ struct Bound {
   const uint8_t* padding;
 };
 
+static bool screens_grouped(const Bound& b);
+
 static int bind_call(const cfm_layer* layer, void* workspace, int32_t capacity,
                      const cfm_call* call, void* stream, Bound* b) {
   if (!layer || !workspace || !call) return CFM_E_NULL;
@@ -1837,8 +1839,7 @@ static int bind_call(const cfm_layer* layer, void* workspace, int32_t capacity,
   if (layer->row_engine < CFM_ROWS_AUTO || layer->row_engine > CFM_ROWS_EXPERT_MAJOR)
     return CFM_E_UNSUPPORTED;
   const bool screened = layer->final_count < layer->top_k * layer->width;
-  if (screened && (!layer->sketch || !layer->statistics || !layer->norms || !layer->signs))
-    return CFM_E_NULL;
+  if (screened && (!layer->statistics || !layer->norms || !layer->signs)) return CFM_E_NULL;
   if (layer->rank && (!layer->encoder || !layer->decoder)) return CFM_E_NULL;
   b->L = device_layer(layer);
   b->ws = bind(layout, workspace, capacity);
@@ -1846,6 +1847,8 @@ static int bind_call(const cfm_layer* layer, void* workspace, int32_t capacity,
   b->T = call->tokens;
   b->row_offset = call->row_offset;
   b->padding = call->padding;
+  // Without a row-major sketch that the expert-major screen can read, the coordinate-major one is.
+  if (screened && !layer->sketch && !screens_grouped(*b)) return CFM_E_NULL;
   return 0;
 }
 

@@ -362,8 +362,8 @@ class ShardedScreenEngine:
 class _HomeScreen:
     """Screen, selection and recovery latent of a rank's own tokens over all experts.
 
-    Holds the replicated part of an expert-parallel layer: the sketch (both kernel
-    layouts), its scales, the down-column norms, the transposed recovery encoder
+    Holds the replicated part of an expert-parallel layer: the sketch (the row-major
+    layout, which the screen reads), its scales, the down-column norms, the transposed recovery encoder
     and the recovery geometry of every expert, gathered from the ranks that built
     them for their own experts, and a workspace for this rank's tokens.
     """
@@ -375,7 +375,6 @@ class _HomeScreen:
         def gather(local: Tensor | None) -> Tensor | None:
             return _all_gather_rows(local.contiguous(), world, group) if local is not None else None
 
-        self.sketch_words = gather(owner.sketch_words)
         self.sketch_grouped_words = gather(owner.sketch_grouped_words)
         # Physical layout of the statistics is [E, B, 2, 2I].
         self.sketch_statistics = gather(owner.sketch_statistics.permute(0, 2, 3, 1))
@@ -396,9 +395,8 @@ class _HomeScreen:
         layer.experts, layer.rank = experts, self.rank
         layer.global_experts, layer.recovery_owner = 0, 1
         layer.gate_up = layer.down = layer.expert_map = None
-        layer.sketch = self.sketch_words.data_ptr()
-        layer.sketch_grouped = (
-            self.sketch_grouped_words.data_ptr() if self.sketch_grouped_words is not None else None)
+        layer.sketch = None
+        layer.sketch_grouped = self.sketch_grouped_words.data_ptr()
         layer.statistics = self.sketch_statistics.data_ptr()
         layer.norms = self.norms.data_ptr()
         layer.geometry = (
@@ -409,7 +407,7 @@ class _HomeScreen:
         self.layer = layer
         self.resident_bytes = sum(
             t.numel() * t.element_size()
-            for t in (self.sketch_words, self.sketch_grouped_words, self.sketch_statistics,
+            for t in (self.sketch_grouped_words, self.sketch_statistics,
                       self.norms, self.encoder, self.recovery_geometry) if t is not None)
 
 
@@ -617,11 +615,9 @@ class ExpertParallelReader:
         local, home = self.reader, self.home
         span = slice(self.rank * gate_up.shape[0], (self.rank + 1) * gate_up.shape[0])
         local.sketch_codes = None
-        local.sketch_words = home.sketch_words[span]
-        local._layer.sketch = local.sketch_words.data_ptr()
-        if local.sketch_grouped_words is not None:
-            local.sketch_grouped_words = home.sketch_grouped_words[span]
-            local._layer.sketch_grouped = local.sketch_grouped_words.data_ptr()
+        local.sketch_words = local._layer.sketch = None
+        local.sketch_grouped_words = home.sketch_grouped_words[span]
+        local._layer.sketch_grouped = local.sketch_grouped_words.data_ptr()
         local.sketch_statistics = home.sketch_statistics[span].permute(0, 3, 1, 2)
         local._layer.statistics = local.sketch_statistics.data_ptr()
         local.sketch_resident_bytes = 0

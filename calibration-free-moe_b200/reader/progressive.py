@@ -228,6 +228,7 @@ class ProgressiveReader:
         ep_group: "dist.ProcessGroup | None" = None,
         recovery_owner: bool | None = None,
         retain_reference_sketch: bool = True,
+        retain_coordinate_sketch: bool | None = None,
         tensor_engine: str = "mma_sync",
         row_engine: str = "auto",
         sketch_builder: str = "torch",
@@ -247,8 +248,11 @@ class ProgressiveReader:
         Keyword-only additions: `ep_group` (process group of the expert-parallel
         ranks; defaults to the world group when `expert_map` is given),
         `recovery_owner` (the rank that adds the decoder term; defaults to rank 0
-        of the group) and `retain_reference_sketch` (keep the reference-layout
-        codes resident beside the kernel layout) and `tensor_engine`, the
+        of the group), `retain_reference_sketch` (keep the reference-layout
+        codes resident beside the kernel layout), `retain_coordinate_sketch` (keep the
+        coordinate-major 2-bit copy resident too, I / 2 bytes per expert and hidden
+        coordinate, which no call of a reader reads but `cfm_screen_static` takes; by
+        default where the reference-layout codes are kept) and `tensor_engine`, the
         tensor-core path of the expert-major screen: "mma_sync" (default: chosen by
         size) or "tcgen05" (tensor-memory accumulators at every size); both give the
         same bits; and `row_engine`, how batches of eight tokens and more read the
@@ -351,14 +355,15 @@ class ProgressiveReader:
 
         self.sketch_signs = block_hadamard_signs(h, device)
         blocks = h // 128
+        if retain_coordinate_sketch is None:
+            retain_coordinate_sketch = retain_reference_sketch
         if sketch is None and sketch_builder == "cuda":
             # One pass of the library's kernel over the weights, straight into the kernel layouts.
-            self.sketch_words, self.sketch_grouped_words, statistics = build_sketch_on_device(
+            words, self.sketch_grouped_words, statistics = build_sketch_on_device(
                 gate_up, self.sketch_signs
             )
-            self.sketch_codes = (
-                codes_from_words(self.sketch_words, 2 * i, h) if retain_reference_sketch else None
-            )
+            self.sketch_codes = codes_from_words(words, 2 * i, h) if retain_reference_sketch else None
+            self.sketch_words = words if retain_coordinate_sketch else None
         else:
             if sketch is None:
                 sketch = build_sketch(gate_up, self.sketch_signs)
@@ -374,14 +379,14 @@ class ProgressiveReader:
                 or statistics.stride() != (4 * i * blocks, 1, 4 * i, 2 * i)
             ):
                 raise ValueError("Sketch must match the local native routed experts")
-            # Kernel layout: two bits per trit, [E, H, 2I/16] words.
-            self.sketch_words = repack_sketch(codes, 2 * i, h)
-            # Row-major copy, which the expert-major screen reads.
+            # Row-major, two bits per trit, which the screen reads.
             self.sketch_grouped_words = repack_sketch_grouped(codes, 2 * i, h)
+            # Coordinate-major, [E, H, 2I/16] words.
+            self.sketch_words = repack_sketch(codes, 2 * i, h) if retain_coordinate_sketch else None
             self.sketch_codes = codes if retain_reference_sketch else None
         self.sketch_statistics = statistics
         self.sketch_resident_bytes = (
-            self.sketch_words.numel() * 4
+            (self.sketch_words.numel() * 4 if self.sketch_words is not None else 0)
             + statistics.numel() * 2
             + self.sketch_grouped_words.numel() * 4
         )
@@ -459,7 +464,7 @@ class ProgressiveReader:
         layer.recovery_owner = int(self.recovery_owner)
         layer.gate_up = self.native_gu.data_ptr()
         layer.down = self.down.data_ptr()
-        layer.sketch = self.sketch_words.data_ptr()
+        layer.sketch = self.sketch_words.data_ptr() if self.sketch_words is not None else None
         layer.sketch_grouped = self.sketch_grouped_words.data_ptr()
         layer.statistics = statistics.data_ptr()
         layer.norms = self.norms.data_ptr()

@@ -71,8 +71,10 @@ typedef struct cfm_layer {
   int32_t reserved;
   const void* gate_up;       /* bf16 [E, 2I, H] contiguous                      */
   const void* down;          /* bf16 physical [E, I, H] (channel-major)         */
-  const uint32_t* sketch;    /* coordinate-major layout [E, H, 2I/16], 2 bits per trit */
-  const uint32_t* sketch_grouped; /* row-major layout [E, B, 2I, 8] or NULL     */
+  const uint32_t* sketch;    /* coordinate-major layout [E, H, 2I/16], 2 bits per trit; read by
+                                cfm_screen_static and for layers without sketch_grouped, NULL
+                                where neither is the case                        */
+  const uint32_t* sketch_grouped; /* row-major layout [E, B, 2I, 8], 16-byte aligned, or NULL */
   const void* statistics;    /* fp16 physical [E, B, 2, 2I]: scale, variance    */
   const float* norms;        /* f32 [E, I], down-column norms                   */
   const float* geometry;     /* f32 [E, I, 2] or NULL (recovery-aware score)    */
