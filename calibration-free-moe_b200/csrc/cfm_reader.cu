@@ -1544,14 +1544,6 @@ __global__ void k_zero_latent(Layer L, Workspace ws) {
 
 #include "cfm_union.cuh"
 
-// One past the last down tile of slot `slot` of token t: a token's tiles lie slot after slot,
-// ceil(count / 64) per local slot, from `tile_starts`.
-__device__ __forceinline__ int down_slot_end(const Layer& L, const Workspace& ws, int t, int slot) {
-  const size_t pair = static_cast<size_t>(t) * L.K + slot;
-  const int tiles = ws.ids[pair] >= 0 ? (ws.counts[pair] + kDownTileRows - 1) / kDownTileRows : 0;
-  return ws.tile_starts[pair] + tiles;
-}
-
 // ---------------------------------------------------------------------------
 // output: router mix + decoder term
 // ---------------------------------------------------------------------------
@@ -2108,13 +2100,20 @@ static bool exact_by_union(const Bound& b) {
 // The expert-major down kernel, on request only: its sums depend in their last FP32 bits on what the
 // other tokens of an expert kept, while the tiles give a token the same bits in every batch.  Where
 // most experts have more than half a pass of sixteen tokens and there is a piece for every second
-// warp: 64 tokens of the 128-expert layer 45 us in all against 37 of the tiles per token and their
-// output, whole calls of 256 tokens 280 against 310 (256-expert layer) and 1494 against 1830 (hidden
-// 4096, width 1536).  (Repeating the sums that the distance could round otherwise, one in a hundred,
-// costs more than the tiles: 3390 us there, most of it for single columns of rows that have left L2.)
+// warp: 64 tokens of the 128-expert layer 45 us with the output against 37 of the tiles, whole calls of
+// 256 tokens 287 against 299 (256-expert layer) and 1535 against 1810 (hidden 4096, width 1536).
+// (Repeating the sums that the distance could round otherwise, one in a hundred, costs more than the
+// tiles: 3390 us there, most of it for single columns of rows that have left L2.)
 static bool down_by_union(const Bound& b) {
   return exact_by_union(b) && b.L.row_engine == CFM_ROWS_EXPERT_MAJOR && shares_decode(b) &&
          static_cast<int64_t>(busy_experts(b)) * (b.L.H / DownUnion::kColumns) >= 148 * 8;
+}
+// Sixteen tokens per CTA of the output after it, and over the tiles of large batches while that gives
+// every SM a CTA: 256 tokens of the 256-expert layer 15 us against 28, of hidden 4096 and width 1536 52
+// against 127; 100 tokens of the 64-expert layer (112 CTAs) 21 against 15.
+static bool mixes_tokens(const Bound& b) {
+  return down_by_union(b) ||
+         (exact_by_union(b) && (b.L.H / 128) * ((b.T + kMixTokens - 1) / kMixTokens) >= 148);
 }
 // The recovery encoder in the expert-major down launch.
 static bool encodes_by_union(const Bound& b) { return down_by_union(b) && encodes(b); }
@@ -2290,14 +2289,19 @@ static int run_output(const Bound& b, const cfm_call* call, bool whole) {
   if (!call->out) return CFM_E_NULL;
   const int latents = !whole || encodes(b);
   auto* out = static_cast<__nv_bfloat16*>(call->out);
-  if (!down_by_union(b)) {
+  if (!mixes_tokens(b)) {
     launch_dependent(k_output, dim3(b.L.H / 128 + whole, b.T), dim3(128), 0, b.stream, b.L, b.ws, b.padding,
                      out, latents, static_cast<int>(whole));
     return launched();
   }
   const int mixed = whole && encodes_by_union(b) ? kLatentsFromSums : latents ? kLatentsGiven : kLatentsNone;
-  launch_dependent(k_mix, dim3(b.L.H / 128 + whole, (b.T + kMixTokens - 1) / kMixTokens), dim3(128), 0, b.stream,
-                   b.L, b.ws, b.padding, b.T, out, mixed, static_cast<int>(whole));
+  const dim3 grid(b.L.H / 128 + whole, (b.T + kMixTokens - 1) / kMixTokens);
+  if (down_by_union(b))
+    launch_dependent(k_mix<false>, grid, dim3(128), 0, b.stream, b.L, b.ws, b.padding, b.T, out, mixed,
+                     static_cast<int>(whole));
+  else
+    launch_dependent(k_mix<true>, grid, dim3(128), 0, b.stream, b.L, b.ws, b.padding, b.T, out, mixed,
+                     static_cast<int>(whole));
   return launched();
 }
 

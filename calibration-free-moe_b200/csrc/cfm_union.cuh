@@ -8,7 +8,7 @@
 //   k_union         per expert the union of its tokens' kept channels; work lists
 //   k_exact_union   gate and up rows of the unions
 //   k_down_union    channel-major down rows of the unions; recovery-encoder rows
-//   k_mix           router mix of the expert sums, latent, decoder term, BF16 store, counters
+//   k_mix           output of large batches: router mix, latent, decoder term, BF16 store, counters
 //
 // The tensor cores are not there for their rate (they idle nine tenths of the time) but for their
 // instruction count: per row and eight tokens a matrix instruction replaces some fifty loads,
@@ -16,7 +16,7 @@
 // A token's gate and up sums depend on its own row and the weights only, in an order fixed by H
 // (quarters of H, columns ascending inside a quarter), and round as the gathers' do; its down and
 // encoder sums go sixteen union rows at a time and depend in their last FP32 bits on the channels
-// the other tokens of an expert kept, which is why the last two kernels run on request only.
+// the other tokens of an expert kept, which is why k_down_union runs on request only.
 // The exact and down kernels are persistent and take their work from flat lists, so experts of
 // very different load keep all SMs busy, and their copies run ahead from one piece of work into
 // the next.  Included by cfm_reader.cu inside namespace cfm.
@@ -823,7 +823,7 @@ __global__ void __launch_bounds__(DownUnion::kThreads, DownUnion::kPerSm)
 }
 
 // ---------------------------------------------------------------------------
-// output after k_down_union
+// output of large batches
 // ---------------------------------------------------------------------------
 // Router mix of the BF16 expert sums of token t at column h, in slot order.
 __device__ __forceinline__ float mix_sums(const Layer& L, const Workspace& ws, int t, int h) {
@@ -843,11 +843,14 @@ __device__ __forceinline__ float mix_sums(const Layer& L, const Workspace& ws, i
 // grid (H / 128, or one more for the tokens' read-cost counters; ceil(T / 16)), 128 threads: sixteen
 // tokens, 32 output columns per warp.  The decoder term is a product of the tokens' latents (BF16)
 // with decoder rows, done by the tensor cores; a sum leaves them after 32 columns of the latent and
-// goes on by ordinary additions.  Columns are dealt to the instruction so that a thread ends up with
-// eight adjacent ones of two tokens, and the order inside sixteen latent columns so that it loads
-// eight adjacent ones of a decoder row.  The expert sums of the first slots are on their way
-// meanwhile.  Bound by latency.  256 tokens of the 256-expert layer 9.2 us, of hidden 4096 and rank 128
-// 13.8 (one column of up to eight tokens per thread and dot products by FMAs: 20 and 44).
+// goes on by ordinary additions, and one whose rounding to BF16 the distance to k_output's chain of
+// FMAs could change is repeated as that chain: the bits are those of k_output.  Columns are dealt to
+// the instruction so that a thread ends up with eight adjacent ones of two tokens, and the order
+// inside sixteen latent columns so that it loads eight adjacent ones of a decoder row.  The expert
+// sums are BF16, one per slot (of the expert-major down kernel; the first slots' are on their way
+// meanwhile), or with TILES the FP32 sums of the down tiles.  Bound by latency, over tiles by their
+// traffic: 256 tokens of the 256-expert layer 9.2 us (tiles 15.4, one token per CTA 27.8), of hidden
+// 4096 and rank 128 13.8 (52, 4.2 TB/s; 127).
 // `latents`: none, the workspace's, or to be mixed here from the encoder's sums.
 constexpr int kLatentsNone = 0, kLatentsGiven = 1, kLatentsFromSums = 2;
 constexpr int kMixTokens = 16;
@@ -863,6 +866,45 @@ __device__ __forceinline__ void add_scaled8(float (&z)[8], const uint4& v, float
   z[6] = fmaf(bf16_lo(v.w), w, z[6]);
   z[7] = fmaf(bf16_hi(v.w), w, z[7]);
 }
+// Eight adjacent columns of a token from its down tiles: per slot the tiles in order, their sum rounded
+// to BF16 times the router weight, slots in order (mix_down_tiles).
+__device__ __forceinline__ void mix_tiles(float (&routed)[8], const float* parts, int H, int used,
+                                          const int* slot_end, const float* slot_weight) {
+  float sum[8] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
+  int slot = 0;
+  auto close = [&]() {
+#pragma unroll
+    for (int c = 0; c < 8; ++c) {
+      routed[c] = fmaf(bf16_round(sum[c]), slot_weight[slot], routed[c]);
+      sum[c] = 0.0f;
+    }
+    ++slot;
+  };
+  constexpr int kTiles = 4;  // on their way at a time
+  for (int base = 0; base < used; base += kTiles) {
+    float4 v[kTiles][2];
+#pragma unroll
+    for (int i = 0; i < kTiles; ++i) {
+      const float4* from = reinterpret_cast<const float4*>(parts + static_cast<size_t>(base + i) * H);
+#pragma unroll
+      for (int c = 0; c < 2; ++c) v[i][c] = base + i < used ? __ldcg(from + c) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    }
+#pragma unroll
+    for (int i = 0; i < kTiles; ++i) {
+      if (base + i >= used) break;
+      while (base + i >= slot_end[slot]) close();
+      sum[0] += v[i][0].x;
+      sum[1] += v[i][0].y;
+      sum[2] += v[i][0].z;
+      sum[3] += v[i][0].w;
+      sum[4] += v[i][1].x;
+      sum[5] += v[i][1].y;
+      sum[6] += v[i][1].z;
+      sum[7] += v[i][1].w;
+    }
+  }
+  if (used > 0) close();
+}
 __device__ __forceinline__ uint4 pack_bf16x8(const float (&z)[8]) {
   uint4 v;
   uint32_t* out = reinterpret_cast<uint32_t*>(&v);
@@ -874,11 +916,26 @@ __device__ __forceinline__ uint4 pack_bf16x8(const float (&z)[8]) {
   return v;
 }
 
+// Largest distance to a chain of FMAs that is provided for, in units of the token's largest running sum
+// over the columns of a warp: 0.27 of it at most and 0.02 RMS in seventeen million sums of latents as
+// the encoder leaves them for normal, outlier and Student-t inputs.
+constexpr float kMixMargin = 1.0f / (1 << 19);
+
+// One past the last down tile of slot `slot` of token t: a token's tiles lie slot after slot,
+// ceil(count / 64) per local slot, from `tile_starts`.
+__device__ __forceinline__ int down_slot_end(const Layer& L, const Workspace& ws, int t, int slot) {
+  const size_t pair = static_cast<size_t>(t) * L.K + slot;
+  const int tiles = ws.ids[pair] >= 0 ? (ws.counts[pair] + kDownTileRows - 1) / kDownTileRows : 0;
+  return ws.tile_starts[pair] + tiles;
+}
+
+template <bool TILES>
 __global__ void __launch_bounds__(128, 4) k_mix(Layer L, Workspace ws, const uint8_t* padding, int tokens,
                                                 __nv_bfloat16* out, int latents, int early) {
   __shared__ __align__(16) __nv_bfloat16 latent[kMixTokens][256 + 32];
   __shared__ float weight[kMixTokens][32];
   __shared__ uint32_t valid[kMixTokens];  // the slots that have sums
+  __shared__ int slot_end[TILES ? kMixTokens : 1][32];  // one past a slot's last down tile
   const int t0 = blockIdx.y * kMixTokens, count = min(kMixTokens, tokens - t0);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, tq = lane & 3;
   if (!early) grid_dependency_wait();
@@ -912,6 +969,7 @@ __global__ void __launch_bounds__(128, 4) k_mix(Layer L, Workspace ws, const uin
       const size_t pair = static_cast<size_t>(t0 + j) * L.K + lane;
       here = ws.ids[pair] >= 0 && !(padding && padding[t0 + j]);
       weight[j][lane] = ws.weights[pair];
+      if (TILES) slot_end[j][lane] = down_slot_end(L, ws, t0 + j, lane);
     }
     const unsigned slots = __ballot_sync(kFull, here);
     if (lane == 0) valid[j] = slots;
@@ -924,7 +982,7 @@ __global__ void __launch_bounds__(128, 4) k_mix(Layer L, Workspace ws, const uin
   uint4 sums[2][kSums];
   const uint4* from[2];
 #pragma unroll
-  for (int i = 0; i < 2; ++i) {
+  for (int i = 0; i < 2 && !TILES; ++i) {
     from[i] = reinterpret_cast<const uint4*>(reinterpret_cast<const __nv_bfloat16*>(ws.down_parts) +
                                              static_cast<size_t>(t0 + min(8 * i + g, count - 1)) * L.K * L.H + h);
 #pragma unroll
@@ -962,6 +1020,7 @@ __global__ void __launch_bounds__(128, 4) k_mix(Layer L, Workspace ws, const uin
     }
     __syncthreads();
   }
+  float size[2] = {0.0f, 0.0f};  // largest running sums of tokens g and g + 8
   float dot[4][4];  // [n][token g, g + 8][columns 2 n, 2 n + 1 of this thread's eight]
 #pragma unroll
   for (int n = 0; n < 4; ++n)
@@ -978,7 +1037,10 @@ __global__ void __launch_bounds__(128, 4) k_mix(Layer L, Workspace ws, const uin
         mma_bf16_first(part, a[0], d[n].x, d[n].y);
         mma_bf16(part, a[1], d[n].z, d[n].w);
 #pragma unroll
-        for (int i = 0; i < 4; ++i) dot[n][i] += part[i];
+        for (int i = 0; i < 4; ++i) {
+          dot[n][i] += part[i];
+          size[i >> 1] = fmaxf(size[i >> 1], fabsf(dot[n][i]));
+        }
       }
     };
     for (int k = 0; k < pieces; k += 8) {
@@ -987,6 +1049,41 @@ __global__ void __launch_bounds__(128, 4) k_mix(Layer L, Workspace ws, const uin
       if (k + 4 < pieces) fold(decoder[1], k + 4);
       load_decoder(decoder[1], k + 12);
     }
+    // Sums in doubt again, a column after the other as the output of the tiles adds them.
+    uint32_t doubt = 0;
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      float margin = size[i];
+      margin = fmaxf(margin, __shfl_xor_sync(kFull, margin, 1));
+      margin = kMixMargin * fmaxf(margin, __shfl_xor_sync(kFull, margin, 2));
+#pragma unroll
+      for (int n = 0; n < 4; ++n)
+#pragma unroll
+        for (int b = 0; b < 2; ++b)
+          doubt |= static_cast<uint32_t>(rounds_either_way(dot[n][2 * i + b], margin)) << (4 * n + 2 * i + b);
+    }
+    for (; doubt; doubt &= doubt - 1) {
+      const int bit = __ffs(doubt) - 1, j = g + 4 * (bit & 2);
+      const uint4* row = reinterpret_cast<const uint4*>(
+          L.decoder + static_cast<size_t>(h + 2 * (bit >> 2) + (bit & 1)) * L.R);
+      const uint4* z = reinterpret_cast<const uint4*>(latent[j]);
+      float sum = 0.0f;
+#pragma unroll 4
+      for (int k = 0; k < pieces; ++k) {
+        const uint4 d = row[k], v = z[k];
+        sum = fmaf(bf16_lo(d.x), bf16_lo(v.x), sum);
+        sum = fmaf(bf16_hi(d.x), bf16_hi(v.x), sum);
+        sum = fmaf(bf16_lo(d.y), bf16_lo(v.y), sum);
+        sum = fmaf(bf16_hi(d.y), bf16_hi(v.y), sum);
+        sum = fmaf(bf16_lo(d.z), bf16_lo(v.z), sum);
+        sum = fmaf(bf16_hi(d.z), bf16_hi(v.z), sum);
+        sum = fmaf(bf16_lo(d.w), bf16_lo(v.w), sum);
+        sum = fmaf(bf16_hi(d.w), bf16_hi(v.w), sum);
+      }
+#pragma unroll
+      for (int i = 0; i < 16; ++i)
+        if (i == bit) dot[i >> 2][i & 3] = sum;
+    }
   }
   const bool aligned = (reinterpret_cast<uintptr_t>(out) & 15) == 0;
 #pragma unroll
@@ -994,10 +1091,12 @@ __global__ void __launch_bounds__(128, 4) k_mix(Layer L, Workspace ws, const uin
     const int j = 8 * i + g;
     if (j >= count) continue;
     float routed[8] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
+    if (TILES) mix_tiles(routed, ws.down_parts + static_cast<size_t>(t0 + j) * ws.down_tiles * L.H + h, L.H,
+                         slot_end[j][L.K - 1], slot_end[j], weight[j]);
 #pragma unroll
-    for (int s = 0; s < kSums; ++s)
+    for (int s = 0; s < kSums && !TILES; ++s)
       if ((valid[j] >> s) & 1u) add_scaled8(routed, sums[i][s], weight[j][s]);
-    for (int s0 = kSums; s0 < L.K; s0 += kSums) {
+    for (int s0 = kSums; s0 < L.K && !TILES; s0 += kSums) {
 #pragma unroll
       for (int s = 0; s < kSums; ++s)
         if (s0 + s < L.K) sums[i][s] = __ldcg(from[i] + static_cast<size_t>(s0 + s) * (L.H / 8));
@@ -1005,10 +1104,12 @@ __global__ void __launch_bounds__(128, 4) k_mix(Layer L, Workspace ws, const uin
       for (int s = 0; s < kSums; ++s)
         if (s0 + s < L.K && ((valid[j] >> (s0 + s)) & 1u)) add_scaled8(routed, sums[i][s], weight[j][s0 + s]);
     }
+    if (!(padding && padding[t0 + j])) {
 #pragma unroll
-    for (int n = 0; n < 4; ++n) {
-      routed[2 * n] += bf16_round(dot[n][2 * i]);
-      routed[2 * n + 1] += bf16_round(dot[n][2 * i + 1]);
+      for (int n = 0; n < 4; ++n) {
+        routed[2 * n] += bf16_round(dot[n][2 * i]);
+        routed[2 * n + 1] += bf16_round(dot[n][2 * i + 1]);
+      }
     }
     __nv_bfloat16* to = out + static_cast<size_t>(t0 + j) * L.H + h;
     if (aligned) {

@@ -455,7 +455,8 @@ class ReplicatedScreenEngine:
         with torch.cuda.device(device):
             if screened:
                 # Routing and the grouping by expert do not depend on the rotated input:
-                # they run on the side stream beside the rotation, as in the whole-layer call.
+                # they run on the side stream beside the rotation (a whole-layer call has both in
+                # one launch).
                 main = torch.cuda.current_stream(device)
                 self._fork.record(main)
                 with torch.cuda.stream(self._side):

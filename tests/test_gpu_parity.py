@@ -173,7 +173,8 @@ def test_tcgen05_screen_gives_the_same_bits(name):
     case = item["case"]
     tokens = case.hidden.shape[0]
     device = torch.device("cuda:0")
-    # Capacity 8 or more switches the screen to the expert-major kernels.
+    # Every screen with a row-major sketch is expert-major; eight rows and more so that experts
+    # have several tokens.
     legacy = make_reader(item, capacity=max(8, tokens))
     modern = make_reader(item, capacity=max(8, tokens), tensor_engine="tcgen05")
     repeat = -(-8 // tokens)

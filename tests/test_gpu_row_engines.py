@@ -233,3 +233,19 @@ def test_a_row_that_is_not_finite_reaches_only_tokens_that_kept_it(engine):
     assert out[~keeps.any(1)].isfinite().all() and not out[keeps.any(1)].isfinite().any()
     assert torch.equal(out.isnan(), want.isnan())
     torch.testing.assert_close(out.float().nan_to_num(), want.float().nan_to_num(), rtol=0.016, atol=2e-3)
+
+
+# hidden, width, experts, top_k, rank, tokens: no map, an eighth of 64 latent columns, the largest rank
+# with a remainder of three tokens, more slots than are on their way at a time.
+@pytest.mark.parametrize("padded", [False, True])
+@pytest.mark.parametrize("shape", [(4096, 16, 20, 5, 0, 80), (4096, 48, 20, 5, 8, 75), (2048, 32, 16, 3, 256, 147),
+                                   (2048, 208, 30, 12, 32, 150)])
+def test_output_of_sixteen_tokens_at_the_edges(shape, padded):
+    h, i, e, k, rank, tokens = shape
+    padding = [t % 7 == 3 or t >= tokens - 2 for t in range(tokens)] if padded else None
+    item = prepared_case(cases._random("mix", h + i, h, i, e, k, rank, tokens, 0.4, 0.5, padding=padding))
+    sixteen, one = (make_reader(item, row_engine=engine) for engine in ("auto", "per_token"))
+    want, out = run_reader(one, item["case"]), run_reader(sixteen, item["case"])
+    assert torch.equal(out, want)
+    if rank:
+        assert torch.equal(sixteen.latent[:tokens], one.latent[:tokens])
