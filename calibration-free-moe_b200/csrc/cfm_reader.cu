@@ -2088,8 +2088,8 @@ static bool encodes(const Bound& b) { return b.L.R > 0 && b.L.F < b.L.N; }
 
 // The expert-major exact kernel, on request and from three tokens per expert and sixteen tokens on:
 // below that the unions of an expert's kept channels are little smaller than their sum.  64 tokens of
-// the 128-expert layer 65 us with the unions against 69 of the gathers, 100 of the 64-expert layer 95
-// against 132, 256 of the 256-expert layer 90 against 155; at two tokens per expert 43 against 39 (32 of
+// the 128-expert layer 67 us with the unions against 69 of the gathers, 100 of the 64-expert layer 100
+// against 132, 256 of the 256-expert layer 96 against 155; at two tokens per expert 43 against 39 (32 of
 // the 128-expert layer) and 141 against 120 (hidden 4096, width 1536).  Under expert parallelism the
 // gathers per token stay, so that a token's bits do not depend on how the experts are spread.
 static bool exact_by_union(const Bound& b) {

@@ -212,10 +212,11 @@ __global__ void __launch_bounds__(kUnionThreads)
 // ways of summing could change a rounding (kExactMargin), the CTA lists the row and repeats the
 // product as the gathers do it when the list is full and at its end, so that the activations are
 // those of the gathers.
-// Bound by the way from L2 to the SMs (9 to 11 TB/s, the tokens' rows included; tiles of sixteen rows
-// carried them twice as often): 100 tokens of the 64-expert layer 89 us (132 the gathers per token),
-// 256 of the 256-expert layer 80 (155), 256 of hidden 4096 and width 1536 580 at 5.3 TB/s of HBM
-// (1431).
+// Bound by the latency of its copies: two warps per scheduler, of 13 cycles per issued instruction four
+// waiting for copies, three for the queue of memory instructions, half a one at barriers; 15 % of the
+// way from L2 to the SMs, DRAM 57 % at 64 tokens of the 128-expert layer (63 us; 69 the gathers per
+// token).  100 tokens of the 64-expert layer 95 us (132), 256 of the 256-expert layer 90 (155), 256 of
+// hidden 4096 and width 1536 616 at 5 TB/s of HBM (1431); without the repeats 61, 89, 80 and 580.
 template <int NT>
 struct ExactUnion {
   static constexpr int kThreads = 128;
