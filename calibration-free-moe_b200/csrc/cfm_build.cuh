@@ -35,37 +35,6 @@
 constexpr int kBuildRows = 16;   // rows per warp = rows per coordinate-major word
 constexpr int kBuildWarps = 8;   // 128 rows per CTA: a coordinate's words leave as 32-byte runs
 
-// Two FP32 values in one 64-bit register and the packed operations on them; each half
-// rounds exactly as the scalar operation does.
-using Pair = unsigned long long;
-__device__ __forceinline__ Pair pair_of(float lo, float hi) {
-  Pair p;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(p) : "f"(lo), "f"(hi));
-  return p;
-}
-__device__ __forceinline__ void pair_split(Pair p, float& lo, float& hi) {
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(p));
-}
-__device__ __forceinline__ Pair pair_add(Pair a, Pair b) {
-  Pair d;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-  return d;
-}
-__device__ __forceinline__ Pair pair_mul(Pair a, Pair b) {
-  Pair d;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-  return d;
-}
-__device__ __forceinline__ Pair pair_fma(Pair a, Pair b, Pair c) {
-  Pair d;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-  return d;
-}
-// a - b: the product with -1 is exact, so the one rounding is that of the subtraction.
-__device__ __forceinline__ Pair pair_sub(Pair a, Pair b) {
-  return pair_fma(b, pair_of(-1.0f, -1.0f), a);
-}
-
 // Sum of a value over the four lanes of a row, in the order of the block sums.
 __device__ __forceinline__ float quad_sum(float x) {
   x = __fadd_rn(x, __shfl_xor_sync(kFull, x, 2));

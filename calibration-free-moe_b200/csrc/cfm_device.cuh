@@ -30,10 +30,8 @@ __device__ __forceinline__ float bf16_round(float x) {
 // exp(x) from Cody-Waite reduction and a degree-7 Horner polynomial.
 // exp(x) = 2^n * p(r), n = rint(x * log2 e), r = x - n * ln 2 (two-term split).
 // Saturates to +inf from 88 and to 0 below -87; NaN propagates.
+// (Without branches, so that several go on at a time; outside of the range the result is replaced.)
 __device__ __forceinline__ float pinned_exp(float x) {
-  if (!(x == x)) return x;
-  if (x >= 88.0f) return __int_as_float(0x7f800000);
-  if (x <= -87.0f) return 0.0f;
   const float n = rintf(__fmul_rn(x, 1.44269502f));
   float r = __fmaf_rn(n, -0.693145752f, x);
   r = __fmaf_rn(n, -1.42860677e-06f, r);
@@ -46,27 +44,46 @@ __device__ __forceinline__ float pinned_exp(float x) {
   p = __fmaf_rn(p, r, 1.0f);
   p = __fmaf_rn(p, r, 1.0f);
   const int e = static_cast<int>(n);  // in [-126, 127]
-  return __fmul_rn(p, __int_as_float((e + 127) << 23));
+  const float y = __fmul_rn(p, __int_as_float((e + 127) << 23));
+  return x >= 88.0f ? __int_as_float(0x7f800000) : x <= -87.0f ? 0.0f : x == x ? y : x;
 }
 
-// SiLU: x / (1 + exp(-x)).
-__device__ __forceinline__ float pinned_silu(float x) {
-  return __fdiv_rn(x, __fadd_rn(1.0f, pinned_exp(-x)));
+// x / d, correctly rounded, for d in [1, inf] and x / d not below 2^-120: Markstein's division
+// (IBM J. Res. Dev. 34, 1990) from the approximate reciprocal, one step on the reciprocal and one on
+// the quotient.  Without branches, so that the five nodes of a risk score and several candidates go
+// on at a time.  Large divisors are scaled for the reciprocal's sake.
+__device__ __forceinline__ float divide_from_one(float x, float d) {
+  const float scale = d > 1.8446744e19f ? 2.3283064e-10f : 1.0f;  // 2^64, 2^-32
+  const float a = __fmul_rn(x, scale), b = __fmul_rn(d, scale);
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(b));
+  y = __fmaf_rn(__fmaf_rn(-b, y, 1.0f), y, y);
+  const float q = __fmul_rn(a, y);
+  return __fmaf_rn(__fmaf_rn(-b, q, a), y, q);
 }
 
-// GELU, tanh form: 0.5 x (1 + tanh(z)), z = sqrt(2/pi) (x + 0.044715 x^3),
-// with tanh(z) = 1 - 2 / (exp(2 z) + 1).
-__device__ __forceinline__ float pinned_gelu_tanh(float x) {
-  const float x3 = __fmul_rn(__fmul_rn(x, x), x);
-  const float inner = __fmaf_rn(0.044715f, x3, x);
-  const float z = __fmul_rn(0.797884583f, inner);
-  const float ez = pinned_exp(__fmul_rn(2.0f, z));
-  const float th = __fsub_rn(1.0f, __fdiv_rn(2.0f, __fadd_rn(ez, 1.0f)));
-  return __fmul_rn(__fmul_rn(0.5f, x), __fadd_rn(1.0f, th));
-}
-
+// SiLU: x / (1 + exp(-x)).  The divisor is 1 from 87 on, 2 about zero, and infinite from -88 down.
+// GELU, tanh form: 0.5 x (1 + tanh(z)), z = sqrt(2/pi) (x + 0.044715 x^3), with
+// tanh(z) = 1 - 2 / (exp(2 z) + 1).
+// Both over one exponential and one division: the risk score has this five times over, and kernels
+// that carried each form apart waited for instructions.  Every one of the 2^32 inputs gives the bits
+// of the IEEE divisions.
 __device__ __forceinline__ float pinned_activate(float x, int activation) {
-  return activation == 1 ? pinned_gelu_tanh(x) : pinned_silu(x);
+  const bool gelu = activation == 1;
+  const float infinity = __int_as_float(0x7f800000);
+  float power = -x;
+  if (gelu) {
+    const float x3 = __fmul_rn(__fmul_rn(x, x), x);
+    power = __fmul_rn(2.0f, __fmul_rn(0.797884583f, __fmaf_rn(0.044715f, x3, x)));
+  }
+  const float e = pinned_exp(power);
+  const float q = divide_from_one(gelu ? 2.0f : x, __fadd_rn(1.0f, e));
+  if (gelu) {
+    const float th = __fsub_rn(1.0f, e < infinity ? q : e == e ? 0.0f : e);
+    return __fmul_rn(__fmul_rn(0.5f, x), __fadd_rn(1.0f, th));
+  }
+  const float edge = x >= 87.0f ? x : x == -infinity ? __int_as_float(0x7fffffff) : -0.0f;
+  return x >= 87.0f || x <= -88.0f ? edge : fabsf(x) < 8.6736174e-19f ? __fmul_rn(x, 0.5f) : q;  // 2^-60
 }
 
 // The gated feature with the reference's rounding points for an exactly
@@ -76,18 +93,15 @@ __device__ __forceinline__ float exact_feature(float g, float u, int activation)
   return bf16_round(__fmul_rn(bf16_round(pinned_activate(gb, activation)), ub));
 }
 
-// The feature of a skipped channel from its sketch projections: one rounding,
+// The feature of a skipped channel from its sketch projections, `active` = phi(bf16 g): one rounding,
 // bf16(phi(bf16 g) * bf16 u).
-__device__ __forceinline__ float sketch_feature(float g, float u, int activation) {
-  const float gb = bf16_round(g), ub = bf16_round(u);
-  return bf16_round(__fmul_rn(pinned_activate(gb, activation), ub));
+__device__ __forceinline__ float sketch_feature(float active, float u) {
+  return bf16_round(__fmul_rn(active, bf16_round(u)));
 }
 
 // Point score: ((norm * phi(g)) * u)^2 * w^2 on BF16-rounded projections.
-__device__ __forceinline__ float point_score(float g, float u, float norm, float w,
-                                             int activation) {
-  const float gb = bf16_round(g), ub = bf16_round(u);
-  const float t = __fmul_rn(__fmul_rn(norm, pinned_activate(gb, activation)), ub);
+__device__ __forceinline__ float point_score(float active, float u, float norm, float w) {
+  const float t = __fmul_rn(__fmul_rn(norm, active), bf16_round(u));
   return __fadd_rn(__fmul_rn(__fmul_rn(t, t), __fmul_rn(w, w)), 0.0f);
 }
 
@@ -96,29 +110,61 @@ __device__ __forceinline__ float point_score(float g, float u, float norm, float
 // nodes), sketch residual variances vg and vu, down-column norm n and the
 // recovery response split into alpha (along the down column) and beta (across):
 //   n^2 max(E[a^2] - E[a]^2, 0) + ((n E[a] - alpha p)^2 + (beta p)^2),
-// p = bf16(phi(g) u), on BF16-rounded projections.
-__device__ __forceinline__ float risk_score(float g, float u, float vg, float vu, float norm,
+// p = bf16(phi(g) u), `active` = phi(g), on BF16-rounded projections.
+__device__ __forceinline__ float risk_score(float g, float active, float u, float vg, float vu, float norm,
                                             float alpha, float beta, float w, int activation) {
   const float gb = bf16_round(g), ub = bf16_round(u);
   const float sg = __fsqrt_rn(vg), su = __fsqrt_rn(vu);
   const float spread = __fadd_rn(__fmul_rn(ub, ub), __fmul_rn(su, su));
-  const float nodes[5] = {-2.85697007f, -1.35562618f, 0.0f, 1.35562618f, 2.85697007f};
-  const float mass[5] = {0.0112574113f, 0.222075922f, 0.533333333f, 0.222075922f,
-                         0.0112574113f};
   float mu = 0.0f, second = 0.0f;
 #pragma unroll
   for (int j = 0; j < 5; ++j) {
-    const float a = pinned_activate(__fadd_rn(gb, __fmul_rn(nodes[j], sg)), activation);
-    mu = __fadd_rn(mu, __fmul_rn(__fmul_rn(mass[j], a), ub));
-    second = __fadd_rn(second, __fmul_rn(__fmul_rn(mass[j], __fmul_rn(a, a)), spread));
+    const float node = j == 0 ? -2.85697007f : j == 1 ? -1.35562618f : j == 2 ? 0.0f : j == 3 ? 1.35562618f : 2.85697007f;
+    const float mass = j == 2 ? 0.533333333f : j == 1 || j == 3 ? 0.222075922f : 0.0112574113f;
+    const float shift = __fmul_rn(node, sg);
+    // The middle node is the gate itself (or NaN with sg).
+    const float a = j == 2 ? __fadd_rn(active, shift) : pinned_activate(__fadd_rn(gb, shift), activation);
+    mu = __fadd_rn(mu, __fmul_rn(__fmul_rn(mass, a), ub));
+    second = __fadd_rn(second, __fmul_rn(__fmul_rn(mass, __fmul_rn(a, a)), spread));
   }
-  const float p = bf16_round(__fmul_rn(pinned_activate(gb, activation), ub));
+  const float p = bf16_round(__fmul_rn(active, ub));
   const float spread_error = fmaxf(__fsub_rn(second, __fmul_rn(mu, mu)), 0.0f);
   float risk = __fmul_rn(__fmul_rn(norm, norm), spread_error);
   const float along = __fsub_rn(__fmul_rn(norm, mu), __fmul_rn(alpha, p));
   const float across = __fmul_rn(beta, p);
   risk = __fadd_rn(risk, __fadd_rn(__fmul_rn(along, along), __fmul_rn(across, across)));
   return __fadd_rn(__fmul_rn(risk, __fmul_rn(w, w)), 0.0f);
+}
+
+// Two FP32 values in one 64-bit register and the packed operations on them; each half
+// rounds exactly as the scalar operation does.
+using Pair = unsigned long long;
+__device__ __forceinline__ Pair pair_of(float lo, float hi) {
+  Pair p;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(p) : "f"(lo), "f"(hi));
+  return p;
+}
+__device__ __forceinline__ void pair_split(Pair p, float& lo, float& hi) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(p));
+}
+__device__ __forceinline__ Pair pair_add(Pair a, Pair b) {
+  Pair d;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ Pair pair_mul(Pair a, Pair b) {
+  Pair d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ Pair pair_fma(Pair a, Pair b, Pair c) {
+  Pair d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+// a - b: the product with -1 is exact, so the one rounding is that of the subtraction.
+__device__ __forceinline__ Pair pair_sub(Pair a, Pair b) {
+  return pair_fma(b, pair_of(-1.0f, -1.0f), a);
 }
 
 // 16-byte read-only load that does not allocate in L1 (streamed weights).
@@ -149,6 +195,13 @@ __device__ __forceinline__ uint32_t shared_u32(const void* p) {
 // 16 bytes global -> shared memory, past L1, in the thread's current cp.async group.
 __device__ __forceinline__ void copy_async16(uint32_t shared, const void* global) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(shared), "l"(global) : "memory");
+}
+template <int AT>
+__device__ __forceinline__ void copy_async8_at(uint32_t shared, const void* global) {
+  asm volatile("cp.async.ca.shared.global [%0+%2], [%1], 8;" ::"r"(shared), "l"(global), "n"(AT) : "memory");
+}
+__device__ __forceinline__ void copy_async4(uint32_t shared, const void* global) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(shared), "l"(global) : "memory");
 }
 __device__ __forceinline__ void copy_async_commit() {
   asm volatile("cp.async.commit_group;" ::: "memory");

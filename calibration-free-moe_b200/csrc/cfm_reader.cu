@@ -519,8 +519,8 @@ __global__ void __launch_bounds__(512) k_screen(Layer L, Workspace ws, const uin
                             static_cast<size_t>(slot) * L.I;
     const bool risk = L.score != CFM_SCORE_POINT;
     for (int c = tid; c < L.I; c += threads)
-      finish_candidate(L, ws, pair, e, c, gate_out[c], up_out[c], risk ? variance[c] : 0.0f,
-                       risk ? variance[L.N + c] : 0.0f);
+      finish_candidate(L, ws, pair, c, candidate_factors(L, e, c), gate_out[c], up_out[c],
+                       risk ? variance[c] : 0.0f, risk ? variance[L.N + c] : 0.0f);
   };
   if (S == 1) {
 #pragma unroll
@@ -1883,21 +1883,24 @@ static bool screens_grouped(const Bound& b) {
   return b.L.F < b.L.N && b.L.sketch_grouped &&
          ((reinterpret_cast<uintptr_t>(b.L.sketch_grouped) | reinterpret_cast<uintptr_t>(b.L.statistics)) & 15) == 0;
 }
-// From 16/3 tokens per expert on average, half of the experts or more fill passes of sixteen
-// tokens, which the tcgen05 screen decodes the sketch once for.
+// More than 16/3 tokens per expert on average.
 static bool shares_decode(const Bound& b) {
   return 3 * static_cast<int64_t>(b.T) * b.L.K > 16 * static_cast<int64_t>(b.L.E);
 }
-// The tcgen05 screen on request, where it shares its decode, or where its CTAs of 64 channels fill
-// the chip (six per SM): 32 tokens of the 128-expert layer 43.7 us against 49.3 of the warp-level
-// kernel, hidden 4096 and width 1536 136.8 against 161.5; with half of that work in flight (8
-// tokens) 24.7 against 23.1.  Its tables have to fit shared memory.
+// The tcgen05 screen on request, where several tokens share its decode, or where its CTAs of 128 channels
+// give every SM one: three tokens of the 128-expert layer 12.6 us against 12.4 of the warp-level kernel, six
+// 15.6 against 19.6, two of hidden 4096 and width 1536 25.9 against 30.6; one token (48 CTAs) 11.8 against 6.1,
+// eight of the 256-expert layer of width 512 14.6 against 13.1.  Its tables have to fit shared memory.
 static bool screens_tc(const Bound& b) {
-  const int64_t ctas = static_cast<int64_t>(busy_experts(b)) * ((b.L.I + 63) / 64);
-  return (b.L.tensor_engine == CFM_ENGINE_TCGEN05 || shares_decode(b) || ctas >= 6 * 148) &&
-         b.L.B <= 512;
+  const int64_t ctas = static_cast<int64_t>(busy_experts(b)) * ((b.L.I + kScreenChannels - 1) / kScreenChannels);
+  return (b.L.tensor_engine == CFM_ENGINE_TCGEN05 || shares_decode(b) || ctas > 148) && b.L.B <= 512;
 }
-static int pass_pairs(const Bound& b) { return screens_tc(b) && shares_decode(b) ? 16 : 8; }
+// Its passes of sixteen tokens from sixteen tokens per expert on: 256 tokens of hidden 4096 and width 1536 240
+// us against 269 of passes of eight; 100 of the 64-expert layer 50 against 47 (recovery-aware score 78 against
+// 66), 256 of the 256-expert layer 59 against 56: fewer warps fit an SM, and fewer passes are full.
+static int pass_pairs(const Bound& b) {
+  return screens_tc(b) && static_cast<int64_t>(b.T) * b.L.K >= 16 * static_cast<int64_t>(b.L.E) ? 16 : 8;
+}
 
 static int group_smem(const Bound& b, size_t* smem) {
   *smem = std::max<size_t>(sizeof(int) * b.L.E, sizeof(float) * kPrepareThreads * 4);
@@ -1961,14 +1964,26 @@ static int launch_screen(const Bound& b, int S) {
   return launched();
 }
 
+// As many CTAs as run at a time, at most `work` of them.
+template <typename... Params, typename... Args>
+static int launch_persistent(void (*kernel)(Params...), int64_t work, int per_sm, int threads, size_t smem,
+                             cudaStream_t stream, Args... args) {
+  const cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               static_cast<int>(smem));
+  if (err != cudaSuccess) return static_cast<int>(err);
+  const unsigned ctas = static_cast<unsigned>(std::max<int64_t>(1, std::min<int64_t>(work, 148 * per_sm)));
+  launch_dependent(kernel, dim3(ctas), dim3(threads), smem, stream, args...);
+  return launched();
+}
+
 template <int TOKENS, bool RISK>
-static int launch_screen_tc(const Bound& b, dim3 grid, int dead) {
-  const size_t smem = Screen<TOKENS>::shared_bytes(b.L.B);
+static int launch_screen_tc(const Bound& b, int rows, int dead) {
+  const size_t smem = Screen<TOKENS, RISK>::shared_bytes(b.L.B);
   const cudaError_t err = cudaFuncSetAttribute(
       k_screen_tc<TOKENS, RISK>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
   if (err != cudaSuccess) return static_cast<int>(err);
-  launch_dependent(k_screen_tc<TOKENS, RISK>, grid, dim3(kScreenThreads), smem, b.stream, b.L, b.ws,
-                   b.padding, dead);
+  launch_dependent(k_screen_tc<TOKENS, RISK>, dim3((b.L.I + kScreenChannels - 1) / kScreenChannels, rows),
+                   dim3(kScreenThreads), smem, b.stream, b.L, b.ws, b.padding, dead);
   return launched();
 }
 
@@ -1994,11 +2009,10 @@ static int run_screen_grouped(const Bound& b) {
   // Passes, at most; one more row of CTAs clears the dead pairs.
   const int rows = static_cast<int>(pairs / pass) + busy_experts(b) + (dead > 0);
   if (screens_tc(b)) {
-    const dim3 grid((b.L.I + kScreenChannels - 1) / kScreenChannels, rows);
     const bool risk = b.L.score == CFM_SCORE_RECOVERY_AWARE;
     if (pass == 16)
-      return risk ? launch_screen_tc<16, true>(b, grid, dead) : launch_screen_tc<16, false>(b, grid, dead);
-    return risk ? launch_screen_tc<8, true>(b, grid, dead) : launch_screen_tc<8, false>(b, grid, dead);
+      return risk ? launch_screen_tc<16, true>(b, rows, dead) : launch_screen_tc<16, false>(b, rows, dead);
+    return risk ? launch_screen_tc<8, true>(b, rows, dead) : launch_screen_tc<8, false>(b, rows, dead);
   }
   // Four warps per tile while one each would not give every SM its sixteen (one token of the
   // 128-expert layer: 6.9 us against 12.3; 8 tokens 24.5 against 23.4).  The products of a tile
@@ -2124,18 +2138,6 @@ static int exact_union_tiles(const Bound& b) {
   int tiles = 1;
   while (tiles < 4 && 3 * static_cast<int64_t>(b.T) * b.L.K > 16 * tiles * static_cast<int64_t>(b.L.E)) tiles *= 2;
   return tiles;
-}
-
-// As many CTAs as run at a time, at most `work` of them.
-template <typename... Params, typename... Args>
-static int launch_persistent(void (*kernel)(Params...), int64_t work, int per_sm, int threads, size_t smem,
-                             cudaStream_t stream, Args... args) {
-  const cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                               static_cast<int>(smem));
-  if (err != cudaSuccess) return static_cast<int>(err);
-  const unsigned ctas = static_cast<unsigned>(std::max<int64_t>(1, std::min<int64_t>(work, 148 * per_sm)));
-  launch_dependent(kernel, dim3(ctas), dim3(threads), smem, stream, args...);
-  return launched();
 }
 
 // `whole`: part of a whole call, which grouped the pairs and cleared the lists' lengths.

@@ -33,24 +33,32 @@ __device__ __forceinline__ float unscale_of(int e) {
   return __uint_as_float(static_cast<uint32_t>(127 + e - kQuantBits) << 23);
 }
 
+// What a channel brings to its candidates' scores.
+struct CandidateFactors {
+  float norm;
+  float2 geometry;
+};
+__device__ __forceinline__ CandidateFactors candidate_factors(const Layer& L, int e, int c) {
+  const size_t channel = static_cast<size_t>(e) * L.I + c;
+  return CandidateFactors{L.norms[channel],
+                          L.score != CFM_SCORE_POINT && L.geometry
+                              ? reinterpret_cast<const float2*>(L.geometry)[channel]
+                              : make_float2(0.0f, 0.0f)};
+}
+
 // What the selection and the recovery encoder take from a live candidate's projections (and
-// their residual variances): channel c of expert e, slot `pair` = (token, slot).
-__device__ __forceinline__ void finish_candidate(const Layer& L, const Workspace& ws, int pair,
-                                                 int e, int c, float gate, float up,
+// their residual variances): channel c, slot `pair` = (token, slot).
+__device__ __forceinline__ void finish_candidate(const Layer& L, const Workspace& ws, int pair, int c,
+                                                 const CandidateFactors& f, float gate, float up,
                                                  float gate_variance, float up_variance) {
-  const size_t channel = static_cast<size_t>(e) * L.I + c, at = static_cast<size_t>(pair) * L.I + c;
-  const float norm = L.norms[channel], weight = ws.weights[pair];
-  float score;
-  if (L.score == CFM_SCORE_POINT) {
-    score = point_score(gate, up, norm, weight, L.activation);
-  } else {
-    const float2 geometry = L.geometry ? reinterpret_cast<const float2*>(L.geometry)[channel]
-                                       : make_float2(0.0f, 0.0f);
-    score = risk_score(gate, up, gate_variance, up_variance, norm, geometry.x, geometry.y, weight,
-                       L.activation);
-  }
-  ws.scores[at] = score;  // N = K I: candidate slot * I + c of the token
-  ws.features[at] = __float2bfloat16_rn(sketch_feature(gate, up, L.activation));
+  const size_t at = static_cast<size_t>(pair) * L.I + c;  // N = K I: candidate slot * I + c of the token
+  const float weight = ws.weights[pair];
+  const float active = pinned_activate(bf16_round(gate), L.activation);
+  ws.features[at] = __float2bfloat16_rn(sketch_feature(active, up));
+  ws.scores[at] = L.score == CFM_SCORE_POINT
+                      ? point_score(active, up, f.norm, weight)
+                      : risk_score(gate, active, up, gate_variance, up_variance, f.norm, f.geometry.x, f.geometry.y,
+                                   weight, L.activation);
 }
 
 // Residual variances of a channel's projections: per block, in block order, the row's FP16
@@ -82,7 +90,7 @@ __device__ __forceinline__ void store_candidate(const Layer& L, const Workspace&
     ws.variances[at] = variance.x;
     ws.variances[at + L.N] = variance.y;
   }
-  finish_candidate(L, ws, pair, e, c, gate, up, variance.x, variance.y);
+  finish_candidate(L, ws, pair, c, candidate_factors(L, e, c), gate, up, variance.x, variance.y);
 }
 
 // Zeroes the projections of channels c0 .. c1 - 1 for every remote or padded pair of the call.

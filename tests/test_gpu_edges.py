@@ -97,6 +97,25 @@ def test_layer_at_the_edges(oracle, name, padded):
     torch.testing.assert_close(gathered.float()[mask], feature[mask], rtol=0.02, atol=1e-3)
 
 
+@pytest.mark.parametrize("score", ["point", "recovery-aware"])
+@pytest.mark.parametrize("tokens", [1, 5, 9, 17, 40])
+@pytest.mark.parametrize("hidden,width", [(128, 16), (256, 112), (384, 128), (640, 144), (1152, 272)])
+def test_tcgen05_screen_at_the_edges_of_its_tiles(oracle, hidden, width, tokens, score):
+    """Channels around 128 per CTA and 32 per warp, blocks around the lengths of its rings, passes of
+    eight and of sixteen tokens with remainders: every projection, variance and score of the oracle."""
+    case = cases._random("tiles", hidden + tokens, hidden, width, 5, 2, 8, tokens, 0.25, 0.75, score=score)
+    item = prepared_case(case)
+    reader = make_reader(item, capacity=tokens, tensor_engine="tcgen05")
+    run_reader(reader, case)
+    assert int(reader.workspace.status.abs().sum()) == 0
+    own = dict(norms=reader.norms.cpu())
+    if reader.recovery_geometry is not None:
+        own["geometry"] = reader.recovery_geometry.cpu()
+    want = run_oracle(oracle, item, **own)
+    assert torch.equal(reader.partial[:tokens].cpu(), want["partial"])
+    assert torch.equal(reader.scores[0][:tokens].cpu(), want["scores"])
+
+
 def test_expert_major_stages_repeat_and_misaligned_output():
     """The stages on their own, twice, and an output that 16-byte stores cannot take."""
     case = cases._random("stages", 5, 1280, 48, 60, 3, 16, 112, 0.25, 0.625)
