@@ -664,16 +664,23 @@ __device__ __forceinline__ uint2 warp_prefix(uint32_t mine, uint32_t* slots) {
 }
 
 constexpr int kSelectListed = 256;  // keys that one warp finishes the search among
+// Bins of keys by their upper thirteen bits but the sign, which scores do not have (keys with it share
+// the last bin).
+constexpr int kSelectBins = 8192, kSelectShift = 18;
+__device__ __forceinline__ uint32_t select_bin(uint32_t key) {
+  return min(key >> kSelectShift, static_cast<uint32_t>(kSelectBins - 1));
+}
 
 // grid (T), 1024 threads, up to PER keys each in registers: candidate 32 (PER warp + j) + lane.
-// The F-th largest key is searched two bits at a time from the top (three counts of the whole
-// CTA per step, one barrier); once at most 256 keys are left between the bounds, they are listed
-// and one warp goes on alone, a bit at a time.  The search ends when exactly F keys reach its
-// bound.  Then ballots give every warp its keys' places in candidate order.  Bound by the latency
-// of one CTA per token: what only ties, remote slots or budgets need is branched around, and the
-// read-cost counters are left to the output kernel where one follows (`account`).  One token of
-// 6144 candidates: 8.4 us with its launch (a histogram of 2048 bins per eleven bits, built with atomics,
-// a contiguous chunk of candidates per thread and the counters: 14 us).
+// The F-th largest key is found by its bin first: 8192 counters in shared memory, one addition per key
+// (equal addresses of a warp are added by the hardware), and a sum over them from the top.  The few
+// keys of its bin (some ten of 6144) are listed and one warp compares each with each; bins with more go
+// on two bits or one bit at a time.  Then ballots give every warp its keys' places in candidate order.
+// Bound by the latency of one CTA per token, most of it code and data that are met for the first time:
+// what only ties, remote slots or budgets need is branched around, and the read-cost counters are left
+// to the output kernel where one follows (`account`).  One token of 6144 candidates 5.2 us with its
+// launch, of 8192 5.6, 32 tokens of 12288 7.2, 256 of them 16.4; by bits from the top, three counts of
+// the whole CTA per two bits, with stores of single bytes and entries, 8.8, 11.3, 17.3 and 31.8.
 // With `peers` (expert parallelism over peer memory; row_offset 0, T = x.tokens) a
 // CTA ends by storing its token's kept list into slot [rank] of every rank's exchange
 // block; the last CTA to arrive releases each destination's flag with the call's epoch.
@@ -689,16 +696,22 @@ __global__ void __launch_bounds__(kSelectThreads, PER <= 4 ? 2 : 1)
              int clear, typename std::conditional<PEERS, Exchange, NoExchange>::type x) {
   constexpr bool peers = PEERS;
   grid_dependency_release();  // the exact gather may be scheduled; it waits for this grid
-  grid_dependency_wait();     // the screen's projections are complete
+  __shared__ __align__(16) uint32_t s_bins[kSelectBins];
   __shared__ uint2 s_counts[2][32];
-  __shared__ uint32_t s_slots[2][32], s_listed[kSelectListed];
+  __shared__ uint32_t s_slots[3][32], s_listed[kSelectListed];
   __shared__ uint32_t s_cut;
-  __shared__ int s_take, s_count;
+  __shared__ int s_take, s_count, s_bin, s_above, s_inside;
   __shared__ int s_route[32], s_tie_start[33], s_budget[32];
   __shared__ uint32_t s_chunk[32 * PER];   // kept candidates of every 32, as bits
   __shared__ uint16_t s_before[32 * PER];  // kept candidates before them
   const int t = blockIdx.x + row_offset, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int N = L.N, F = L.F, K = L.K, I = L.I;
+  constexpr int kOwnBins = kSelectBins / kSelectThreads;
+#pragma unroll
+  for (int j = 0; j < kOwnBins; j += 4)
+    *reinterpret_cast<uint4*>(s_bins + 4 * tid + 4 * kSelectThreads * (j / 4)) = make_uint4(0, 0, 0, 0);
+  if (tid == 0) s_count = s_inside = 0;
+  grid_dependency_wait();  // the screen's projections are complete
   const bool cut_given = scores_ready == 2, cut_only = scores_ready == 3;
   int32_t* counts = ws.counts + static_cast<size_t>(t) * K;
   int32_t* starts = ws.starts + static_cast<size_t>(t) * K;
@@ -752,7 +765,6 @@ __global__ void __launch_bounds__(kSelectThreads, PER <= 4 ? 2 : 1)
   if (tid < 32) {
     s_route[tid] = tid < K ? ws.ids[static_cast<size_t>(t) * K + tid] : -1;
   }
-  if (tid == 0) s_count = 0;
   const int first = 32 * PER * warp + lane;  // this thread's candidates: first, first + 32, ...
   float* score = ws.scores + static_cast<size_t>(t) * N;
   uint32_t key[PER];
@@ -776,89 +788,150 @@ __global__ void __launch_bounds__(kSelectThreads, PER <= 4 ? 2 : 1)
   uint32_t cut = 0;
   int take_ties = 0;
   if (screened && !cut_given) {
-    int reached = N, above = 0;  // keys from `cut` up, and beyond the current bounds
-    bool found = false;
-    int shift = 30;
-    for (int step = 0; shift >= 0; shift -= 2, ++step) {
-      uint32_t low = 0, high = 0;  // counts from one and two steps up, from three steps up
+    // The bin of the F-th largest key: the thread whose bins, from the top, take the count past F.
 #pragma unroll
-      for (int j = 0; j < PER; ++j) {
-        low += (key[j] >= (cut | (1u << shift)) ? 1u : 0u) + (key[j] >= (cut | (2u << shift)) ? 0x10000u : 0u);
-        high += key[j] >= (cut | (3u << shift)) ? 1u : 0u;
+    for (int j = 0; j < PER; ++j)
+      if (first + 32 * j < N && key[j]) atomicAdd(&s_bins[select_bin(key[j])], 1u);
+    __syncthreads();
+    uint32_t own[kOwnBins], sum = 0;  // counts, from the top
+#pragma unroll
+    for (int j = 0; j < kOwnBins; j += 4) {
+      const uint4 four = *reinterpret_cast<const uint4*>(s_bins + kSelectBins - kOwnBins * (tid + 1) + kOwnBins - 4 - j);
+      own[j] = four.w;
+      own[j + 1] = four.z;
+      own[j + 2] = four.y;
+      own[j + 3] = four.x;
+      sum += (four.x + four.y) + (four.z + four.w);
+    }
+    uint32_t scan = sum;
+#pragma unroll
+    for (int w = 1; w < 32; w <<= 1) {
+      const uint32_t o = __shfl_up_sync(kFull, scan, w);
+      if (lane >= w) scan += o;
+    }
+    const uint2 totals = warp_prefix(__shfl_sync(kFull, scan, 31), s_slots[2]);
+    uint32_t upto = totals.x + scan - sum;  // keys in higher bins
+    if (upto < static_cast<uint32_t>(F) && upto + sum >= static_cast<uint32_t>(F)) {
+#pragma unroll
+      for (int j = 0; j < kOwnBins; ++j) {
+        if (upto < static_cast<uint32_t>(F) && upto + own[j] >= static_cast<uint32_t>(F)) {
+          s_bin = kSelectBins - 1 - kOwnBins * tid - j;
+          s_above = upto;
+          s_inside = own[j];
+        }
+        upto += own[j];
       }
-      low = __reduce_add_sync(kFull, low);
-      high = __reduce_add_sync(kFull, high);
-      if (lane == 0) s_counts[step & 1][warp] = make_uint2(low, high);
-      __syncthreads();
-      const uint2 c = s_counts[step & 1][lane];
-      low = __reduce_add_sync(kFull, c.x);
-      const int c3 = __reduce_add_sync(kFull, c.y), c2 = low >> 16, c1 = low & 0xffff;
-      if (c3 >= F) {
-        cut |= 3u << shift;
-        reached = c3;
-      } else if (c2 >= F) {
-        cut |= 2u << shift;
-        reached = c2;
-        above = c3;
-      } else if (c1 >= F) {
-        cut |= 1u << shift;
-        reached = c1;
-        above = c2;
-      } else {
-        above = c1;
-      }
-      if (reached == F) {  // exactly the keys from the cut up
-        cut -= 1;
+    }
+    __syncthreads();
+    int above = s_above, reached = above + s_inside;  // keys beyond the bounds, keys from `cut` up
+    int shift = kSelectShift;
+    bool found = false;
+    if (s_inside == 0) {  // fewer than F keys differ from zero: zeros tie for the rest
+      above = totals.y;
+      shift = 0;
+    } else {
+      cut = static_cast<uint32_t>(s_bin) << kSelectShift;
+      if (reached == F) {  // exactly the keys from the cut up, none of them zero
+        cut = max(cut, 1u) - 1u;
         found = true;
-        break;
+      } else if (s_bin == kSelectBins - 1 || s_inside > kSelectListed) {
+        if (s_bin == kSelectBins - 1) {  // whatever has its sign
+          cut = 0;
+          above = 0;
+          reached = N;
+          shift = 32;
+        }
+        // Two bits per step: three counts of the whole CTA, one barrier.
+        for (int step = 0; shift > 0; ++step) {
+          shift -= 2;
+          uint32_t low = 0, high = 0;  // counts from one and two steps up, from three steps up
+#pragma unroll
+          for (int j = 0; j < PER; ++j) {
+            low += (key[j] >= (cut | (1u << shift)) ? 1u : 0u) + (key[j] >= (cut | (2u << shift)) ? 0x10000u : 0u);
+            high += key[j] >= (cut | (3u << shift)) ? 1u : 0u;
+          }
+          low = __reduce_add_sync(kFull, low);
+          high = __reduce_add_sync(kFull, high);
+          if (lane == 0) s_counts[step & 1][warp] = make_uint2(low, high);
+          __syncthreads();
+          const uint2 c = s_counts[step & 1][lane];
+          low = __reduce_add_sync(kFull, c.x);
+          const int c3 = __reduce_add_sync(kFull, c.y), c2 = low >> 16, c1 = low & 0xffff;
+          if (c3 >= F) {
+            cut |= 3u << shift;
+            reached = c3;
+          } else if (c2 >= F) {
+            cut |= 2u << shift;
+            reached = c2;
+            above = c3;
+          } else if (c1 >= F) {
+            cut |= 1u << shift;
+            reached = c1;
+            above = c2;
+          } else {
+            above = c1;
+          }
+          if (reached == F) {  // exactly the keys from the cut up
+            cut -= 1;
+            found = true;
+            break;
+          }
+          if (shift > 0 && reached - above <= kSelectListed) break;
+        }
       }
-      if (shift > 0 && reached - above <= kSelectListed) break;
     }
     if (!found && shift <= 0) {
       take_ties = F - above;  // the cut is the F-th largest key
     } else if (!found) {
-      const uint32_t top = cut + ((1u << shift) - 1);  // largest key within the bounds
+      const uint32_t low = max(cut, 1u), top = cut + ((1u << shift) - 1);  // bounds; the cut is no zero
       int inside = 0;
 #pragma unroll
       for (int j = 0; j < PER; ++j)
-        inside += first + 32 * j < N && key[j] >= cut && key[j] <= top;
-      // Any order will do: a place for every thread's keys from one addition per warp.
-      int scan = inside;
-#pragma unroll
-      for (int w = 1; w < 32; w <<= 1) {
-        const int o = __shfl_up_sync(kFull, scan, w);
-        if (lane >= w) scan += o;
-      }
-      int at = 0;
-      if (lane == 31 && scan) at = atomicAdd(&s_count, scan);
-      at = __shfl_sync(kFull, at, 31) + scan - inside;
-      if (inside) {
+        inside += key[j] >= low && key[j] <= top;
+      if (inside) {  // any order will do
+        int at = atomicAdd(&s_count, inside);
 #pragma unroll
         for (int j = 0; j < PER; ++j)
-          if (first + 32 * j < N && key[j] >= cut && key[j] <= top) s_listed[at++] = key[j];
+          if (key[j] >= low && key[j] <= top) s_listed[at++] = key[j];
       }
       __syncthreads();
       if (warp == 0) {
         const int listed = s_count, wanted = F - above;
-        uint32_t k[kSelectListed / 32];
+        if (listed <= 32) {
+          // Every key against every other: the one that `wanted` keys reach is the cut.
+          const uint32_t own_key = lane < listed ? s_listed[lane] : 0u;
+          int more = 0, same = 0;
+          for (int i = 0; i < listed; ++i) {
+            const uint32_t other = s_listed[i];
+            more += other > own_key;
+            same += other == own_key;
+          }
+          if (more < wanted && more + same >= wanted) {  // one lane, or several with the same key
+            const bool all = more + same == wanted;
+            s_cut = all ? own_key - 1 : own_key;
+            s_take = all ? 0 : wanted - more;
+          }
+        } else {
+          uint32_t k[kSelectListed / 32];
 #pragma unroll
-        for (int j = 0; j < kSelectListed / 32; ++j) k[j] = 32 * j + lane < listed ? s_listed[32 * j + lane] : 0u;
-        auto count_from = [&](uint32_t bound) {
-          int n = 0;
+          for (int j = 0; j < kSelectListed / 32; ++j) k[j] = 32 * j + lane < listed ? s_listed[32 * j + lane] : 0u;
+          auto count_from = [&](uint32_t bound) {
+            int n = 0;
 #pragma unroll
-          for (int j = 0; j < kSelectListed / 32; ++j) n += k[j] >= bound;
-          return __reduce_add_sync(kFull, n);
-        };
-        for (int bit = shift - 1; bit >= 0 && !found; --bit) {
-          const uint32_t trial = cut | (1u << bit);
-          const int n = count_from(trial);
-          if (n >= wanted) cut = trial;
-          found = n == wanted;
-        }
-        const int ties = found ? 0 : wanted - count_from(cut + 1);
-        if (lane == 0) {
-          s_cut = found ? cut - 1 : cut;
-          s_take = ties;
+            for (int j = 0; j < kSelectListed / 32; ++j) n += k[j] >= bound;
+            return __reduce_add_sync(kFull, n);
+          };
+          for (int bit = shift - 1; bit >= 0 && !found; --bit) {
+            const uint32_t trial = cut | (1u << bit);
+            const int n = count_from(trial);
+            if (n >= wanted) cut = trial;
+            found = n == wanted;
+          }
+          const int ties = found ? 0 : wanted - count_from(cut + 1);
+          if (lane == 0) {
+            s_cut = found ? cut - 1 : cut;
+            s_take = ties;
+          }
         }
       }
       __syncthreads();
@@ -922,7 +995,7 @@ __global__ void __launch_bounds__(kSelectThreads, PER <= 4 ? 2 : 1)
   uint32_t kept = 0;  // bit j: this thread keeps its candidate j
 #pragma unroll
   for (int j = 0; j < PER; ++j)
-    kept |= static_cast<uint32_t>(first + 32 * j < N && (!screened || key[j] > cut)) << j;
+    kept |= static_cast<uint32_t>(screened ? key[j] > cut : first + 32 * j < N) << j;
   if (tied_keys) {
     uint32_t running = ties.x;
 #pragma unroll
@@ -944,43 +1017,53 @@ __global__ void __launch_bounds__(kSelectThreads, PER <= 4 ? 2 : 1)
     for (int j = 0; j < PER; ++j)
       if (first + 32 * j < N && s_route[slot_of(L, first + 32 * j)] < 0) kept &= ~(1u << j);
   }
-  mine = 0;
+  // Lane j of a warp goes on with the mask of its candidates 32 j ..: the masks' places, then masks,
+  // lists and bytes by as many threads as there are words of each.  (Byte and entry at a time from the
+  // candidates' threads, stores took half of the kernel's time.)
+  uint32_t word = 0;
 #pragma unroll
-  for (int j = 0; j < PER; ++j) mine += __popc(__ballot_sync(kFull, (kept >> j) & 1u));
-  const uint2 kept_counts = warp_prefix(mine, s_slots[1]);
+  for (int j = 0; j < PER; ++j) {
+    const uint32_t ballot = __ballot_sync(kFull, (kept >> j) & 1u);
+    if (lane == j) word = ballot;
+  }
+  uint32_t scan = __popc(word);
+#pragma unroll
+  for (int w = 1; w < PER; w <<= 1) {
+    const uint32_t o = __shfl_up_sync(kFull, scan, w);
+    if (lane >= w) scan += o;
+  }
+  const uint2 kept_counts = warp_prefix(__shfl_sync(kFull, scan, PER - 1), s_slots[1]);
   const int total_kept = kept_counts.y;
-  uint8_t* selected = ws.selected + static_cast<size_t>(t) * N;
-  uint8_t* completed = ws.completed + static_cast<size_t>(t) * N;
+  if (lane < PER) {
+    s_chunk[warp * PER + lane] = word;
+    s_before[warp * PER + lane] = static_cast<uint16_t>(kept_counts.x + scan - __popc(word));
+  }
+  __syncthreads();
   int32_t* list = ws.candidate_ids + static_cast<size_t>(t) * F;
-  {
-    int running = kept_counts.x;
-#pragma unroll
-    for (int j = 0; j < PER; ++j) {
-      const int i = first + 32 * j;
-      const bool keep = (kept >> j) & 1u;
-      const unsigned ballot = __ballot_sync(kFull, keep);
-      if (lane == 0) {
-        const int word = warp * PER + j;
-        s_chunk[word] = ballot;
-        s_before[word] = static_cast<uint16_t>(running);
-        if (32 * word < N) {
-          ws.kept_bits[static_cast<size_t>(t) * kept_words(N) + word] = ballot;
-          ws.kept_before[static_cast<size_t>(t) * kept_words(N) + word] = static_cast<uint16_t>(running);
-        }
-      }
-      if (i < N) {
-        selected[i] = keep;
-        completed[i] = keep && (!remote || s_route[slot_of(L, i)] >= 0);
-        if (keep) {
-          list[running + __popc(ballot & before)] = i;
-          if (clear) ws.features[static_cast<size_t>(t) * N + i] = __float2bfloat16_rn(0.0f);
-        }
-      }
-      running += __popc(ballot);
+  if (32 * tid < N) {
+    uint32_t bits = s_chunk[tid];
+    int at = s_before[tid];
+    ws.kept_bits[static_cast<size_t>(t) * kept_words(N) + tid] = bits;
+    ws.kept_before[static_cast<size_t>(t) * kept_words(N) + tid] = static_cast<uint16_t>(at);
+    for (; bits; bits &= bits - 1, ++at) {
+      const int i = 32 * tid + __ffs(bits) - 1;
+      list[at] = i;
+      if (clear) ws.features[static_cast<size_t>(t) * N + i] = __float2bfloat16_rn(0.0f);
     }
   }
   for (int i = total_kept + tid; i < F; i += kSelectThreads) list[i] = -1;
-  __syncthreads();
+  // Sixteen candidates' bytes at a time, from the last thread on: N = K I is a multiple of sixteen, and
+  // a slot's first candidate too.
+  for (int i = 16 * (kSelectThreads - 1 - tid); i < N; i += 16 * kSelectThreads) {
+    const uint32_t bits = s_chunk[i >> 5] >> (i & 16);
+    auto bytes = [&](int from) {  // four bits to four bytes
+      return (((bits >> from) & 15u) * 0x00204081u) & 0x01010101u;
+    };
+    const uint4 four = make_uint4(bytes(0), bytes(4), bytes(8), bytes(12));
+    *reinterpret_cast<uint4*>(ws.selected + static_cast<size_t>(t) * N + i) = four;
+    *reinterpret_cast<uint4*>(ws.completed + static_cast<size_t>(t) * N + i) =
+        !remote || s_route[slot_of(L, i)] >= 0 ? four : make_uint4(0, 0, 0, 0);
+  }
   if (warp == 0) {
     const bool live = lane < K;
     const int from = min(lane, K) * I, chunk = from / 32;  // the slot's first candidate

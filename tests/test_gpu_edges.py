@@ -150,3 +150,36 @@ def test_selection_at_every_number_of_keys_per_thread(width):
         torch.cuda.synchronize()
         order = scores.sort(dim=1, descending=True, stable=True).indices[:, : case.plan.final_count]
         assert torch.equal(reader.candidate_ids[-1][:2].long(), order.sort(dim=1).values)
+
+
+@pytest.mark.parametrize("width", [256, 768, 1536, 2048])
+@pytest.mark.parametrize("kind", ["one-bin", "crowded-bin", "few-not-zero", "any-bits"])
+def test_selection_by_bins(kind, width):
+    """Keys that all fall into one bin of the selection, more of them in the cut's bin than one warp
+    compares and than the list takes, fewer than are kept that differ from zero, and any 32 bits."""
+    case = cases._random("bins", width, 128, width, 8, 8, 0, 2, 0.125, 0.5)
+    reader = make_reader(prepared_case(case))
+    run_reader(reader, case)
+    scores = reader.scores[0][:2]
+    n, f = scores.shape[1], case.plan.final_count
+    g = torch.Generator().manual_seed(width)
+    if kind == "one-bin":
+        keys = 0x3F800000 + torch.randperm(0x3FFFF, generator=g)[: 2 * n].view(2, n)
+    elif kind == "crowded-bin":  # some 60 or 200 keys about the cut share a bin
+        keys = 0x3F800000 + (torch.randperm(n * 16, generator=g)[: 2 * n] * (0x40000 // (60 * 16 * (1 + 2 * (width > 768))))).view(2, n)
+    elif kind == "few-not-zero":
+        keys = torch.where(torch.rand(2, n, generator=g) < 0.5 * f / n, 0x3F800000 + torch.arange(n), 0)
+    else:
+        keys = torch.randint(0, 1 << 32, (2, n), generator=g)
+        keys[:, ::3] = keys[:, ::3] % 5 + 0xFFFFFFF0
+    signed = torch.where(keys >= 1 << 31, keys - (1 << 32), keys).int()
+    scores.view(torch.int32).copy_(signed)
+    call = reader._call_struct(2, *(t.cuda() for t in (case.hidden, case.ids, case.weights)), None,
+                               torch.empty(2, 128, dtype=torch.bfloat16, device="cuda"), False)
+    call.scores_ready = 1
+    reader._stage("cfm_select", call)
+    torch.cuda.synchronize()
+    kept = keys.sort(dim=1, descending=True, stable=True).indices[:, :f].sort(dim=1).values
+    assert torch.equal(reader.candidate_ids[-1][:2].cpu().long(), kept)
+    mask = torch.zeros(2, n, dtype=torch.uint8).scatter_(1, kept, 1)
+    assert torch.equal(reader.workspace.selected[:2].cpu().view(2, n).to(torch.uint8), mask)
