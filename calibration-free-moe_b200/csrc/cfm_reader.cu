@@ -164,7 +164,7 @@ static int make_layout(const cfm_layer* l, int32_t capacity, cfm_workspace_layou
   o->variances = take(4 * C * 2 * N);
   const int64_t E = std::max<int64_t>(l->experts, 1);
   o->features = take(2 * C * N);
-  o->pass_work = take(16 * (C * K / 8 + std::min(E, C * K)));  // of at least eight pairs
+  o->pass_work = take(16 * (C * K / 4 + std::min(E, C * K)));  // of at least four pairs
   o->busy_experts = take(4 * E);
   o->work_counts = take(32);
   o->tile_list = take(32 * C * ((F + kDownTileRows - 1) / kDownTileRows + K));
@@ -1971,18 +1971,24 @@ static bool shares_decode(const Bound& b) {
   return 3 * static_cast<int64_t>(b.T) * b.L.K > 16 * static_cast<int64_t>(b.L.E);
 }
 // The tcgen05 screen on request, where several tokens share its decode, or where its CTAs of 128 channels
-// give every SM one: three tokens of the 128-expert layer 12.6 us against 12.4 of the warp-level kernel, six
-// 15.6 against 19.6, two of hidden 4096 and width 1536 25.9 against 30.6; one token (48 CTAs) 11.8 against 6.1,
-// eight of the 256-expert layer of width 512 14.6 against 13.1.  Its tables have to fit shared memory.
+// give most SMs one or the rows are long: three tokens of the 128-expert layer (144 CTAs) 10.0 us against 12.4
+// of the warp-level kernel, two of the 64-expert layer (128) 9.8 against 11.5, one of hidden 4096 and width
+// 1536 (96 CTAs, 32 blocks) 17.1 against 19.4; two of the 128-expert layer (96, 16 blocks) 9.9 against 8.3,
+// four of the 256-expert layer of width 512 (128) 10.5 against 8.4.  Its tables have to fit shared memory.
 static bool screens_tc(const Bound& b) {
   const int64_t ctas = static_cast<int64_t>(busy_experts(b)) * ((b.L.I + kScreenChannels - 1) / kScreenChannels);
-  return (b.L.tensor_engine == CFM_ENGINE_TCGEN05 || shares_decode(b) || ctas > 148) && b.L.B <= 512;
+  return (b.L.tensor_engine == CFM_ENGINE_TCGEN05 || shares_decode(b) || ctas >= 128 || ctas * b.L.B >= 96 * 32) &&
+         b.L.B <= 512;
 }
-// Its passes of sixteen tokens from sixteen tokens per expert on: 256 tokens of hidden 4096 and width 1536 240
-// us against 269 of passes of eight; 100 of the 64-expert layer 50 against 47 (recovery-aware score 78 against
-// 66), 256 of the 256-expert layer 59 against 56: fewer warps fit an SM, and fewer passes are full.
+// Its passes.  Of four tokens, five CTAs per SM and fewer instructions for empty places, up to four tokens per
+// expert: 32 tokens of the 128-expert layer 24.5 us against 30.4 of passes of eight, 64 of them (4 per expert)
+// 35.1 against 37.8, 50 of the 64-expert layer (6.3) 43 against 38.  Of sixteen from sixteen tokens per expert
+// on: 256 tokens of hidden 4096 and width 1536 240 us against 269 of eight; 100 of the 64-expert layer (12.5)
+// 50 against 47 (recovery-aware score 78 against 66), for fewer warps fit an SM and fewer passes are full.
 static int pass_pairs(const Bound& b) {
-  return screens_tc(b) && static_cast<int64_t>(b.T) * b.L.K >= 16 * static_cast<int64_t>(b.L.E) ? 16 : 8;
+  if (!screens_tc(b)) return 8;
+  const int64_t pairs = static_cast<int64_t>(b.T) * b.L.K, experts = b.L.E;
+  return pairs >= 16 * experts ? 16 : pairs <= 4 * experts ? 4 : 8;
 }
 
 static int group_smem(const Bound& b, size_t* smem) {
@@ -2093,9 +2099,11 @@ static int run_screen_grouped(const Bound& b) {
   const int rows = static_cast<int>(pairs / pass) + busy_experts(b) + (dead > 0);
   if (screens_tc(b)) {
     const bool risk = b.L.score == CFM_SCORE_RECOVERY_AWARE;
-    if (pass == 16)
-      return risk ? launch_screen_tc<16, true>(b, rows, dead) : launch_screen_tc<16, false>(b, rows, dead);
-    return risk ? launch_screen_tc<8, true>(b, rows, dead) : launch_screen_tc<8, false>(b, rows, dead);
+    switch (pass) {
+      case 4: return risk ? launch_screen_tc<4, true>(b, rows, dead) : launch_screen_tc<4, false>(b, rows, dead);
+      case 8: return risk ? launch_screen_tc<8, true>(b, rows, dead) : launch_screen_tc<8, false>(b, rows, dead);
+      default: return risk ? launch_screen_tc<16, true>(b, rows, dead) : launch_screen_tc<16, false>(b, rows, dead);
+    }
   }
   // Four warps per tile while one each would not give every SM its sixteen (one token of the
   // 128-expert layer: 6.9 us against 12.3; 8 tokens 24.5 against 23.4).  The products of a tile

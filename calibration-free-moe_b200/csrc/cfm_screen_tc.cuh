@@ -20,10 +20,10 @@
 // wait for one another.
 // Bound by instruction issue, some 150 per warp and tile with four tokens, 56 of them the decode's (0.8
 // of the issue slots while four CTAs share an SM), and by the last CTAs of a launch, alone on their SM.
-// 64 tokens of the 128-expert layer (100 MB of codes: 15 us of HBM) 37 us, 32 tokens 32, 8 tokens 19,
-// 256 tokens of hidden 4096 and width 1536 240, against 56, 44, 27 and 404 of 64 channels per CTA whose
-// threads copied, waited for their product and met at a barrier once per block.  Persistent CTAs with
-// units of 64 channels, whose two places in tensor memory alternate between blocks, took 59 us at 64
+// 64 tokens of the 128-expert layer (100 MB of codes: 15 us of HBM) 35 us, 32 tokens 24.5, 8 tokens
+// 15, 256 tokens of hidden 4096 and width 1536 240, against 56, 44, 27 and 404 of 64 channels per CTA
+// whose threads copied, waited for their product and met at a barrier once per block.  Persistent CTAs
+// with units of 64 channels, whose two places in tensor memory alternate between blocks, took 59 us at 64
 // tokens (140 instructions per block and warp for copies and waits that a pair of tiles shares here);
 // one driver for all copies and products, 45.
 // Included by cfm_reader.cu inside namespace cfm.
@@ -36,16 +36,17 @@ constexpr int kScreenAhead = 4;  // blocks whose variances are on their way toge
 
 template <int TOKENS, bool RISK>
 struct Screen {
-  static constexpr int kColumns = TOKENS == 8 ? 32 : 3 * TOKENS;  // N: three digits per token
+  static constexpr int kColumns = TOKENS == 16 ? 48 : 4 * TOKENS;  // N: three digits per token, a multiple of 16
   static constexpr int kDigitStep = kColumns * 32;             // bytes of one K = 32 step
   static constexpr int kDigitBytes = 4 * kDigitStep;           // of a block
   static constexpr int kCodeBytes = kScreenChannels * 68;      // gate codes, up codes, gate scales, up scales
-  static constexpr int kCodeRing = TOKENS == 8 ? 4 : 3;        // blocks
+  static constexpr int kCodeRing = TOKENS == 16 ? 3 : 4;       // blocks
   static constexpr int kDigitRing = 3;                         // the next two are on their way
-  // Tensor memory: the first operand of the gate tile, then 128 columns that begin with that of the up
-  // tile (eight tokens: all in the 128), then the tiles' sums.
-  static constexpr int kSumsStep = TOKENS == 8 ? 32 : 48;      // between the tiles' sums
-  static constexpr int kPerSm = TOKENS == 8 ? 4 : 3;
+  // Tensor memory, for each tile 32 columns of its product's first operand and the sums, in two pieces:
+  // four tokens 32 (sums) and 64, eight 128, sixteen 32 (first operand of the gate tile) and 128.
+  static constexpr int kSumsStep = kColumns;
+  static constexpr int kSmall = TOKENS == 8 ? 0 : 32, kLarge = TOKENS == 4 ? 64 : 128;
+  static constexpr int kPerSm = TOKENS == 4 ? 5 : TOKENS == 8 ? 4 : 3;
   static constexpr int kStride = kScreenChannels * (RISK ? 4 : 2);  // floats per token of the end
   static constexpr size_t kCopies = static_cast<size_t>(kCodeRing) * kCodeBytes + kDigitRing * kDigitBytes;
   static constexpr size_t kEnd = static_cast<size_t>(TOKENS) * kStride * sizeof(float);
@@ -273,10 +274,11 @@ __global__ void __launch_bounds__(kScreenThreads, Screen<TOKENS, RISK>::kPerSm)
   }
   // The small piece first: were the large ones held by CTAs that wait for a small one, none would end.
   if (warp == 4) {
-    if (TOKENS == 16)
+    if (S::kSmall)
       asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 32;" ::"r"(shared_u32(tmem_holder + 1))
                    : "memory");
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 128;" ::"r"(shared_u32(tmem_holder))
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(shared_u32(tmem_holder)),
+                 "n"(S::kLarge)
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
@@ -285,7 +287,7 @@ __global__ void __launch_bounds__(kScreenThreads, Screen<TOKENS, RISK>::kPerSm)
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   // First operands of the gate and the up tile, sums.
   const uint32_t tmem_rows[2] = {TOKENS == 16 ? tmem_holder[1] : tmem_holder[0], tmem_holder[0] + (TOKENS == 16 ? 0 : 32)};
-  const uint32_t tmem_sums = tmem_rows[1] + 32;
+  const uint32_t tmem_sums = TOKENS == 4 ? tmem_holder[1] : tmem_rows[1] + 32;
   // Per block and two tokens the scales of the fixed point and the sums of the values; energies.
   int4* factor = reinterpret_cast<int4*>(screen_shared + S::kRing);
   float* energy = reinterpret_cast<float*>(factor + TOKENS / 2 * B);
@@ -418,7 +420,7 @@ __global__ void __launch_bounds__(kScreenThreads, Screen<TOKENS, RISK>::kPerSm)
       auto load_sums = [&](int tile, int half, int (&c)[24]) {
         const uint32_t sums = tmem_sums + lanes + tile * S::kSumsStep + 24 * half;
         load_columns16(sums, c);
-        if (count > 8 * half + 4) load_columns8(sums + 16, c + 16);
+        if (TOKENS > 4 && count > 8 * half + 4) load_columns8(sums + 16, c + 16);
       };
       // Adds them, block b, to the projections, four tokens at a time.
       auto rescale = [&](auto which, int half, int b, const int (&c)[24]) {
@@ -426,8 +428,8 @@ __global__ void __launch_bounds__(kScreenThreads, Screen<TOKENS, RISK>::kPerSm)
         const Pair scales = pair_of(scale[tile], scale[tile]);
         const int4* factors = factor + (b * TOKENS + 8 * half) / 2;
 #pragma unroll
-        for (int four = 0; four < 2; ++four) {
-          if (8 * half + 4 * four >= count) break;
+        for (int four = 0; four < (TOKENS > 4 ? 2 : 1); ++four) {
+          if (TOKENS > 4 && 8 * half + 4 * four >= count) break;
 #pragma unroll
           for (int two = 2 * four; two < 2 * four + 2; ++two) {
             const int4 f = factors[two];
@@ -490,7 +492,7 @@ __global__ void __launch_bounds__(kScreenThreads, Screen<TOKENS, RISK>::kPerSm)
         barrier_wait(done + 8 * tile, (B - 1) & 1, abort);
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
-        for (int half = 0; half < TOKENS / 8; ++half) {
+        for (int half = 0; half < (TOKENS + 7) / 8; ++half) {
           if (8 * half >= count) break;
           load_sums(tile, half, c);
           load_wait();
@@ -596,8 +598,9 @@ __global__ void __launch_bounds__(kScreenThreads, Screen<TOKENS, RISK>::kPerSm)
   if (warp == 4) {
     if (abort_flag && lane == 0) atomicExch(&ws.status[0], 1);
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 128;" ::"r"(tmem_holder[0]) : "memory");
-    if (TOKENS == 16)
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_holder[0]), "n"(S::kLarge)
+                 : "memory");
+    if (S::kSmall)
       asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 32;" ::"r"(tmem_holder[1]) : "memory");
   }
 }

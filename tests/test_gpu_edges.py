@@ -102,7 +102,7 @@ def test_layer_at_the_edges(oracle, name, padded):
 @pytest.mark.parametrize("hidden,width", [(128, 16), (256, 112), (384, 128), (640, 144), (1152, 272)])
 def test_tcgen05_screen_at_the_edges_of_its_tiles(oracle, hidden, width, tokens, score):
     """Channels around 128 per CTA and 32 per warp, blocks around the lengths of its rings, passes of
-    eight and of sixteen tokens with remainders: every projection, variance and score of the oracle."""
+    four, eight and sixteen tokens with remainders: every projection and score of the oracle."""
     case = cases._random("tiles", hidden + tokens, hidden, width, 5, 2, 8, tokens, 0.25, 0.75, score=score)
     item = prepared_case(case)
     reader = make_reader(item, capacity=tokens, tensor_engine="tcgen05")
