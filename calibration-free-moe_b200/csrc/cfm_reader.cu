@@ -1318,6 +1318,38 @@ __global__ void __launch_bounds__(kExactWarps * 32, STRIDED ? 4 : 5) k_exact_pai
 // 13 us for 64).  `shared`: 256 + 4 * 256 floats.
 constexpr int kEncodeThreads = 128;
 
+// The latent of a token whose encoder sums are all there, by 128 threads.
+__device__ __forceinline__ void mix_latent(const Layer& L, const Workspace& ws, int t) {
+  const int tid = threadIdx.x, R = L.R;
+  // Per slot the sums in tile order, rounded to BF16, times the router weight, in slot order.
+  const int parts_of_slot = ws.encoder_tiles, all_parts = L.K * parts_of_slot;
+  const size_t pair0 = static_cast<size_t>(t) * L.K;
+  for (int r = tid; r < R; r += kEncodeThreads) {
+    const float* p = ws.encoder_parts + pair0 * parts_of_slot * R + r;
+    float latent = 0.0f, sum = 0.0f;
+    int slot2 = 0, left = parts_of_slot;
+    for (int n0 = 0; n0 < all_parts; n0 += 8) {
+      float v[8];  // on their way together
+#pragma unroll
+      for (int n = 0; n < 8; ++n)
+        v[n] = n0 + n < all_parts ? __ldcg(p + static_cast<size_t>(n0 + n) * R) : 0.0f;
+#pragma unroll
+      for (int n = 0; n < 8; ++n) {
+        if (n0 + n >= all_parts) break;
+        sum += v[n];
+        if (--left == 0) {
+          if (ws.ids[pair0 + slot2] >= 0)
+            latent = fmaf(bf16_round(sum), ws.weights[pair0 + slot2], latent);
+          sum = 0.0f;
+          left = parts_of_slot;
+          ++slot2;
+        }
+      }
+    }
+    ws.latent[static_cast<size_t>(t) * R + r] = latent;
+  }
+}
+
 __device__ __forceinline__ void encode_tile(const Layer& L, const Workspace& ws,
                                             const uint8_t* padding, int index, float* shared) {
   float* feature = shared;
@@ -1394,32 +1426,139 @@ __device__ __forceinline__ void encode_tile(const Layer& L, const Workspace& ws,
   __syncthreads();
   if (shared[0] == 0.0f) return;
   __threadfence();
-  // Per slot the sums in tile order, rounded to BF16, times the router weight, in slot order.
-  const int parts_of_slot = ws.encoder_tiles, all_parts = L.K * parts_of_slot;
-  const size_t pair0 = static_cast<size_t>(t) * L.K;
-  for (int r = tid; r < R; r += kEncodeThreads) {
-    const float* p = ws.encoder_parts + pair0 * parts_of_slot * R + r;
-    float latent = 0.0f, sum = 0.0f;
-    int slot2 = 0, left = parts_of_slot;
-    for (int n0 = 0; n0 < all_parts; n0 += 8) {
-      float v[8];  // on their way together
+  mix_latent(L, ws, t);
+}
+
+// The same sums for up to four pairs of an expert at a time: its rows are read and widened once for all
+// of them (a pair at a time they came from L2 once per pair, 0.8 GB for 256 tokens of hidden 4096 and width
+// 1536), and a pair's product is one packed instruction per two columns.  Rows, their order and every
+// rounding are encode_tile's.  `index` = (pass * subs + part of the pass) * tiles + tile; after those, CTAs
+// whose threads zero the latents of tokens without a live pair.  `shared`: 4 x 256 pairs of floats, 4 x 4 x
+// 256 floats, 4 words.
+constexpr int kEncodePairs = 4;
+constexpr int kEncodeGroupBytes = kEncodePairs * (kEncodeTileRows * 8 + 4 * 256 * 4) + 16;
+
+template <int N>
+__device__ __forceinline__ void encode_rows(const __nv_bfloat16* rows, const Pair* feature, int c0, int c1, int R,
+                                            int group, int groups, float (*red)[4][256], int col, int lpr) {
+  constexpr int U = 8;
+  Pair acc[N][4];
 #pragma unroll
-      for (int n = 0; n < 8; ++n)
-        v[n] = n0 + n < all_parts ? __ldcg(p + static_cast<size_t>(n0 + n) * R) : 0.0f;
+  for (int n = 0; n < N; ++n)
 #pragma unroll
-      for (int n = 0; n < 8; ++n) {
-        if (n0 + n >= all_parts) break;
-        sum += v[n];
-        if (--left == 0) {
-          if (ws.ids[pair0 + slot2] >= 0)
-            latent = fmaf(bf16_round(sum), ws.weights[pair0 + slot2], latent);
-          sum = 0.0f;
-          left = parts_of_slot;
-          ++slot2;
-        }
+    for (int j = 0; j < 4; ++j) acc[n][j] = 0;
+  for (int base = c0 + group; base < c1; base += groups * U) {
+    uint4 w[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int c = base + u * groups;
+      w[u] = c < c1 ? *reinterpret_cast<const uint4*>(rows + static_cast<size_t>(c) * R) : make_uint4(0, 0, 0, 0);
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int c = min(base + u * groups, c1 - 1) - c0;
+      const bool there = base + u * groups < c1;
+      const Pair v[4] = {pair_of(bf16_lo(w[u].x), bf16_hi(w[u].x)), pair_of(bf16_lo(w[u].y), bf16_hi(w[u].y)),
+                         pair_of(bf16_lo(w[u].z), bf16_hi(w[u].z)), pair_of(bf16_lo(w[u].w), bf16_hi(w[u].w))};
+#pragma unroll
+      for (int n = 0; n < N; ++n) {
+        const Pair a = there ? feature[n * kEncodeTileRows + c] : 0;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc[n][j] = pair_fma(v[j], a, acc[n][j]);
       }
     }
-    ws.latent[static_cast<size_t>(t) * R + r] = latent;
+  }
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+  for (int n = 0; n < N; ++n) {
+    float sum[8];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) pair_split(acc[n][j], sum[2 * j], sum[2 * j + 1]);
+    for (int w = lpr; w < 32; w <<= 1) {  // the row groups that share a warp
+#pragma unroll
+      for (int j = 0; j < 8; ++j) sum[j] += __shfl_xor_sync(kFull, sum[j], w);
+    }
+    if (lane < lpr) {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) red[n][warp][col + j] = sum[j];
+    }
+  }
+}
+
+__device__ __forceinline__ void encode_group(const Layer& L, const Workspace& ws, const uint8_t* padding, int index,
+                                             int subs, int group_ctas, int tokens, uint8_t* shared) {
+  const int tid = threadIdx.x, lane = tid & 31, R = L.R, I = L.I, tiles = ws.encoder_tiles;
+  if (index >= group_ctas) {
+    const int t = (index - group_ctas) * kEncodeThreads + tid;
+    bool live = t >= tokens;
+    for (int k = 0; k < L.K && !live; ++k)
+      live = !(padding && padding[t]) && ws.ids[static_cast<size_t>(t) * L.K + k] >= 0;
+    if (!live)
+      for (int r = 0; r < R; ++r) ws.latent[static_cast<size_t>(t) * R + r] = 0.0f;
+    return;
+  }
+  const int tile = index % tiles, part = index / tiles % subs, number = index / tiles / subs;
+  if (number >= ws.work_counts[kPassCount]) return;
+  const int4 pass = *reinterpret_cast<const int4*>(ws.pass_work + number);
+  const int e = pass.x, first = pass.y + kEncodePairs * part, count = min(kEncodePairs, pass.z - kEncodePairs * part);
+  if (count <= 0) return;
+  Pair* feature = reinterpret_cast<Pair*>(shared);
+  float(*red)[4][256] = reinterpret_cast<float(*)[4][256]>(shared + kEncodePairs * kEncodeTileRows * 8);
+  int* last = reinterpret_cast<int*>(shared + kEncodePairs * (kEncodeTileRows * 8 + 4 * 256 * 4));
+  const int c0 = tile * kEncodeTileRows, c1 = min(I, c0 + kEncodeTileRows);
+  int pairs[kEncodePairs];
+#pragma unroll
+  for (int n = 0; n < kEncodePairs; ++n) pairs[n] = ws.group_pairs[first + min(n, count - 1)];
+#pragma unroll
+  for (int i = 0; i < kEncodeTileRows / kEncodeThreads; ++i) {
+    const int c = min(c0 + tid + i * kEncodeThreads, c1 - 1);
+    uint8_t kept[kEncodePairs];
+    __nv_bfloat16 f[kEncodePairs];
+#pragma unroll
+    for (int n = 0; n < kEncodePairs; ++n) {
+      const size_t at = static_cast<size_t>(pairs[n]) * I + c;  // (t K + slot) I = t N + slot I
+      kept[n] = ws.selected[at];
+      f[n] = ws.features[at];
+    }
+#pragma unroll
+    for (int n = 0; n < kEncodePairs; ++n) {
+      const float v = kept[n] ? 0.0f : __bfloat162float(f[n]);
+      feature[n * kEncodeTileRows + c - c0] = pair_of(v, v);
+    }
+  }
+  __syncthreads();
+  const int lpr = R / 8, groups = kEncodeThreads / lpr, group = tid / lpr, col = (tid - group * lpr) * 8;
+  const __nv_bfloat16* rows = L.encoder + static_cast<size_t>(e) * I * R + col;
+  switch (count) {
+    case 1: encode_rows<1>(rows, feature, c0, c1, R, group, groups, red, col, lpr); break;
+    case 2: encode_rows<2>(rows, feature, c0, c1, R, group, groups, red, col, lpr); break;
+    default: encode_rows<4>(rows, feature, c0, c1, R, group, groups, red, col, lpr); break;
+  }
+  __syncthreads();
+  for (int i = tid; i < count * R; i += kEncodeThreads) {
+    const int n = i / R, r = i - n * R;
+    const float(*own)[256] = red[n];
+    const int pair = n == 0 ? pairs[0] : n == 1 ? pairs[1] : n == 2 ? pairs[2] : pairs[3];
+    ws.encoder_parts[(static_cast<size_t>(pair) * tiles + tile) * R + r] =
+        ((own[0][r] + own[1][r]) + own[2][r]) + own[3][r];
+  }
+  __threadfence();
+  __syncthreads();
+  // The last to arrive of a token's live pairs and their tiles mixes its latent.
+  if (tid < count) {
+    const int t = (tid == 0 ? pairs[0] : tid == 1 ? pairs[1] : tid == 2 ? pairs[2] : pairs[3]) / L.K;
+    int live = 0;
+    for (int k = 0; k < L.K; ++k) live += ws.ids[static_cast<size_t>(t) * L.K + k] >= 0;
+    uint32_t* counter = ws.counters + 2 * static_cast<size_t>(ws.capacity) * L.K + t;
+    const bool done = atomicAdd(counter, 1u) == static_cast<unsigned>(live * tiles - 1);
+    if (done) *counter = 0;
+    last[tid] = done ? t : -1;
+  }
+  __syncthreads();
+  for (int n = 0; n < count; ++n) {
+    if (last[n] < 0) continue;
+    __threadfence();
+    mix_latent(L, ws, last[n]);
   }
 }
 
@@ -1434,6 +1573,7 @@ __global__ void __launch_bounds__(kEncodeThreads) k_encode(Layer L, Workspace ws
 // down: gathered channel-major down rows
 // ---------------------------------------------------------------------------
 constexpr int kDownRingBytes = 32 * 1024;  // per CTA
+static_assert(kEncodeGroupBytes <= kDownRingBytes, "the encoder's arrays lie in the ring");
 
 // 128 threads, kDownRingBytes of dynamic shared memory.  A CTA sums up to 64 kept rows of one
 // expert, each scaled by its activation, over 256 CHUNKS output columns.  A warp takes every fourth
@@ -1537,6 +1677,7 @@ __device__ __forceinline__ void down_tile(const Layer& L, const Workspace& ws, i
 // `columns` CTAs per tile.
 struct DownGrid {
   int encode_ctas, columns, tiles;
+  int encode_subs, group_ctas, tokens;  // parts of a screen pass that share encoder rows (0: none do)
 };
 
 // The tiles of every token in turn: 1D grid of encode_ctas + T * tiles * columns CTAs.  Under expert
@@ -1599,14 +1740,17 @@ __global__ void __launch_bounds__(128, 4) k_down(Layer L, Workspace ws, const ui
 // (cfm_select.cuh): 1D grid of encode_ctas + tiles * columns CTAs.  A CTA reads its 32-byte record
 // and goes straight to the tile's rows.  Same tiles, same sums, same bits as k_down.
 template <int CHUNKS>
-__global__ void __launch_bounds__(128, 4) k_down_tiles(Layer L, Workspace ws, const uint8_t* padding,
+__global__ void __launch_bounds__(128, 5) k_down_tiles(Layer L, Workspace ws, const uint8_t* padding,
                                                        DownGrid d) {
   extern __shared__ __align__(128) uint8_t down_ring[];
   __shared__ int tile_channel[kDownTileRows];
   __shared__ float tile_activation[kDownTileRows];
   if (static_cast<int>(blockIdx.x) < d.encode_ctas) {
     grid_dependency_release();
-    encode_tile(L, ws, padding, blockIdx.x, reinterpret_cast<float*>(down_ring));
+    if (d.encode_subs)
+      encode_group(L, ws, padding, blockIdx.x, d.encode_subs, d.group_ctas, d.tokens, down_ring);
+    else
+      encode_tile(L, ws, padding, blockIdx.x, reinterpret_cast<float*>(down_ring));
     return;
   }
   grid_dependency_wait();     // the activations and the list are complete
@@ -2327,6 +2471,16 @@ static int run_exact(const Bound& b, const cfm_call* call, bool whole) {
   return launched();
 }
 
+// The encoder for four pairs of an expert at a time, from four tokens per expert on where the gathers beside
+// it are long enough to cover its chain of loads, a quarter of a gigabyte: 96 tokens of the 128-expert layer
+// (0.3 GB) 38 us against 45 of a pair at a time, 100 of the 64-expert layer 46 against 57, 243 of the 256-expert
+// layer 52 against 70, hidden 4096 and width 1536 with 64 tokens 103 against 117 and with 256 522 against 597;
+// 64 tokens of the 128-expert layer (0.2 GB) 34 against 33, 50 of the 64-expert layer 38 against 33.
+static bool shares_encoder(const Bound& b) {
+  const int64_t pairs = static_cast<int64_t>(b.T) * b.L.K;
+  return pairs_grouped(b) && !b.L.expert_map && pairs >= 4 * static_cast<int64_t>(b.L.E) &&
+         2 * static_cast<int64_t>(b.T) * b.L.F * b.L.H >= 240000000;
+}
 // `encode`: run the recovery encoder too.  `whole`: part of a whole call.
 static int run_down(const Bound& b, bool encode, bool whole) {
   if (!b.L.down) return CFM_E_NULL;
@@ -2344,8 +2498,16 @@ static int run_down(const Bound& b, bool encode, bool whole) {
   const int64_t expected = static_cast<int64_t>(b.T) * (b.L.F / kDownTileRows + b.L.K / 2 + 1);
   int chunks = 4;
   while (chunks > 1 && expected * ((b.L.H + 256 * chunks - 1) / (256 * chunks)) < 2 * 148) chunks /= 2;
-  DownGrid d;
+  DownGrid d = {};
   d.encode_ctas = encode ? b.T * b.L.K * b.ws.encoder_tiles : 0;
+  if (encode && whole && shares_encoder(b)) {
+    const int pass = pass_pairs(b);
+    const int64_t passes = static_cast<int64_t>(b.T) * b.L.K / pass + busy_experts(b);
+    d.encode_subs = pass / kEncodePairs;
+    d.group_ctas = static_cast<int>(passes * d.encode_subs * b.ws.encoder_tiles);
+    d.tokens = b.T;
+    d.encode_ctas = d.group_ctas + (b.T + kEncodeThreads - 1) / kEncodeThreads;
+  }
   d.columns = (b.L.H + 256 * chunks - 1) / (256 * chunks);
   d.tiles = static_cast<int>(tiles);
   const unsigned ctas = static_cast<unsigned>(d.encode_ctas + tiles * d.columns * (listed ? 1 : b.T));

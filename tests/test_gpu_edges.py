@@ -183,3 +183,24 @@ def test_selection_by_bins(kind, width):
     assert torch.equal(reader.candidate_ids[-1][:2].cpu().long(), kept)
     mask = torch.zeros(2, n, dtype=torch.uint8).scatter_(1, kept, 1)
     assert torch.equal(reader.workspace.selected[:2].cpu().view(2, n).to(torch.uint8), mask)
+
+
+@pytest.mark.parametrize("rank,width,tokens", [(8, 400, 26), (64, 272, 40), (256, 256, 42)])
+def test_encoder_rows_shared_by_an_experts_pairs(rank, width, tokens):
+    """Large calls sum the encoder for several pairs of an expert at a time; the stage on its own takes a
+    pair at a time.  The same latents, with padding and with passes that are not full."""
+    hidden, experts, top_k = 4096, 6, 5
+    case = cases._random("shared", rank, hidden, width, experts, top_k, rank, tokens, 0.7, 0.625,
+                         padding=[t % 7 == 3 for t in range(tokens)])
+    assert 2 * tokens * case.plan.final_count * hidden >= 240_000_000
+    reader = make_reader(prepared_case(case))
+    run_reader(reader, case)
+    device = reader.latent.device
+    whole = reader.latent[:tokens].clone()
+    assert whole.abs().sum() > 0
+    reader.latent.fill_(float("nan"))
+    call = reader._call_struct(tokens, *(t.to(device) for t in (case.hidden, case.ids, case.weights, case.padding)),
+                               torch.empty(tokens, hidden, dtype=torch.bfloat16, device=device), False)
+    reader._stage("cfm_encode", call)
+    torch.cuda.synchronize()
+    assert torch.equal(whole, reader.latent[:tokens])
