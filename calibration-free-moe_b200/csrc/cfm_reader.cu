@@ -1169,14 +1169,19 @@ __device__ __forceinline__ void exact_dot(const uint4* gate, const uint4* up, co
   u_out = u;
 }
 
-// grid (ceil(F / 4), T), 128 threads; one warp per kept candidate.
-__global__ void __launch_bounds__(kExactWarps * 32) k_exact(Layer L, Workspace ws,
+// grid (ceil(F / 4), T), 128 threads; one warp per kept candidate.  With `list` one more CTA row, the
+// first, lists the down tiles meanwhile.
+__global__ void __launch_bounds__(kExactWarps * 32, 5) k_exact(Layer L, Workspace ws,
                                                             const __nv_bfloat16* hidden,
-                                                            const uint8_t* padding) {
+                                                            const uint8_t* padding, int list_tiles) {
   grid_dependency_wait();     // the selection is complete
   grid_dependency_release();  // the down kernel may be scheduled: its encoder needs no more than that
   extern __shared__ uint4 xs[];  // H bf16 values of the token
-  const int t = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  if (list_tiles && blockIdx.y == 0) {
+    if (blockIdx.x == 0) list_down_tiles(L, ws, reinterpret_cast<int*>(xs));
+    return;
+  }
+  const int t = blockIdx.y - list_tiles, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   if (padding && padding[t]) return;
   const int32_t* list = ws.candidate_ids + static_cast<size_t>(t) * L.F;
   const bool strided = gridDim.x * kExactWarps < L.F;  // CTAs walk the list in strides
@@ -2419,6 +2424,11 @@ static int run_down_union(const Bound& b, bool encode, bool whole) {
                            static_cast<uint32_t>((1ull << 32) / (b.L.H / X::kColumns) + 1));
 }
 
+// The gather that walks pairs in expert order, from twelve tokens on: with fewer the tokens share few rows, and
+// every CTA's way to its rows is longer (8 tokens of the 128-expert layer 12.5 us and 8.7 of the down tiles against
+// 14.9 and 7.7, of hidden 4096 and width 1536 38.4 and 21.3 against 40.4 and 20.9; 12 of the 64-expert layer 25.5 and
+// 13.3 against 23.7 and 11.8).
+static bool gathers_by_pair(const Bound& b) { return pairs_grouped(b) && (b.L.expert_map || b.T >= 12); }
 // `whole`: part of a whole call; the down tiles are listed too where the down kernel needs them.
 static int run_exact(const Bound& b, const cfm_call* call, bool whole) {
   if (!call->hidden || !b.L.gate_up) return CFM_E_NULL;
@@ -2436,7 +2446,7 @@ static int run_exact(const Bound& b, const cfm_call* call, bool whole) {
                                  static_cast<int>(smem));
     if (err != cudaSuccess) return static_cast<int>(err);
   }
-  if (pairs_grouped(b)) {
+  if (gathers_by_pair(b)) {
     const bool list = whole;
     // One warp per kept row of a pair when the pair keeps the mean number of rows.
     const int per_pair = (b.L.F + b.L.K - 1) / b.L.K;
@@ -2466,8 +2476,9 @@ static int run_exact(const Bound& b, const cfm_call* call, bool whole) {
     const int64_t share = (2LL * ctas * b.L.E + b.L.global_experts - 1) / b.L.global_experts;
     ctas = static_cast<int>(std::max<int64_t>(8, std::min<int64_t>(ctas, share)));
   }
-  launch_dependent(k_exact, dim3(ctas, b.T), dim3(kExactWarps * 32), smem, b.stream, b.L, b.ws,
-                   static_cast<const __nv_bfloat16*>(call->hidden), b.padding);
+  const int list = whole && pairs_grouped(b);
+  launch_dependent(k_exact, dim3(ctas, b.T + list), dim3(kExactWarps * 32), smem, b.stream, b.L, b.ws,
+                   static_cast<const __nv_bfloat16*>(call->hidden), b.padding, list);
   return launched();
 }
 
