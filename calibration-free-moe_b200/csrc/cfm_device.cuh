@@ -43,8 +43,8 @@ __device__ __forceinline__ float pinned_exp(float x) {
   p = __fmaf_rn(p, r, 0.5f);
   p = __fmaf_rn(p, r, 1.0f);
   p = __fmaf_rn(p, r, 1.0f);
-  const int e = static_cast<int>(n);  // in [-126, 127]
-  const float y = __fmul_rn(p, __int_as_float((e + 127) << 23));
+  const uint32_t e = static_cast<uint32_t>(static_cast<int>(n)) + 127u;  // in [1, 254]
+  const float y = __fmul_rn(p, __uint_as_float(e << 23));
   return x >= 88.0f ? __int_as_float(0x7f800000) : x <= -87.0f ? 0.0f : x == x ? y : x;
 }
 

@@ -242,6 +242,7 @@ __global__ void __launch_bounds__(kScreenThreads, Screen<TOKENS, RISK>::kPerSm)
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
+  __syncwarp();  // the warp's elected thread uses them before the CTA meets
   grid_dependency_wait();  // the digits and the passes are complete
   if (pairs && blockIdx.y == gridDim.y - 1) {
     clear_dead(L, ws, padding, pairs, c0, c0 + channels);
