@@ -2335,8 +2335,8 @@ static int run_score(const Bound& b) {
   return launched();
 }
 
-// Batch size from which the native rows are read in expert order (the groups come from route and
-// adopt).
+// Batch size from which the down rows are read in expert order (the groups come from route and
+// adopt); the gate and up rows see gathers_by_pair.
 constexpr int kGroupedTokens = 8;
 static bool pairs_grouped(const Bound& b) { return b.T >= kGroupedTokens; }
 
