@@ -1492,7 +1492,7 @@ __device__ __forceinline__ void encode_rows(const __nv_bfloat16* rows, const Pai
 
 __device__ __forceinline__ void encode_group(const Layer& L, const Workspace& ws, const uint8_t* padding, int index,
                                              int subs, int group_ctas, int tokens, uint8_t* shared) {
-  const int tid = threadIdx.x, lane = tid & 31, R = L.R, I = L.I, tiles = ws.encoder_tiles;
+  const int tid = threadIdx.x, R = L.R, I = L.I, tiles = ws.encoder_tiles;
   if (index >= group_ctas) {
     const int t = (index - group_ctas) * kEncodeThreads + tid;
     bool live = t >= tokens;

@@ -419,7 +419,7 @@ __global__ void __launch_bounds__(kScreenThreads, Screen<TOKENS, RISK>::kPerSm)
     asm volatile("bar.sync 1, 128;" ::: "memory");
     if (warp < busy_warps) {
       const uint32_t lanes = static_cast<uint32_t>(warp * 32) << 16;
-      float run[2][TOKENS], scale[2];
+      float run[2][TOKENS], scale[2] = {0.0f, 0.0f};
       int leader;  // of the warp
       asm volatile("{\n\t.reg .pred p;\n\tsetp.eq.s32 p, %1, 0;\n\tselp.s32 %0, 1, 0, p;\n\t}" : "=r"(leader) : "r"(lane));
 #pragma unroll
