@@ -48,18 +48,30 @@ __device__ __forceinline__ float pinned_exp(float x) {
   return x >= 88.0f ? __int_as_float(0x7f800000) : x <= -87.0f ? 0.0f : x == x ? y : x;
 }
 
-// x / d, correctly rounded, for d in [1, inf] and x / d not below 2^-120: Markstein's division
-// (IBM J. Res. Dev. 34, 1990) from the approximate reciprocal, one step on the reciprocal and one on
-// the quotient.  Without branches, so that the five nodes of a risk score and several candidates go
-// on at a time.  Large divisors are scaled for the reciprocal's sake.
+// x / d, correctly rounded, from a value y within one unit in the last place of 1 / d: Markstein's
+// division (IBM J. Res. Dev. 34, 1990), one step on the reciprocal and one on the quotient.  The step
+// rounds the reciprocal correctly or leaves a quotient that the second one does, except where the
+// significand of d is all ones: there 1 / d lies just above the middle of two values and the step ends
+// on the lower one.  The upper one is (1/2 + 2^-24) 2^-k for d = (2 - 2^-23) 2^k.
+// (Checked for every significand of d with both neighbours of 1 / d, and where the reciprocal does not
+// round correctly, for every significand of x.)
+__device__ __forceinline__ float divide_by_reciprocal(float x, float d, float y) {
+  y = __fmaf_rn(__fmaf_rn(-d, y, 1.0f), y, y);
+  const uint32_t bits = __float_as_uint(d);
+  y = (~bits & 0x7fffffu) == 0 ? __uint_as_float(0x7f000000u - bits) : y;
+  const float q = __fmul_rn(x, y);
+  return __fmaf_rn(__fmaf_rn(-d, q, x), y, q);
+}
+
+// x / d, correctly rounded, for d in [1, inf] and x / d not below 2^-120.  Without branches, so that the
+// five nodes of a risk score and several candidates go on at a time.  Large divisors are scaled for the
+// reciprocal's sake.
 __device__ __forceinline__ float divide_from_one(float x, float d) {
   const float scale = d > 1.8446744e19f ? 2.3283064e-10f : 1.0f;  // 2^64, 2^-32
   const float a = __fmul_rn(x, scale), b = __fmul_rn(d, scale);
   float y;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(b));
-  y = __fmaf_rn(__fmaf_rn(-b, y, 1.0f), y, y);
-  const float q = __fmul_rn(a, y);
-  return __fmaf_rn(__fmaf_rn(-b, q, a), y, q);
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(b));  // within one unit in the last place
+  return divide_by_reciprocal(a, b, y);
 }
 
 // SiLU: x / (1 + exp(-x)).  The divisor is 1 from 87 on, 2 about zero, and infinite from -88 down.

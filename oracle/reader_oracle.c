@@ -155,6 +155,11 @@ static float activate(float x, int activation) {
   return x / (1.0f + pinned_exp(-x)); /* SiLU */
 }
 
+/* The activation of `n` values on its own. */
+void oracle_activate(const float* x, float* out, int64_t n, int activation) {
+  for (int64_t i = 0; i < n; ++i) out[i] = activate(x[i], activation);
+}
+
 /* Recovery-aware score (reference tests/test_progressive_reader.py:146-182,
  * progressive.py:1304-1353): five-node Gauss-Hermite expectation over the gate. */
 static float risk_score(float g, float u, float vg, float vu, float norm, float alpha, float beta,
