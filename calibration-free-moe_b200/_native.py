@@ -19,6 +19,7 @@ HEADERS = [PACKAGE / "csrc" / "cfm_device.cuh", PACKAGE / "csrc" / "cfm_union.cu
            PACKAGE / "csrc" / "cfm_exchange.cuh", PACKAGE / "csrc" / "cfm_select.cuh",
            PACKAGE / "csrc" / "cfm_build.cuh", PACKAGE / "csrc" / "cfm_screen.cuh",
            PACKAGE / "csrc" / "cfm_screen_tc.cuh", PACKAGE / "csrc" / "cfm_prepare.cuh",
+           PACKAGE / "csrc" / "cfm_rules.cuh",
            PACKAGE.parent / "include" / "cfm_b200.h"]
 LIBRARY = PACKAGE / "libcfm_b200.so"
 ABI_VERSION = 12
