@@ -2188,14 +2188,22 @@ static int launch_persistent(void (*kernel)(Params...), int64_t work, int per_sm
   return launched();
 }
 
+// Rows of CTAs that clear dead pairs, eight pairs per CTA: with one row, six CTAs of the 128-expert layer walked
+// all pairs of the call, and that was most of the screen on a rank of eight (256 tokens: 409 us, 28 now; 32 tokens 54 and 17).
+static int dead_rows(int pairs, int columns) {
+  return pairs ? std::min(std::max((pairs + 8 * columns - 1) / (8 * columns), 1), 64) : 0;
+}
+
+// `rows`: most passes of the call; `dead`: its pairs, where some may be dead.
 template <int TOKENS, bool RISK>
 static int launch_screen_tc(const Bound& b, int rows, int dead) {
   const size_t smem = Screen<TOKENS, RISK>::shared_bytes(b.L.B);
   const cudaError_t err = cudaFuncSetAttribute(
       k_screen_tc<TOKENS, RISK>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
   if (err != cudaSuccess) return static_cast<int>(err);
-  launch_dependent(k_screen_tc<TOKENS, RISK>, dim3((b.L.I + kScreenChannels - 1) / kScreenChannels, rows),
-                   dim3(kScreenThreads), smem, b.stream, b.L, b.ws, b.padding, dead);
+  const int columns = (b.L.I + kScreenChannels - 1) / kScreenChannels, clearing = dead_rows(dead, columns);
+  launch_dependent(k_screen_tc<TOKENS, RISK>, dim3(columns, rows + clearing), dim3(kScreenThreads), smem, b.stream,
+                   b.L, b.ws, b.padding, dead, clearing);
   return launched();
 }
 
@@ -2208,9 +2216,9 @@ static int launch_screen_tiles(const Bound& b, int rows, int dead) {
         k_screen_tiles<W>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
     if (err != cudaSuccess) return static_cast<int>(err);
   }
-  const int channels = 16 * S::kTiles;
-  launch_dependent(k_screen_tiles<W>, dim3((b.L.I + channels - 1) / channels, rows),
-                   dim3(S::kThreads), smem, b.stream, b.L, b.ws, b.padding, dead);
+  const int channels = 16 * S::kTiles, columns = (b.L.I + channels - 1) / channels, clearing = dead_rows(dead, columns);
+  launch_dependent(k_screen_tiles<W>, dim3(columns, rows + clearing), dim3(S::kThreads), smem, b.stream, b.L, b.ws,
+                   b.padding, dead, clearing);
   return launched();
 }
 
@@ -2218,8 +2226,7 @@ static int run_screen_grouped(const Bound& b) {
   const int64_t pairs = static_cast<int64_t>(b.T) * b.L.K;
   const int dead = b.padding || b.L.expert_map ? static_cast<int>(pairs) : 0;
   const int pass = pass_pairs(b);
-  // Passes, at most; one more row of CTAs clears the dead pairs.
-  const int rows = static_cast<int>(pairs / pass) + busy_experts(b) + (dead > 0);
+  const int rows = static_cast<int>(pairs / pass) + busy_experts(b);  // passes, at most
   if (screens_tc(b)) {
     const bool risk = b.L.score == CFM_SCORE_RECOVERY_AWARE;
     switch (pass) {

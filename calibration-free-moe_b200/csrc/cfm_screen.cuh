@@ -93,14 +93,18 @@ __device__ __forceinline__ void store_candidate(const Layer& L, const Workspace&
   finish_candidate(L, ws, pair, c, candidate_factors(L, e, c), gate, up, variance.x, variance.y);
 }
 
-// Zeroes the projections of channels c0 .. c1 - 1 for every remote or padded pair of the call.
-__device__ __forceinline__ void clear_dead(const Layer& L, const Workspace& ws,
-                                           const uint8_t* padding, int pairs, int c0, int c1) {
-  for (int p = threadIdx.x; p < pairs; p += blockDim.x) {
+// The last rows of CTAs of a screen, `rows` of them: zero the projections of every remote or padded pair
+// of the call, a pair at a time by all threads of a CTA.
+__device__ __forceinline__ void clear_dead(const Layer& L, const Workspace& ws, const uint8_t* padding, int pairs,
+                                           int rows) {
+  const int row = blockIdx.y - (gridDim.y - rows);
+  for (int p = row * gridDim.x + blockIdx.x; p < pairs; p += rows * gridDim.x) {
     const int t = p / L.K;
     if (ws.ids[p] >= 0 && !(padding && padding[t])) continue;
-    float* gate = ws.partial + static_cast<size_t>(t) * L.N + static_cast<size_t>(p) * L.I;
-    for (int c = c0; c < c1; ++c) gate[c] = gate[L.N + c] = 0.0f;
+    // I is a multiple of 16, and so is the offset of a pair.
+    float4* gate = reinterpret_cast<float4*>(ws.partial + static_cast<size_t>(t) * L.N + static_cast<size_t>(p) * L.I);
+    for (int i = threadIdx.x; i < L.I / 4; i += blockDim.x)
+      gate[i] = gate[L.N / 4 + i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
   }
 }
 
@@ -130,11 +134,11 @@ struct ScreenTiles {
   }
 };
 
-// grid (ceil(I / (16 tiles)), most passes of eight tokens); with `pairs` one more row of CTAs that
-// clears the projections of the call's dead pairs.
+// grid (ceil(I / (16 tiles)), most passes of eight tokens); `dead_rows` more rows of CTAs clear the
+// projections of the dead ones of the call's `pairs`.
 template <int W>
 __global__ void __launch_bounds__(ScreenTiles<W>::kThreads, 16 / ScreenTiles<W>::kWarps)
-    k_screen_tiles(Layer L, Workspace ws, const uint8_t* padding, int pairs) {
+    k_screen_tiles(Layer L, Workspace ws, const uint8_t* padding, int pairs, int dead_rows) {
   using S = ScreenTiles<W>;
   extern __shared__ __align__(128) uint8_t tiles_shared[];
   float* products = reinterpret_cast<float*>(tiles_shared + S::kRingBytes);  // [tile][block][8][lane]
@@ -142,9 +146,8 @@ __global__ void __launch_bounds__(ScreenTiles<W>::kThreads, 16 / ScreenTiles<W>:
   grid_dependency_wait();     // the digits and the passes are complete
   grid_dependency_release();  // the selection may be scheduled; it waits for this grid
   const int I = L.I, B = L.B, rows = 2 * I;
-  if (pairs && blockIdx.y == gridDim.y - 1) {
-    const int c0 = blockIdx.x * 16 * S::kTiles;
-    clear_dead(L, ws, padding, pairs, c0, min(I, c0 + 16 * S::kTiles));
+  if (blockIdx.y + dead_rows >= gridDim.y) {
+    clear_dead(L, ws, padding, pairs, dead_rows);
     return;
   }
   if (static_cast<int>(blockIdx.y) >= ws.work_counts[kPassCount]) return;

@@ -209,11 +209,11 @@ __device__ __forceinline__ void load_wait() {
 
 }  // namespace tc
 
-// grid (ceil(I / 128), most passes of TOKENS tokens), 192 threads; with `pairs` one more row of CTAs
-// that clears the projections of the call's dead pairs.
+// grid (ceil(I / 128), most passes of TOKENS tokens), 192 threads; `dead_rows` more rows of CTAs
+// clear the projections of the dead ones of the call's `pairs`.
 template <int TOKENS, bool RISK>
 __global__ void __launch_bounds__(kScreenThreads, Screen<TOKENS, RISK>::kPerSm)
-    k_screen_tc(Layer L, Workspace ws, const uint8_t* padding, int pairs) {
+    k_screen_tc(Layer L, Workspace ws, const uint8_t* padding, int pairs, int dead_rows) {
   using S = Screen<TOKENS, RISK>;
   using namespace tc;
   extern __shared__ __align__(1024) uint8_t screen_shared[];
@@ -244,8 +244,8 @@ __global__ void __launch_bounds__(kScreenThreads, Screen<TOKENS, RISK>::kPerSm)
   }
   __syncwarp();  // the warp's elected thread uses them before the CTA meets
   grid_dependency_wait();  // the digits and the passes are complete
-  if (pairs && blockIdx.y == gridDim.y - 1) {
-    clear_dead(L, ws, padding, pairs, c0, c0 + channels);
+  if (blockIdx.y + dead_rows >= gridDim.y) {
+    clear_dead(L, ws, padding, pairs, dead_rows);
     return;
   }
   const int4 pass = *reinterpret_cast<const int4*>(ws.pass_work + blockIdx.y);
