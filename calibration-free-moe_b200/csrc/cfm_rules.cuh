@@ -7,17 +7,20 @@
 static int busy_experts(const Bound& b) {
   return static_cast<int>(std::min<int64_t>(b.L.E, static_cast<int64_t>(b.T) * b.L.K));
 }
-// More than 16/3 tokens per expert on average.
-static bool shares_decode(const Bound& b) {
-  return 3 * static_cast<int64_t>(b.T) * b.L.K > 16 * static_cast<int64_t>(b.L.E);
+// Pairs that this device's experts can expect of the call: all, or under expert parallelism their share.
+static int64_t expected_pairs(const Bound& b) {
+  const int64_t pairs = static_cast<int64_t>(b.T) * b.L.K;
+  return b.L.expert_map && b.L.global_experts > 0 ? (pairs * b.L.E + b.L.global_experts - 1) / b.L.global_experts : pairs;
 }
+// More than 16/3 tokens per expert on average.
+static bool shares_decode(const Bound& b) { return 3 * expected_pairs(b) > 16 * static_cast<int64_t>(b.L.E); }
 // The tcgen05 screen on request, where several tokens share its decode, or where its CTAs of 128 channels
 // give most SMs one or the rows are long: three tokens of the 128-expert layer (144 CTAs) 10.0 us against 12.4
 // of the warp-level kernel, two of the 64-expert layer (128) 9.8 against 11.5, one of hidden 4096 and width
 // 1536 (96 CTAs, 32 blocks) 17.1 against 19.4; two of the 128-expert layer (96, 16 blocks) 9.9 against 8.3,
 // four of the 256-expert layer of width 512 (128) 10.5 against 8.4.  Its tables have to fit shared memory.
 static bool screens_tc(const Bound& b) {
-  const int64_t ctas = static_cast<int64_t>(busy_experts(b)) * ((b.L.I + kScreenChannels - 1) / kScreenChannels);
+  const int64_t ctas = std::min<int64_t>(b.L.E, expected_pairs(b)) * ((b.L.I + kScreenChannels - 1) / kScreenChannels);
   return (b.L.tensor_engine == CFM_ENGINE_TCGEN05 || shares_decode(b) || ctas >= 128 || ctas * b.L.B >= 96 * 32) &&
          b.L.B <= 512;
 }
@@ -26,9 +29,11 @@ static bool screens_tc(const Bound& b) {
 // 35.1 against 37.8, 50 of the 64-expert layer (6.3) 43 against 38.  Of sixteen from sixteen tokens per expert
 // on: 256 tokens of hidden 4096 and width 1536 240 us against 269 of eight; 100 of the 64-expert layer (12.5)
 // 50 against 47 (recovery-aware score 78 against 66), for fewer warps fit an SM and fewer passes are full.
+// (One of eight ranks with 64 and 256 tokens of all of the 256-expert layer, two and eight per expert: passes of
+// four 13.9 against 18.1 of sixteen, of eight 24.7 against 27.3.)
 static int pass_pairs(const Bound& b) {
   if (!screens_tc(b)) return 8;
-  const int64_t pairs = static_cast<int64_t>(b.T) * b.L.K, experts = b.L.E;
+  const int64_t pairs = expected_pairs(b), experts = b.L.E;
   return pairs >= 16 * experts ? 16 : pairs <= 4 * experts ? 4 : 8;
 }
 
