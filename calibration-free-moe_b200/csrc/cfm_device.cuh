@@ -63,9 +63,10 @@ __device__ __forceinline__ float divide_by_reciprocal(float x, float d, float y)
   return __fmaf_rn(__fmaf_rn(-d, q, x), y, q);
 }
 
-// x / d, correctly rounded, for d in [1, inf] and x / d not below 2^-120.  Without branches, so that the
-// five nodes of a risk score and several candidates go on at a time.  Large divisors are scaled for the
-// reciprocal's sake.
+// x / d, correctly rounded, for finite d from 1 on, |x| from 2^-60 on and quotients from 2^-126 on, the smallest
+// normal one (SiLU comes down to 88 / e^88, 2^-120.5; GELU to 2 / (1 + e^88), just above 2^-126).  An infinite
+// divisor gives NaN, which the activations replace.  Without branches, so that the five nodes of a risk score and
+// several candidates go on at a time.  Large divisors are scaled for the reciprocal's sake.
 __device__ __forceinline__ float divide_from_one(float x, float d) {
   const float scale = d > 1.8446744e19f ? 2.3283064e-10f : 1.0f;  // 2^64, 2^-32
   const float a = __fmul_rn(x, scale), b = __fmul_rn(d, scale);
@@ -207,13 +208,6 @@ __device__ __forceinline__ uint32_t shared_u32(const void* p) {
 // 16 bytes global -> shared memory, past L1, in the thread's current cp.async group.
 __device__ __forceinline__ void copy_async16(uint32_t shared, const void* global) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(shared), "l"(global) : "memory");
-}
-template <int AT>
-__device__ __forceinline__ void copy_async8_at(uint32_t shared, const void* global) {
-  asm volatile("cp.async.ca.shared.global [%0+%2], [%1], 8;" ::"r"(shared), "l"(global), "n"(AT) : "memory");
-}
-__device__ __forceinline__ void copy_async4(uint32_t shared, const void* global) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(shared), "l"(global) : "memory");
 }
 __device__ __forceinline__ void copy_async_commit() {
   asm volatile("cp.async.commit_group;" ::: "memory");

@@ -49,6 +49,10 @@ __device__ __forceinline__ void copy_async16_at(uint32_t shared, const void* glo
   asm volatile("cp.async.cg.shared.global [%0+%2], [%1], 16;" ::"r"(shared), "l"(global), "n"(AT) : "memory");
 }
 template <int AT>
+__device__ __forceinline__ void copy_async8_at(uint32_t shared, const void* global) {
+  asm volatile("cp.async.ca.shared.global [%0+%2], [%1], 8;" ::"r"(shared), "l"(global), "n"(AT) : "memory");
+}
+template <int AT>
 __device__ __forceinline__ uint2 load_shared8_at(uint32_t address) {
   uint2 v;
   asm volatile("ld.shared.v2.u32 {%0,%1}, [%2+%3];" : "=r"(v.x), "=r"(v.y) : "r"(address), "n"(AT) : "memory");
