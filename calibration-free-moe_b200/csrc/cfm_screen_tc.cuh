@@ -29,8 +29,15 @@
 // Included by cfm_reader.cu inside namespace cfm.
 #pragma once
 
+// How long a wait goes on, in nanoseconds, and how it asks.  (A build for tests has short waits run out.)
+#ifndef CFM_SCREEN_WAIT_NS
+#define CFM_SCREEN_WAIT_NS 1000000000u
+#define CFM_SCREEN_WAIT "try_wait"
+#endif
+
 constexpr int kScreenThreads = 192;
 constexpr int kScreenChannels = 128;
+constexpr uint32_t kScreenDrain = 1000000000u;  // nanoseconds for what is still in flight at the end
 constexpr int kScreenAhead = 4;  // blocks whose variances are on their way together (16: 83 us against 78 for 100
                                  // tokens of the 64-expert layer; the code outgrows its cache)
 
@@ -86,31 +93,36 @@ __device__ __forceinline__ void barrier_init(uint32_t bar, int count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
 }
 
-// Waits for the phase with the given parity.  After four million tries (some half a second), or when
-// another thread has given up, the word at `abort` is set and the wait ends.  Returns whether it has
-// come to that.
-__device__ __forceinline__ int barrier_wait(uint32_t bar, uint32_t parity, uint32_t abort) {
-  int gone;
+// Waits for the phase with the given parity, `limit` nanoseconds at most: then the word at `abort` is set.
+// A thread that gives up, because its time ran out or another thread's has, clears `alive`; a phase that
+// is complete counts all the same.
+__device__ __forceinline__ void barrier_wait(uint32_t bar, uint32_t parity, uint32_t abort, int& alive,
+                                             uint32_t limit = CFM_SCREEN_WAIT_NS) {
   asm volatile(
-      "{\n\t.reg .pred p;\n\t.reg .u32 tries;\n\t"
-      "mov.u32 %0, 0;\n\t"
-      "mov.u32 tries, 0;\n"
+      "{\n\t.reg .pred p;\n\t.reg .u32 start, now;\n\t"
+      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "@p bra done;\n\t"
+      "ld.volatile.shared.u32 now, [%3];\n\t"
+      "setp.ne.u32 p, now, 0;\n\t"
+      "@p bra gone;\n\t"
+      "mov.u32 start, %%globaltimer_lo;\n"
       "again:\n\t"
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "mbarrier." CFM_SCREEN_WAIT ".parity.shared::cta.b64 p, [%1], %2;\n\t"
       "@p bra done;\n\t"
-      "ld.volatile.shared.u32 %0, [%3];\n\t"
-      "setp.ne.u32 p, %0, 0;\n\t"
-      "@p bra done;\n\t"
-      "add.u32 tries, tries, 1;\n\t"
-      "setp.lt.u32 p, tries, 4000000;\n\t"
+      "ld.volatile.shared.u32 now, [%3];\n\t"
+      "setp.ne.u32 p, now, 0;\n\t"
+      "@p bra gone;\n\t"
+      "mov.u32 now, %%globaltimer_lo;\n\t"
+      "sub.u32 now, now, start;\n\t"
+      "setp.lt.u32 p, now, %4;\n\t"
       "@p bra again;\n\t"
-      "mov.u32 %0, 1;\n\t"
       "st.volatile.shared.u32 [%3], 1;\n"
+      "gone:\n\t"
+      "mov.u32 %0, 0;\n"
       "done:\n\t}"
-      : "=&r"(gone)
-      : "r"(bar), "r"(parity), "r"(abort)
+      : "+r"(alive)
+      : "r"(bar), "r"(parity), "r"(abort), "r"(limit)
       : "memory");
-  return gone;
 }
 
 // One lane of the warp, known to the compiler as one (instructions of a single thread then need no
@@ -222,7 +234,7 @@ __global__ void __launch_bounds__(kScreenThreads, Screen<TOKENS, RISK>::kPerSm)
   __shared__ int abort_flag, late_flag, s_pair[TOKENS], s_token[TOKENS];
   const int tid = threadIdx.x, lane = tid & 31;
   const int warp = __shfl_sync(kFull, tid >> 5, 0);  // known to be the same in all lanes
-  const uint32_t abort = shared_u32(&abort_flag);
+  const uint32_t abort = shared_u32(&abort_flag), late = shared_u32(&late_flag);
   const int I = L.I, B = L.B, rows = 2 * I, c0 = blockIdx.x * kScreenChannels;
   const int channels = min(kScreenChannels, I - c0);
   const int busy_warps = (channels + 31) / 32;  // that hold channels
@@ -338,17 +350,21 @@ __global__ void __launch_bounds__(kScreenThreads, Screen<TOKENS, RISK>::kPerSm)
     }
     int place = 0, refill = S::kDigitRing - 1, turn = 0;
     uint32_t second = static_cast<uint32_t>(second_base);
+    int alive = 1, issued = 0;
     for (int b = 0; b < B; ++b) {
       copy_async_wait<S::kDigitRing - 2>();
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       __syncwarp();  // the block's digits have landed, for all lanes
       barrier_arrive(digits_landed + 8 * place, lane == 0);
-      if (__any_sync(kFull, barrier_wait(ready, b & 1, abort))) break;
+      barrier_wait(ready, b & 1, abort, alive);
+      if (!__all_sync(kFull, alive)) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       if (elect_lane()) issue(gate, second);
       __syncwarp();
+      ++issued;
       if (b + S::kDigitRing - 1 < B) {  // into the place of the block before this one
-        if (b && __any_sync(kFull, barrier_wait(digits_free + 8 * refill, turn, abort))) break;
+        if (b) barrier_wait(digits_free + 8 * refill, turn, abort, alive);
+        if (!__all_sync(kFull, alive)) break;
         fetch(refill);
       }
       copy_async_commit();
@@ -357,18 +373,22 @@ __global__ void __launch_bounds__(kScreenThreads, Screen<TOKENS, RISK>::kPerSm)
       refill = refill + 1 == S::kDigitRing ? 0 : refill + 1;
       if (refill == 0 && b) turn ^= 1;
     }
+    // Nothing of the driver's may outlive the CTA, whatever became of its waits: the copies, the last product.
     copy_async_wait<0>();
+    if (issued) barrier_wait(done, (issued - 1) & 1, late, alive, kScreenDrain);
   } else if (warp == 5) {
     // ---- codes and scales, and the products of the up tile ----
     if (elect_lane()) {
-      int gone = 0;
+      int alive = 1, issued = 0;
       uint32_t place = codes, bar = landed, free = digits_free + 8 * (S::kDigitRing - 1), turn = 0;
       uint32_t second = static_cast<uint32_t>(second_base), digit_bar = digits_landed;
       for (int b = 0; b < B; ++b) {
-        gone |= barrier_wait(digit_bar, turn, abort) | barrier_wait(ready + 8, b & 1, abort);
-        if (gone) break;
+        barrier_wait(digit_bar, turn, abort, alive);
+        barrier_wait(ready + 8, b & 1, abort, alive);
+        if (!alive) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         issue(up, second);
+        ++issued;
         // The rows of this block came after the products of the one before, whose digits may go.
         if (b) barrier_arrive(free, 1);
         if (fetched < B) {  // the block's codes have been read
@@ -390,9 +410,10 @@ __global__ void __launch_bounds__(kScreenThreads, Screen<TOKENS, RISK>::kPerSm)
           turn ^= 1;
         }
       }
-      if (gone)  // codes may be on their way still: each place's last block, for a limited time
-        for (int p = 0; p < min(fetched, S::kCodeRing); ++p)
-          barrier_wait(landed + 8 * p, ((fetched - p - 1) / S::kCodeRing) & 1, shared_u32(&late_flag));
+      // As above: the last product, and each place's last codes.
+      if (issued) barrier_wait(done + 8, (issued - 1) & 1, late, alive, kScreenDrain);
+      for (int p = 0; p < min(fetched, S::kCodeRing); ++p)
+        barrier_wait(landed + 8 * p, ((fetched - p - 1) / S::kCodeRing) & 1, late, alive, kScreenDrain);
     }
     __syncwarp();
   } else {
@@ -420,8 +441,13 @@ __global__ void __launch_bounds__(kScreenThreads, Screen<TOKENS, RISK>::kPerSm)
     if (warp < busy_warps) {
       const uint32_t lanes = static_cast<uint32_t>(warp * 32) << 16;
       float run[2][TOKENS], scale[2] = {0.0f, 0.0f};
-      int leader;  // of the warp
-      asm volatile("{\n\t.reg .pred p;\n\tsetp.eq.s32 p, %1, 0;\n\tselp.s32 %0, 1, 0, p;\n\t}" : "=r"(leader) : "r"(lane));
+      // kLeads in the warp's leader, kFollows in its other threads, 0 once a wait has run out.  A leader that
+      // has given up arrives no more, so a product is issued only while every warp's waits have ended in
+      // time, and a thread that saw the last product's end knows that all copies have landed.
+      constexpr int kFollows = 1, kLeads = 2;
+      int state;
+      asm volatile("{\n\t.reg .pred p;\n\tsetp.eq.s32 p, %1, 0;\n\tselp.s32 %0, %2, %3, p;\n\t}"
+                   : "=r"(state) : "r"(lane), "n"(kLeads), "n"(kFollows));
 #pragma unroll
       for (int t = 0; t < TOKENS; ++t) run[0][t] = run[1][t] = 0.0f;
       // The sums of eight tokens of the tile's product before the next one; load_wait() completes them.
@@ -458,7 +484,8 @@ __global__ void __launch_bounds__(kScreenThreads, Screen<TOKENS, RISK>::kPerSm)
         constexpr bool kFirst = decltype(begin)::value;  // block 0
         int c[24];
         if constexpr (!kFirst) {
-          barrier_wait(done + 8 * tile, (b - 1) & 1, abort);
+          barrier_wait(done + 8 * tile, (b - 1) & 1, abort, state);
+          if (!__any_sync(kFull, state)) return;  // the product may read the rows still
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
           load_sums(tile, 0, c);
         }
@@ -492,12 +519,13 @@ __global__ void __launch_bounds__(kScreenThreads, Screen<TOKENS, RISK>::kPerSm)
         asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
         __syncwarp();
-        barrier_arrive(ready + 8 * tile, leader);  // the rows are in place, the sums read
+        barrier_arrive(ready + 8 * tile, state == kLeads);  // the rows are in place, the sums read
       };
       auto finish = [&](auto which) {  // the last block's product
         constexpr int tile = decltype(which)::value;
         int c[24];
-        barrier_wait(done + 8 * tile, (B - 1) & 1, abort);
+        barrier_wait(done + 8 * tile, (B - 1) & 1, abort, state);
+        if (!__any_sync(kFull, state)) return;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
         for (int half = 0; half < (TOKENS + 7) / 8; ++half) {
@@ -507,13 +535,13 @@ __global__ void __launch_bounds__(kScreenThreads, Screen<TOKENS, RISK>::kPerSm)
           rescale(which, half, B - 1, c);
         }
       };
-      barrier_wait(landed, 0, abort);
+      barrier_wait(landed, 0, abort, state);
       step(gate, std::true_type{}, 0, codes);
       step(up, std::true_type{}, 0, codes);
       uint32_t place = codes + S::kCodeBytes, bar = landed + 8, parity = 0;
 #pragma unroll 1
       for (int b = 1; b < B; ++b) {
-        barrier_wait(bar, parity, abort);
+        barrier_wait(bar, parity, abort, state);
         step(gate, std::false_type{}, b, place);
         step(up, std::false_type{}, b, place);
         place += S::kCodeBytes;
@@ -529,15 +557,16 @@ __global__ void __launch_bounds__(kScreenThreads, Screen<TOKENS, RISK>::kPerSm)
       grid_dependency_release();  // the selection may be scheduled; it waits for this grid
 
       // Projections out, scores and features of the pass's tokens in turn: the sums go through shared
-      // memory, so that the code is there once.  The ring has been read by every warp.
-      float* mine = reinterpret_cast<float*>(screen_shared) + tid;
-#pragma unroll
-      for (int t = 0; t < TOKENS; ++t) {
-        mine[t * S::kStride] = run[0][t];
-        mine[t * S::kStride + kScreenChannels] = run[1][t];
-      }
+      // memory, so that the code is there once.  The ring has been read by every warp.  A channel whose sums
+      // did not come in time leaves nothing.
       const int channel = c0 + tid;
-      if (tid < channels) {
+      if (tid < channels && state) {
+        float* mine = reinterpret_cast<float*>(screen_shared) + tid;
+#pragma unroll
+        for (int t = 0; t < TOKENS; ++t) {
+          mine[t * S::kStride] = run[0][t];
+          mine[t * S::kStride + kScreenChannels] = run[1][t];
+        }
         if (RISK) {
           // Residual variances: per block, in block order, the row's times the energy of the token's
           // kept coordinates.
@@ -604,7 +633,7 @@ __global__ void __launch_bounds__(kScreenThreads, Screen<TOKENS, RISK>::kPerSm)
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   if (warp == 4) {
-    if (abort_flag && lane == 0) atomicExch(&ws.status[0], 1);
+    if ((abort_flag || late_flag) && lane == 0) atomicExch(&ws.status[0], 1);
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_holder[0]), "n"(S::kLarge)
                  : "memory");

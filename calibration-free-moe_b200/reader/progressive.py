@@ -639,10 +639,10 @@ class ProgressiveReader:
     def check_status(self) -> None:
         """Raise if a kernel of this reader's workspace reported a device-side error.
 
-        The tensor-memory screen (`tensor_engine="tcgen05"`) bounds every barrier wait;
-        a wait that runs out sets a flag in the workspace and leaves the projections
-        of that call unwritten, so the kept channels of that call are not to be
-        trusted.  Reading the flag synchronises with the device: call this at points
+        The tensor-memory screen (taken by size, or with `tensor_engine="tcgen05"`)
+        bounds every wait: after a second it sets a flag in the workspace.
+        Projections whose sums had not come by then are left as they were, so the
+        kept channels of that call are not to be trusted.  Reading the flag synchronises with the device: call this at points
         where the host waits anyway (after a decode step, before reading a report).
         """
         status = self.workspace.status.cpu().tolist()

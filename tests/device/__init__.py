@@ -1,4 +1,4 @@
-"""Builds and loads checks.cu and rules.cpp: parts of the library, called on chosen values."""
+"""Builds and loads checks.cu, rules.cpp and impatient.cu: parts of the library, called on chosen values."""
 
 import ctypes
 import subprocess
@@ -16,7 +16,7 @@ def _load(source: str, *compiler: str) -> ctypes.CDLL:
     """The source as a library, compiled again where it or a header is newer."""
     path = HERE / source
     library = path.with_name(f"lib{path.stem}.so")
-    newest = max(p.stat().st_mtime for p in [path, *_native.HEADERS])
+    newest = max(p.stat().st_mtime for p in [path, *_native.HEADERS, *_native.SOURCES])
     if not library.exists() or library.stat().st_mtime < newest:
         subprocess.run([*compiler, *INCLUDES, "-o", str(library), str(path)], check=True, capture_output=True)
     return ctypes.CDLL(str(library))
@@ -29,6 +29,13 @@ def call(name: str, *arguments) -> None:
         ctypes.c_void_p(a.data_ptr()) if hasattr(a, "data_ptr") else ctypes.c_int(a)
         for a in arguments))
     assert code == 0, f"{name}: CUDA error {code}"
+
+
+def impatient_screen():
+    """`cfm_screen` of a library whose waits run out within microseconds."""
+    function = _load("impatient.cu", _native.nvcc(), *_native.NVCC_FLAGS).cfm_screen
+    function.restype, function.argtypes = _native.load().cfm_screen.restype, _native.load().cfm_screen.argtypes
+    return function
 
 
 def dispatch(tokens: int, **sizes: int) -> dict[str, int]:
