@@ -4,6 +4,7 @@ import pytest
 import torch
 
 import cases
+from device import dispatch
 from cfm_b200.reader.sketch import (
     block_hadamard_signs, build_sketch, build_sketch_on_device, repack_sketch,
     repack_sketch_grouped,
@@ -189,10 +190,29 @@ def test_selection_by_bins(kind, width):
 def test_encoder_rows_shared_by_an_experts_pairs(rank, width, tokens):
     """Large calls sum the encoder for several pairs of an expert at a time; the stage on its own takes a
     pair at a time.  The same latents, with padding and with passes that are not full."""
-    hidden, experts, top_k = 4096, 6, 5
+    _shared_encoder(rank, width, tokens, experts=6, top_k=5, passes=16)
+
+
+@pytest.mark.parametrize("rank,width,tokens,experts,passes", [
+    (64, 176, 48, 60, 4),   # four pairs per expert: the rule's edge, one part per pass
+    (16, 272, 33, 20, 8),
+    (128, 176, 50, 16, 8),  # just below sixteen
+])
+def test_encoder_rows_shared_by_fewer_pairs(rank, width, tokens, experts, passes):
+    """The same in passes of four and eight pairs, with some experts' load far above the others'."""
+    generator = torch.Generator().manual_seed(experts)
+    load = 1.0 / (3.0 + torch.arange(experts))
+    routes = torch.multinomial(load.expand(tokens, -1), 5, generator=generator).tolist()
+    _shared_encoder(rank, width, tokens, experts=experts, top_k=5, passes=passes, routes=routes)
+
+
+def _shared_encoder(rank, width, tokens, experts, top_k, passes, routes=None):
+    hidden = 4096
     case = cases._random("shared", rank, hidden, width, experts, top_k, rank, tokens, 0.7, 0.625,
-                         padding=[t % 7 == 3 for t in range(tokens)])
-    assert 2 * tokens * case.plan.final_count * hidden >= 240_000_000
+                         routes=routes, padding=[t % 7 == 3 for t in range(tokens)])
+    took = dispatch(tokens, hidden=hidden, width=width, experts=experts, top_k=top_k, rank=rank,
+                    final_count=case.plan.final_count)
+    assert took["shares_encoder"] and took["pass_pairs"] == passes
     reader = make_reader(prepared_case(case))
     run_reader(reader, case)
     device = reader.latent.device
