@@ -2235,11 +2235,9 @@ static int run_screen_grouped(const Bound& b) {
       default: return risk ? launch_screen_tc<16, true>(b, rows, dead) : launch_screen_tc<16, false>(b, rows, dead);
     }
   }
-  // Four warps per tile while one each would not give every SM its sixteen (one token of the
-  // 128-expert layer: 6.9 us against 12.3; 8 tokens 24.5 against 23.4).  The products of a tile
-  // have to fit shared memory.
-  const int64_t tiles = static_cast<int64_t>(busy_experts(b)) * (b.L.I / 16);
-  if (tiles < 148 * 16 && b.L.B <= 128) return launch_screen_tiles<4>(b, rows, dead);
+  // Four warps per tile: the calls that come here would not give every SM its sixteen with one each (one token
+  // of the 128-expert layer 6.9 us against 12.3).  The products of a tile have to fit shared memory.
+  if (b.L.B <= 128) return launch_screen_tiles<4>(b, rows, dead);
   return launch_screen_tiles<1>(b, rows, dead);
 }
 

@@ -21,6 +21,7 @@ static bool shares_decode(const Bound& b) { return 3 * expected_pairs(b) > 16 * 
 // four of the 256-expert layer of width 512 (128) 10.5 against 8.4.  Its tables have to fit shared memory.
 static bool screens_tc(const Bound& b) {
   const int64_t ctas = std::min<int64_t>(b.L.E, expected_pairs(b)) * ((b.L.I + kScreenChannels - 1) / kScreenChannels);
+  if (b.L.tensor_engine == CFM_ENGINE_WARP) return false;
   return (b.L.tensor_engine == CFM_ENGINE_TCGEN05 || shares_decode(b) || ctas >= 128 || ctas * b.L.B >= 96 * 32) &&
          b.L.B <= 512;
 }

@@ -42,8 +42,9 @@ extern "C" {
 #define CFM_ACT_GELU_TANH 1
 #define CFM_SCORE_POINT 0
 #define CFM_SCORE_RECOVERY_AWARE 1
-#define CFM_ENGINE_MMA_SYNC 0 /* warp-level mma.sync.m16n8k32 (default: measured faster) */
-#define CFM_ENGINE_TCGEN05 1  /* tcgen05.mma kind::i8, accumulators in tensor memory     */
+#define CFM_ENGINE_MMA_SYNC 0 /* default: warp-level mma.sync.m16n8k32 in calls too small for the next */
+#define CFM_ENGINE_TCGEN05 1  /* tcgen05.mma kind::i8, accumulators in tensor memory, in every call    */
+#define CFM_ENGINE_WARP 2     /* the warp-level one in every call, to compare the two (same bits)      */
 #define CFM_ROWS_AUTO 0        /* the library's choice; a token's output bits do not depend on it
                                   or on the batch                                         */
 #define CFM_ROWS_PER_TOKEN 1   /* native rows always gathered per token                 */

@@ -117,6 +117,32 @@ def test_tcgen05_screen_at_the_edges_of_its_tiles(oracle, hidden, width, tokens,
     assert torch.equal(reader.scores[0][:tokens].cpu(), want["scores"])
 
 
+# 129 blocks: the products of a tile no longer fit shared memory, and a warp has a tile to itself.
+@pytest.mark.parametrize("score", ["point", "recovery-aware"])
+@pytest.mark.parametrize("hidden,width,experts,top_k,tokens", [
+    (4096, 1536, 8, 8, 1), (4096, 1536, 8, 4, 9), (2048, 512, 32, 8, 4), (16384, 48, 3, 2, 5),
+    (16512, 16, 3, 2, 1), (16512, 80, 4, 3, 11),
+])
+def test_the_two_expert_major_screens_agree(oracle, hidden, width, experts, top_k, tokens, score):
+    """Warp-level and tcgen05 screen at sizes where a call by itself takes one of them only."""
+    case = cases._random("screens", hidden + tokens, hidden, width, experts, top_k, 8, tokens, 0.25, 0.625,
+                         score=score)
+    item = prepared_case(case)
+    want = None
+    for engine in (1, 2):  # CFM_ENGINE_TCGEN05, CFM_ENGINE_WARP
+        reader = make_reader(item, capacity=tokens)
+        reader._layer.tensor_engine = engine
+        run_reader(reader, case)
+        reader.check_status()
+        if want is None:
+            own = dict(norms=reader.norms.cpu())
+            if reader.recovery_geometry is not None:
+                own["geometry"] = reader.recovery_geometry.cpu()
+            want = run_oracle(oracle, item, **own)
+        assert torch.equal(reader.partial[:tokens].cpu(), want["partial"])
+        assert torch.equal(reader.scores[0][:tokens].cpu(), want["scores"])
+
+
 def test_expert_major_stages_repeat_and_misaligned_output():
     """The stages on their own, twice, and an output that 16-byte stores cannot take."""
     case = cases._random("stages", 5, 1280, 48, 60, 3, 16, 112, 0.25, 0.625)
