@@ -18,8 +18,9 @@
 // So no thread waits for a product's latency (450 cycles alone, 1000 beside three other CTAs; a thread
 // needs 54 cycles for each of its four instructions, whatever N up to 64), and the four warps never
 // wait for one another.
-// Bound by instruction issue, some 150 per warp and tile with four tokens, 56 of them the decode's (0.8
-// of the issue slots while four CTAs share an SM), and by the last CTAs of a launch, alone on their SM.
+// Bound by instruction issue and the latency between instructions: some 160 per warp and tile with four
+// tokens, 56 of them the decode's, issued at 0.64 per scheduler and active cycle with five CTAs per SM (0.56
+// with four and passes of eight); and by the last CTAs of a launch, alone on their SM.
 // 64 tokens of the 128-expert layer (100 MB of codes: 15 us of HBM) 35 us, 32 tokens 24.5, 8 tokens
 // 15, 256 tokens of hidden 4096 and width 1536 240, against 56, 44, 27 and 404 of 64 channels per CTA
 // whose threads copied, waited for their product and met at a barrier once per block.  Persistent CTAs
