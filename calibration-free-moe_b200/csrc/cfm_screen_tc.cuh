@@ -30,15 +30,16 @@
 // Included by cfm_reader.cu inside namespace cfm.
 #pragma once
 
-// How long a wait goes on, in nanoseconds, and how it asks.  (A build for tests has short waits run out.)
+// How long a wait goes on, how long, once one has run out, those for what is still in flight do, in
+// nanoseconds, and how they ask.  (A build for tests has short waits run out.)
 #ifndef CFM_SCREEN_WAIT_NS
 #define CFM_SCREEN_WAIT_NS 1000000000u
+#define CFM_SCREEN_DRAIN_NS 1000000000u
 #define CFM_SCREEN_WAIT "try_wait"
 #endif
 
 constexpr int kScreenThreads = 192;
 constexpr int kScreenChannels = 128;
-constexpr uint32_t kScreenDrain = 1000000000u;  // nanoseconds for what is still in flight at the end
 constexpr int kScreenAhead = 4;  // blocks whose variances are on their way together (16: 83 us against 78 for 100
                                  // tokens of the 64-expert layer; the code outgrows its cache)
 
@@ -96,23 +97,20 @@ __device__ __forceinline__ void barrier_init(uint32_t bar, int count) {
 
 // Waits for the phase with the given parity, `limit` nanoseconds at most: then the word at `abort` is set.
 // A thread that gives up, because its time ran out or another thread's has, clears `alive`; a phase that
-// is complete counts all the same.
+// is complete counts all the same.  (One try suspends for up to 4 us.)
 __device__ __forceinline__ void barrier_wait(uint32_t bar, uint32_t parity, uint32_t abort, int& alive,
                                              uint32_t limit = CFM_SCREEN_WAIT_NS) {
   asm volatile(
       "{\n\t.reg .pred p;\n\t.reg .u32 start, now;\n\t"
-      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-      "@p bra done;\n\t"
-      "ld.volatile.shared.u32 now, [%3];\n\t"
-      "setp.ne.u32 p, now, 0;\n\t"
-      "@p bra gone;\n\t"
-      "mov.u32 start, %%globaltimer_lo;\n"
-      "again:\n\t"
       "mbarrier." CFM_SCREEN_WAIT ".parity.shared::cta.b64 p, [%1], %2;\n\t"
       "@p bra done;\n\t"
+      "mov.u32 start, %%globaltimer_lo;\n"
+      "again:\n\t"
       "ld.volatile.shared.u32 now, [%3];\n\t"
       "setp.ne.u32 p, now, 0;\n\t"
       "@p bra gone;\n\t"
+      "mbarrier." CFM_SCREEN_WAIT ".parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "@p bra done;\n\t"
       "mov.u32 now, %%globaltimer_lo;\n\t"
       "sub.u32 now, now, start;\n\t"
       "setp.lt.u32 p, now, %4;\n\t"
@@ -123,6 +121,48 @@ __device__ __forceinline__ void barrier_wait(uint32_t bar, uint32_t parity, uint
       "done:\n\t}"
       : "+r"(alive)
       : "r"(bar), "r"(parity), "r"(abort), "r"(limit)
+      : "memory");
+}
+
+// The same for the end of a product, whose rows and sums the thread is about to touch: having given up it
+// goes on waiting, until the word at `late` is set or, after CFM_SCREEN_DRAIN_NS, sets that.  (By then no driver
+// issues a product any more.  A vote of the warp before it goes on, instead, cost 2 us of 55.)
+__device__ __forceinline__ void barrier_wait_product(uint32_t bar, uint32_t parity, uint32_t abort, uint32_t late,
+                                                     int& alive) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t.reg .u32 start, now;\n\t"
+      "mbarrier." CFM_SCREEN_WAIT ".parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "@p bra done;\n\t"
+      "mov.u32 start, %%globaltimer_lo;\n"
+      "again:\n\t"
+      "ld.volatile.shared.u32 now, [%3];\n\t"
+      "setp.ne.u32 p, now, 0;\n\t"
+      "@p bra gone;\n\t"
+      "mbarrier." CFM_SCREEN_WAIT ".parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "@p bra done;\n\t"
+      "mov.u32 now, %%globaltimer_lo;\n\t"
+      "sub.u32 now, now, start;\n\t"
+      "setp.lt.u32 p, now, %5;\n\t"
+      "@p bra again;\n\t"
+      "st.volatile.shared.u32 [%3], 1;\n"
+      "gone:\n\t"
+      "mov.u32 %0, 0;\n\t"
+      "mov.u32 start, %%globaltimer_lo;\n"
+      "drain:\n\t"
+      "mbarrier." CFM_SCREEN_WAIT ".parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "@p bra done;\n\t"
+      "ld.volatile.shared.u32 now, [%4];\n\t"
+      "setp.ne.u32 p, now, 0;\n\t"
+      "@p bra done;\n\t"
+      "mov.u32 now, %%globaltimer_lo;\n\t"
+      "sub.u32 now, now, start;\n\t"
+      "setp.lt.u32 p, now, %6;\n\t"
+      "@p bra drain;\n\t"
+      "st.volatile.shared.u32 [%4], 1;\n"
+      "done:\n\t}"
+      : "+r"(alive)
+      : "r"(bar), "r"(parity), "r"(abort), "r"(late), "r"(static_cast<uint32_t>(CFM_SCREEN_WAIT_NS)),
+        "r"(CFM_SCREEN_DRAIN_NS)
       : "memory");
 }
 
@@ -232,7 +272,7 @@ __global__ void __launch_bounds__(kScreenThreads, Screen<TOKENS, RISK>::kPerSm)
   extern __shared__ __align__(1024) uint8_t screen_shared[];
   __shared__ uint64_t barriers[S::kCodeRing + 4 + 2 * S::kDigitRing];
   __shared__ uint32_t tmem_holder[2];
-  __shared__ int abort_flag, late_flag, s_pair[TOKENS], s_token[TOKENS];
+  __shared__ int abort_flag, late_flag, s_issued[2], s_fetched, s_pair[TOKENS], s_token[TOKENS];
   const int tid = threadIdx.x, lane = tid & 31;
   const int warp = __shfl_sync(kFull, tid >> 5, 0);  // known to be the same in all lanes
   const uint32_t abort = shared_u32(&abort_flag), late = shared_u32(&late_flag);
@@ -374,9 +414,8 @@ __global__ void __launch_bounds__(kScreenThreads, Screen<TOKENS, RISK>::kPerSm)
       refill = refill + 1 == S::kDigitRing ? 0 : refill + 1;
       if (refill == 0 && b) turn ^= 1;
     }
-    // Nothing of the driver's may outlive the CTA, whatever became of its waits: the copies, the last product.
     copy_async_wait<0>();
-    if (issued) barrier_wait(done, (issued - 1) & 1, late, alive, kScreenDrain);
+    if (lane == 0) s_issued[0] = issued;
   } else if (warp == 5) {
     // ---- codes and scales, and the products of the up tile ----
     if (elect_lane()) {
@@ -411,10 +450,8 @@ __global__ void __launch_bounds__(kScreenThreads, Screen<TOKENS, RISK>::kPerSm)
           turn ^= 1;
         }
       }
-      // As above: the last product, and each place's last codes.
-      if (issued) barrier_wait(done + 8, (issued - 1) & 1, late, alive, kScreenDrain);
-      for (int p = 0; p < min(fetched, S::kCodeRing); ++p)
-        barrier_wait(landed + 8 * p, ((fetched - p - 1) / S::kCodeRing) & 1, late, alive, kScreenDrain);
+      s_issued[1] = issued;
+      s_fetched = fetched;
     }
     __syncwarp();
   } else {
@@ -485,8 +522,7 @@ __global__ void __launch_bounds__(kScreenThreads, Screen<TOKENS, RISK>::kPerSm)
         constexpr bool kFirst = decltype(begin)::value;  // block 0
         int c[24];
         if constexpr (!kFirst) {
-          barrier_wait(done + 8 * tile, (b - 1) & 1, abort, state);
-          if (!__any_sync(kFull, state)) return;  // the product may read the rows still
+          barrier_wait_product(done + 8 * tile, (b - 1) & 1, abort, late, state);
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
           load_sums(tile, 0, c);
         }
@@ -525,8 +561,7 @@ __global__ void __launch_bounds__(kScreenThreads, Screen<TOKENS, RISK>::kPerSm)
       auto finish = [&](auto which) {  // the last block's product
         constexpr int tile = decltype(which)::value;
         int c[24];
-        barrier_wait(done + 8 * tile, (B - 1) & 1, abort, state);
-        if (!__any_sync(kFull, state)) return;
+        barrier_wait_product(done + 8 * tile, (B - 1) & 1, abort, late, state);
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
         for (int half = 0; half < (TOKENS + 7) / 8; ++half) {
@@ -634,7 +669,18 @@ __global__ void __launch_bounds__(kScreenThreads, Screen<TOKENS, RISK>::kPerSm)
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   if (warp == 4) {
-    if ((abort_flag || late_flag) && lane == 0) atomicExch(&ws.status[0], 1);
+    if (abort_flag) {
+      // Nothing may outlive the CTA: the last products, each place's last codes.  (Where no wait ran out, the
+      // decoding warps have seen the end of all.)
+      int alive = 1;
+      for (int tile = 0; tile < 2; ++tile)
+        if (s_issued[tile])
+          barrier_wait(done + 8 * tile, (s_issued[tile] - 1) & 1, late, alive, CFM_SCREEN_DRAIN_NS);
+      for (int p = 0; p < min(s_fetched, S::kCodeRing); ++p)
+        barrier_wait(landed + 8 * p, ((s_fetched - p - 1) / S::kCodeRing) & 1, late, alive, CFM_SCREEN_DRAIN_NS);
+      __syncwarp();
+      if (lane == 0) atomicExch(&ws.status[0], 1);
+    }
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_holder[0]), "n"(S::kLarge)
                  : "memory");
