@@ -930,6 +930,7 @@ __device__ __forceinline__ int down_slot_end(const Layer& L, const Workspace& ws
   return ws.tile_starts[pair] + tiles;
 }
 
+// Without tiles (after the union down kernel) seven registers are spilled for the four CTAs per SM.
 template <bool TILES>
 __global__ void __launch_bounds__(128, 4) k_mix(Layer L, Workspace ws, const uint8_t* padding, int tokens,
                                                 __nv_bfloat16* out, int latents, int early) {
