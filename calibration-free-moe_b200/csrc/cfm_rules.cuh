@@ -15,10 +15,12 @@ static int64_t expected_pairs(const Bound& b) {
 // More than 16/3 tokens per expert on average.
 static bool shares_decode(const Bound& b) { return 3 * expected_pairs(b) > 16 * static_cast<int64_t>(b.L.E); }
 // The tcgen05 screen on request, where several tokens share its decode, or where its CTAs of 128 channels
-// give most SMs one or the rows are long: three tokens of the 128-expert layer (144 CTAs) 10.0 us against 12.4
-// of the warp-level kernel, two of the 64-expert layer (128) 9.8 against 11.5, one of hidden 4096 and width
-// 1536 (96 CTAs, 32 blocks) 17.1 against 19.4; two of the 128-expert layer (96, 16 blocks) 9.9 against 8.3,
-// four of the 256-expert layer of width 512 (128) 10.5 against 8.4.  Its tables have to fit shared memory.
+// give most SMs one or the rows are long.  Whole calls, us per layer, with it and with the warp-level kernel, which lets
+// the selection be scheduled earlier: two tokens of the 128-expert layer (96 CTAs, 16 blocks) 36.7 and 34.8, of the
+// 64-expert layer (128) 39.3 and 39.7; three and four of the 256-expert layer of width 512 (96, 128) 36.2 and 34.3, 37.3
+// and 37.9, four with the recovery-aware score 41.0 and 45.4; three of the 128-expert layer (144) 38.9 and 40.0; four of a layer
+// of 64 experts, hidden 1152 and width 704 (144, 9 blocks) 36.3 and 37.7; one token of hidden 4096 and width 1536 (96, 32 blocks) 54.9 and
+// 54.8, three of hidden 4096, width 512 (96, 32) 46.1 and 50.1, two (64, 32) 43.6 and 39.0.  Its tables have to fit shared memory.
 static bool screens_tc(const Bound& b) {
   const int64_t ctas = std::min<int64_t>(b.L.E, expected_pairs(b)) * ((b.L.I + kScreenChannels - 1) / kScreenChannels);
   if (b.L.tensor_engine == CFM_ENGINE_WARP) return false;
