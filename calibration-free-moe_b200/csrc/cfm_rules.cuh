@@ -87,11 +87,17 @@ static int exact_union_tiles(const Bound& b) {
   return tiles;
 }
 
-// The gather that walks pairs in expert order, from twelve tokens on: with fewer the tokens share few rows, and
-// every CTA's way to its rows is longer (8 tokens of the 128-expert layer 12.5 us and 8.7 of the down tiles against
-// 14.9 and 7.7, of hidden 4096 and width 1536 38.4 and 21.3 against 40.4 and 20.9; 12 of the 64-expert layer 25.5 and
-// 13.3 against 23.7 and 11.8).
-static bool gathers_by_pair(const Bound& b) { return pairs_grouped(b) && (b.L.expert_map || b.T >= 12); }
+// The gather that walks pairs in expert order, from twelve tokens and one token per expert on: below that the tokens
+// share few rows, and every CTA's way to its rows is longer.  Whole calls, us per layer, this gather and the one that
+// walks tokens: 9 tokens of the 128-expert layer (0.6 per expert) 58.3 and 56.2, of a layer of 32 experts (2.3) 52.7 and 51.1,
+// of hidden 4096 and width 1536 132.3 and 129.8, of the 64-expert layer (1.1) 65.7 and 66.6; 12 of the 256-expert layer
+// of width 512 (0.4) 53.5 and 52.4, 24 (0.8) 71.8 and 71.1, 40 (1.3) 94.0 and 94.4, 95 (3.0) 166.7 and 169.2; 16 of the
+// 64-expert layer (2.0) 82.8 and 84.8; 12 of the 128-expert layer (0.8) 64.4 and 61.0, 24 (1.5) 87.9 and 86.9, 32 (2.0) 100.6 and 101.7,
+// 47 (2.9) 126.0 and 129.2; 32 of hidden 4096 and width 1536 (2.0) 304.7 and 312.0.  Layers of few or short rows would
+// rather walk tokens for longer: 12 tokens of 32 experts (3.0) 58.8 and 56.5, 28 of 100 experts of width 640 (1.7) 90.8 and 86.9.
+static bool gathers_by_pair(const Bound& b) {
+  return pairs_grouped(b) && (b.L.expert_map || (b.T >= 12 && static_cast<int64_t>(b.T) * b.L.K >= b.L.E));
+}
 
 // The encoder for four pairs of an expert at a time, from four tokens per expert on where the gathers beside
 // it are long enough to cover its chain of loads, a quarter of a gigabyte: 96 tokens of the 128-expert layer

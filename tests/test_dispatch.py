@@ -37,3 +37,17 @@ def test_screen_of_a_rank(layer, ranks, tokens, tcgen05, pairs):
     share = dict(layer, experts=layer["experts"] // ranks, global_experts=layer["experts"])
     took = device.dispatch(tokens, **share)
     assert (took["tcgen05"], took["pass_pairs"]) == (tcgen05, pairs)
+
+
+@pytest.mark.parametrize("layer,tokens,by_pair", [
+    (QWEN3, 12, 0), (QWEN3, 15, 0), (QWEN3, 16, 1), (OLMOE, 8, 0), (OLMOE, 11, 0), (OLMOE, 12, 1),
+    (SMALL, 31, 0), (SMALL, 32, 1), (WIDE, 32, 1),
+])
+def test_exact_rows_by_pair_from_one_token_per_expert_on(layer, tokens, by_pair):
+    assert device.dispatch(tokens, **layer)["by_pair"] == by_pair
+
+
+@pytest.mark.parametrize("tokens", [8, 12, 64])
+def test_a_rank_walks_pairs_from_eight_tokens_on(tokens):
+    share = dict(SMALL, experts=SMALL["experts"] // 8, global_experts=SMALL["experts"])
+    assert device.dispatch(tokens, **share)["by_pair"]

@@ -43,6 +43,9 @@ LAYERS = {
     "down-listed": (1152, 208, 32, 3, 64, 8, 0.5, 0.625, "gelu_tanh", "point", {}),
     # Expert-major exact with the tiles per token: three tokens per expert and more, up to 16 / 3.
     "union-exact-only": (640, 112, 12, 3, 16, 18, 0.25, 0.625, "silu", "point", {}),
+    # Twelve tokens and more, just below one token per expert and at it: exact rows by token, by pair.
+    "exact-by-token": (384, 48, 64, 2, 16, 31, 0.3, 0.625, "silu", "point", {}),
+    "exact-by-pair": (384, 48, 64, 2, 16, 32, 0.3, 0.625, "silu", "point", {}),
     # One step per quarter of the columns, fewer rows than a tile; a quarter that is no whole turn.
     "union-one-step": (128, 16, 4, 2, 8, 16, 0.25, 1.0, "silu", "point", {}),
     "union-part-turn": (640, 176, 6, 5, 128, 33, 0.3, 0.625, "gelu_tanh", "point", {}),
