@@ -16,9 +16,11 @@
 // The readers take either sketch; parity tests use the reference builder's.
 //
 // What bounds it: 2 + 1/2 bytes per weight cross HBM, but every weight also takes seven
-// butterfly stages, the threshold rule and two 2-bit codes, so the kernel is bound by
-// instruction issue (24 instructions per weight and lane, spread over the FMA, ALU and
-// shuffle pipes, each about half busy).  Hence the split: four lanes share a row's block,
+// butterfly stages, the threshold rule and two 2-bit codes, 0.75 warp instructions in all (24
+// per weight and lane), of which the rotation is about a third.  They are issued at 0.62 per
+// scheduler and cycle: four warps per scheduler, which 128 registers leave room for, do not
+// cover what a warp waits for between two of its own, 5.2 cycles (fixed latencies 0.9, loads
+// 0.75, shuffles 0.7, busy pipes 0.7; no pipe is more than 0.45 busy).  Hence the split: four lanes share a row's block,
 // lane q holding the chunks 16 j + 4 q .. + 3 of it (j = 0 .. 7).  Five of the seven stages
 // and all but two steps of every sum then stay inside a lane, where they run as packed
 // pairs (chunks j and j + 4 of a lane in one f32x2 operation); a warp per row spent 42
